@@ -7,7 +7,7 @@ namespace st {
 
 cudaError_t configure_gemv_kernels();
 cudaError_t configure_gemm_tc_kernels();
-cudaError_t configure_gemm_pair_kernels();
+cudaError_t configure_gemm_dense_kernels();
 cudaError_t configure_grouped_kernels();
 
 // SM count of the current device, looked up once per device ordinal.
@@ -27,7 +27,7 @@ int device_sm_count() {
 cudaError_t configure_device() {
     cudaError_t e = configure_gemv_kernels();
     if (e == cudaSuccess) e = configure_gemm_tc_kernels();
-    if (e == cudaSuccess) e = configure_gemm_pair_kernels();
+    if (e == cudaSuccess) e = configure_gemm_dense_kernels();
     if (e == cudaSuccess) e = configure_grouped_kernels();
     return e;
 }

@@ -1,0 +1,480 @@
+// Prefill GEMM for many rows: weights decoded ONCE per call into binary16 tiles in the caller's
+// workspace, then a dense tcgen05 GEMM over pairs of CTAs with the output stages in its epilogue.
+// It stands in for the reference's tiled core at large row counts (src/wmma_tiled.hip:87-269,
+// src/gemm.hip:15-76).
+//
+// Why two passes: decoding costs about 40 issue clocks per 16x16 tile per SM sub-partition
+// whatever the row count.  A kernel that decodes on the fly repeats it for every row tile (512 rows
+// was the most tensor memory allows), which at 8192 rows is sixteen decodes of every weight in an
+// SM that is also feeding the tensor pipe, and it fills tensor memory with one tile's
+// accumulators, so that no epilogue can overlap the next tile.  With decoded tiles the stage is two
+// bulk copies, accumulators are double-buffered and the decode is paid once.
+//
+// Launch 1 (dense_prologue_kernel) decodes and runs the input stages, side by side in one grid.
+// Bound by memory: K4, 4096 -> 12288, 8192 rows: 67 MB read, 167 MB written in 64 us.
+// Launch 2 (gemm_dense_kernel): persistent CTA pairs (tcgen05 cta_group::2).  A pair's tile is
+// 256 rows x NB column blocks of 128; each CTA holds 128 rows of it, loads its own activation
+// image and its half of the weight image, the MMA reads the other half from the partner.
+// Bound by the tensor pipe: 8192 rows 549 us (1.50 PFLOP/s at the capped clock); the kernel before,
+// which decoded on the fly in 512 x 256 tiles, took 950 us.  What mattered most: the partner CTA's
+// "my stage has landed" must not be a release-arrival on the leader's barrier (1250-1750 clocks each
+// beside bulk copies, longer than a K step); a four-byte st.async that counts as transaction bytes
+// took the same kernel from 950 to 557 us.
+// A wide output is cut into column ranges so that the decoded tiles stay under kDenseScratch.
+//
+// K order: the 16 inputs of an MMA step may come in any order as long as both operands agree.
+// A lane of the decoder holds inputs 2q, 2q+1, 2q+8, 2q+9 of its column, so position 8q+4t+j of a
+// 32-input group is element {2q, 2q+1, 2q+8, 2q+9}[j] of k-tile t: eight weights of two k-tiles are
+// one 16-byte store, and so are an activation lane's.
+#include "backend.h"
+#include "hadamard.cuh"
+#include "sync_primitives.cuh"
+#include "tcgen05.cuh"
+#include "trellis_decode.cuh"
+
+namespace st {
+
+namespace {
+constexpr int kTileBytes = 128 * 64 * 2;      // one operand image: 128 rows x 64 binary16, SWIZZLE_128B
+constexpr int kEpiWarpsD = 8;                 // two per tensor-memory lane quarter
+constexpr int kThreadsD = (2 + kEpiWarpsD) * 32;
+constexpr uint32_t kTmemColsD = 512;
+constexpr size_t kRingBytesD = 192 * 1024;
+constexpr size_t kSmemD = 1024 + kRingBytesD + 512;
+
+template <int NB> struct DenseShape {
+    static constexpr int kStage = kTileBytes + NB * kTileBytes / 2;  // own rows, own half of the columns
+    static constexpr int kStages = (int)(kRingBytesD / kStage);
+};
+
+struct DenseArgs {
+    LinearCall call;
+    const unsigned char* a_tiles;  // [rows padded to 256 / 128][I/64][16 KB]
+    const unsigned char* b_tiles;  // [column blocks of this range][I/64][16 KB]
+    int nb_first, nb_count;        // column blocks of this range
+    int m_tiles;                   // ceil(rows / 256)
+    int n_tiles;                   // ceil(nb_count / NB)
+};
+
+// 16-byte chunk (8 k positions) `chunk` of row `row` in an operand image
+__device__ __forceinline__ uint32_t image_chunk(uint32_t row, uint32_t chunk) {
+    return (row >> 3) * 1024u + (row & 7u) * 128u + (((chunk ^ row) & 7u) << 4);
+}
+}  // namespace
+
+// ---- launch 1: weights and activations into operand images ---------------------------------
+// Jobs of eight warps: the first `decode_jobs` decode one 128-column x 64-input weight image each
+// (one warp per 16-column tile), the others run the input stages of 32 rows of one
+// 128-block.
+template <int K, int CB>
+__global__ void __launch_bounds__(256) dense_prologue_kernel(const DenseArgs args, unsigned char* a_tiles,
+                                                             unsigned char* b_tiles, int decode_jobs, int jobs, int sms) {
+    const LinearCall& c = args.call;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int kt64 = c.w.inputs / 64, blocks = c.w.inputs / 128;
+    const int g = lane >> 2, q = lane & 3;
+    const LaneGeom<K> geom(lane);
+    const bool aligned = quads_aligned(c.x, c.x_dtype, c.x_stride);
+    pdl_launch_dependents();
+    pdl_wait_prior_grid();  // x may come from the launch before, and the images may still be read by it
+
+    // Weight images: a warp decodes one 16-column tile of four k-tiles, with the ring words of its
+    // next job already on their way (a job is a DRAM round trip and only 200 instructions).
+    auto decode = [&] {
+        const uint32_t* first = c.w.packed + ((size_t)args.nb_first * kt64 * 32 + warp) * tile_words(K);
+        uint32_t w[4][3], next[4][3];
+        auto fetch = [&](int job, uint32_t (&words)[4][3]) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) load_window<K>(first + ((size_t)job * 32 + t * 8) * tile_words(K), geom, words[t]);
+        };
+        int job = blockIdx.x;
+        if (job < decode_jobs) fetch(job, next);
+        for (; job < decode_jobs; job += gridDim.x) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) w[t][i] = next[t][i];
+            if (job + (int)gridDim.x < decode_jobs) fetch(job + gridDim.x, next);
+            unsigned char* image = b_tiles + (size_t)job * kTileBytes;
+#pragma unroll
+            for (int t = 0; t < 4; t += 2) {
+                uint32_t lo[4], hi[4];
+                decode_words_frag<K, CB>(w[t], geom, lo);
+                decode_words_frag<K, CB>(w[t + 1], geom, hi);
+                const uint32_t chunk = 2 * t + q, row = warp * 16 + g;
+                *reinterpret_cast<uint4*>(image + image_chunk(row, chunk)) = make_uint4(lo[0], lo[2], hi[0], hi[2]);
+                *reinterpret_cast<uint4*>(image + image_chunk(row + 8, chunk)) = make_uint4(lo[1], lo[3], hi[1], hi[3]);
+            }
+        }
+    };
+    // Activation images: 32 rows of one 128-block per job, four rows per warp, eight lanes per row.
+    auto stage = [&] {
+        const int jobs_in = jobs - decode_jobs;
+        for (int job = blockIdx.x; job < jobs_in; job += gridDim.x) {
+            const int row_group = job / blocks, blk = job - row_group * blocks;
+            const int row = row_group * 32 + warp * 4 + (lane >> 3), l8 = lane & 7;
+            float v[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0.f;
+                if (row < c.rows) load_quad(c.x, c.x_dtype, (long long)row * c.x_stride + blk * 128 + 32 * i + 4 * l8, aligned, v[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                scale_quad(v[i], *reinterpret_cast<const uint2*>(c.w.suh + blk * 128 + 32 * i + 4 * l8));
+            hadamard128_oct(v, lane);
+            // lane pairs (h = 0, 1) of a 16-input k-tile swap halves: {4p .. 4p+3} and {4p+8 .. 4p+11}
+            // become {4p, 4p+1, 4p+8, 4p+9} and {4p+2, 4p+3, 4p+10, 4p+11}, positions of one chunk
+            const int t = l8 >> 2, h = (l8 >> 1) & 1, q2 = 2 * (l8 & 1) + h;
+            unsigned char* image = a_tiles + ((size_t)(row >> 7) * kt64 + blk * 2) * kTileBytes + 8 * t;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t lo = as_u32(__floats2half2_rn(v[i][0], v[i][1])), hi = as_u32(__floats2half2_rn(v[i][2], v[i][3]));
+                const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, h ? lo : hi, 2);
+                *reinterpret_cast<uint2*>(image + (i >> 1) * kTileBytes + image_chunk(row & 127, (i & 1) * 4 + q2)) =
+                    h ? make_uint2(got, hi) : make_uint2(lo, got);
+            }
+        }
+    };
+    // Decoding is bound by issue slots, the input stages by memory: an SM should be at both at once.
+    for (int turn = 0; turn < 2; ++turn) {
+        if (((int)blockIdx.x / sms + turn) & 1) decode();
+        else stage();
+    }
+}
+
+// ---- launch 2: the dense GEMM ---------------------------------------------------------------
+template <int NB>
+__global__ void __launch_bounds__(kThreadsD, 1) gemm_dense_kernel(const DenseArgs args) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    constexpr int kStages = DenseShape<NB>::kStages, kStage = DenseShape<NB>::kStage;
+    const LinearCall& c = args.call;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();  // 0 = leader
+    const int kt64 = c.w.inputs / 64;
+    const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const int tiles = args.m_tiles * args.n_tiles;
+    const int my_tiles = tiles > pair ? (tiles - pair + pairs - 1) / pairs : 0;
+    // Row tiles fastest, in bands of eight: pairs that run together share weight images and the
+    // band's activation images, both L2 hits.
+    constexpr int kBand = 8;
+    auto place = [&](int lt, int& m, int& n) {
+        const int t = pair + lt * pairs, per_band = kBand * args.n_tiles;
+        const int band = t / per_band, in_band = t - band * per_band;
+        const int left = args.m_tiles - band * kBand, high = left < kBand ? left : kBand;
+        n = in_band / high;
+        m = band * kBand + in_band - n * high;
+    };
+
+    const uint32_t ring0 = smem_u32(ring);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ring + kRingBytesD);
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_abort;
+    __shared__ __align__(16) uint32_t s_sink[4];
+    const uint32_t full = smem_u32(bars), empty = smem_u32(bars + kStages), tmem_full = smem_u32(bars + 2 * kStages),
+                   tmem_empty = smem_u32(bars + 2 * kStages + 2);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kStages; ++i) {
+            mbar_init(full + 8 * i, 1);
+            mbar_init(empty + 8 * i, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(tmem_full + 8 * b, 1);
+            mbar_init(tmem_empty + 8 * b, 2 * (NB == 2 ? kEpiWarpsD : kEpiWarpsD / 2));
+        }
+        mbar_fence_init();
+        s_abort = 0;
+    }
+    if (warp == 1) tmem_alloc_pair(smem_u32(&s_tmem_base), kTmemColsD);
+    tc_fence_before_sync();
+    cluster_sync_all();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = s_tmem_base;
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        // ---- producer: this CTA's activation image and half of the weight image per K step ------
+        if (lane == 0) {
+            pdl_wait_prior_grid();  // the images belong to the launch before
+            int st = 0, issued = 0;
+            uint32_t prev_use = 1;  // parity of the slot's previous use
+            for (int lt = 0; lt < my_tiles && !s_abort; ++lt) {
+                int m, n;
+                place(lt, m, n);
+                const int nb = n * NB + (NB == 2 ? (int)rank : 0);
+                const bool live = nb < args.nb_count;  // odd block count: the last tile's second half is padding
+                const unsigned char* a = args.a_tiles + (size_t)(m * 2 + (int)rank) * kt64 * kTileBytes;
+                const unsigned char* b = args.b_tiles + (size_t)nb * kt64 * kTileBytes + (NB == 1 ? rank * (kTileBytes / 2) : 0);
+                for (int ks = 0; ks < kt64; ++ks) {
+                    if (issued >= kStages && !mbar_wait(empty + 8 * st, prev_use, c.status, kTimeoutTensorPipe)) {
+                        s_abort = 1;
+                        break;
+                    }
+                    const uint32_t dst = ring0 + st * kStage;
+                    // the leader's stage also counts the partner's signal
+                    mbar_expect_tx(full + 8 * st, (live ? kStage : kTileBytes) + (rank == 0 ? 4 : 0));
+                    bulk_load(dst, a + (size_t)ks * kTileBytes, kTileBytes, full + 8 * st);
+                    if (live) bulk_load(dst + kTileBytes, b + (size_t)ks * kTileBytes, NB * kTileBytes / 2, full + 8 * st);
+                    ++issued;
+                    if (++st == kStages) { st = 0; prev_use ^= 1; }
+                }
+            }
+            for (int i = (issued > kStages ? issued - kStages : 0); i < issued; ++i)  // nothing still landing at exit
+                mbar_wait(full + 8 * (i % kStages), (uint32_t)(i / kStages) & 1, c.status, kTimeoutDrain);
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            // ---- MMA issuer (leader CTA) --------------------------------------------------------
+            constexpr uint32_t idesc = umma_idesc_f16_f32(256, NB * 128);
+            int st = 0;
+            uint32_t use = 0;
+            for (int lt = 0; lt < my_tiles && !s_abort; ++lt) {
+                const int buf = lt & 1;
+                if (lt >= 2 && !mbar_wait(tmem_empty + 8 * buf, (uint32_t)((lt >> 1) - 1) & 1, c.status, kTimeoutTensorPipe)) {
+                    s_abort = 1;
+                    break;
+                }
+                tc_fence_after_sync();
+                for (int ks = 0; ks < kt64; ++ks) {
+                    if (!mbar_wait(full + 8 * st, use, c.status, kTimeoutTensorPipe)) {
+                        s_abort = 1;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    const uint32_t base = ring0 + st * kStage;
+                    const uint64_t adesc = umma_desc_k_major_sw128(base), bdesc = umma_desc_k_major_sw128(base + kTileBytes);
+#pragma unroll
+                    for (int k4 = 0; k4 < 4; ++k4)
+                        umma_f16_pair(tmem_base + buf * NB * 128, adesc + 2 * k4, bdesc + 2 * k4, idesc, (ks | k4) != 0);
+                    umma_commit_pair(empty + 8 * st, 3);
+                    if (++st == kStages) { st = 0; use ^= 1; }
+                }
+                umma_commit_pair(tmem_full + 8 * buf, 3);
+            }
+        } else if (lane == 0) {
+            // ---- partner CTA: one signal per stage once its copies have landed ---------------------
+            const uint32_t leader_full = map_to_rank(full, 0), leader_sink = map_to_rank(smem_u32(s_sink), 0);
+            const int iters = my_tiles * kt64;
+            int st = 0;
+            uint32_t use = 0;
+            for (int it = 0; it < iters; ++it) {
+                if (!mbar_wait(full + 8 * st, use, c.status, kTimeoutTensorPipe)) {
+                    s_abort = 1;
+                    break;
+                }
+                signal_cluster_tx(leader_full + 8 * st, leader_sink);
+                if (++st == kStages) { st = 0; use ^= 1; }
+            }
+        }
+    } else {
+        // ---- epilogue: one thread has one row of a 128-column block, H128 runs in its registers ----
+        const int quarter = warp & 3, part = (warp - 2) >> 2;
+        const uint32_t leader_tmem_empty = map_to_rank(tmem_empty, 0);
+        const bool wide = c.y_dtype == DT_F32
+            ? (c.y_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(c.y) & 15) == 0
+            : (c.y_stride & 7) == 0 && (reinterpret_cast<uintptr_t>(c.y) & 15) == 0;
+        for (int lt = 0; lt < my_tiles; ++lt) {
+            const int buf = lt & 1;
+            if (NB == 1 && part != buf) continue;  // one block per tile: the two warp sets take turns
+            int m, n;
+            place(lt, m, n);
+            const int nb = n * NB + (NB == 2 ? part : 0);
+            if (s_abort || !mbar_wait(tmem_full + 8 * buf, (uint32_t)(lt >> 1) & 1, c.status, kTimeoutTensorPipe)) {
+                s_abort = 1;
+                break;
+            }
+            __syncwarp();  // rows beyond the call left the last tile early
+            tc_fence_after_sync();
+            float v[128];
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * NB * 128 + (NB == 2 ? part * 128 : 0);
+            {
+                uint32_t r[4][32];
+#pragma unroll
+                for (int ch = 0; ch < 4; ++ch) tmem_ld_32x32(taddr + ch * 32, r[ch]);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 128; ++i) {
+                    asm volatile("" : "+r"(r[i >> 5][i & 31]));  // not before the wait
+                    v[i] = __uint_as_float(r[i >> 5][i & 31]);
+                }
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(leader_tmem_empty + 8 * buf);  // the values are in registers
+            const int row = (m * 2 + (int)rank) * 128 + quarter * 32 + lane;
+            if (nb >= args.nb_count || row >= c.rows) continue;
+            hadamard128_thread(v);
+            const int col0 = (args.nb_first + nb) * 128;
+            const long long at = (long long)row * c.y_stride + col0;
+#pragma unroll
+            for (int j8 = 0; j8 < 16; ++j8) {
+                const uint4 s8 = *reinterpret_cast<const uint4*>(c.w.svh + col0 + 8 * j8);
+                const uint32_t sw[4] = {s8.x, s8.y, s8.z, s8.w};
+                float o[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    o[j] = __fmul_rn(v[8 * j8 + j], half_bits_to_float((uint16_t)(sw[j >> 1] >> (16 * (j & 1)))));
+                    if (c.w.bias) o[j] = __fadd_rn(o[j], c.w.bias[col0 + 8 * j8 + j]);
+                }
+                if (!wide || c.beta != 0.0f) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) scale_and_store(c.y, c.y_dtype, at + 8 * j8 + j, o[j], c.alpha, c.beta);
+                    continue;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] = __fmul_rn(o[j], c.alpha);
+                if (c.y_dtype == DT_F32) {
+                    float4* out = reinterpret_cast<float4*>(c.y + at + 8 * j8);
+                    out[0] = make_float4(o[0], o[1], o[2], o[3]);
+                    out[1] = make_float4(o[4], o[5], o[6], o[7]);
+                } else {
+                    uint32_t p[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (c.y_dtype == DT_F16) {
+                            p[j] = as_u32(__floats2half2_rn(o[2 * j], o[2 * j + 1]));
+                        } else {
+                            const __nv_bfloat162 b = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
+                            p[j] = *reinterpret_cast<const uint32_t*>(&b);
+                        }
+                    }
+                    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(c.y) + at + 8 * j8) = make_uint4(p[0], p[1], p[2], p[3]);
+                }
+            }
+        }
+    }
+
+    // ---- common exit: both CTAs are done with each other's memory before anything is freed ----
+    tc_fence_before_sync();
+    cluster_sync_all();
+    if (warp == 1) {
+        tc_fence_after_sync();
+        tmem_dealloc_pair(tmem_base, kTmemColsD);
+    }
+}
+
+// ---- host side ---------------------------------------------------------------------------------
+namespace {
+constexpr size_t kDenseScratch = (size_t)256 << 20;  // decoded weight images of one column range
+
+// Column blocks of one range: as few ranges as fit the scratch, of equal (even) size.
+int dense_range(const DeviceWeights& w) {
+    const int nblocks = w.outputs / 128;
+    const size_t block = (size_t)w.inputs * 256;
+    const int most = (int)(kDenseScratch / block) < 2 ? 2 : (int)(kDenseScratch / block);
+    const int ranges = (nblocks + most - 1) / most;
+    int per = (nblocks + ranges - 1) / ranges;
+    per += per & 1;
+    return per < nblocks ? per : nblocks;
+}
+
+template <int K, int CB>
+cudaError_t launch_prologue(const DenseArgs& args, unsigned char* a, unsigned char* b, bool inputs, int rows_padded,
+                            bool programmatic, cudaStream_t stream) {
+    const long long decode_jobs = (long long)args.nb_count * (args.call.w.inputs / 64);
+    const long long jobs = decode_jobs + (inputs ? (long long)(rows_padded / 32) * (args.call.w.inputs / 128) : 0);
+    if (jobs > 0x3FFFFFFF) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(streaming_grid(jobs, 4));  // 64 registers x 256 threads: four CTAs per SM are resident
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = programmatic ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, dense_prologue_kernel<K, CB>, args, a, b, (int)decode_jobs, (int)jobs, device_sm_count());
+}
+template <int CB>
+cudaError_t launch_prologue_bits(const DenseArgs& args, unsigned char* a, unsigned char* b, bool inputs, int padded,
+                                 bool pdl, cudaStream_t s) {
+    switch (args.call.w.bits) {
+    case 1: return launch_prologue<1, CB>(args, a, b, inputs, padded, pdl, s);
+    case 2: return launch_prologue<2, CB>(args, a, b, inputs, padded, pdl, s);
+    case 3: return launch_prologue<3, CB>(args, a, b, inputs, padded, pdl, s);
+    case 4: return launch_prologue<4, CB>(args, a, b, inputs, padded, pdl, s);
+    case 5: return launch_prologue<5, CB>(args, a, b, inputs, padded, pdl, s);
+    case 6: return launch_prologue<6, CB>(args, a, b, inputs, padded, pdl, s);
+    case 7: return launch_prologue<7, CB>(args, a, b, inputs, padded, pdl, s);
+    case 8: return launch_prologue<8, CB>(args, a, b, inputs, padded, pdl, s);
+    case 9: case 10: case 11:  // 1.5 / 2.5 / 3.5 bits per weight exist for mul1 only
+        if constexpr (CB == CB_MUL1) {
+            if (args.call.w.bits == 9) return launch_prologue<9, CB>(args, a, b, inputs, padded, pdl, s);
+            if (args.call.w.bits == 10) return launch_prologue<10, CB>(args, a, b, inputs, padded, pdl, s);
+            return launch_prologue<11, CB>(args, a, b, inputs, padded, pdl, s);
+        }
+        return cudaErrorInvalidValue;
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template <int NB>
+cudaError_t launch_dense(const DenseArgs& args, int sm_count, bool programmatic, cudaStream_t stream) {
+    const int tiles = args.m_tiles * args.n_tiles, pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = dim3(kThreadsD);
+    cfg.dynamicSmemBytes = kSmemD;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = programmatic ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, gemm_dense_kernel<NB>, args);
+}
+}  // namespace
+
+int gemm_dense_rows_padded(int rows) { return (rows + 255) / 256 * 256; }
+size_t gemm_dense_scratch(const DeviceWeights& w) { return (size_t)dense_range(w) * w.inputs * 256; }
+
+// Opt-in dynamic shared memory is a per-device function attribute: set when a context is created
+// on a device (configure_device), never on the launch path.
+cudaError_t configure_gemm_dense_kernels() {
+    cudaError_t e = cudaFuncSetAttribute(gemm_dense_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemD);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_dense_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemD);
+    return e;
+}
+
+// `workspace`: activation images, then (256-byte aligned) the decoded weight images of one range.
+cudaError_t launch_gemm_dense(const LinearCall& call, unsigned char* workspace, int sm_count, bool programmatic,
+                              cudaStream_t stream) {
+    DenseArgs args{};
+    args.call = call;
+    const int rows_padded = gemm_dense_rows_padded(call.rows), nblocks = call.w.outputs / 128, range = dense_range(call.w);
+    unsigned char* b = workspace + align_up((size_t)rows_padded * call.w.inputs * 2);
+    args.a_tiles = workspace;
+    args.b_tiles = b;
+    args.m_tiles = rows_padded / 256;
+    if (sm_count < 2 || (long long)args.m_tiles * nblocks > 0x3FFFFFFF) return cudaErrorInvalidValue;
+    for (int nb = 0; nb < nblocks; nb += range) {
+        args.nb_first = nb;
+        args.nb_count = nblocks - nb < range ? nblocks - nb : range;
+        cudaError_t e;
+        switch (call.w.codebook) {
+        case CB_3INST: e = launch_prologue_bits<CB_3INST>(args, workspace, b, nb == 0, rows_padded, programmatic, stream); break;
+        case CB_MCG: e = launch_prologue_bits<CB_MCG>(args, workspace, b, nb == 0, rows_padded, programmatic, stream); break;
+        case CB_MUL1: e = launch_prologue_bits<CB_MUL1>(args, workspace, b, nb == 0, rows_padded, programmatic, stream); break;
+        default: return cudaErrorInvalidValue;
+        }
+        if (e != cudaSuccess) return e;
+        // A K step of a 256 x 256 tile takes about 4/3 of that of a 256 x 128 tile (measured 0.46
+        // and 0.35 us: half the flops for three quarters of the loads), so narrow tiles pay only
+        // where they save that much in the last wave.
+        const int pairs = sm_count / 2;
+        const int wide = (args.m_tiles * ((args.nb_count + 1) / 2) + pairs - 1) / pairs;
+        const int narrow = (args.m_tiles * args.nb_count + pairs - 1) / pairs;
+        const bool two = 4 * wide <= 3 * narrow;
+        args.n_tiles = two ? (args.nb_count + 1) / 2 : args.nb_count;
+        e = two ? launch_dense<2>(args, sm_count, programmatic, stream) : launch_dense<1>(args, sm_count, programmatic, stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+}  // namespace st

@@ -448,9 +448,11 @@ GemmPlan plan_gemm_chunked(const DeviceWeights& w, int rows, int sm_count);
 cudaError_t launch_gemm_chunked(const LinearCall& call, int sm_count, void* workspace, bool programmatic_launch,
                                 cudaStream_t stream);
 
-// gemm_tc_pair.cu: two CTAs per 512 x 256 tile
-int gemm_pair_rows_padded(int rows);
-cudaError_t launch_gemm_pair(const LinearCall& call, const unsigned char* a_tiles, int sm_count, cudaStream_t stream);
+// gemm_dense.cu: weights decoded once, then a dense GEMM
+int gemm_dense_rows_padded(int rows);
+size_t gemm_dense_scratch(const DeviceWeights& w);
+cudaError_t launch_gemm_dense(const LinearCall& call, unsigned char* workspace, int sm_count, bool programmatic,
+                              cudaStream_t stream);
 
 GemmPlan plan_gemm(const DeviceWeights& w, int rows, int sm_count) {
     // Up to two 8-row chunks of the fused GEMV are faster than the three launches of the
@@ -459,14 +461,15 @@ GemmPlan plan_gemm(const DeviceWeights& w, int rows, int sm_count) {
     // tensor-core route wins or ties on every benchmark shape.
     if (rows <= kChunkedMaxRows) return plan_gemm_chunked(w, rows, sm_count);
     GemmPlan plan{};
-    const bool pair = rows > kBM * kMT && sm_count >= 2;
-    const int rows_padded = pair ? gemm_pair_rows_padded(rows) : (rows + kBM * kMT - 1) / (kBM * kMT) * (kBM * kMT);
+    const bool dense = rows > kBM * kMT && sm_count >= 2;
+    const int rows_padded = (rows + kBM * kMT - 1) / (kBM * kMT) * (kBM * kMT);
     plan.act_bytes = (size_t)rows_padded * w.inputs * 2;
     plan.workspace_bytes = align_up(plan.act_bytes);
-    plan.tile_m = pair ? 2 * kBM * kMT : kBM * kMT;
+    if (dense) plan.workspace_bytes += gemm_dense_scratch(w);
+    plan.tile_m = dense ? 2 * kBM * kMT : kBM * kMT;
     // One row tile leaves most SMs without a column tile: partition K so that every SM has work.
     plan.k_splits = 1;
-    if (!pair && rows_padded == kBM * kMT) {
+    if (!dense && rows_padded == kBM * kMT) {
         const int n_pairs = (w.outputs / 128 + kBN / 128 - 1) / (kBN / 128);
         int splits = sm_count / n_pairs;
         if (splits > 4) splits = 4;
@@ -553,9 +556,10 @@ cudaError_t launch_gemm(const LinearCall& call, const GemmPlan& plan, void* work
     // later launches to it programmatically.
     if (!plan.tensor_core) return launch_gemm_chunked(call, plan.sm_count, workspace, programmatic_launch, stream);
     if (!workspace) return cudaErrorInvalidValue;
-    const bool pair = plan.tile_m == 2 * kBM * kMT;
+    if (plan.tile_m == 2 * kBM * kMT)
+        return launch_gemm_dense(call, static_cast<unsigned char*>(workspace), plan.sm_count, programmatic_launch, stream);
     const int m_pairs = (call.rows + kBM * kMT - 1) / (kBM * kMT);
-    const int rows_padded = pair ? gemm_pair_rows_padded(call.rows) : m_pairs * kBM * kMT;
+    const int rows_padded = m_pairs * kBM * kMT;
     {
         const long long groups = (long long)rows_padded * (call.w.inputs / 128);
         const long long want = (groups + 7) / 8;
@@ -565,7 +569,6 @@ cudaError_t launch_gemm(const LinearCall& call, const GemmPlan& plan, void* work
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    if (pair) return launch_gemm_pair(call, static_cast<const unsigned char*>(workspace), plan.sm_count, stream);
     GemmArgs args{};
     args.call = call;
     args.a_tiles = static_cast<const unsigned char*>(workspace);

@@ -71,6 +71,14 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// Signals a barrier of another CTA of the cluster by four transaction bytes (a word stored to
+// `sink` there).  Unlike an arrival with release semantics it does not wait for anything this SM
+// has in flight: measured 1250 - 1750 clocks per remote release-arrival beside bulk copies.  For
+// signals that order no generic-proxy writes.
+__device__ __forceinline__ void signal_cluster_tx(uint32_t cluster_bar, uint32_t cluster_sink) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
+                 ::"r"(cluster_sink), "r"(1u), "r"(cluster_bar) : "memory");
+}
 // Word-granular publication between CTAs of one grid: a 32-bit word is either the "empty"
 // pattern or a value, so neither a fence nor a flag is needed around it.
 __device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
