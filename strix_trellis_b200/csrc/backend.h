@@ -105,14 +105,12 @@ cudaError_t reset_gemv_scratch(void* workspace, const GemvPlan& plan, cudaStream
 cudaError_t launch_gemv(const LinearCall& call, const GemvPlan& plan, void* workspace,
                         bool programmatic_launch, cudaStream_t stream);
 
-// ---- prefill GEMM (rows > 8): input stage kernel + tcgen05 core with fused epilogue ---
+// ---- GEMM (rows > 8) --------------------------------------------------------------------
 struct GemmPlan {
-    size_t act_bytes;       // binary16 [rows_padded][I] core input
+    size_t act_bytes;        // core input as binary16 operand images
     size_t workspace_bytes;
-    int tile_m, tile_n;
     int sm_count;
-    int k_splits;           // K partitions per output tile (> 1: raw partial accumulators in the workspace)
-    bool tensor_core;       // tcgen05 prefill kernel selected (else 8-row GEMV chunks)
+    bool dense;  // weights decoded once, dense GEMM (else decoded on the fly)
 };
 GemmPlan plan_gemm(const DeviceWeights& w, int rows, int sm_count);
 cudaError_t launch_gemm(const LinearCall& call, const GemmPlan& plan, void* workspace,

@@ -55,11 +55,6 @@ struct DenseArgs {
     int m_tiles;                   // ceil(rows / 256)
     int n_tiles;                   // ceil(nb_count / NB)
 };
-
-// 16-byte chunk (8 k positions) `chunk` of row `row` in an operand image
-__device__ __forceinline__ uint32_t image_chunk(uint32_t row, uint32_t chunk) {
-    return (row >> 3) * 1024u + (row & 7u) * 128u + (((chunk ^ row) & 7u) << 4);
-}
 }  // namespace
 
 // ---- launch 1: weights and activations into operand images ---------------------------------
@@ -102,8 +97,8 @@ __global__ void __launch_bounds__(256) dense_prologue_kernel(const DenseArgs arg
                 decode_words_frag<K, CB>(w[t], geom, lo);
                 decode_words_frag<K, CB>(w[t + 1], geom, hi);
                 const uint32_t chunk = 2 * t + q, row = warp * 16 + g;
-                *reinterpret_cast<uint4*>(image + image_chunk(row, chunk)) = make_uint4(lo[0], lo[2], hi[0], hi[2]);
-                *reinterpret_cast<uint4*>(image + image_chunk(row + 8, chunk)) = make_uint4(lo[1], lo[3], hi[1], hi[3]);
+                *reinterpret_cast<uint4*>(image + sw128_chunk(row, chunk)) = make_uint4(lo[0], lo[2], hi[0], hi[2]);
+                *reinterpret_cast<uint4*>(image + sw128_chunk(row + 8, chunk)) = make_uint4(lo[1], lo[3], hi[1], hi[3]);
             }
         }
     };
@@ -131,7 +126,7 @@ __global__ void __launch_bounds__(256) dense_prologue_kernel(const DenseArgs arg
             for (int i = 0; i < 4; ++i) {
                 const uint32_t lo = as_u32(__floats2half2_rn(v[i][0], v[i][1])), hi = as_u32(__floats2half2_rn(v[i][2], v[i][3]));
                 const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, h ? lo : hi, 2);
-                *reinterpret_cast<uint2*>(image + (i >> 1) * kTileBytes + image_chunk(row & 127, (i & 1) * 4 + q2)) =
+                *reinterpret_cast<uint2*>(image + (i >> 1) * kTileBytes + sw128_chunk(row & 127, (i & 1) * 4 + q2)) =
                     h ? make_uint2(got, hi) : make_uint2(lo, got);
             }
         }
@@ -147,10 +142,10 @@ __global__ void __launch_bounds__(256) dense_prologue_kernel(const DenseArgs arg
 template <int NB>
 __global__ void __launch_bounds__(kThreadsD, 1) gemm_dense_kernel(const DenseArgs args) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* ring = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (still a shared-memory pointer to the compiler)
     constexpr int kStages = DenseShape<NB>::kStages, kStage = DenseShape<NB>::kStage;
     const LinearCall& c = args.call;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();  // 0 = leader
     const int kt64 = c.w.inputs / 64;
     const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
@@ -224,34 +219,36 @@ __global__ void __launch_bounds__(kThreadsD, 1) gemm_dense_kernel(const DenseArg
                 mbar_wait(full + 8 * (i % kStages), (uint32_t)(i / kStages) & 1, c.status, kTimeoutDrain);
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            // ---- MMA issuer (leader CTA) --------------------------------------------------------
+        if (rank == 0) {
+            // ---- MMA issuer (leader CTA): the whole warp walks, an elected lane issues -----------
             constexpr uint32_t idesc = umma_idesc_f16_f32(256, NB * 128);
             int st = 0;
             uint32_t use = 0;
-            for (int lt = 0; lt < my_tiles && !s_abort; ++lt) {
+            bool ok = true;
+            for (int lt = 0; lt < my_tiles && ok; ++lt) {
                 const int buf = lt & 1;
-                if (lt >= 2 && !mbar_wait(tmem_empty + 8 * buf, (uint32_t)((lt >> 1) - 1) & 1, c.status, kTimeoutTensorPipe)) {
-                    s_abort = 1;
-                    break;
-                }
+                if (lt >= 2 && !mbar_wait(tmem_empty + 8 * buf, (uint32_t)((lt >> 1) - 1) & 1, c.status, kTimeoutTensorPipe)) break;
                 tc_fence_after_sync();
                 for (int ks = 0; ks < kt64; ++ks) {
                     if (!mbar_wait(full + 8 * st, use, c.status, kTimeoutTensorPipe)) {
-                        s_abort = 1;
+                        ok = false;
                         break;
                     }
                     tc_fence_after_sync();
                     const uint32_t base = ring0 + st * kStage;
                     const uint64_t adesc = umma_desc_k_major_sw128(base), bdesc = umma_desc_k_major_sw128(base + kTileBytes);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4)
-                        umma_f16_pair(tmem_base + buf * NB * 128, adesc + 2 * k4, bdesc + 2 * k4, idesc, (ks | k4) != 0);
-                    umma_commit_pair(empty + 8 * st, 3);
+                        for (int k4 = 0; k4 < 4; ++k4)
+                            umma_f16_pair(tmem_base + buf * NB * 128, adesc + 2 * k4, bdesc + 2 * k4, idesc, (ks | k4) != 0);
+                        umma_commit_pair(empty + 8 * st, 3);
+                    }
+                    __syncwarp();
                     if (++st == kStages) { st = 0; use ^= 1; }
                 }
-                umma_commit_pair(tmem_full + 8 * buf, 3);
+                if (elect_one()) umma_commit_pair(tmem_full + 8 * buf, 3);
             }
+            if (!ok) s_abort = 1;
         } else if (lane == 0) {
             // ---- partner CTA: one signal per stage once its copies have landed ---------------------
             const uint32_t leader_full = map_to_rank(full, 0), leader_sink = map_to_rank(smem_u32(s_sink), 0);

@@ -147,6 +147,32 @@ __device__ __forceinline__ void load_quad(const void* base, int dtype, long long
         }
     }
 }
+// scale_and_store of four neighbours.
+__device__ __forceinline__ void scale_and_store_quad(void* y, int dtype, long long index, bool aligned, float (&v)[4],
+                                                     float alpha, float beta) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __fmul_rn(v[j], alpha);
+    if (beta != 0.0f) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = __fadd_rn(v[j], __fmul_rn(beta, load_element(y, dtype, index + j)));
+    }
+    if (!aligned) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) store_element(y, dtype, index + j, v[j]);
+    } else if (dtype == DT_F32) {
+        *reinterpret_cast<float4*>(static_cast<float*>(y) + index) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+        uint2 out;
+        if (dtype == DT_F16) {
+            const __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
+            out = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        } else {
+            const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+            out = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        }
+        *reinterpret_cast<uint2*>(static_cast<uint16_t*>(y) + index) = out;
+    }
+}
 // The four input scales that go with load_quad (weights: always aligned).
 __device__ __forceinline__ void scale_quad(float (&v)[4], uint2 suh) {
     v[0] = __half2float(scale_input(v[0], (uint16_t)suh.x));

@@ -30,6 +30,17 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
+// The warp index as a value the compiler knows to be the same in every lane, and one elected lane
+// of a converged warp.  A role that issues tensor-core work runs its whole loop converged and
+// elects the issuing lane per batch: descriptors and counters then live in uniform registers,
+// where tcgen05 instructions read them.  (In a loop under `if (lane == 0)` every operand is moved
+// there first: measured 110 clocks per issued MMA.)
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t is;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
+    return is != 0;
+}
 // Hardware-suspended wait: the thread sleeps inside try_wait for up to ~2 us per call,
 // so a waiting warp costs no issue slots.
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {

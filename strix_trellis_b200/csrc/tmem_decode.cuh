@@ -1,0 +1,107 @@
+// The decode side of the tensor-memory kernels (gemv_tmem.cu, wide_linear.cu): packed tiles from a
+// shared-memory ring into stages of tensor memory, where they are the A operand of tcgen05.mma.
+//
+// A unit is (one 128-column block) x (one H128 block of K): 64 tiles, 128 lanes x 64 columns of
+// tensor memory once decoded.  Eight warps decode a unit, one column tile each; kUnitGroups such
+// groups take turns.  A warp may only write its own lane quarter (warp % 4), so warp w has column
+// tiles 2(w % 4) and 2(w % 4) + 1 among its group of eight.
+//
+// Measured with nothing else running (clocks per 16x16 tile per SM sub-partition, K2 / K4 / K5 / K6):
+// 45 / 43 / 50 / 54, against 51 / 48 / 56 / 58 with each tile fed to mma.sync, which holds the
+// issue port of its scheduler for most of its eight clocks.
+#pragma once
+#include "sync_primitives.cuh"
+#include "tcgen05.cuh"
+#include "trellis_decode.cuh"
+
+namespace st {
+
+constexpr int kUnitGroups = 2;
+constexpr int kMaxAStages = 7;  // decoded units in tensor memory
+
+// Decodes this warp's column tile of the units of its turn in one segment: two K = 64 halves per
+// unit, four tiles each, one tensor-memory store per half.
+struct DecodeState {
+    int unit;      // counter over the CTA's range: the next unit of this warp's turn
+    int stage;     // its tensor-memory stage
+    uint32_t a_prev;  // parity of the stage's previous use
+    bool a_used;   // whether there was one
+    int slot;      // its ring slot
+    uint32_t use;  // and the slot's use parity
+};
+template <int K, int CB>
+__device__ __forceinline__ bool decode_segment(DecodeState& s, int until, const unsigned char* ring, int w_slots, int w_stride,
+                                               uint32_t w_full, uint32_t w_empty, uint32_t a_full, uint32_t a_empty,
+                                               uint32_t taddr, int a_stages, int ctile, int lane, unsigned int* status) {
+    const LaneGeom<K> geom(lane);
+    for (; s.unit < until; s.unit += kUnitGroups) {
+        const int stage = s.stage;
+        if (!mbar_wait(w_full + 8 * s.slot, s.use, status, kTimeoutRingFull)) return false;
+        if (s.a_used && !mbar_wait(a_empty + 8 * stage, s.a_prev, status, kTimeoutTensorPipe))
+            return false;
+        tc_fence_after_sync();
+        const uint32_t* tiles = reinterpret_cast<const uint32_t*>(ring + (size_t)s.slot * w_stride) + ctile * tile_words(K);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            uint32_t r[16];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                uint32_t f[4];
+                decode_tile_frag<K, CB>(tiles + (half * 4 + t) * 8 * tile_words(K), geom, f);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) r[4 * t + j] = f[j];
+            }
+            tmem_st_16x32(taddr + stage * 64 + half * 32, r);
+        }
+        if (lane == 0) mbar_arrive(w_empty + 8 * s.slot);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(a_full + 8 * stage);
+        s.slot += kUnitGroups;
+        while (s.slot >= w_slots) { s.slot -= w_slots; s.use ^= 1; }
+        s.stage += kUnitGroups;
+        if (s.stage >= a_stages) { s.stage -= a_stages; s.a_prev ^= 1; s.a_used = true; }
+    }
+    return true;
+}
+
+// The same for a run-time rate.
+template <int CB>
+__device__ __forceinline__ bool decode_segment_rate(int bits, DecodeState& s, int until, const unsigned char* ring, int w_slots,
+                                                    int w_stride, uint32_t w_full, uint32_t w_empty, uint32_t a_full,
+                                                    uint32_t a_empty, uint32_t taddr, int a_stages, int ctile, int lane,
+                                                    unsigned int* status) {
+#define ST_DECODE(K) decode_segment<K, CB>(s, until, ring, w_slots, w_stride, w_full, w_empty, a_full, a_empty, taddr, a_stages, ctile, lane, status)
+    switch (bits) {
+    case 1: return ST_DECODE(1);
+    case 2: return ST_DECODE(2);
+    case 3: return ST_DECODE(3);
+    case 4: return ST_DECODE(4);
+    case 5: return ST_DECODE(5);
+    case 6: return ST_DECODE(6);
+    case 7: return ST_DECODE(7);
+    case 8: return ST_DECODE(8);
+    default:  // half-integer rates exist for mul1 only
+        if constexpr (CB == CB_MUL1) {
+            if (bits == 9) return ST_DECODE(9);
+            if (bits == 10) return ST_DECODE(10);
+            return ST_DECODE(11);
+        }
+        return false;
+    }
+#undef ST_DECODE
+}
+
+// Barrier of one warp group (128 threads) that also tells every thread whether any brought `pred`.
+__device__ __forceinline__ bool group_any(int id, bool pred) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, %2, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any) : "r"((uint32_t)pred), "r"(id) : "memory");
+    return any != 0;
+}
+}  // namespace st
