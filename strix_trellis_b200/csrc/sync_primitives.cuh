@@ -41,9 +41,19 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
     return is != 0;
 }
-// Hardware-suspended wait: the thread sleeps inside try_wait for up to ~2 us per call,
-// so a waiting warp costs no issue slots.
+// One try_wait without a time hint: about 12 clocks when the phase is over.  The form with a
+// suspend-time hint costs about 105 clocks even then (measured), so it is kept for long waits, where
+// the hardware lets the thread sleep for up to the hinted 2 us per call.
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_try_sleep(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -55,26 +65,13 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // Bounded: gives up after about a quarter of a second and reports it in `status`.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned int* status,
                                           unsigned int fail_bit) {
-    for (uint32_t i = 0; i < (1u << 17); ++i)
+    if (mbar_try(bar, parity)) return true;  // the usual case, kept apart from the loops' set-up
+#pragma unroll 1
+    for (uint32_t i = 0; i < 64; ++i)
         if (mbar_try(bar, parity)) return true;
-    if (status) atomicOr(status, fail_bit);
-    return false;
-}
-// Cluster-scope variants for barriers that another CTA of the cluster arrives on.
-constexpr uint32_t kClusterWaitHintNs = 100;  // suspend-time hint of one try_wait
-__device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "r"(kClusterWaitHintNs) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, unsigned int* status,
-                                                  unsigned int fail_bit) {
-    for (uint32_t i = 0; i < (1u << 21); ++i)  // short sleeps: about the same quarter second in total
-        if (mbar_try_cluster(bar, parity)) return true;
+#pragma unroll 1
+    for (uint32_t i = 0; i < (1u << 17); ++i)
+        if (mbar_try_sleep(bar, parity)) return true;
     if (status) atomicOr(status, fail_bit);
     return false;
 }
