@@ -89,15 +89,15 @@ cudaError_t launch_decode_rate(const DeviceWeights& w, int iters, int warps, int
 struct GemvPlan {
     int grid;            // persistent CTAs (one per SM, fewer for tiny layers)
     int splits;          // typical number of CTAs that share one column block
-    int stages;          // shared-memory ring depth
-    int act_blocks;      // H128 blocks of core input staged at a time
+    int stages;          // weight ring depth, in units
+    int act_blocks;      // H128 blocks of core input a CTA holds
     size_t smem_bytes;
     size_t counter_bytes;   // reserved area at the start of the workspace (0: the fold needs no counters)
-    size_t partial_bytes;   // float [grid][2][rows][128] after the counters
+    size_t partial_bytes;   // partial planes after the counters
+    bool row_kernel;        // one row through gemv_row.cu (else gemv_tmem.cu)
 };
 GemvPlan plan_gemv(const DeviceWeights& w, int rows, int sm_count);
-// `workspace` must be 256-byte aligned and hold counter_bytes + partial_bytes.  The
-// counters must be zero when the kernel starts; it leaves them zero.
+// `workspace` must be 256-byte aligned and hold counter_bytes + partial_bytes.
 // Marks every partial-plane word of a GEMV scratch area "empty".  A completed launch leaves
 // the area empty again, so this is needed once per scratch area (plans) or before a launch
 // on scratch of unknown content (direct calls).

@@ -6,6 +6,7 @@
 namespace st {
 
 cudaError_t configure_gemv_kernels();
+cudaError_t configure_gemv_row_kernels();
 cudaError_t configure_wide_kernels();
 cudaError_t configure_gemm_dense_kernels();
 cudaError_t configure_grouped_kernels();
@@ -26,6 +27,7 @@ int device_sm_count() {
 
 cudaError_t configure_device() {
     cudaError_t e = configure_gemv_kernels();
+    if (e == cudaSuccess) e = configure_gemv_row_kernels();
     if (e == cudaSuccess) e = configure_wide_kernels();
     if (e == cudaSuccess) e = configure_gemm_dense_kernels();
     if (e == cudaSuccess) e = configure_grouped_kernels();

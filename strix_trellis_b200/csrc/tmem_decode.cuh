@@ -2,8 +2,8 @@
 // shared-memory ring into stages of tensor memory, where they are the A operand of tcgen05.mma.
 //
 // A unit is (one 128-column block) x (one H128 block of K): 64 tiles, 128 lanes x 64 columns of
-// tensor memory once decoded.  Eight warps decode a unit, one column tile each; kUnitGroups such
-// groups take turns.  A warp may only write its own lane quarter (warp % 4), so warp w has column
+// tensor memory once decoded.  Eight warps decode a unit, one column tile each; one or several
+// such groups take turns.  A warp may only write its own lane quarter (warp % 4), so warp w has column
 // tiles 2(w % 4) and 2(w % 4) + 1 among its group of eight.
 //
 // Measured with nothing else running (clocks per 16x16 tile per SM sub-partition, K2 / K4 / K5 / K6):
@@ -16,7 +16,6 @@
 
 namespace st {
 
-constexpr int kUnitGroups = 2;
 constexpr int kMaxAStages = 7;  // decoded units in tensor memory
 
 // Decodes this warp's column tile of the units of its turn in one segment: two K = 64 halves per
@@ -29,12 +28,13 @@ struct DecodeState {
     int slot;      // its ring slot
     uint32_t use;  // and the slot's use parity
 };
-template <int K, int CB>
+// GROUPS of eight warps take turns.
+template <int K, int CB, int GROUPS>
 __device__ __forceinline__ bool decode_segment(DecodeState& s, int until, const unsigned char* ring, int w_slots, int w_stride,
                                                uint32_t w_full, uint32_t w_empty, uint32_t a_full, uint32_t a_empty,
                                                uint32_t taddr, int a_stages, int ctile, int lane, unsigned int* status) {
     const LaneGeom<K> geom(lane);
-    for (; s.unit < until; s.unit += kUnitGroups) {
+    for (; s.unit < until; s.unit += GROUPS) {
         const int stage = s.stage;
         if (!mbar_wait(w_full + 8 * s.slot, s.use, status, kTimeoutRingFull)) return false;
         if (s.a_used && !mbar_wait(a_empty + 8 * stage, s.a_prev, status, kTimeoutTensorPipe))
@@ -58,21 +58,21 @@ __device__ __forceinline__ bool decode_segment(DecodeState& s, int until, const 
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(a_full + 8 * stage);
-        s.slot += kUnitGroups;
+        s.slot += GROUPS;
         while (s.slot >= w_slots) { s.slot -= w_slots; s.use ^= 1; }
-        s.stage += kUnitGroups;
+        s.stage += GROUPS;
         if (s.stage >= a_stages) { s.stage -= a_stages; s.a_prev ^= 1; s.a_used = true; }
     }
     return true;
 }
 
 // The same for a run-time rate.
-template <int CB>
+template <int CB, int GROUPS>
 __device__ __forceinline__ bool decode_segment_rate(int bits, DecodeState& s, int until, const unsigned char* ring, int w_slots,
                                                     int w_stride, uint32_t w_full, uint32_t w_empty, uint32_t a_full,
                                                     uint32_t a_empty, uint32_t taddr, int a_stages, int ctile, int lane,
                                                     unsigned int* status) {
-#define ST_DECODE(K) decode_segment<K, CB>(s, until, ring, w_slots, w_stride, w_full, w_empty, a_full, a_empty, taddr, a_stages, ctile, lane, status)
+#define ST_DECODE(K) decode_segment<K, CB, GROUPS>(s, until, ring, w_slots, w_stride, w_full, w_empty, a_full, a_empty, taddr, a_stages, ctile, lane, status)
     switch (bits) {
     case 1: return ST_DECODE(1);
     case 2: return ST_DECODE(2);

@@ -30,7 +30,7 @@
 namespace st {
 
 namespace {
-constexpr int kDecodeW = 8 * kUnitGroups, kEpiW = 4;
+constexpr int kUnitGroups = 2, kDecodeW = 8 * kUnitGroups, kEpiW = 4;
 constexpr int kWarpMma = kDecodeW + kEpiW, kWarpWeights = kWarpMma + 1, kWarpRows = kWarpMma + 2;
 constexpr int kThreadsW = (kWarpRows + 1) * 32;
 constexpr int kChunkRows = 16;                       // rows of one epilogue chunk
@@ -369,7 +369,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             const int len = w.length(args);
             until += len;
             const int bits = args.table ? args.table[w.p].w.bits : args.one.w.bits;
-            ok = decode_segment_rate<CB>(bits, s, until, w_ring, args.w_slots, args.w_stride, w_full, w_empty, a_full, a_empty,
+            ok = decode_segment_rate<CB, kUnitGroups>(bits, s, until, w_ring, args.w_slots, args.w_stride, w_full, w_empty, a_full, a_empty,
                                          taddr, a_stages, ctile, lane, args.status);
             if (!ok || until >= my_units) break;
             w.next(args, len);
