@@ -335,11 +335,11 @@ static strix_status grouped_views(strix_context c, const strix_grouped_gemv_desc
         v.push_back(view);
         offsets.push_back(total);
     }
-    // one grouped launch: [problem table][per group: arrival counters, partial planes]
+    // one grouped launch: [problem table][flags and planes][per group: core input tiles]
     const st::DeviceWeights& w0 = d->weights[0]->device;
-    const st::GroupedPlan gp = st::plan_grouped(w0.inputs, w0.outputs, w0.bits, (int)d->group_count, c->sm_count);
-    total = st::align_up(d->group_count * sizeof(st::GroupedProblem)) +
-            d->group_count * (gp.counter_bytes_per_problem + gp.partial_bytes_per_problem);
+    const st::GroupedPlan gp = st::plan_grouped(w0.inputs, w0.outputs, w0.bits, (int)d->rows, c->sm_count, (int)d->group_count);
+    total = st::align_up(d->group_count * sizeof(st::GroupedProblem)) + st::align_up(gp.shared_bytes) +
+            d->group_count * gp.partial_bytes_per_problem;
     return STRIX_SUCCESS;
 }
 
@@ -377,13 +377,14 @@ strix_status strix_grouped_gemv_plan_create(strix_context c, const strix_grouped
     p->stream = cs;
     {
         const st::DeviceWeights& w0 = m[0].weights->device;
-        p->grouped = st::plan_grouped(w0.inputs, w0.outputs, w0.bits, (int)m.size(), c->sm_count);
+        p->grouped = st::plan_grouped(w0.inputs, w0.outputs, w0.bits, (int)d->rows, c->sm_count, (int)m.size());
         p->inputs = w0.inputs; p->outputs = w0.outputs; p->codebook = w0.codebook;
         p->problem_count = (int)m.size();
         unsigned char* base = static_cast<unsigned char*>(d->workspace);
         p->problems = reinterpret_cast<st::GroupedProblem*>(base);
         const size_t table = st::align_up(m.size() * sizeof(st::GroupedProblem));
-        const size_t each = p->grouped.counter_bytes_per_problem + p->grouped.partial_bytes_per_problem;
+        p->grouped.shared = base + table;
+        unsigned char* tiles = base + table + st::align_up(p->grouped.shared_bytes);
         std::vector<st::GroupedProblem> host(m.size());
         for (size_t g = 0; g < m.size(); ++g) {
             st::GroupedProblem& pr = host[g];
@@ -395,14 +396,14 @@ strix_status strix_grouped_gemv_plan_create(strix_context c, const strix_grouped
             pr.y_stride = (long long)v[g].y_stride;
             pr.rows = v[g].rows;
             for (int k = 0; k < pr.rows; ++k) pr.x_row[k] = pr.y_row[k] = k;
-            pr.counters = reinterpret_cast<unsigned int*>(base + table + g * each);
-            pr.partials = reinterpret_cast<float*>(base + table + g * each + p->grouped.counter_bytes_per_problem);
+            pr.tiles = tiles + g * p->grouped.partial_bytes_per_problem;
+            pr.alpha = 1.0f;
+            st::bind_rows(pr, p->problems + g);
         }
-        cudaError_t e = cudaMemsetAsync(base + table, 0, m.size() * each, cs);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(p->problems, host.data(), host.size() * sizeof(st::GroupedProblem),
-                                cudaMemcpyHostToDevice, cs);
-        const cudaError_t done = cudaStreamSynchronize(cs);  // `host` leaves scope; counters are zero for every replay
+        host[0].live = (int)m.size();
+        const cudaError_t e = cudaMemcpyAsync(p->problems, host.data(), host.size() * sizeof(st::GroupedProblem),
+                                              cudaMemcpyHostToDevice, cs);
+        const cudaError_t done = cudaStreamSynchronize(cs);  // `host` leaves scope
         s = cuda_status(e != cudaSuccess ? e : done);
     }
     if (s != STRIX_SUCCESS) { delete p; return s; }

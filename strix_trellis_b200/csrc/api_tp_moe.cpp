@@ -29,6 +29,7 @@ struct strix_tp_moe_plan_impl {
     int* row_valid = nullptr;                 // device (device-routed plans)
     float *hidden = nullptr, *g = nullptr, *u = nullptr, *each = nullptr;
     st::GroupedPlan gu_plan{}, down_plan{};
+    unsigned char *gu_tiles = nullptr, *down_tiles = nullptr;
     float* y = nullptr;
     long long y_stride = 0;
     float alpha = 1.f, beta = 0.f;
@@ -114,24 +115,17 @@ struct Carver {  // bump allocator over one device block (sizes only when base =
     }
 };
 
-// Problems a step is expected to have when `routes` routes spread evenly over `bank` experts,
-// eight rows per problem.
-int expected_problems(int routes, int bank) {
-    if (routes < 1) routes = 1;
-    const int chunks = (routes + bank * st::kGroupRows - 1) / (bank * st::kGroupRows);
-    return std::min(routes, bank * chunks);
-}
-
 void fill_problem(st::GroupedProblem& p, const st::DeviceWeights& w, const float* x, long long xs, float* y,
-                  long long ys, unsigned int* counters, float* partials) {
+                  long long ys, const st::GroupedProblem* device, unsigned char* tiles) {
     p = st::GroupedProblem{};
     p.w = w;
     p.x = x;
     p.y = y;
     p.x_stride = xs;
     p.y_stride = ys;
-    p.counters = counters;
-    p.partials = partials;
+    p.tiles = tiles;
+    p.alpha = 1.0f;
+    st::bind_rows(p, device);
 }
 
 // Lays out the plan-owned block and (when `p->block` is set) fills pointers.
@@ -147,34 +141,12 @@ size_t layout_block(strix_tp_moe_plan_impl* p, int gu_slots, int down_slots, boo
     p->g = c.take<float>(routes * p->inter);
     p->u = c.take<float>(routes * p->inter);
     p->each = c.take<float>(routes * p->model);
-    // per-problem scratch: counters then partial planes
-    unsigned char* gu_scratch = c.take<unsigned char>(
-        (size_t)gu_slots * (p->gu_plan.counter_bytes_per_problem + p->gu_plan.partial_bytes_per_problem));
-    unsigned char* dn_scratch = c.take<unsigned char>(
-        (size_t)down_slots * (p->down_plan.counter_bytes_per_problem + p->down_plan.partial_bytes_per_problem));
-    (void)gu_scratch;
-    (void)dn_scratch;
+    // the two launches run one after the other: they share flags and planes
+    unsigned char* shared = c.take<unsigned char>(std::max(p->gu_plan.shared_bytes, p->down_plan.shared_bytes));
+    p->gu_plan.shared = p->down_plan.shared = shared;
+    p->gu_tiles = c.take<unsigned char>((size_t)gu_slots * p->gu_plan.partial_bytes_per_problem);
+    p->down_tiles = c.take<unsigned char>((size_t)down_slots * p->down_plan.partial_bytes_per_problem);
     return st::align_up(c.used);
-}
-
-unsigned char* scratch_of(strix_tp_moe_plan_impl* p, bool down, int slot) {
-    // recompute the scratch base the same way layout_block did
-    Carver c{static_cast<unsigned char*>(p->block)};
-    const size_t routes = (size_t)p->tokens * p->top_k;
-    const int gu_slots = p->gu_count, down_slots = p->down_count;
-    c.take<st::GroupedProblem>(gu_slots);
-    c.take<st::GroupedProblem>(down_slots);
-    c.take<st::MoeBankEntry>(p->bank_count);
-    c.take<int>(p->device_routed ? p->tokens : 0);
-    c.take<float>(p->device_routed ? 0 : routes);
-    c.take<float>(routes * p->inter);
-    c.take<float>(routes * p->inter);
-    c.take<float>(routes * p->model);
-    const size_t gu_each = p->gu_plan.counter_bytes_per_problem + p->gu_plan.partial_bytes_per_problem;
-    const size_t dn_each = p->down_plan.counter_bytes_per_problem + p->down_plan.partial_bytes_per_problem;
-    unsigned char* gu_scratch = c.take<unsigned char>((size_t)gu_slots * gu_each);
-    unsigned char* dn_scratch = c.take<unsigned char>((size_t)down_slots * dn_each);
-    return down ? dn_scratch + (size_t)slot * dn_each : gu_scratch + (size_t)slot * gu_each;
 }
 
 void destroy_plan(strix_tp_moe_plan_impl* p) {
@@ -296,7 +268,7 @@ strix_status create_host(strix_context c, const strix_tp_moe_desc* d, const stri
     s = host_routing(d, tokens, top_k, route_expert);
     if (s != STRIX_SUCCESS) return s;
 
-    // group routes by expert, eight rows per problem (all routes for gate/up, scored ones for down)
+    // group routes by expert, kGroupRows rows per problem (all routes for gate/up, scored ones for down)
     const int experts = (int)d->expert_count, routes = tokens * top_k;
     std::vector<std::vector<int>> by_expert(experts);
     for (int r = 0; r < routes; ++r) by_expert[route_expert[r]].push_back(r);
@@ -318,8 +290,8 @@ strix_status create_host(strix_context c, const strix_tp_moe_desc* d, const stri
     p->tokens = tokens; p->top_k = top_k; p->model = g.model; p->inter = g.inter; p->codebook = g.codebook;
     p->gu_count = 2 * (int)gu_chunks.size();
     p->down_count = (int)down_chunks.size();
-    p->gu_plan = st::plan_grouped(g.model, g.inter, g.max_bits, p->gu_count, c->sm_count);
-    p->down_plan = st::plan_grouped(g.inter, g.model, g.max_bits, std::max(p->down_count, 1), c->sm_count);
+    p->gu_plan = st::plan_grouped(g.model, g.inter, g.max_bits, tokens, c->sm_count, p->gu_count);
+    p->down_plan = st::plan_grouped(g.inter, g.model, g.max_bits, tokens, c->sm_count, p->down_count);
     const size_t bytes = layout_block(p, p->gu_count, p->down_count, true);
     cudaError_t e = cudaMalloc(&p->block, bytes);
     if (e != cudaSuccess) { (void)cudaGetLastError(); delete p; return cuda_status(e); }
@@ -335,10 +307,8 @@ strix_status create_host(strix_context c, const strix_tp_moe_desc* d, const stri
         const strix_tp_expert_desc& ex = d->experts[gu_chunks[i].expert];
         for (int half = 0; half < 2; ++half) {
             st::GroupedProblem& pr = host_gu[2 * i + half];
-            unsigned char* sc = scratch_of(p, false, (int)(2 * i + half));
             fill_problem(pr, half ? ex.up->device : ex.gate->device, x, (long long)xs, half ? p->u : p->g, g.inter,
-                         reinterpret_cast<unsigned int*>(sc),
-                         reinterpret_cast<float*>(sc + p->gu_plan.counter_bytes_per_problem));
+                         p->gu + 2 * i + half, p->gu_tiles + (2 * i + half) * p->gu_plan.partial_bytes_per_problem);
             pr.rows = (int)gu_chunks[i].routes.size();
             for (int k = 0; k < pr.rows; ++k) {
                 pr.x_row[k] = gu_chunks[i].routes[k] / top_k;  // token
@@ -349,13 +319,14 @@ strix_status create_host(strix_context c, const strix_tp_moe_desc* d, const stri
     for (size_t i = 0; i < down_chunks.size(); ++i) {
         const strix_tp_expert_desc& ex = d->experts[down_chunks[i].expert];
         st::GroupedProblem& pr = host_dn[i];
-        unsigned char* sc = scratch_of(p, true, (int)i);
-        fill_problem(pr, ex.down->device, p->hidden, g.inter, p->each, g.model, reinterpret_cast<unsigned int*>(sc),
-                     reinterpret_cast<float*>(sc + p->down_plan.counter_bytes_per_problem));
+        fill_problem(pr, ex.down->device, p->hidden, g.inter, p->each, g.model, p->down + i,
+                     p->down_tiles + i * p->down_plan.partial_bytes_per_problem);
         pr.rows = (int)down_chunks[i].routes.size();
         for (int k = 0; k < pr.rows; ++k) pr.x_row[k] = pr.y_row[k] = down_chunks[i].routes[k];
     }
-    // zero the whole block (counters must start at zero), then upload tables and scores
+    if (p->gu_count) host_gu[0].live = p->gu_count;
+    if (p->down_count) host_dn[0].live = p->down_count;
+    // zero the whole block (rows that no problem writes read as zero), then upload tables and scores
     e = cudaMemsetAsync(p->block, 0, bytes, cs);
     if (e == cudaSuccess && p->gu_count)
         e = cudaMemcpyAsync(p->gu, host_gu.data(), host_gu.size() * sizeof(st::GroupedProblem), cudaMemcpyHostToDevice, cs);
@@ -414,24 +385,12 @@ strix_status create_device(strix_context c, const strix_tp_moe_device_desc* d, c
     const int routes = tokens * top_k;
     p->owner = c; p->stream = cs; p->device_routed = true;
     p->tokens = tokens; p->top_k = top_k; p->model = g.model; p->inter = g.inter; p->codebook = g.codebook;
-    p->gu_count = 2 * routes;
-    p->down_count = routes;
     p->bank_count = (int)d->expert_count;
+    p->down_count = st::max_problems(routes, p->bank_count);
+    p->gu_count = 2 * p->down_count;
     p->window = st::MoeWindow{0, p->bank_count};
-    // the K partition is planned for the problems a step is EXPECTED to have (routes spread evenly
-    // over the bank, eight rows per problem), not for the slots it may have at most
-    const int spread = expected_problems(routes, p->bank_count);
-    p->max_bits = g.max_bits;
-    // Scratch for up to four times the planned partitions (while it stays under 128 MB): a
-    // window set later means fewer local routes, and fewer problems want more partitions.
-    int headroom = 4;
-    for (;; headroom /= 2) {
-        p->gu_plan = st::plan_grouped(g.model, g.inter, g.max_bits, 2 * spread, c->sm_count, headroom);
-        p->down_plan = st::plan_grouped(g.inter, g.model, g.max_bits, spread, c->sm_count, headroom);
-        const size_t scratch = (size_t)p->gu_count * p->gu_plan.partial_bytes_per_problem +
-                               (size_t)p->down_count * p->down_plan.partial_bytes_per_problem;
-        if (headroom == 1 || scratch <= ((size_t)128 << 20)) break;
-    }
+    p->gu_plan = st::plan_grouped(g.model, g.inter, g.max_bits, tokens, c->sm_count, p->gu_count);
+    p->down_plan = st::plan_grouped(g.inter, g.model, g.max_bits, tokens, c->sm_count, p->down_count);
     const size_t bytes = layout_block(p, p->gu_count, p->down_count, false);
     cudaError_t e = cudaMalloc(&p->block, bytes);
     if (e != cudaSuccess) { (void)cudaGetLastError(); delete p; return cuda_status(e); }
@@ -442,26 +401,16 @@ strix_status create_device(strix_context c, const strix_tp_moe_device_desc* d, c
     p->y = static_cast<float*>(d->output.data);
     p->y_stride = (long long)ys;
     p->alpha = d->alpha; p->beta = d->beta;
-    // static part of every per-route slot; the device routing kernel fills weights and rows
+    // static part of every record; the device routing kernel fills weights, rows and counts
     std::vector<st::GroupedProblem> host_gu(p->gu_count), host_dn(p->down_count);
     std::vector<st::MoeBankEntry> bank(p->bank_count);
     const float* x = static_cast<const float*>(d->input.data);
-    for (int route = 0; route < routes; ++route) {
-        for (int half = 0; half < 2; ++half) {
-            st::GroupedProblem& pr = host_gu[2 * route + half];
-            unsigned char* sc = scratch_of(p, false, 2 * route + half);
-            fill_problem(pr, st::DeviceWeights{}, x, (long long)xs, half ? p->u : p->g, g.inter,
-                         reinterpret_cast<unsigned int*>(sc),
-                         reinterpret_cast<float*>(sc + p->gu_plan.counter_bytes_per_problem));
-            pr.x_row[0] = route / top_k;
-            pr.y_row[0] = route;
-        }
-        st::GroupedProblem& pr = host_dn[route];
-        unsigned char* sc = scratch_of(p, true, route);
-        fill_problem(pr, st::DeviceWeights{}, p->hidden, g.inter, p->each, g.model, reinterpret_cast<unsigned int*>(sc),
-                     reinterpret_cast<float*>(sc + p->down_plan.counter_bytes_per_problem));
-        pr.x_row[0] = pr.y_row[0] = route;
-    }
+    for (int i = 0; i < p->gu_count; ++i)
+        fill_problem(host_gu[i], st::DeviceWeights{}, x, (long long)xs, i & 1 ? p->u : p->g, g.inter, p->gu + i,
+                     p->gu_tiles + i * p->gu_plan.partial_bytes_per_problem);
+    for (int i = 0; i < p->down_count; ++i)
+        fill_problem(host_dn[i], st::DeviceWeights{}, p->hidden, g.inter, p->each, g.model, p->down + i,
+                     p->down_tiles + i * p->down_plan.partial_bytes_per_problem);
     for (int i = 0; i < p->bank_count; ++i)
         bank[i] = st::MoeBankEntry{d->experts[i].gate->device, d->experts[i].up->device, d->experts[i].down->device};
     e = cudaMemsetAsync(p->block, 0, bytes, cs);
@@ -555,13 +504,6 @@ strix_status strix_b200_moe_plan_set_window(strix_tp_moe_plan p, uint32_t first_
     if (experts_total > INT_MAX || (uint64_t)first_expert + (uint64_t)p->bank_count > experts_total)
         return STRIX_ERROR_INVALID_ARGUMENT;
     p->window = st::MoeWindow{(int)first_expert, (int)experts_total};
-    // of all routes, about bank / experts_total are this rank's: plan the partitions for those
-    const long long routes = (long long)p->tokens * p->top_k;
-    const int local = (int)std::max<long long>(1, (routes * p->bank_count + experts_total - 1) / experts_total);
-    const int spread = expected_problems(local, p->bank_count);
-    const int sms = p->owner->sm_count;
-    p->gu_plan = st::replan_grouped(p->gu_plan, p->model, p->inter, p->max_bits, 2 * spread, sms);
-    p->down_plan = st::replan_grouped(p->down_plan, p->inter, p->model, p->max_bits, spread, sms);
     return STRIX_SUCCESS;
 }
 // Routing, gate/up, SwiGLU and down of the routes this rank owns; no combine.
@@ -624,9 +566,9 @@ static strix_status swiglu_shape(strix_context c, const strix_tp_swiglu_desc* d,
     s = row_view(d->input, rows, g.inputs, xs, xb);
     if (s == STRIX_SUCCESS) s = row_view(d->hidden_output, rows, g.outputs, hs, hb);
     if (s != STRIX_SUCCESS) return s;
-    const st::GroupedPlan plan = st::plan_grouped(g.inputs, g.outputs, st::heavier_rate(g.bits, u.bits), 2, c->sm_count);
+    const st::GroupedPlan plan = st::plan_grouped(g.inputs, g.outputs, st::heavier_rate(g.bits, u.bits), rows, c->sm_count, 2);
     need = st::align_up((uint64_t)2 * rows * g.outputs * 4) +
-           2 * (plan.counter_bytes_per_problem + plan.partial_bytes_per_problem) + st::align_up(2 * sizeof(st::GroupedProblem));
+           st::align_up(2 * plan.partial_bytes_per_problem) + st::align_up(plan.shared_bytes) + st::align_up(2 * sizeof(st::GroupedProblem));
     return STRIX_SUCCESS;
 }
 
@@ -681,28 +623,28 @@ strix_status strix_tp_swiglu_plan_create(strix_context c, const strix_tp_swiglu_
     const st::DeviceWeights &g = d->gate->device, &u = d->up->device;
     p->owner = c; p->stream = cs; p->gate = d->gate; p->up = d->up; p->is_swiglu = true;
     p->rows = rows; p->inter = g.outputs; p->inputs = g.inputs; p->codebook = g.codebook;
-    p->plan = st::plan_grouped(g.inputs, g.outputs, st::heavier_rate(g.bits, u.bits), 2, c->sm_count);
+    p->plan = st::plan_grouped(g.inputs, g.outputs, st::heavier_rate(g.bits, u.bits), rows, c->sm_count, 2);
     Carver carve{static_cast<unsigned char*>(d->workspace)};
     p->g = carve.take<float>((size_t)rows * g.outputs);
     p->u = p->g + (size_t)rows * g.outputs;
     carve.used = st::align_up((size_t)2 * rows * g.outputs * 4);
     if (d->diagnostic_gate) p->g = d->diagnostic_gate;
     if (d->diagnostic_up) p->u = d->diagnostic_up;
-    const size_t each = p->plan.counter_bytes_per_problem + p->plan.partial_bytes_per_problem;
-    unsigned char* scratch = carve.take<unsigned char>(2 * each);
+    const size_t each = p->plan.partial_bytes_per_problem;
+    unsigned char* tiles = carve.take<unsigned char>(2 * each);
+    p->plan.shared = carve.take<unsigned char>(p->plan.shared_bytes);
     p->problems = carve.take<st::GroupedProblem>(2);
     p->hidden = static_cast<float*>(d->hidden_output.data);
     p->hidden_stride = (long long)hs;
     st::GroupedProblem host[2];
     for (int half = 0; half < 2; ++half) {
         fill_problem(host[half], half ? u : g, static_cast<const float*>(d->input.data), (long long)xs, half ? p->u : p->g,
-                     g.outputs, reinterpret_cast<unsigned int*>(scratch + half * each),
-                     reinterpret_cast<float*>(scratch + half * each + p->plan.counter_bytes_per_problem));
+                     g.outputs, p->problems + half, tiles + half * each);
         host[half].rows = rows;
         for (int k = 0; k < rows; ++k) host[half].x_row[k] = host[half].y_row[k] = k;
     }
-    cudaError_t e = cudaMemsetAsync(scratch, 0, 2 * each, cs);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(p->problems, host, sizeof(host), cudaMemcpyHostToDevice, cs);
+    host[0].live = 2;
+    cudaError_t e = cudaMemcpyAsync(p->problems, host, sizeof(host), cudaMemcpyHostToDevice, cs);
     const cudaError_t done = cudaStreamSynchronize(cs);
     if (e != cudaSuccess || done != cudaSuccess) { delete p; return cuda_status(e != cudaSuccess ? e : done); }
     ++d->gate->plan_refs;

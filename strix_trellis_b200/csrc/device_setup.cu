@@ -9,7 +9,6 @@ cudaError_t configure_gemv_kernels();
 cudaError_t configure_gemv_row_kernels();
 cudaError_t configure_wide_kernels();
 cudaError_t configure_gemm_dense_kernels();
-cudaError_t configure_grouped_kernels();
 
 // SM count of the current device, looked up once per device ordinal.
 int device_sm_count() {
@@ -30,7 +29,6 @@ cudaError_t configure_device() {
     if (e == cudaSuccess) e = configure_gemv_row_kernels();
     if (e == cudaSuccess) e = configure_wide_kernels();
     if (e == cudaSuccess) e = configure_gemm_dense_kernels();
-    if (e == cudaSuccess) e = configure_grouped_kernels();
     return e;
 }
 

@@ -1,43 +1,41 @@
 // Grouped linears: many independent complete linears of ONE geometry (inputs, outputs)
-// in one launch, each with its own weights (any rate 1..8), its own gathered input rows and
-// scattered output rows.  Building block of the routed-expert, SwiGLU and grouped-GEMV plans.
+// in one launch of wide_linear.cu, each with its own weights (any rate), its own gathered input
+// rows and scattered output rows.  Building block of the routed-expert, SwiGLU and grouped-GEMV plans.
 #pragma once
 #include "backend.h"
+#include "wide_linear.h"
 
 namespace st {
 
-constexpr int kGroupRows = 8;
+constexpr int kGroupRows = 128;  // most rows of one problem: its weights are decoded once for all of them
 
-// One problem.  rows == 0 marks an unused slot (its CTAs exit at once).
-// Input row r is x + x_row[r]*x_stride, output row r is y + y_row[r]*y_stride.
-struct GroupedProblem {
-    DeviceWeights w;
-    const float* x;
-    float* y;
-    long long x_stride, y_stride;
-    int rows;
+// One problem of a table in device memory.  Input row r is x + x_row[r]*x_stride, output row r is
+// y + y_row[r]*y_stride (x_rows / y_rows point at the arrays of the record itself, see bind_rows).
+struct GroupedProblem : WideProblem {
+    int live;  // in the table's FIRST record: how many of its records a launch runs
     int x_row[kGroupRows];
     int y_row[kGroupRows];
-    unsigned int* counters;  // [outputs/128], zero between launches
-    float* partials;         // [outputs/128][splits][rows][128]
 };
+// Points a host copy's row arrays at those of the device record it will be copied to.
+inline void bind_rows(GroupedProblem& host, const GroupedProblem* device) {
+    host.x_rows = device->x_row;
+    host.y_rows = device->y_row;
+}
 
 struct GroupedPlan {
-    int splits;          // K partitions per column block of a launch
-    int scratch_splits;  // partitions the per-problem scratch is sized for (>= splits)
-    int stages;
-    int ctas_per_problem;
-    int stage_stride;
-    size_t smem_bytes;
-    size_t counter_bytes_per_problem;
-    size_t partial_bytes_per_problem;  // for kGroupRows rows
+    int splits;            // typical number of CTAs that share one column block
+    int scratch_splits;    // planes of partial sums per CTA
+    int stages;            // weight ring slots
+    int ctas_per_problem;  // CTAs of a launch of one problem
+    WidePlan wide;
+    size_t counter_bytes_per_problem;  // 0: nothing is counted per problem
+    size_t partial_bytes_per_problem;  // core input tiles of one problem
+    size_t shared_bytes;               // flags and planes of a launch
+    unsigned char* shared;             // the caller's memory for them
 };
-// `problems` = the number of problems a launch is EXPECTED to have live (it sets the partition
-// count).  `headroom` sizes the scratch for that many times the planned partitions, so that
-// replan_grouped may choose more of them later, when the expectation changes.
-GroupedPlan plan_grouped(int inputs, int outputs, int max_bits, int problems, int sm_count, int headroom = 1);
-GroupedPlan replan_grouped(const GroupedPlan& sized, int inputs, int outputs, int max_bits, int problems, int sm_count);
-// `problems` lives in device memory; slots with rows == 0 are skipped on the device.
+// `rows` = most rows of one problem, `problems` = most problems of a launch.
+GroupedPlan plan_grouped(int inputs, int outputs, int max_bits, int rows, int sm_count, int problems);
+// `problems` lives in device memory; problems[0].live of its `problem_count` records are run.
 cudaError_t launch_grouped(const GroupedProblem* problems, int problem_count, int inputs, int outputs,
                            int codebook, const GroupedPlan& plan, unsigned int* status, bool programmatic,
                            cudaStream_t stream);
@@ -48,8 +46,12 @@ cudaError_t launch_swiglu(const float* gate, const float* up, float* hidden, int
                           long long out_stride, bool programmatic, cudaStream_t stream);
 
 // Device-side routing for a persistent expert bank: validates each token's route row and
-// groups the valid routes by expert into problem slots of up to kGroupRows rows each
-// (slot tables hold tokens*top_k slots; unused ones get rows = 0).
+// groups the valid routes by expert into problems of up to kGroupRows rows each, the first records of
+// the tables, and sets their `live` counts.  The tables hold max_problems(...) (gate/up: twice that).
+inline int max_problems(int routes, int bank) {
+    const long long most = (long long)bank + routes / kGroupRows;  // one remainder per expert, full ones beyond
+    return (int)(most < routes ? most : routes);
+}
 struct MoeBankEntry { DeviceWeights gate, up, down; };
 // The bank is a window of the router's id space: id g is bank entry g - first_expert when that
 // lies in [0, bank_count), belongs to another rank when g < experts_total (its slot runs nothing

@@ -42,24 +42,29 @@ constexpr int kRingMin = kDecodeW / 4 * kStageFloats * 4;       // the decode gr
 
 struct WideArgs {
     const WideProblem* table;
+    size_t table_stride;
     const int* live;
     WideProblem one;
     int count, hblocks, nblocks;
     int n_max, w_slots, w_stride, b_slots, b_stride;
-    int a_stages, d_bufs;  // tensor memory: a_stages x 64 columns of A, d_bufs accumulators of n_max
+    // tensor memory: a_stages x 64 columns of A, then d_bufs buffers of d_accs accumulators of n_max
+    int a_stages, d_bufs, d_accs;
     unsigned int* flags;
     float* planes;
     unsigned int* status;
 };
 
 // Problem p of the set: from the table, or row group p of the one layer.
+__device__ __forceinline__ const WideProblem& problem(const WideArgs& a, int p) {
+    return a.table ? *reinterpret_cast<const WideProblem*>(reinterpret_cast<const unsigned char*>(a.table) + p * a.table_stride) : a.one;
+}
 __device__ __forceinline__ int problem_rows(const WideArgs& a, int p) {
-    if (a.table) return a.table[p].rows;
+    if (a.table) return problem(a, p).rows;
     const int left = a.one.rows - p * kWideRows;
     return left < kWideRows ? left : kWideRows;
 }
 __device__ __forceinline__ const unsigned char* problem_tiles(const WideArgs& a, int p) {
-    return a.table ? a.table[p].tiles : a.one.tiles + (size_t)p * a.hblocks * wide_tile_bytes(kWideRows);
+    return a.table ? problem(a, p).tiles : a.one.tiles + (size_t)p * a.hblocks * wide_tile_bytes(kWideRows);
 }
 
 // Position in a CTA's unit range; every role walks it segment by segment (a segment ends with a
@@ -113,7 +118,7 @@ struct Epilogue {
         int last = cta;
         if (!contributor && w.hb + len < a.hblocks) last = owner(split, hi - 1);
         (void)mine;
-        const WideProblem& pr = a.table ? a.table[w.p] : a.one;
+        const WideProblem& pr = problem(a, w.p);
         // The flag of CTA c counts the chunks of its plane that are there.
         bool late = false;
         for (int c = cta + 1; c <= last && !late; ++c) {
@@ -135,6 +140,16 @@ struct Epilogue {
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(r[j]));  // not before the wait
+            if (a.d_accs == 2) {
+                uint32_t q[16];
+                tmem_ld_32x16(taddr + a.n_max + ch * kChunkRows, q);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    asm volatile("" : "+r"(q[j]));
+                    r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(q[j])));
+                }
+            }
             if (contributor) {
                 float* plane = a.planes + ((size_t)cta * a.n_max + ch * kChunkRows) * 128 + col;
 #pragma unroll
@@ -246,7 +261,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     const uint32_t tmem = s_tmem_base;
     pdl_launch_dependents();
 
-    auto d_column = [&](int seg) { return a_stages * 64 + (d_bufs == 2 ? (seg & 1) * args.n_max : 0); };
+    auto d_column = [&](int seg) { return a_stages * 64 + (d_bufs == 2 ? (seg & 1) * args.d_accs * args.n_max : 0); };
     auto d_parity = [&](int seg) { return (uint32_t)(d_bufs == 2 ? seg >> 1 : seg) & 1; };  // of the seg-th use
     auto d_index = [&](int seg) { return d_bufs == 2 ? seg & 1 : 0; };
 
@@ -257,7 +272,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             bool ok = true;
             for (Walk w(args, mine); w.unit < w.end && ok;) {
                 const int len = w.length(args);
-                const DeviceWeights& dw = args.table ? args.table[w.p].w : args.one.w;
+                const DeviceWeights& dw = problem(args, w.p).w;
                 const uint32_t bytes = unit_bytes(dw.bits);
                 const unsigned char* src = reinterpret_cast<const unsigned char*>(dw.packed) +
                                            ((size_t)w.nb * args.hblocks + w.hb) * bytes;
@@ -309,6 +324,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         for (Walk w(args, mine); w.unit < w.end && ok; ++seg) {
             const int len = w.length(args), n = wide_n(problem_rows(args, w.p));
             const uint32_t idesc = umma_idesc_f16_f32(128, n), dcol = tmem + d_column(seg);
+            const uint32_t odd = args.d_accs == 2 ? args.n_max : 0;  // accumulator of the odd K steps
             if (seg >= d_bufs && !mbar_wait(d_empty + 8 * d_index(seg), d_parity(seg) ^ 1, args.status, kTimeoutTensorPipe)) break;
             for (int i = 0; i < len; ++i) {
                 if (!mbar_wait(b_full + 8 * slot, use, args.status, kTimeoutTensorPipe) ||
@@ -322,7 +338,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        umma_f16_ts(dcol, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, (i | k) != 0);
+                        umma_f16_ts(dcol + (k & 1) * odd, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, i != 0 || k >= args.d_accs);
                     umma_commit(a_empty + 8 * stage);
                     umma_commit(b_empty + 8 * slot);
                 }
@@ -339,7 +355,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         // Output scales and bias are cold in DRAM and needed at the very end: ask the L2 for them now.
         for (int b = mine.begin / args.hblocks + (warp & 3), e = (mine.end - 1) / args.hblocks; b <= e; b += kEpiW) {
             const int p = b / args.nblocks, nb = b - p * args.nblocks;
-            const DeviceWeights& dw = args.table ? args.table[p].w : args.one.w;
+            const DeviceWeights& dw = problem(args, p).w;
             if (lane < 2) prefetch_line_l2(dw.svh + (size_t)nb * 128 + lane * 64);
             else if (lane < 6 && dw.bias) prefetch_line_l2(dw.bias + (size_t)nb * 128 + (lane - 2) * 32);
         }
@@ -368,7 +384,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         while (true) {
             const int len = w.length(args);
             until += len;
-            const int bits = args.table ? args.table[w.p].w.bits : args.one.w.bits;
+            const int bits = problem(args, w.p).w.bits;
             ok = decode_segment_rate<CB, kUnitGroups>(bits, s, until, w_ring, args.w_slots, args.w_stride, w_full, w_empty, a_full, a_empty,
                                          taddr, a_stages, ctile, lane, args.status);
             if (!ok || until >= my_units) break;
@@ -423,7 +439,7 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
         for (int i = threadIdx.x; i < grid_ctas; i += blockDim.x) args.flags[i] = 0;
     const int count = args.live ? *args.live : args.count;
     for (int p = blockIdx.y; p < count; p += gridDim.y) {
-        const WideProblem& pr = args.table ? args.table[p] : args.one;
+        const WideProblem& pr = problem(args, p);
         const int rows = problem_rows(args, p), quads = (rows + 3) / 4;
         const size_t tile_bytes = wide_tile_bytes(rows);
         unsigned char* tiles = const_cast<unsigned char*>(problem_tiles(args, p));
@@ -479,6 +495,7 @@ WidePlan plan_wide(int inputs, int heaviest, int rows_max, long long units, int 
 static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int* flags, float* planes, unsigned int* status) {
     WideArgs a{};
     a.table = set.table;
+    a.table_stride = set.table_stride;
     a.live = set.live;
     a.one = set.one;
     a.count = set.count;
@@ -489,10 +506,11 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     a.w_stride = plan.w_stride;
     a.b_slots = plan.b_slots;
     a.b_stride = plan.b_stride;
-    // A second accumulator lets the MMAs of the next segment start under this one's epilogue; it is
-    // worth less than two more stages of A, so it exists where there is room for both.
+    // Even and odd K steps have accumulators of their own where there is room: half the roundings in
+    // a row.  A second buffer lets the MMAs of the next segment start under this one's epilogue.
+    a.d_accs = plan.n_max <= 128 ? 2 : 1;
     a.d_bufs = plan.n_max <= 64 ? 2 : 1;
-    a.a_stages = (512 - a.d_bufs * plan.n_max) / 64;
+    a.a_stages = (512 - a.d_bufs * a.d_accs * plan.n_max) / 64;
     if (a.a_stages > kMaxAStages) a.a_stages = kMaxAStages;
     a.flags = flags;
     a.planes = planes;

@@ -22,8 +22,8 @@ struct WideProblem {
     float alpha, beta;
 };
 
-__host__ __device__ inline int wide_n(int rows) { return rows <= 16 ? 16 : (rows + 15) & ~15; }  // MMA N
-__host__ __device__ inline size_t wide_tile_bytes(int rows) { return (size_t)wide_n(rows) * 256; }
+ST_RATE_FN int wide_n(int rows) { return rows <= 16 ? 16 : (rows + 15) & ~15; }  // MMA N
+ST_RATE_FN size_t wide_tile_bytes(int rows) { return (size_t)wide_n(rows) * 256; }
 
 struct WidePlan {
     int grid;
@@ -37,11 +37,12 @@ struct WidePlan {
 // `heaviest`: the rate code with the largest tiles among the problems.
 WidePlan plan_wide(int inputs, int heaviest, int rows_max, long long units, int sm_count);
 
-// A set of problems of one geometry.  `table` (device memory) holds them; without a table the set is
-// ONE layer whose `one.rows` rows are cut into problems of kWideRows rows.  `live` (device memory,
-// may be null) overrides `count` at run time.
+// A set of problems of one geometry.  `table` (device memory) holds them, `table_stride` bytes apart;
+// without a table the set is ONE layer whose `one.rows` rows are cut into problems of kWideRows rows.
+// `live` (device memory, may be null) overrides `count` at run time.
 struct WideSet {
     const WideProblem* table;
+    size_t table_stride;
     const int* live;
     WideProblem one;
     int count;
