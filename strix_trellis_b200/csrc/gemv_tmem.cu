@@ -34,7 +34,7 @@
 namespace st {
 
 namespace {
-constexpr int kUnitGroups = 2, kDecodeT = 8 * kUnitGroups, kHelpersT = 8;
+constexpr int kUnitGroups = 4, kDecodeT = 4 * kUnitGroups, kHelpersT = 8;
 constexpr int kWarpMmaT = kDecodeT + kHelpersT, kWarpWeightsT = kWarpMmaT + 1;
 constexpr int kThreadsT = (kWarpWeightsT + 1) * 32;
 constexpr int kRowsT = 16;                       // the MMA's N: the smallest it has; rows beyond the call's are never read
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
                   reinterpret_cast<const unsigned char*>(c.w.packed) + (size_t)(mine.begin + unit) * w_stride, w_stride, w_full + 8 * slot);
     };
     if (warp == kWarpWeightsT) {
-        if (lane < args.w_slots) { mbar_init(w_full + 8 * lane, 1); mbar_init(w_empty + 8 * lane, 8); }
+        if (lane < args.w_slots) { mbar_init(w_full + 8 * lane, 1); mbar_init(w_empty + 8 * lane, 4); }
         mbar_fence_init();
         __syncwarp();
         if (lane == 0)
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
     } else {  // one decode thread per barrier
         const int t = threadIdx.x;
         if (t < args.b_slots) { mbar_init(b_full + 8 * t, rows); mbar_init(b_empty + 8 * t, 1); }
-        if (t < kMaxAStages) { mbar_init(a_full + 8 * t, 8); mbar_init(a_empty + 8 * t, 1); }
+        if (t < kMaxAStages) { mbar_init(a_full + 8 * t, 4); mbar_init(a_empty + 8 * t, 1); }
         if (t < 2) { mbar_init(d_full + 8 * t, 1); mbar_init(d_empty + 8 * t, 4); }
         mbar_fence_init();
     }
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
         }
     } else if (warp < kDecodeT) {
         // ---- decode warps ---------------------------------------------------------------------------
-        const int turn = warp >> 3, ctile = 2 * (warp & 3) + ((warp >> 2) & 1);
+        const int turn = warp >> 2, ctile = 2 * (warp & 3);
         DecodeState s{turn, turn, 1, false, turn % args.w_slots, (uint32_t)(turn / args.w_slots) & 1};
         decode_segment_rate<CB, kUnitGroups>(c.w.bits, s, my_units, w_ring, args.w_slots, w_stride, w_full, w_empty, a_full, a_empty,
                                              tmem + ((uint32_t)(ctile * 16) << 16), kMaxAStages, ctile, lane, c.status);

@@ -2,9 +2,11 @@
 // shared-memory ring into stages of tensor memory, where they are the A operand of tcgen05.mma.
 //
 // A unit is (one 128-column block) x (one H128 block of K): 64 tiles, 128 lanes x 64 columns of
-// tensor memory once decoded.  Eight warps decode a unit, one column tile each; one or several
-// such groups take turns.  A warp may only write its own lane quarter (warp % 4), so warp w has column
-// tiles 2(w % 4) and 2(w % 4) + 1 among its group of eight.
+// tensor memory once decoded.  A warp may only write its own lane quarter (warp % 4), so the four
+// warps of a group decode column tiles 2q and 2q + 1 of a unit each, sixteen tiles between two
+// rounds of barriers; several groups take turns.  (Eight warps per unit, eight tiles each, took
+// 129 against 115 us for 4096 -> 129280 at K5: the barriers, slot and stage arithmetic are about
+// sixty instructions per round.)
 //
 // Measured with nothing else running (clocks per 16x16 tile per SM sub-partition, K2 / K4 / K5 / K6):
 // 45 / 43 / 50 / 54, against 51 / 48 / 56 / 58 with each tile fed to mma.sync, which holds the
@@ -18,8 +20,8 @@ namespace st {
 
 constexpr int kMaxAStages = 7;  // decoded units in tensor memory
 
-// Decodes this warp's column tile of the units of its turn in one segment: two K = 64 halves per
-// unit, four tiles each, one tensor-memory store per half.
+// Decodes this warp's two column tiles of the units of its turn in one segment:
+// two K = 64 halves per column tile, four tiles each, one tensor-memory store per half.
 struct DecodeState {
     int unit;      // counter over the CTA's range: the next unit of this warp's turn
     int stage;     // its tensor-memory stage
@@ -28,7 +30,7 @@ struct DecodeState {
     int slot;      // its ring slot
     uint32_t use;  // and the slot's use parity
 };
-// GROUPS of eight warps take turns.
+// GROUPS of four warps take turns.
 template <int K, int CB, int GROUPS>
 __device__ __forceinline__ bool decode_segment(DecodeState& s, int until, const unsigned char* ring, int w_slots, int w_stride,
                                                uint32_t w_full, uint32_t w_empty, uint32_t a_full, uint32_t a_empty,
@@ -41,17 +43,21 @@ __device__ __forceinline__ bool decode_segment(DecodeState& s, int until, const 
             return false;
         tc_fence_after_sync();
         const uint32_t* tiles = reinterpret_cast<const uint32_t*>(ring + (size_t)s.slot * w_stride) + ctile * tile_words(K);
+        uint32_t to = taddr + stage * 64;
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c, tiles += tile_words(K), to += 16u << 16) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            uint32_t r[16];
+            for (int half = 0; half < 2; ++half) {
+                uint32_t r[16];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                uint32_t f[4];
-                decode_tile_frag<K, CB>(tiles + (half * 4 + t) * 8 * tile_words(K), geom, f);
+                for (int t = 0; t < 4; ++t) {
+                    uint32_t f[4];
+                    decode_tile_frag<K, CB>(tiles + (half * 4 + t) * 8 * tile_words(K), geom, f);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) r[4 * t + j] = f[j];
+                    for (int j = 0; j < 4; ++j) r[4 * t + j] = f[j];
+                }
+                tmem_st_16x32(to + half * 32, r);
             }
-            tmem_st_16x32(taddr + stage * 64 + half * 32, r);
         }
         if (lane == 0) mbar_arrive(w_empty + 8 * s.slot);
         tmem_st_wait();

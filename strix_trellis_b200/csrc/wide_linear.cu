@@ -13,7 +13,7 @@
 // ordered problem, column block, K; the grid is one persistent CTA per SM and CTA c owns a
 // contiguous range of units (gemv_partition.h), whatever the shapes are.
 // Roles: 16 decode warps (warp w feeds tensor-memory lane quarter w % 4, i.e. column tiles
-// 2(w % 4) and +1, of every second unit), 4 epilogue warps, one producer thread each for
+// 2(w % 4) and +1, of every fourth unit), 4 epilogue warps, one producer thread each for
 // the weight ring and the activation ring, one MMA issuer.
 // Fold: a CTA whose range BEGINS inside a column block dumps its raw sums to its plane in global
 // scratch (that is its first segment, done early) and counts the chunks in its flag; the CTA whose
@@ -30,7 +30,7 @@
 namespace st {
 
 namespace {
-constexpr int kUnitGroups = 2, kDecodeW = 8 * kUnitGroups, kEpiW = 4;
+constexpr int kUnitGroups = 4, kDecodeW = 4 * kUnitGroups, kEpiW = 4;
 constexpr int kWarpMma = kDecodeW + kEpiW, kWarpWeights = kWarpMma + 1, kWarpRows = kWarpMma + 2;
 constexpr int kThreadsW = (kWarpRows + 1) * 32;
 constexpr int kChunkRows = 16;                       // rows of one epilogue chunk
@@ -247,9 +247,9 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                    b_empty = b_full + 8 * kMaxBSlots, a_full = b_empty + 8 * kMaxBSlots, a_empty = a_full + 8 * kMaxAStages,
                    d_full = a_empty + 8 * kMaxAStages, d_empty = d_full + 16, all_done = d_empty + 16;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < args.w_slots; ++i) { mbar_init(w_full + 8 * i, 1); mbar_init(w_empty + 8 * i, 8); }
+        for (int i = 0; i < args.w_slots; ++i) { mbar_init(w_full + 8 * i, 1); mbar_init(w_empty + 8 * i, 4); }
         for (int i = 0; i < args.b_slots; ++i) { mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, 1); }
-        for (int i = 0; i < a_stages; ++i) { mbar_init(a_full + 8 * i, 8); mbar_init(a_empty + 8 * i, 1); }
+        for (int i = 0; i < a_stages; ++i) { mbar_init(a_full + 8 * i, 4); mbar_init(a_empty + 8 * i, 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, 1); mbar_init(d_empty + 8 * i, kEpiW); }
         mbar_init(all_done, 1);
         mbar_fence_init();
@@ -375,7 +375,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         }
     } else {
         // ---- decode warps ---------------------------------------------------------------------------
-        const int turn = warp >> 3, ctile = 2 * (warp & 3) + ((warp >> 2) & 1);
+        const int turn = warp >> 2, ctile = 2 * (warp & 3);
         const uint32_t taddr = tmem + ((uint32_t)(ctile * 16) << 16);
         DecodeState s{turn, turn, 1, false, turn % args.w_slots, (uint32_t)(turn / args.w_slots) & 1};
         bool ok = true;
