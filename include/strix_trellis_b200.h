@@ -258,6 +258,25 @@ strix_status strix_b200_peer_return_routes(strix_b200_peer_group group,
 strix_status strix_b200_gemv_noalloc(strix_context context, const strix_matmul_desc *desc,
                                      const strix_stream *stream);
 
+/* strix_gemv / strix_gemm (operation = STRIX_OPERATION_GEMV / _GEMM) from plain arguments, for
+ * bindings whose cost per call is the filling of descriptors.  A tensor of rank 1 has `width`
+ * elements, one of rank 2 `rows` x `width`; strides in elements; the span it covers must lie in
+ * one device allocation.  `stream` is the stream handle itself.
+ * With a workspace the call is strix_gemv / strix_gemm.  Without one (NULL/0) a call of up to eight
+ * rows uses a scratch area that the context keeps for the stream (made on the first such call on it,
+ * freed with the context); where there is none to use -- more rows, a stream that is being captured,
+ * more streams than the context keeps areas for -- it returns STRIX_ERROR_INSUFFICIENT_BUFFER with
+ * nothing enqueued, and the caller brings a workspace. */
+typedef struct strix_b200_tensor {
+    void *data;
+    uint64_t rows, width, row_stride, column_stride;
+    uint32_t dtype, rank;
+} strix_b200_tensor;
+strix_status strix_b200_linear_call(strix_context context, strix_weights weights, uint32_t operation,
+                                    const strix_b200_tensor *input, const strix_b200_tensor *output,
+                                    float alpha, float beta, void *workspace, uint64_t workspace_bytes,
+                                    void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -291,6 +291,7 @@ strix_status strix_context_create(const strix_context_desc* d, strix_context* ou
 
 strix_status strix_context_destroy(strix_context c) {
     if (!c || c->weights_count) return STRIX_ERROR_INVALID_ARGUMENT;
+    for (const auto& s : c->stream_scratch) (void)cudaFree(s.area);
     (void)cudaFree(c->status);
     delete c;
     return STRIX_SUCCESS;

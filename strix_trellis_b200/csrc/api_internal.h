@@ -3,6 +3,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -16,6 +17,11 @@ struct strix_context_impl {
     size_t weights_count = 0;
     unsigned int* status = nullptr;  // device word: bounded-wait failures of any kernel
     bool programmatic_launch = true;
+    // Scratch areas of immediate calls that bring no workspace (direct_call.cu), one per stream, every
+    // word empty between launches; freed with the context.
+    struct StreamScratch { cudaStream_t stream; void* area; };
+    std::vector<StreamScratch> stream_scratch;
+    std::mutex scratch_lock;
 };
 
 struct strix_weights_impl {

@@ -154,6 +154,12 @@ class PeerReturnDesc(C.Structure):
                 ("region", u64), ("reserved", u64 * 2)]
 
 
+class Tensor(C.Structure):
+    """strix_b200_tensor: a tensor as strix_b200_linear_call takes it."""
+    _fields_ = [("data", vp), ("rows", u64), ("width", u64), ("row_stride", u64), ("column_stride", u64),
+                ("dtype", u32), ("rank", u32)]
+
+
 PROTOTYPES = {
     "strix_get_abi_version": (u32, []),
     "strix_status_string": (C.c_char_p, [C.c_int]),
@@ -238,6 +244,7 @@ PROTOTYPES = {
     "strix_b200_device_status": (C.c_int, [vp, P(u32)]),
     "strix_b200_set_programmatic_launch": (C.c_int, [vp, u32]),
     "strix_b200_gemv_noalloc": (C.c_int, [vp, P(MatmulDesc), P(Stream)]),
+    "strix_b200_linear_call": (C.c_int, [vp, vp, u32, P(Tensor), P(Tensor), f32, f32, vp, u64, vp]),
 }
 
 _LIB = None

@@ -15,6 +15,9 @@ def _cur_stream(stream=None):
     return N.stream_desc(stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream))
 
 
+_DTYPES = {torch.float32: N.DTYPE_F32, torch.float16: N.DTYPE_F16, torch.bfloat16: N.DTYPE_BF16}
+
+
 class Context:
     """strix_context for one device (must be the calling thread's current device)."""
 
@@ -129,6 +132,7 @@ class Weights:
             N.check(st, "strix_weights_prepare_parts")
         del keep
         self.packed_bytes = tb
+        self._needs = {}  # workspace bytes by row count (a function of the geometry alone)
 
     def close(self):
         if self.handle:
@@ -150,8 +154,7 @@ class Weights:
             strides = None if t.dim() == 1 else (t.stride(0), t.stride(1))
             size = t.element_size()
             nbytes = 0 if t.numel() == 0 else ((shape[0] - 1) * t.stride(0) + shape[-1]) * size if t.dim() == 2 else t.numel() * size
-            dtype = {torch.float32: N.DTYPE_F32, torch.float16: N.DTYPE_F16, torch.bfloat16: N.DTYPE_BF16}[t.dtype]
-            setattr(d, desc_name, N.tensor_desc(t.data_ptr() if t.numel() else 0, nbytes, shape, strides, dtype))
+            setattr(d, desc_name, N.tensor_desc(t.data_ptr() if t.numel() else 0, nbytes, shape, strides, _DTYPES[t.dtype]))
         d.alpha, d.beta = alpha, beta
         if workspace is not None and workspace.numel():
             d.workspace, d.workspace_bytes = workspace.data_ptr(), workspace.numel() * workspace.element_size()
@@ -167,25 +170,53 @@ class Weights:
         n = self.workspace_bytes(x, y)
         return torch.empty(max(n, 1), dtype=torch.uint8, device=x.device) if n else None
 
+    def _call(self, operation, where, x, y, alpha, beta, workspace, stream):
+        """One immediate call.  Without a workspace the library's scratch of this stream serves a GEMV;
+        where it has none (many rows, graph capture) the call is repeated with a workspace of its own."""
+        if x.dim() not in (1, 2) or y.dim() not in (1, 2):
+            N.check(N.UNSUPPORTED_FORMAT, where)
+        if stream is None:
+            handle = torch.cuda.current_stream().cuda_stream
+        else:
+            handle = stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
+        tensors = []
+        for t in (x, y):
+            if t.dim() == 2:
+                (rows, width), (row_stride, column_stride) = t.shape, t.stride()
+            else:
+                rows, width, row_stride, column_stride = 1, t.shape[0], t.shape[0], t.stride(0)
+            tensors.append(N.Tensor(t.data_ptr() if rows and width else None, rows, width, row_stride, column_stride,
+                                    _DTYPES[t.dtype], t.dim()))
+        call, xt, yt = self.lib.strix_b200_linear_call, C.byref(tensors[0]), C.byref(tensors[1])
+        if workspace is None:
+            need = 0
+            if operation == N.OP_GEMM and x.dim() == 2 and x.shape[0] > 8:
+                need = self._needs.get(x.shape[0])
+                if need is None:
+                    need = self.workspace_bytes(x, y)
+                    if len(self._needs) < 64:
+                        self._needs[x.shape[0]] = need
+            if not need:
+                status = call(self.ctx.handle, self.handle, operation, xt, yt, alpha, beta, None, 0, handle)
+                if status != N.INSUFFICIENT_BUFFER:
+                    return N.check(status, where)
+                need = self.workspace_bytes(x, y)
+            workspace = torch.empty(max(need, 1), dtype=torch.uint8, device=x.device)
+        size = workspace.numel() * workspace.element_size()
+        N.check(call(self.ctx.handle, self.handle, operation, xt, yt, alpha, beta, workspace.data_ptr() if size else None, size,
+                     handle), where)
+
     def gemv(self, x, y=None, alpha=1.0, beta=0.0, workspace=None, stream=None):
         """x, y: float32, float16 or bfloat16 CUDA tensors (each on its own); y defaults to float32."""
         if y is None:
             y = torch.empty(x.shape[:-1] + (self.outputs,), dtype=torch.float32, device=x.device)
-        if workspace is None:
-            workspace = self._workspace(x, y)
-        d = self.matmul_desc(x, y, alpha, beta, workspace)
-        sd = _cur_stream(stream)
-        N.check(self.lib.strix_gemv(self.ctx.handle, C.byref(d), C.byref(sd)), "strix_gemv")
+        self._call(N.OP_GEMV, "strix_gemv", x, y, alpha, beta, workspace, stream)
         return y
 
     def gemm(self, x, y=None, alpha=1.0, beta=0.0, workspace=None, stream=None):
         if y is None:
             y = torch.empty((x.shape[0], self.outputs), dtype=torch.float32, device=x.device)
-        if workspace is None:
-            workspace = self._workspace(x, y)
-        d = self.matmul_desc(x, y, alpha, beta, workspace)
-        sd = _cur_stream(stream)
-        N.check(self.lib.strix_gemm(self.ctx.handle, C.byref(d), C.byref(sd)), "strix_gemm")
+        self._call(N.OP_GEMM, "strix_gemm", x, y, alpha, beta, workspace, stream)
         return y
 
     def plan(self, x, y, operation=N.OP_GEMV, alpha=1.0, beta=0.0, workspace=None, stream=None):
