@@ -45,7 +45,7 @@ struct WideArgs {
     size_t table_stride;
     const int* live;
     WideProblem one;
-    int count, hblocks, nblocks;
+    int count, group_rows, hblocks, nblocks;
     int n_max, w_slots, w_stride, b_slots, b_stride;
     // tensor memory: a_stages x 64 columns of A, then d_bufs buffers of d_accs accumulators of n_max
     int a_stages, d_bufs, d_accs;
@@ -60,11 +60,11 @@ __device__ __forceinline__ const WideProblem& problem(const WideArgs& a, int p) 
 }
 __device__ __forceinline__ int problem_rows(const WideArgs& a, int p) {
     if (a.table) return problem(a, p).rows;
-    const int left = a.one.rows - p * kWideRows;
-    return left < kWideRows ? left : kWideRows;
+    const int left = a.one.rows - p * a.group_rows;
+    return left < a.group_rows ? left : a.group_rows;
 }
 __device__ __forceinline__ const unsigned char* problem_tiles(const WideArgs& a, int p) {
-    return a.table ? problem(a, p).tiles : a.one.tiles + (size_t)p * a.hblocks * wide_tile_bytes(kWideRows);
+    return a.table ? problem(a, p).tiles : a.one.tiles + (size_t)p * a.hblocks * wide_tile_bytes(a.group_rows);
 }
 
 // Position in a CTA's unit range; every role walks it segment by segment (a segment ends with a
@@ -201,7 +201,7 @@ struct Epilogue {
             sv[i] = __ldg(reinterpret_cast<const uint2*>(pr.w.svh + c0));
             bi[i] = pr.w.bias ? __ldg(reinterpret_cast<const float4*>(pr.w.bias + c0)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        const int out_row = a.table ? (pr.y_rows ? pr.y_rows[r] : r) : w.p * kWideRows + r;
+        const int out_row = a.table ? (pr.y_rows ? pr.y_rows[r] : r) : w.p * a.group_rows + r;
         const bool aligned = quads_aligned(pr.y, pr.y_dtype, pr.y_stride);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
         const int row_bytes = args.one.x_dtype == DT_F32 ? 512 : 256;  // of this block
         if (row < rows && l8 * 128 < row_bytes)
             prefetch_line_l2(static_cast<const unsigned char*>(args.one.x) +
-                             ((size_t)(p * kWideRows + row) * args.one.x_stride + blk * 128) * (row_bytes / 128) + l8 * 128);
+                             ((size_t)(p * args.group_rows + row) * args.one.x_stride + blk * 128) * (row_bytes / 128) + l8 * 128);
     }
     pdl_wait_prior_grid();  // x may come from the launch before; the tiles may still be read by it
     if (blockIdx.x == 0 && blockIdx.y == 0)
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
         for (int item = first; item < quads * args.hblocks; item += gridDim.x * kInputWarps) {
             const int quad = item / args.hblocks, blk = item - quad * args.hblocks;
             const int row = quad * 4 + (lane >> 3);
-            const int x_row = row >= rows ? 0 : !args.table ? p * kWideRows + row : pr.x_rows ? pr.x_rows[row] : row;
+            const int x_row = row >= rows ? 0 : !args.table ? p * args.group_rows + row : pr.x_rows ? pr.x_rows[row] : row;
             float v[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -499,6 +499,7 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     a.live = set.live;
     a.one = set.one;
     a.count = set.count;
+    a.group_rows = set.group_rows;
     a.hblocks = set.inputs / 128;
     a.nblocks = set.outputs / 128;
     a.n_max = plan.n_max;

@@ -38,14 +38,14 @@ struct WidePlan {
 WidePlan plan_wide(int inputs, int heaviest, int rows_max, long long units, int sm_count);
 
 // A set of problems of one geometry.  `table` (device memory) holds them, `table_stride` bytes apart;
-// without a table the set is ONE layer whose `one.rows` rows are cut into problems of kWideRows rows.
+// without a table the set is ONE layer whose `one.rows` rows are cut into problems of group_rows rows.
 // `live` (device memory, may be null) overrides `count` at run time.
 struct WideSet {
     const WideProblem* table;
     size_t table_stride;
     const int* live;
     WideProblem one;
-    int count;
+    int count, group_rows;
     int inputs, outputs, codebook;
 };
 // Input stages of every row of every problem into its tiles; also zeroes the flags.
