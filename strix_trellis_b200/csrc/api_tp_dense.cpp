@@ -401,8 +401,9 @@ strix_status strix_grouped_gemv_plan_create(strix_context c, const strix_grouped
             st::bind_rows(pr, p->problems + g);
         }
         host[0].live = (int)m.size();
-        const cudaError_t e = cudaMemcpyAsync(p->problems, host.data(), host.size() * sizeof(st::GroupedProblem),
-                                              cudaMemcpyHostToDevice, cs);
+        cudaError_t e = cudaMemsetAsync(tiles, 0, m.size() * p->grouped.partial_bytes_per_problem, cs);  // a direct plan's counters
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(p->problems, host.data(), host.size() * sizeof(st::GroupedProblem), cudaMemcpyHostToDevice, cs);
         const cudaError_t done = cudaStreamSynchronize(cs);  // `host` leaves scope
         s = cuda_status(e != cudaSuccess ? e : done);
     }

@@ -33,7 +33,7 @@ struct strix_tp_moe_plan_impl {
     float* y = nullptr;
     long long y_stride = 0;
     float alpha = 1.f, beta = 0.f;
-    st::MoeWindow window{0, 0};  // device-routed plans: where the bank sits in the router's id space
+    st::MoeWindow window{0, 0, 0};  // device-routed plans: where the bank sits in the router's id space
 };
 
 // A dense pair-style plan with SwiGLU: two grouped problems + the activation.
@@ -234,6 +234,44 @@ strix_status enqueue_gate_up(strix_tp_moe_plan_impl* p) {
     return cuda_status(e);
 }
 
+// Groups of at most eight rows when `routes` are spread evenly over a bank.
+long long spread_groups(long long routes, int bank) {
+    if (routes < 1) routes = 1;
+    return std::min<long long>(routes, bank * ((routes + 8ll * bank - 1) / (8ll * bank)));
+}
+// Plans of the projections for an expected number of groups of at most eight rows.
+void expect_groups(strix_tp_moe_plan_impl* p, long long groups, int sm_count) {
+    st::expect_row_groups(p->gu_plan, p->model, p->inter, p->max_bits, 2 * groups, sm_count);
+    st::expect_row_groups(p->down_plan, p->inter, p->model, p->max_bits, groups, sm_count);
+}
+// The projections share one grouping of the routes: rows per problem, for expected `groups` of at most
+// eight rows over `experts` live experts.
+int rows_per_problem(const Geometry& g, long long groups, long long experts, int sm_count) {
+    return st::direct_pays(3 * groups, 3 * experts, g.model, g.inter, 2, sm_count) ? st::kDirectRows : st::kGroupRows;
+}
+void plan_projections(strix_tp_moe_plan_impl* p, const Geometry& g, int group_rows, long long groups, int sm_count) {
+    p->max_bits = g.max_bits;
+    const int rows = std::max(p->tokens, st::kDirectRows + 1);  // (wide plans; of up to 16 rows all are alike)
+    p->gu_plan = st::plan_grouped(g.model, g.inter, g.max_bits, rows, sm_count, p->gu_count);
+    p->down_plan = st::plan_grouped(g.inter, g.model, g.max_bits, rows, sm_count, p->down_count);
+    if (group_rows == st::kDirectRows) {
+        // Planes for up to four times the partitions while they stay under 128 MB: a window set later
+        // means fewer local routes, and fewer groups want more partitions.
+        const st::GroupedPlan gu = p->gu_plan, down = p->down_plan;
+        for (int headroom = 4; headroom >= 1; headroom /= 2) {
+            p->gu_plan = gu;
+            p->down_plan = down;
+            st::plan_direct(p->gu_plan, g.model, g.inter, g.max_bits, 2 * groups, sm_count, headroom);
+            st::plan_direct(p->down_plan, g.inter, g.model, g.max_bits, groups, sm_count, headroom);
+            if (p->gu_count * p->gu_plan.partial_bytes_per_problem + p->down_count * p->down_plan.partial_bytes_per_problem <=
+                ((size_t)128 << 20))
+                break;
+        }
+    } else {
+        expect_groups(p, groups, sm_count);
+    }
+}
+
 strix_status enqueue_down(strix_tp_moe_plan_impl* p, bool combine = true) {
     cudaError_t e = st::launch_grouped(p->down, p->down_count, p->inter, p->model, p->codebook, p->down_plan,
                                        p->owner->status, p->owner->programmatic_launch, p->stream);
@@ -268,20 +306,23 @@ strix_status create_host(strix_context c, const strix_tp_moe_desc* d, const stri
     s = host_routing(d, tokens, top_k, route_expert);
     if (s != STRIX_SUCCESS) return s;
 
-    // group routes by expert, kGroupRows rows per problem (all routes for gate/up, scored ones for down)
+    // group routes by expert (all routes for gate/up, scored ones for down)
     const int experts = (int)d->expert_count, routes = tokens * top_k;
     std::vector<std::vector<int>> by_expert(experts);
     for (int r = 0; r < routes; ++r) by_expert[route_expert[r]].push_back(r);
+    long long groups = 0;
+    for (const auto& of : by_expert) groups += ((long long)of.size() + 7) / 8;
+    const int group_rows = rows_per_problem(g, groups, experts, c->sm_count);
     struct Chunk { int expert; std::vector<int> routes; };
     std::vector<Chunk> gu_chunks, down_chunks;
     for (int e = 0; e < experts; ++e) {
         std::vector<int> scored;
         for (int r : by_expert[e])
             if (d->route_scores[r] != 0.0f) scored.push_back(r);
-        for (size_t i = 0; i < by_expert[e].size(); i += st::kGroupRows)
-            gu_chunks.push_back({e, {by_expert[e].begin() + i, by_expert[e].begin() + std::min(by_expert[e].size(), i + st::kGroupRows)}});
-        for (size_t i = 0; i < scored.size(); i += st::kGroupRows)
-            down_chunks.push_back({e, {scored.begin() + i, scored.begin() + std::min(scored.size(), i + st::kGroupRows)}});
+        for (size_t i = 0; i < by_expert[e].size(); i += group_rows)
+            gu_chunks.push_back({e, {by_expert[e].begin() + i, by_expert[e].begin() + std::min(by_expert[e].size(), i + group_rows)}});
+        for (size_t i = 0; i < scored.size(); i += group_rows)
+            down_chunks.push_back({e, {scored.begin() + i, scored.begin() + std::min(scored.size(), i + group_rows)}});
     }
     strix_tp_moe_plan_impl* p = new (std::nothrow) strix_tp_moe_plan_impl;
     if (!p) return STRIX_ERROR_OUT_OF_MEMORY;
@@ -290,8 +331,7 @@ strix_status create_host(strix_context c, const strix_tp_moe_desc* d, const stri
     p->tokens = tokens; p->top_k = top_k; p->model = g.model; p->inter = g.inter; p->codebook = g.codebook;
     p->gu_count = 2 * (int)gu_chunks.size();
     p->down_count = (int)down_chunks.size();
-    p->gu_plan = st::plan_grouped(g.model, g.inter, g.max_bits, tokens, c->sm_count, p->gu_count);
-    p->down_plan = st::plan_grouped(g.inter, g.model, g.max_bits, tokens, c->sm_count, p->down_count);
+    plan_projections(p, g, group_rows, groups, c->sm_count);
     const size_t bytes = layout_block(p, p->gu_count, p->down_count, true);
     cudaError_t e = cudaMalloc(&p->block, bytes);
     if (e != cudaSuccess) { (void)cudaGetLastError(); delete p; return cuda_status(e); }
@@ -386,11 +426,12 @@ strix_status create_device(strix_context c, const strix_tp_moe_device_desc* d, c
     p->owner = c; p->stream = cs; p->device_routed = true;
     p->tokens = tokens; p->top_k = top_k; p->model = g.model; p->inter = g.inter; p->codebook = g.codebook;
     p->bank_count = (int)d->expert_count;
-    p->down_count = st::max_problems(routes, p->bank_count);
+    const long long groups = spread_groups(routes, p->bank_count);
+    const int group_rows = rows_per_problem(g, groups, std::min(routes, p->bank_count), c->sm_count);
+    p->down_count = st::max_problems(routes, p->bank_count, group_rows);
     p->gu_count = 2 * p->down_count;
-    p->window = st::MoeWindow{0, p->bank_count};
-    p->gu_plan = st::plan_grouped(g.model, g.inter, g.max_bits, tokens, c->sm_count, p->gu_count);
-    p->down_plan = st::plan_grouped(g.inter, g.model, g.max_bits, tokens, c->sm_count, p->down_count);
+    p->window = st::MoeWindow{0, p->bank_count, group_rows};
+    plan_projections(p, g, group_rows, groups, c->sm_count);
     const size_t bytes = layout_block(p, p->gu_count, p->down_count, false);
     cudaError_t e = cudaMalloc(&p->block, bytes);
     if (e != cudaSuccess) { (void)cudaGetLastError(); delete p; return cuda_status(e); }
@@ -503,7 +544,10 @@ strix_status strix_b200_moe_plan_set_window(strix_tp_moe_plan p, uint32_t first_
     if (!p || !p->device_routed) return STRIX_ERROR_INVALID_ARGUMENT;
     if (experts_total > INT_MAX || (uint64_t)first_expert + (uint64_t)p->bank_count > experts_total)
         return STRIX_ERROR_INVALID_ARGUMENT;
-    p->window = st::MoeWindow{(int)first_expert, (int)experts_total};
+    p->window = st::MoeWindow{(int)first_expert, (int)experts_total, p->window.group_rows};
+    // of all routes, about bank / experts_total are this rank's
+    const long long routes = (long long)p->tokens * p->top_k;
+    expect_groups(p, spread_groups((routes * p->bank_count + experts_total - 1) / experts_total, p->bank_count), p->owner->sm_count);
     return STRIX_SUCCESS;
 }
 // Routing, gate/up, SwiGLU and down of the routes this rank owns; no combine.
@@ -644,7 +688,8 @@ strix_status strix_tp_swiglu_plan_create(strix_context c, const strix_tp_swiglu_
         for (int k = 0; k < rows; ++k) host[half].x_row[k] = host[half].y_row[k] = k;
     }
     host[0].live = 2;
-    cudaError_t e = cudaMemcpyAsync(p->problems, host, sizeof(host), cudaMemcpyHostToDevice, cs);
+    cudaError_t e = cudaMemsetAsync(tiles, 0, 2 * each, cs);  // a direct plan's counters
+    if (e == cudaSuccess) e = cudaMemcpyAsync(p->problems, host, sizeof(host), cudaMemcpyHostToDevice, cs);
     const cudaError_t done = cudaStreamSynchronize(cs);
     if (e != cudaSuccess || done != cudaSuccess) { delete p; return cuda_status(e != cudaSuccess ? e : done); }
     ++d->gate->plan_refs;

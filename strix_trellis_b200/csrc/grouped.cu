@@ -16,12 +16,15 @@ GroupedPlan plan_grouped(int inputs, int outputs, int max_bits, int rows, int sm
     if (rows > kGroupRows) rows = kGroupRows;
     if (problems < 1) problems = 1;
     plan.wide = plan_wide(inputs, max_bits, rows, (long long)problems * nblocks * hblocks, sm_count);
+    expect_row_groups(plan, inputs, outputs, max_bits, (long long)problems * ((rows + 7) / 8), sm_count);
     plan.splits = (plan.wide.grid + problems * nblocks - 1) / (problems * nblocks);
     plan.scratch_splits = 1;
     plan.stages = plan.wide.w_slots;
     plan.ctas_per_problem = nblocks * hblocks < plan.wide.grid ? nblocks * hblocks : plan.wide.grid;
     plan.partial_bytes_per_problem = align_up((size_t)hblocks * wide_tile_bytes(rows));
     plan.shared_bytes = plan.wide.flag_bytes + plan.wide.plane_bytes;
+    if (rows <= kDirectRows && direct_pays(problems, problems, inputs, outputs, 1, sm_count))
+        plan_direct(plan, inputs, outputs, max_bits, problems, sm_count, 1);
     return plan;
 }
 
@@ -29,6 +32,8 @@ cudaError_t launch_grouped(const GroupedProblem* problems, int problem_count, in
                            int codebook, const GroupedPlan& plan, unsigned int* status, bool programmatic,
                            cudaStream_t stream) {
     if (problem_count <= 0) return cudaSuccess;
+    if (plan.direct)
+        return launch_grouped_direct(problems, problem_count, inputs, outputs, codebook, plan, status, programmatic, stream);
     if (!plan.shared) return cudaErrorInvalidValue;
     WideSet set{};
     set.table = problems;
@@ -87,7 +92,7 @@ cudaError_t launch_swiglu(const float* gate, const float* up, float* hidden, int
 
 // Device-side routing, one CTA.  A row is valid when its ids are in range and distinct and
 // its scores are finite and non-negative (src/tp_moe_routes.hpp:46-61); slots of invalid
-// rows run nothing.  Valid routes are grouped by expert into problems of up to kGroupRows rows,
+// rows run nothing.  Valid routes are grouped by expert into problems of up to `window.group_rows` rows,
 // so an expert's weights are streamed once per that many routed rows, not once per route.  A
 // row's result does not depend on which problem slot or row position carries it.
 // Zero-score routes are computed like any other; the combine skips them.
@@ -97,7 +102,7 @@ __global__ void __launch_bounds__(1024) moe_route_kernel(const unsigned int* __r
                                                          const MoeWindow window, GroupedProblem* gate_up,
                                                          GroupedProblem* down, int* row_valid) {
     __shared__ int count[1024], first_problem[1024], cursor[1024], warp_total[32];
-    const int tid = threadIdx.x, routes = tokens * top_k;
+    const int tid = threadIdx.x, routes = tokens * top_k, group = window.group_rows;
     count[tid] = 0;
     cursor[tid] = 0;
     pdl_wait_prior_grid();  // ids and scores may come from the launch before
@@ -121,7 +126,7 @@ __global__ void __launch_bounds__(1024) moe_route_kernel(const unsigned int* __r
     }
     __syncthreads();
     const int n = tid < bank_count ? count[tid] : 0;
-    const int problems = (n + kGroupRows - 1) / kGroupRows;
+    const int problems = (n + group - 1) / group;
     // inclusive scan of problems per expert: within a warp by shuffles, then over the 32 warp totals
     int incl = problems;
 #pragma unroll
@@ -146,13 +151,13 @@ __global__ void __launch_bounds__(1024) moe_route_kernel(const unsigned int* __r
     first_problem[tid] = begin;
     for (int k = 0; k < problems; ++k) {
         const int q = begin + k;
-        const int rows = n - k * kGroupRows < kGroupRows ? n - k * kGroupRows : kGroupRows;
+        const int rows = n - k * group < group ? n - k * group : group;
         gate_up[2 * q].rows = gate_up[2 * q + 1].rows = down[q].rows = rows;
         gate_up[2 * q].w = bank[tid].gate;
         gate_up[2 * q + 1].w = bank[tid].up;
         down[q].w = bank[tid].down;
     }
-    if (tid == 0) {
+    if (tid == 0 && group <= kDirectRows) {  // grouped_direct.cu waits for this whole launch
         gate_up[0].live = 2 * total;
         down[0].live = total;
     }
@@ -164,17 +169,25 @@ __global__ void __launch_bounds__(1024) moe_route_kernel(const unsigned int* __r
         if (local >= (unsigned int)bank_count) continue;
         const int e = (int)local;
         const int pos = atomicAdd(&cursor[e], 1);
-        const int q = first_problem[e] + pos / kGroupRows, j = pos % kGroupRows;
+        const int q = first_problem[e] + pos / group, j = pos % group;
         gate_up[2 * q].x_row[j] = gate_up[2 * q + 1].x_row[j] = t;
         gate_up[2 * q].y_row[j] = gate_up[2 * q + 1].y_row[j] = r;
         down[q].x_row[j] = down[q].y_row[j] = r;
+    }
+    // Last, and released: a wide_linear.cu kernel that acquires its table's count has the table.
+    if (group <= kDirectRows) return;
+    __syncthreads();
+    if (tid == 0) {
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&gate_up[0].live), "r"(2 * total) : "memory");
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&down[0].live), "r"(total) : "memory");
     }
 }
 
 cudaError_t launch_moe_route(const unsigned int* route_ids, const float* route_scores, int tokens, int top_k,
                              const MoeBankEntry* bank, int bank_count, MoeWindow window, GroupedProblem* gate_up,
                              GroupedProblem* down, int* row_valid, bool programmatic, cudaStream_t stream) {
-    if (bank_count > 1024 || window.first_expert < 0 || window.experts_total < window.first_expert + bank_count)
+    if (bank_count > 1024 || window.first_expert < 0 || window.experts_total < window.first_expert + bank_count ||
+        window.group_rows < 1 || window.group_rows > kGroupRows)
         return cudaErrorInvalidValue;
     return launch_small(moe_route_kernel, 1, 1024, programmatic, stream, route_ids, route_scores, tokens, top_k, bank,
                         bank_count, window, gate_up, down, row_valid);

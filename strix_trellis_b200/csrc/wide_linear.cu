@@ -47,8 +47,8 @@ struct WideArgs {
     WideProblem one;
     int count, group_rows, hblocks, nblocks;
     int n_max, w_slots, w_stride, b_slots, b_stride;
-    // tensor memory: a_stages x 64 columns of A, then d_bufs buffers of d_accs accumulators of n_max
-    int a_stages, d_bufs, d_accs;
+    // tensor memory: a_stages x 64 columns of A, then d_bufs buffers of `parts` times d_accs accumulators of n_max
+    int a_stages, d_bufs, d_accs, parts, parts_log2;
     unsigned int* flags;
     float* planes;
     unsigned int* status;
@@ -65,6 +65,14 @@ __device__ __forceinline__ int problem_rows(const WideArgs& a, int p) {
 }
 __device__ __forceinline__ const unsigned char* problem_tiles(const WideArgs& a, int p) {
     return a.table ? problem(a, p).tiles : a.one.tiles + (size_t)p * a.hblocks * wide_tile_bytes(a.group_rows);
+}
+
+// First block of K part s: the blocks [part_begin(s), part_begin(s + 1)) have accumulators of their own.
+__device__ __forceinline__ int part_begin(const WideArgs& a, int s) { return (a.hblocks * s) >> a.parts_log2; }
+__device__ __forceinline__ int part_of(const WideArgs& a, int hb) {
+    int part = 0;
+    while (part_begin(a, part + 1) <= hb) ++part;
+    return part;
 }
 
 // Position in a CTA's unit range; every role walks it segment by segment (a segment ends with a
@@ -132,23 +140,35 @@ struct Epilogue {
         }
         const int col = quarter * 32 + lane;
         const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + dcol;
+        const int first_part = part_of(a, w.hb), last_part = part_of(a, w.hb + len - 1);  // of this segment
         int dumped = 0;
         for (int ch = first_chunk; ch < chunks; ch += step) {
             uint32_t r[16];
-            __syncwarp();
-            tmem_ld_32x16(taddr + ch * kChunkRows, r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(r[j]));  // not before the wait
-            if (a.d_accs == 2) {
-                uint32_t q[16];
-                tmem_ld_32x16(taddr + a.n_max + ch * kChunkRows, q);
+            // Parts in ascending K order; the running sum of a column waits in its place in `stage`.
+#pragma unroll 1
+            for (int part = first_part; part <= last_part; ++part) {
+                const uint32_t at = taddr + part * a.d_accs * a.n_max + ch * kChunkRows;
+                __syncwarp();
+                tmem_ld_32x16(at, r);
                 tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    asm volatile("" : "+r"(q[j]));
-                    r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(q[j])));
+                for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(r[j]));  // not before the wait
+                if (a.d_accs == 2) {
+                    uint32_t q[16];
+                    tmem_ld_32x16(at + a.n_max, q);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        asm volatile("" : "+r"(q[j]));
+                        r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(q[j])));
+                    }
                 }
+                if (part != first_part)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__fadd_rn(stage[j * 128 + col], __uint_as_float(r[j])));
+                if (part != last_part)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) stage[j * 128 + col] = __uint_as_float(r[j]);
             }
             if (contributor) {
                 float* plane = a.planes + ((size_t)cta * a.n_max + ch * kChunkRows) * 128 + col;
@@ -226,10 +246,10 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (still a shared-memory pointer to the compiler)
     const int warp = uniform_warp(), lane = threadIdx.x & 31, cta = (int)blockIdx.x;
-    // A table may be the work of the launch before; one layer's weights are immutable, so there only
-    // the activation producer waits.
-    if (args.table) pdl_wait_prior_grid();
-    const int count = args.live ? *args.live : args.count;
+    // Weights are immutable and a table is there before the launch before lets this one start (its own
+    // wait comes first, see wide_inputs_kernel; acquiring the count acquires the table), so only the
+    // activation producer waits.
+    const int count = args.live ? (int)ld_acquire_gpu(reinterpret_cast<const unsigned int*>(args.live)) : args.count;
     const int units = count * args.nblocks * args.hblocks;
     const int grid = units < (int)gridDim.x ? units : (int)gridDim.x;
     if (cta >= grid) return;
@@ -261,7 +281,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     const uint32_t tmem = s_tmem_base;
     pdl_launch_dependents();
 
-    auto d_column = [&](int seg) { return a_stages * 64 + (d_bufs == 2 ? (seg & 1) * args.d_accs * args.n_max : 0); };
+    auto d_column = [&](int seg) { return a_stages * 64 + (d_bufs == 2 ? (seg & 1) * args.parts * args.d_accs * args.n_max : 0); };
     auto d_parity = [&](int seg) { return (uint32_t)(d_bufs == 2 ? seg >> 1 : seg) & 1; };  // of the seg-th use
     auto d_index = [&](int seg) { return d_bufs == 2 ? seg & 1 : 0; };
 
@@ -326,7 +346,10 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             const uint32_t idesc = umma_idesc_f16_f32(128, n), dcol = tmem + d_column(seg);
             const uint32_t odd = args.d_accs == 2 ? args.n_max : 0;  // accumulator of the odd K steps
             if (seg >= d_bufs && !mbar_wait(d_empty + 8 * d_index(seg), d_parity(seg) ^ 1, args.status, kTimeoutTensorPipe)) break;
+            int part = part_of(args, w.hb), fresh = 1;
             for (int i = 0; i < len; ++i) {
+                if (part_begin(args, part + 1) == w.hb + i) { ++part; fresh = 1; }
+                const uint32_t acc = dcol + part * args.d_accs * args.n_max;
                 if (!mbar_wait(b_full + 8 * slot, use, args.status, kTimeoutTensorPipe) ||
                     !mbar_wait(a_full + 8 * stage, a_use, args.status, kTimeoutTensorPipe)) {
                     ok = false;
@@ -338,11 +361,12 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        umma_f16_ts(dcol + (k & 1) * odd, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, i != 0 || k >= args.d_accs);
+                        umma_f16_ts(acc + (k & 1) * odd, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, !fresh || k >= args.d_accs);
                     umma_commit(a_empty + 8 * stage);
                     umma_commit(b_empty + 8 * slot);
                 }
                 __syncwarp();
+                fresh = 0;
                 if (++slot == args.b_slots) { slot = 0; use ^= 1; }
                 if (++stage == a_stages) { stage = 0; a_use ^= 1; }
             }
@@ -417,7 +441,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
 // ---- input stages: four rows of one 128-block per warp, eight lanes per row --------------------
 constexpr int kInputWarps = 4;
 __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const WideArgs args, int grid_ctas) {
-    pdl_launch_dependents();
+    if (!args.table) pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l8 = lane & 7;
     const int first = blockIdx.x * kInputWarps + warp;
     uint2 su[4];
@@ -435,6 +459,7 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
                              ((size_t)(p * args.group_rows + row) * args.one.x_stride + blk * 128) * (row_bytes / 128) + l8 * 128);
     }
     pdl_wait_prior_grid();  // x may come from the launch before; the tiles may still be read by it
+    if (args.table) pdl_launch_dependents();  // not earlier: that launch reads the table at once
     if (blockIdx.x == 0 && blockIdx.y == 0)
         for (int i = threadIdx.x; i < grid_ctas; i += blockDim.x) args.flags[i] = 0;
     const int count = args.live ? *args.live : args.count;
@@ -478,6 +503,7 @@ WidePlan plan_wide(int inputs, int heaviest, int rows_max, long long units, int 
     WidePlan plan{};
     plan.grid = (int)(units < sm_count ? units : sm_count);
     plan.n_max = wide_n(rows_max < kWideRows ? rows_max : kWideRows);
+    plan.parts = 1;
     plan.w_stride = unit_bytes(heaviest);
     plan.w_slots = (64 * 1024) / plan.w_stride;
     if (plan.w_slots > kMaxWSlots) plan.w_slots = kMaxWSlots;
@@ -509,9 +535,13 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     a.b_stride = plan.b_stride;
     // Even and odd K steps have accumulators of their own where there is room: half the roundings in
     // a row.  A second buffer lets the MMAs of the next segment start under this one's epilogue.
+    // Four A stages (one for each decode group) are enough, half of the columns are the accumulators'.
     a.d_accs = plan.n_max <= 128 ? 2 : 1;
-    a.d_bufs = plan.n_max <= 64 ? 2 : 1;
-    a.a_stages = (512 - a.d_bufs * a.d_accs * plan.n_max) / 64;
+    a.parts = plan.parts;
+    while (a.parts > 1 && a.parts * a.d_accs * plan.n_max > 256) a.parts /= 2;
+    while ((1 << a.parts_log2) < a.parts) ++a.parts_log2;
+    a.d_bufs = 2 * a.parts * a.d_accs * plan.n_max <= 256 ? 2 : 1;
+    a.a_stages = (512 - a.d_bufs * a.parts * a.d_accs * plan.n_max) / 64;
     if (a.a_stages > kMaxAStages) a.a_stages = kMaxAStages;
     a.flags = flags;
     a.planes = planes;

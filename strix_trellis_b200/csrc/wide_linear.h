@@ -30,10 +30,27 @@ struct WidePlan {
     int n_max;              // widest problem's N
     int w_slots, w_stride;  // weight ring: slots of one unit, bytes apart
     int b_slots, b_stride;  // activation ring
+    int parts;              // K parts that are summed apart (accumulator_parts), 1, 2 or 4
     size_t smem_bytes;
     size_t flag_bytes;      // [grid] counters, zeroed by launch_wide_inputs
     size_t plane_bytes;     // [grid][n_max][128] partial sums
 };
+// K parts, each with accumulators of its own, for `groups` problems of at most eight rows.  The tensor
+// cores truncate as they accumulate, so the error of a sum grows with the steps it is made of, and a
+// routed expert rounds these sums to binary16 twice more: hidden rows that differ by 2.4e-6 (one sum of
+// K = 4096 against two) move its outputs by 3.4e-4.  The parts are those of a grid of one CTA per (group,
+// column block, part) that balances its last wave against its longest CTA, so results do not depend on
+// how this kernel cuts K between CTAs beyond the blocks that it cuts.
+ST_RATE_FN int accumulator_parts(int hblocks, int nblocks, long long groups, int sm_count) {
+    int parts = 1;
+    double best = -1.0;
+    for (int s = hblocks > 32 ? 2 : 1; s <= hblocks && s <= 4; s *= 2) {
+        const double each = (double)((hblocks + s - 1) / s) + 1.0;
+        const double cost = (double)groups * nblocks * s * each / sm_count + 0.5 * each;
+        if (best < 0.0 || cost < best) { best = cost; parts = s; }
+    }
+    return parts;
+}
 // `heaviest`: the rate code with the largest tiles among the problems.
 WidePlan plan_wide(int inputs, int heaviest, int rows_max, long long units, int sm_count);
 
