@@ -94,7 +94,8 @@ struct GemvPlan {
     size_t smem_bytes;
     size_t counter_bytes;   // reserved area at the start of the workspace (0: the fold needs no counters)
     size_t partial_bytes;   // partial planes after the counters
-    bool row_kernel;        // one row through gemv_row.cu (else gemv_tmem.cu)
+    bool row_kernel;        // one row through gemv_row.cu
+    bool few_kernel;        // 2..8 rows through gemv_few.cu (else gemv_tmem.cu)
 };
 GemvPlan plan_gemv(const DeviceWeights& w, int rows, int sm_count);
 // `workspace` must be 256-byte aligned and hold counter_bytes + partial_bytes.

@@ -7,6 +7,7 @@ namespace st {
 
 cudaError_t configure_gemv_kernels();
 cudaError_t configure_gemv_row_kernels();
+cudaError_t configure_gemv_few_kernels();
 cudaError_t configure_wide_kernels();
 cudaError_t configure_direct_kernels();
 cudaError_t configure_gemm_dense_kernels();
@@ -28,6 +29,7 @@ int device_sm_count() {
 cudaError_t configure_device() {
     cudaError_t e = configure_gemv_kernels();
     if (e == cudaSuccess) e = configure_gemv_row_kernels();
+    if (e == cudaSuccess) e = configure_gemv_few_kernels();
     if (e == cudaSuccess) e = configure_wide_kernels();
     if (e == cudaSuccess) e = configure_direct_kernels();
     if (e == cudaSuccess) e = configure_gemm_dense_kernels();

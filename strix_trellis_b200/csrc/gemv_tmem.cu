@@ -382,12 +382,17 @@ __global__ void __launch_bounds__(256) empty_planes_kernel(uint4* planes, int co
 // ---- host side -------------------------------------------------------------------------
 // gemv_row.cu: one row, few units per CTA
 bool plan_gemv_row(const DeviceWeights& w, GemvPlan& plan);
+// gemv_few.cu: 2..8 rows, very few units per CTA
+void plan_gemv_few(const DeviceWeights& w, int rows, GemvPlan& plan);
+cudaError_t launch_gemv_few(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream);
 cudaError_t launch_gemv_row(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream);
 
 // One row with this many units per CTA takes this kernel: the decode loop then outweighs the longer
 // way from the last tile to the fold (measured, one row: 24 units of K4 15.4 against 16.5 us for
 // gemv_row.cu, 218 units of K5 126 against 129 us the other way round).
 constexpr int kTmemUnits = 96;
+// Two or more rows with at most this many units per CTA go to gemv_few.cu.
+constexpr int kFewUnits = 4;
 
 GemvPlan plan_gemv(const DeviceWeights& w, int rows, int sm_count) {
     GemvPlan plan{};
@@ -416,6 +421,8 @@ GemvPlan plan_gemv(const DeviceWeights& w, int rows, int sm_count) {
     plan.counter_bytes = 0;  // the fold needs no counters
     plan.partial_bytes = align_up((size_t)grid * rows * 128 * sizeof(float));
     plan.row_kernel = rows == 1 && per_cta < kTmemUnits && plan_gemv_row(w, plan);
+    plan.few_kernel = rows > 1 && per_cta <= kFewUnits;
+    if (plan.few_kernel) plan_gemv_few(w, rows, plan);
     return plan;
 }
 
@@ -454,6 +461,7 @@ cudaError_t launch_gemv(const LinearCall& call, const GemvPlan& plan, void* work
     args.row_magic = call.rows == 1 ? 0 : (uint32_t)((0x100000000ull + call.rows - 1) / call.rows);
     args.planes = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + plan.counter_bytes);
     if (plan.row_kernel) return launch_gemv_row(call, plan, args.split, args.planes, programmatic_launch, stream);
+    if (plan.few_kernel) return launch_gemv_few(call, plan, args.split, args.planes, programmatic_launch, stream);
     switch (call.w.codebook) {
     case CB_3INST: return launch_pdl(gemv_tmem_kernel<CB_3INST>, plan.grid, kThreadsT, plan.smem_bytes, programmatic_launch, stream, args);
     case CB_MCG: return launch_pdl(gemv_tmem_kernel<CB_MCG>, plan.grid, kThreadsT, plan.smem_bytes, programmatic_launch, stream, args);
