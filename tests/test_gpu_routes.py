@@ -1,0 +1,123 @@
+"""Each kernel route of the linears at the edges of its range, against the CPU contract."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import dev, gate, host
+from oracle import c_oracle
+from strix_trellis_b200 import synthetic
+from test_gpu_moe import MOE_NRMSE, MOE_REL, make_experts, oracle_block
+
+pytestmark = pytest.mark.gpu
+CODEBOOK = {"3inst": 0, "mcg": 1, "mul1": 2}
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from strix_trellis_b200.runtime import Context
+    c = Context(0)
+    yield c
+    assert c.device_status() == 0
+    c.close()
+
+
+def check(ctx, rows, inputs, outputs, bits=4, codebook="mul1", bias=False):
+    layer = synthetic.make_layer(inputs, outputs, bits, seed=9000 + rows, codebook=codebook, bias=bias)
+    x = synthetic.make_activations(rows, inputs, seed=9001)
+    want = c_oracle.linear(layer.trellis, layer.suh, layer.svh, layer.bias, bits, CODEBOOK[codebook], x)
+    w = ctx.prepare(layer)
+    run = w.gemv if rows <= 8 else w.gemm
+    for again in range(2):  # the second call finds the scratch as the first one left it
+        gate(host(run(dev(x))), want, f"{rows} rows {inputs}x{outputs} call {again}")
+    w.close()
+
+
+@pytest.mark.parametrize("rows,inputs,outputs,bits,codebook", [
+    (2, 128, 128, 4, "mul1"), (8, 4736, 2048, 3, "mcg"), (3, 5120, 1920, 8, "3inst"),      # up to four units per CTA
+    (2, 4736, 2176, 3, "mcg"), (8, 5120, 2048, 8, "3inst"), (5, 3072, 4096, 1, "mul1"),    # five and more
+    (1, 6144, 14720, 2, "mul1"), (3, 6144, 14720, 2, "mul1"), (8, 16384, 4224, 3, "mul1")])  # rings, many units, long rows
+def test_decode_routes(ctx, rows, inputs, outputs, bits, codebook):
+    check(ctx, rows, inputs, outputs, bits, codebook, bias=rows & 1 == 1)
+
+
+@pytest.mark.parametrize("rows", [9, 16, 17, 64, 128, 129, 176, 177, 256])
+@pytest.mark.parametrize("inputs,outputs", [(128, 128), (3072, 256), (640, 5120)])
+def test_wide_row_groups(ctx, rows, inputs, outputs):
+    """One group or several, blocks with one CTA or with many, and CTAs with several blocks."""
+    check(ctx, rows, inputs, outputs, bits=5, bias=inputs == 640)
+
+
+@pytest.mark.parametrize("rows", [257, 511, 513])
+@pytest.mark.parametrize("inputs,outputs,bits,codebook", [(128, 128, 2, "mul1"), (1152, 384, 6, "mcg"), (256, 4480, 4, "3inst")])
+def test_dense_tiles(ctx, rows, inputs, outputs, bits, codebook):
+    check(ctx, rows, inputs, outputs, bits, codebook, bias=True)
+
+
+@pytest.mark.parametrize("rows", [1, 6, 40, 300])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rows_off_a_vector_boundary(ctx, rows, dtype):
+    """Tensors that start one element into a buffer, in and out; what lies around them stays as it was."""
+    inputs, outputs = 384, 256
+    layer = synthetic.make_layer(inputs, outputs, 4, seed=9100)
+    w = ctx.prepare(layer)
+    x = torch.zeros(rows * inputs + 2, dtype=dtype, device="cuda")
+    y = torch.full((rows * outputs + 2,), 7.0, dtype=dtype, device="cuda")
+    xv, yv = x[1:-1].view(rows, inputs), y[1:-1].view(rows, outputs)
+    xv.copy_(dev(synthetic.make_activations(rows, inputs, seed=9101)))
+    (w.gemv if rows <= 8 else w.gemm)(xv, yv)
+    want = c_oracle.linear(layer.trellis, layer.suh, layer.svh, None, 4, 2, host(xv.float()))
+    if dtype == torch.float32:
+        gate(host(yv), want, f"offset {rows}")
+    else:
+        np.testing.assert_allclose(host(yv.float()), want, rtol=2.0 ** -8, atol=1e-3 * np.abs(want).max())
+    assert y[0] == 7 and y[-1] == 7
+    w.close()
+
+
+@pytest.mark.parametrize("tokens,n_exp,top_k", [(5, 16, 2), (17, 2, 1), (150, 1, 1), (130, 2, 2)])
+def test_routed_rows_per_expert(ctx, tokens, n_exp, top_k):
+    """One to 150 rows of an expert: groups of eight, and of 128 with remainders; routes on either side."""
+    from strix_trellis_b200.runtime import MoePlan
+    model, inter = 512, 256
+    layers = make_experts(n_exp, model, inter, 9200)
+    ws = [tuple(ctx.prepare(l[k]) for k in ("gate", "up", "down")) for l in layers]
+    x = synthetic.make_activations(tokens, model, seed=9201)
+    ids, scores = synthetic.make_routes(tokens, n_exp, top_k, seed=9202)
+    want, _ = oracle_block(x, layers, ids, scores, 1.0, 0.0, None)
+    used = sorted(set(int(i) for i in ids.ravel()))
+    for device_routed in (False, True):
+        y = torch.full((tokens, model), float("nan"), device="cuda")
+        if device_routed:
+            plan = MoePlan(ctx, ws, dev(x), y, dev(ids.astype(np.uint32).view(np.int32)), dev(scores), device_routed=True)
+        else:
+            plan = MoePlan(ctx, [ws[e] for e in used], dev(x), y, ids, scores, expert_ids=used)
+        for _ in range(2):
+            plan.submit()
+        torch.cuda.synchronize()
+        gate(host(y), want, f"moe {tokens} device {device_routed}", MOE_REL, MOE_NRMSE)
+        plan.close()
+    for t in ws:
+        for w in t:
+            w.close()
+
+
+def test_immediate_calls_share_scratch_between_shapes(ctx):
+    """Calls of changing shape, in turn on two streams; each stream's scratch serves them all."""
+    shapes = [(1, 1152, 4096), (8, 2048, 640), (40, 512, 1280), (1, 256, 128), (300, 256, 384), (2, 6144, 2560)]
+    cases = []
+    for k, (rows, i, n) in enumerate(shapes):
+        layer = synthetic.make_layer(i, n, 4, seed=9300 + k)
+        x = synthetic.make_activations(rows, i, seed=9310 + k)
+        cases.append((ctx.prepare(layer), dev(x), c_oracle.linear(layer.trellis, layer.suh, layer.svh, None, 4, 2, x)))
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    results = []
+    for turn in range(4):
+        with torch.cuda.stream(streams[turn & 1]):
+            for w, x, want in cases:
+                results.append(((w.gemv if x.shape[0] <= 8 else w.gemm)(x), want))
+    torch.cuda.synchronize()
+    for y, want in results:
+        gate(host(y), want, "immediate")
+    for w, *_ in cases:
+        w.close()
