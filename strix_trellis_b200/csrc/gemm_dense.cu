@@ -427,6 +427,14 @@ cudaError_t launch_dense(const DenseArgs& args, int sm_count, bool programmatic,
 }
 }  // namespace
 
+// A K step of a 256 x 256 tile takes about 4/3 of that of a 256 x 128 tile (measured 0.46 and 0.35 us:
+// half the flops for three quarters of the loads), so narrow tiles pay only where they save that much
+// in the last wave.
+bool gemm_dense_narrow(int m_tiles, int nblocks, int pairs) {
+    const int wide = (m_tiles * ((nblocks + 1) / 2) + pairs - 1) / pairs;
+    const int narrow = (m_tiles * nblocks + pairs - 1) / pairs;
+    return 4 * wide > 3 * narrow;
+}
 int gemm_dense_rows_padded(int rows) { return (rows + 255) / 256 * 256; }
 size_t gemm_dense_scratch(const DeviceWeights& w) { return (size_t)dense_range(w) * w.inputs * 256; }
 
@@ -460,13 +468,7 @@ cudaError_t launch_gemm_dense(const LinearCall& call, unsigned char* workspace, 
         default: return cudaErrorInvalidValue;
         }
         if (e != cudaSuccess) return e;
-        // A K step of a 256 x 256 tile takes about 4/3 of that of a 256 x 128 tile (measured 0.46
-        // and 0.35 us: half the flops for three quarters of the loads), so narrow tiles pay only
-        // where they save that much in the last wave.
-        const int pairs = sm_count / 2;
-        const int wide = (args.m_tiles * ((args.nb_count + 1) / 2) + pairs - 1) / pairs;
-        const int narrow = (args.m_tiles * args.nb_count + pairs - 1) / pairs;
-        const bool two = 4 * wide <= 3 * narrow;
+        const bool two = !gemm_dense_narrow(args.m_tiles, args.nb_count, sm_count / 2);
         args.n_tiles = two ? (args.nb_count + 1) / 2 : args.nb_count;
         e = two ? launch_dense<2>(args, sm_count, programmatic, stream) : launch_dense<1>(args, sm_count, programmatic, stream);
         if (e != cudaSuccess) return e;
