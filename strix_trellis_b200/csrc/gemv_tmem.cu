@@ -22,8 +22,8 @@
 // for another, measured 2.6 us per layer slower: the extra launch boundary costs more.)
 //
 // Measured in a chain of launches against the kernel before, which fed mma.sync and staged its rows
-// four 2-byte stores at a time: 16 layers, four rows, K2..K6 226 -> 180 us; 16384 -> 4096, eight
-// rows, K5 29.6 -> 23.4 us; 4096 -> 129280, one row, K5 133 -> 126 us.
+// four 2-byte stores at a time: 16 layers, four rows, K2..K6 226 -> 178 us; 16384 -> 4096, eight
+// rows, K5 29.6 -> 21.6 us; 4096 -> 129280, one row, K5 133 -> 116 us.
 #include <type_traits>
 
 #include "backend.h"
@@ -389,7 +389,7 @@ cudaError_t launch_gemv_row(const LinearCall& call, const GemvPlan& plan, Split 
 
 // One row with this many units per CTA takes this kernel: the decode loop then outweighs the longer
 // way from the last tile to the fold (measured, one row: 24 units of K4 15.4 against 16.5 us for
-// gemv_row.cu, 218 units of K5 126 against 129 us the other way round).
+// gemv_row.cu, 218 units of K5 115 against 129 us the other way round).
 constexpr int kTmemUnits = 96;
 // Two or more rows with at most this many units per CTA go to gemv_few.cu.
 constexpr int kFewUnits = 4;

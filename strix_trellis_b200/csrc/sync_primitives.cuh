@@ -105,11 +105,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void* src, ui
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
         ::"r"(dst_smem), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-// Asks the L2 to fetch `bytes` (a multiple of 16) at the 16-byte aligned `src`; nothing waits
-// for it and nothing depends on it.
-__device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
 // Asks the L2 for the 128-byte line that holds `p`.  The L2 is the point of coherence of the
 // device, so a line fetched early and written by another SM afterwards is still read correctly
 // from the L2 later.
@@ -144,11 +139,6 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t ran
     uint32_t out;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_addr), "r"(rank));
     return out;
-}
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-    return v;
 }
 
 // Not volatile: the compiler may interleave independent decodes around it.

@@ -41,15 +41,6 @@ __device__ __forceinline__ uint64_t umma_desc_k_major_sw128(uint32_t smem_addr) 
 __host__ __device__ constexpr uint32_t umma_idesc_f16_f32(int m, int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by ONE thread.
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
 // Arrive on an mbarrier once every previously issued MMA of this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
@@ -126,12 +117,6 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
 }
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Byte offset of element (row, k) inside a [rows][64] binary16 tile in the 128-byte
-// swizzled K-major layout the descriptors above describe.
-__host__ __device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t k) {
-    return (row >> 3) * 1024u + (row & 7u) * 128u + ((((k >> 3) ^ row) & 7u) << 4) + (k & 7u) * 2u;
 }
 
 // The 16-byte chunk (8 k) `chunk` of row `row` in such a tile.
