@@ -111,6 +111,7 @@ __device__ __forceinline__ void red_release_gpu(unsigned int* p, unsigned int v)
 // chunk, adds the other CTAs' planes (finisher) or stores the sums to this CTA's plane
 // (contributor); for outputs the chunk is transposed through `stage` and each warp finishes four
 // rows, eight lanes per row.
+template <bool PARTS>  // K in more than one part
 struct Epilogue {
     const WideArgs& a;
     int cta, quarter, lane, bar;
@@ -140,7 +141,7 @@ struct Epilogue {
         }
         const int col = quarter * 32 + lane;
         const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + dcol;
-        const int first_part = part_of(a, w.hb), last_part = part_of(a, w.hb + len - 1);  // of this segment
+        const int first_part = PARTS ? part_of(a, w.hb) : 0, last_part = PARTS ? part_of(a, w.hb + len - 1) : 0;  // of this segment
         int dumped = 0;
         for (int ch = first_chunk; ch < chunks; ch += step) {
             uint32_t r[16];
@@ -163,10 +164,10 @@ struct Epilogue {
                         r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(q[j])));
                     }
                 }
-                if (part != first_part)
+                if (PARTS && part != first_part)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__fadd_rn(stage[j * 128 + col], __uint_as_float(r[j])));
-                if (part != last_part)
+                if (PARTS && part != last_part)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) stage[j * 128 + col] = __uint_as_float(r[j]);
             }
@@ -241,7 +242,7 @@ struct Epilogue {
 
 // At most 72 registers: a CTA of the next call's input stages (128 threads) then fits beside this
 // kernel's, is resident and has its operands in the L2 when this kernel ends.
-template <int CB>
+template <int CB, bool PARTS>
 __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (still a shared-memory pointer to the compiler)
@@ -346,9 +347,9 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             const uint32_t idesc = umma_idesc_f16_f32(128, n), dcol = tmem + d_column(seg);
             const uint32_t odd = args.d_accs == 2 ? args.n_max : 0;  // accumulator of the odd K steps
             if (seg >= d_bufs && !mbar_wait(d_empty + 8 * d_index(seg), d_parity(seg) ^ 1, args.status, kTimeoutTensorPipe)) break;
-            int part = part_of(args, w.hb), fresh = 1;
+            int part = PARTS ? part_of(args, w.hb) : 0, fresh = 1;
             for (int i = 0; i < len; ++i) {
-                if (part_begin(args, part + 1) == w.hb + i) { ++part; fresh = 1; }
+                if (PARTS && part_begin(args, part + 1) == w.hb + i) { ++part; fresh = 1; }
                 const uint32_t acc = dcol + part * args.d_accs * args.n_max;
                 if (!mbar_wait(b_full + 8 * slot, use, args.status, kTimeoutTensorPipe) ||
                     !mbar_wait(a_full + 8 * stage, a_use, args.status, kTimeoutTensorPipe)) {
@@ -383,7 +384,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             if (lane < 2) prefetch_line_l2(dw.svh + (size_t)nb * 128 + lane * 64);
             else if (lane < 6 && dw.bias) prefetch_line_l2(dw.bias + (size_t)nb * 128 + (lane - 2) * 32);
         }
-        const Epilogue epi{args, cta, warp & 3, lane, 1, epi_stage, tmem};
+        const Epilogue<PARTS> epi{args, cta, warp & 3, lane, 1, epi_stage, tmem};
         int seg = 0;
         for (Walk w(args, mine); w.unit < w.end; ++seg) {
             const int len = w.length(args);
@@ -423,7 +424,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         if (ok) ok = mbar_wait(all_done, 0, args.status, kTimeoutTensorPipe);
         if (!group_any(2 + group, !ok)) {
             tc_fence_after_sync();
-            const Epilogue epi{args, cta, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, tmem};
+            const Epilogue<PARTS> epi{args, cta, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, tmem};
             epi.segment(split, mine, w, w.length(args), d_column(seg), 1 + group, 1 + kDecodeW / 4);
             tc_fence_before_sync();
         }
@@ -576,6 +577,12 @@ cudaError_t launch_wide_inputs(const WideSet& set, const WidePlan& plan, unsigne
     return launch_pdl(wide_inputs_kernel, dim3(x, y), 32 * kInputWarps, 0, programmatic, stream, a, plan.grid);
 }
 
+template <int CB>
+static cudaError_t launch_wide_cb(const WideArgs& a, const WidePlan& plan, bool programmatic, cudaStream_t stream) {
+    if (a.parts > 1) return launch_pdl(wide_linear_kernel<CB, true>, dim3(plan.grid), kThreadsW, plan.smem_bytes, programmatic, stream, a);
+    return launch_pdl(wide_linear_kernel<CB, false>, dim3(plan.grid), kThreadsW, plan.smem_bytes, programmatic, stream, a);
+}
+
 cudaError_t launch_wide(const WideSet& set, const WidePlan& plan, unsigned int* flags, float* planes, unsigned int* status,
                         bool programmatic, cudaStream_t stream) {
     const WideArgs a = wide_args(set, plan, flags, planes, status);
@@ -584,21 +591,25 @@ cudaError_t launch_wide(const WideSet& set, const WidePlan& plan, unsigned int* 
         (size_t)plan.w_slots * plan.w_stride < kRingMin)
         return cudaErrorInvalidValue;
     switch (set.codebook) {
-    case CB_3INST: return launch_pdl(wide_linear_kernel<CB_3INST>, dim3(plan.grid), kThreadsW, plan.smem_bytes, programmatic, stream, a);
-    case CB_MCG: return launch_pdl(wide_linear_kernel<CB_MCG>, dim3(plan.grid), kThreadsW, plan.smem_bytes, programmatic, stream, a);
-    case CB_MUL1: return launch_pdl(wide_linear_kernel<CB_MUL1>, dim3(plan.grid), kThreadsW, plan.smem_bytes, programmatic, stream, a);
+    case CB_3INST: return launch_wide_cb<CB_3INST>(a, plan, programmatic, stream);
+    case CB_MCG: return launch_wide_cb<CB_MCG>(a, plan, programmatic, stream);
+    case CB_MUL1: return launch_wide_cb<CB_MUL1>(a, plan, programmatic, stream);
     default: return cudaErrorInvalidValue;
     }
 }
 
 // Opt-in dynamic shared memory is a per-device function attribute: set when a context is created
 // on a device (configure_device), never on the launch path.
+template <int CB>
+static cudaError_t configure_wide_cb() {
+    const cudaError_t e = cudaFuncSetAttribute(wide_linear_kernel<CB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(wide_linear_kernel<CB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+}
 cudaError_t configure_wide_kernels() {
-    cudaError_t e = cudaFuncSetAttribute(wide_linear_kernel<CB_3INST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(wide_linear_kernel<CB_MCG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(wide_linear_kernel<CB_MUL1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    cudaError_t e = configure_wide_cb<CB_3INST>();
+    if (e == cudaSuccess) e = configure_wide_cb<CB_MCG>();
+    if (e == cudaSuccess) e = configure_wide_cb<CB_MUL1>();
     // The same shared-memory carve-out as the kernel that follows: an SM that has to change its split
     // between L1 and shared memory drains first, and nothing of the two launches overlaps.
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_inputs_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
