@@ -35,7 +35,7 @@ constexpr int kWarpMma = kDecodeW + kEpiW, kWarpWeights = kWarpMma + 1, kWarpRow
 constexpr int kThreadsW = (kWarpRows + 1) * 32;
 constexpr int kChunkRows = 16;                       // rows of one epilogue chunk
 constexpr int kStageFloats = kChunkRows * 128;       // 8 KB of transposition space per warp group
-constexpr int kHeaderW = 1024 + kStageFloats * 4;    // barriers, the epilogue group's staging
+constexpr int kHeaderW = 1024 + 2 * kStageFloats * 4;  // barriers, the epilogue group's two staging areas
 constexpr size_t kSmemLimitW = 224 * 1024;
 constexpr int kMaxWSlots = 24, kMaxBSlots = 8;
 constexpr int kRingMin = kDecodeW / 4 * kStageFloats * 4;       // the decode groups' staging of the last segment
@@ -115,18 +115,17 @@ template <bool PARTS>  // K in more than one part
 struct Epilogue {
     const WideArgs& a;
     int cta, quarter, lane, bar;
-    float* stage;
-    uint32_t tmem;  // tensor-memory base
+    float* areas;      // staging: two areas in turn (one barrier per chunk instead of two), or one
+    int area_floats;   // from one to the other; 0: one
 
     // false: a wait ran out (the whole group returns together)
-    __device__ __forceinline__ bool segment(const Split& split, const Range& mine, const Walk& w, int len, uint32_t dcol,
-                                            int first_chunk, int step) const {
+    __device__ __forceinline__ bool segment(const Split& split, const Walk& w, int len, uint32_t dcol, int first_chunk, int step,
+                                            uint32_t d_empty) const {
         const int rows = problem_rows(a, w.p), chunks = (rows + kChunkRows - 1) / kChunkRows;
         const int lo = (w.p * a.nblocks + w.nb) * a.hblocks, hi = lo + a.hblocks;
         const bool contributor = w.hb != 0;
         int last = cta;
         if (!contributor && w.hb + len < a.hblocks) last = owner(split, hi - 1);
-        (void)mine;
         const WideProblem& pr = problem(a, w.p);
         // The flag of CTA c counts the chunks of its plane that are there.
         bool late = false;
@@ -140,7 +139,8 @@ struct Epilogue {
             return false;
         }
         const int col = quarter * 32 + lane;
-        const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + dcol;
+        const uint32_t taddr = ((uint32_t)(quarter * 32) << 16) + dcol;
+        float* stage = areas;
         const int first_part = PARTS ? part_of(a, w.hb) : 0, last_part = PARTS ? part_of(a, w.hb + len - 1) : 0;  // of this segment
         int dumped = 0;
         for (int ch = first_chunk; ch < chunks; ch += step) {
@@ -151,18 +151,19 @@ struct Epilogue {
                 const uint32_t at = taddr + part * a.d_accs * a.n_max + ch * kChunkRows;
                 __syncwarp();
                 tmem_ld_32x16(at, r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(r[j]));  // not before the wait
                 if (a.d_accs == 2) {
                     uint32_t q[16];
                     tmem_ld_32x16(at + a.n_max, q);
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        asm volatile("" : "+r"(q[j]));
+                        asm volatile("" : "+r"(r[j]), "+r"(q[j]));  // not before the wait
                         r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(q[j])));
                     }
+                } else {
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(r[j]));
                 }
                 if (PARTS && part != first_part)
 #pragma unroll
@@ -170,6 +171,11 @@ struct Epilogue {
                 if (PARTS && part != last_part)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) stage[j * 128 + col] = __uint_as_float(r[j]);
+            }
+            if (d_empty && ch + step >= chunks) {  // the accumulators are in registers: the next segment's MMAs may start
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(d_empty);
             }
             if (contributor) {
                 float* plane = a.planes + ((size_t)cta * a.n_max + ch * kChunkRows) * 128 + col;
@@ -192,8 +198,9 @@ struct Epilogue {
 #pragma unroll
             for (int j = 0; j < 16; ++j) stage[j * 128 + col] = v[j];
             named_barrier(bar, 128);
-            finish_rows(pr, w, ch, rows);
-            named_barrier(bar, 128);
+            finish_rows(pr, w, ch, rows, stage);
+            if (!area_floats) named_barrier(bar, 128);  // (two areas: the next chunk's barrier does)
+            stage = stage == areas ? areas + area_floats : areas;
         }
         if (contributor && dumped) {
             named_barrier(bar, 128);  // the group's stores are ordered before the count below
@@ -202,7 +209,7 @@ struct Epilogue {
         return true;
     }
 
-    __device__ __forceinline__ void finish_rows(const WideProblem& pr, const Walk& w, int ch, int rows) const {
+    __device__ __forceinline__ void finish_rows(const WideProblem& pr, const Walk& w, int ch, int rows, const float* stage) const {
         const int l8 = lane & 7;
         const int in_chunk = quarter * 4 + (lane >> 3);
         float v[4][4];
@@ -384,7 +391,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             if (lane < 2) prefetch_line_l2(dw.svh + (size_t)nb * 128 + lane * 64);
             else if (lane < 6 && dw.bias) prefetch_line_l2(dw.bias + (size_t)nb * 128 + (lane - 2) * 32);
         }
-        const Epilogue<PARTS> epi{args, cta, warp & 3, lane, 1, epi_stage, tmem};
+        const Epilogue<PARTS> epi{args, cta, warp & 3, lane, 1, epi_stage, kStageFloats};
         int seg = 0;
         for (Walk w(args, mine); w.unit < w.end; ++seg) {
             const int len = w.length(args);
@@ -392,10 +399,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             const bool ok = mbar_wait(d_full + 8 * d_index(seg), d_parity(seg), args.status, kTimeoutTensorPipe);
             if (group_any(1, !ok)) break;
             tc_fence_after_sync();
-            if (!epi.segment(split, mine, w, len, d_column(seg), 0, final ? 1 + kDecodeW / 4 : 1)) break;
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(d_empty + 8 * d_index(seg));
+            if (!epi.segment(split, w, len, tmem + d_column(seg), 0, final ? 1 + kDecodeW / 4 : 1, d_empty + 8 * d_index(seg))) break;
             w.next(args, len);
         }
     } else {
@@ -424,8 +428,8 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         if (ok) ok = mbar_wait(all_done, 0, args.status, kTimeoutTensorPipe);
         if (!group_any(2 + group, !ok)) {
             tc_fence_after_sync();
-            const Epilogue<PARTS> epi{args, cta, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, tmem};
-            epi.segment(split, mine, w, w.length(args), d_column(seg), 1 + group, 1 + kDecodeW / 4);
+            const Epilogue<PARTS> epi{args, cta, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, 0};
+            epi.segment(split, w, w.length(args), tmem + d_column(seg), 1 + group, 1 + kDecodeW / 4, 0);
             tc_fence_before_sync();
         }
     }
