@@ -10,7 +10,7 @@ namespace st {
 constexpr int kGroupRows = 128;  // most rows of one problem: its weights are decoded once for all of them
 constexpr int kDirectRows = 8;   // most rows of one problem of grouped_direct.cu
 constexpr int kDirectStages = 16, kDirectSplits = 16;
-constexpr double kWideStart = 14.0;  // us of a wide launch pair beyond its units, see direct_pays
+constexpr double kWideStart = 10.0;  // us of a wide launch pair beyond its units, see direct_pays
 constexpr size_t kDirectSmemLimit = 110 * 1024;  // two CTAs per SM
 
 // One problem of a table in device memory.  Input row r is x + x_row[r]*x_stride, output row r is
