@@ -15,13 +15,13 @@ cudaError_t launch_gemm_dense(const LinearCall& call, unsigned char* workspace, 
                               cudaStream_t stream);
 
 namespace {
-// At 512 rows two decodes of a unit and one dense step over it take the same time.
-constexpr int kWideMaxRows = 512;
+// As far as the estimates are fitted and measured; beyond, four and more decodes of a unit hardly pay.
+constexpr int kWideMaxRows = 1024;
 
 // How a call's rows are cut into groups that each decode the weights, and how many CTAs run them: one
 // group and every SM, unless so few column blocks are left that many CTAs share one and the CTA that
 // finishes it adds all their planes (178 rows on 3072 -> 2048, nine CTAs a block: 51 us in one group,
-// 22 us in three).  Estimates in us, fitted to 150 shapes of 9 to 512 rows (rms error 10 %): a unit 0.6
+// 22 us in three).  Estimates in us, fitted to 150 shapes of 9 to 512 rows (rms error 10 %) and checked to 1024: a unit 0.6
 // + 0.0023 a row (its activation tile comes from the L2 for every unit); a segment that is not a
 // CTA's last 1.4 a chunk of 16 rows, 1.6 where its accumulators have no second buffer; in the last one
 // a plane's chunk 0.9, five warp groups side by side.  With s CTAs a block that is (unit * hblocks +

@@ -40,7 +40,7 @@ def test_decode_routes(ctx, rows, inputs, outputs, bits, codebook):
     check(ctx, rows, inputs, outputs, bits, codebook, bias=rows & 1 == 1)
 
 
-@pytest.mark.parametrize("rows", [9, 16, 17, 64, 128, 129, 176, 177, 256, 257, 512])
+@pytest.mark.parametrize("rows", [9, 16, 17, 64, 128, 129, 176, 177, 256, 257, 513, 1024])
 @pytest.mark.parametrize("inputs,outputs", [(128, 128), (3072, 256), (640, 5120)])
 def test_wide_row_groups(ctx, rows, inputs, outputs):
     """One group or several, blocks with one CTA or with many, CTAs with several blocks, and up to
@@ -48,7 +48,7 @@ def test_wide_row_groups(ctx, rows, inputs, outputs):
     check(ctx, rows, inputs, outputs, bits=5, bias=inputs == 640)
 
 
-@pytest.mark.parametrize("rows", [513, 767, 1025])
+@pytest.mark.parametrize("rows", [1025, 1151, 1281])
 @pytest.mark.parametrize("inputs,outputs,bits,codebook", [(128, 128, 2, "mul1"), (1152, 384, 6, "mcg"), (256, 4480, 4, "3inst")])
 def test_dense_tiles(ctx, rows, inputs, outputs, bits, codebook):
     check(ctx, rows, inputs, outputs, bits, codebook, bias=True)
