@@ -10,7 +10,7 @@
 // per 16 inputs.  Here the activation operand is made by the CTA itself, in shared memory: eight
 // helper warps run the input stages of the blocks its range touches while the decode warps are
 // already at work (weights are immutable, so they do not wait for the previous kernel; only the
-// MMAs wait for the activations, and the decode is up to seven units ahead of them).
+// MMAs wait for the activations, and the decode is up to six units ahead of them).
 //
 // Fold: a column block that several CTAs share is finished by the CTA that holds its FIRST K range
 // (the end of its own range).  The others publish their sums word by word in global planes, where
@@ -39,6 +39,14 @@ constexpr int kWarpMmaT = kDecodeT + kHelpersT, kWarpWeightsT = kWarpMmaT + 1;
 constexpr int kThreadsT = (kWarpWeightsT + 1) * 32;
 constexpr int kRowsT = 16;                       // the MMA's N: the smallest it has; rows beyond the call's are never read
 constexpr int kMaxRowsT = 8;
+// A column is summed in four chains (parity of the unit, parity of the K step), each with an accumulator
+// of its own, twice for the segments in turn: 128 of the 512 columns, the other 384 are six A stages.  The
+// tensor cores truncate as they accumulate, so the error of a chain grows with the 1.5th power of its
+// steps.  Distance from the sum in 64 bits, one chain and four, of the result's norm: 4096 -> 129280, one
+// row 4.8e-6 and 1.2e-6; 16384 -> 4096, eight rows 4.0e-6 and 1.0e-6; 5120 -> 5120, four rows 1.6e-6 and
+// 4.5e-7.  Four take 119.2 us instead of 118.0 for the first of these and 22.0 instead of 21.65 for the second.
+constexpr int kChains = 4, kAStagesT = 6;
+static_assert(kAStagesT * 64 + 2 * kChains * kRowsT <= 512 && kAStagesT >= kUnitGroups && kAStagesT <= kMaxAStages, "tensor memory");
 constexpr int kSlotBytesT = kRowsT * 256;        // activation operand of one H128 block
 constexpr int kStageFloats = kMaxRowsT * 128;    // transposition space of one helper group
 constexpr int kMaxWSlotsT = 32, kMaxBSlotsT = 48;
@@ -46,7 +54,7 @@ constexpr int kHeaderT = 2048 + 2 * kStageFloats * 4;
 constexpr size_t kSmemLimitT = 224 * 1024;
 constexpr uint32_t kEmptyWord = 0xFFFFFFFFu;      // a plane word nobody has written yet
 constexpr int kMinBRing = 4 * kHelpersT;          // units of one staging step of one row
-static_assert((2 * kMaxWSlotsT + 2 * kMaxBSlotsT + 2 * kMaxAStages + 4) * 8 <= 2048, "barriers fit the header");
+static_assert((2 * kMaxWSlotsT + 2 * kMaxBSlotsT + 2 * kAStagesT + 4) * 8 <= 2048, "barriers fit the header");
 
 struct TmemArgs {
     LinearCall call;
@@ -73,8 +81,8 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
     unsigned char* w_ring = b_ring + (size_t)args.b_slots * kSlotBytesT;
     __shared__ uint32_t s_tmem_base;
     const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * kMaxWSlotsT, b_full = w_empty + 8 * kMaxWSlotsT,
-                   b_empty = b_full + 8 * kMaxBSlotsT, a_full = b_empty + 8 * kMaxBSlotsT, a_empty = a_full + 8 * kMaxAStages,
-                   d_full = a_empty + 8 * kMaxAStages, d_empty = d_full + 16;
+                   b_empty = b_full + 8 * kMaxBSlotsT, a_full = b_empty + 8 * kMaxBSlotsT, a_empty = a_full + 8 * kAStagesT,
+                   d_full = a_empty + 8 * kAStagesT, d_empty = d_full + 16;
 
     // The activation operand is staged per H128 block.  `resident`: every block the range touches has
     // a slot of its own and is staged once; else the slots are a ring in unit order.
@@ -130,14 +138,14 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
     } else {  // one decode thread per barrier
         const int t = threadIdx.x;
         if (t < args.b_slots) { mbar_init(b_full + 8 * t, rows); mbar_init(b_empty + 8 * t, 1); }
-        if (t < kMaxAStages) { mbar_init(a_full + 8 * t, 4); mbar_init(a_empty + 8 * t, 1); }
+        if (t < kAStagesT) { mbar_init(a_full + 8 * t, 4); mbar_init(a_empty + 8 * t, 1); }
         if (t < 2) { mbar_init(d_full + 8 * t, 1); mbar_init(d_empty + 8 * t, 4); }
         mbar_fence_init();
     }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = s_tmem_base, d_col = kMaxAStages * 64;
+    const uint32_t tmem = s_tmem_base, d_col = kAStagesT * 64;
     pdl_launch_dependents();
 
     if (warp == kWarpWeightsT) {
@@ -164,7 +172,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
         bool ok = true;
         for (int done = 0, hb = first_hb; done < my_units && ok; ++seg, hb = 0) {
             const int left = my_units - done, len = left < hblocks - hb ? left : hblocks - hb;
-            const uint32_t dcol = tmem + d_col + (seg & 1) * kRowsT;
+            const uint32_t dcol = tmem + d_col + (seg & 1) * kChains * kRowsT;
             if (seg >= 2 && !mbar_wait(d_empty + 8 * (seg & 1), (uint32_t)((seg >> 1) - 1) & 1, c.status, kTimeoutTensorPipe)) break;
             for (int i = 0; i < len; ++i) {
                 if (!mbar_wait(b_full + 8 * slot, use, c.status, kTimeoutTensorPipe) ||
@@ -174,17 +182,17 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
                 }
                 tc_fence_after_sync();
                 const uint64_t b0 = b_desc + (uint32_t)(slot * (kSlotBytesT / 16));  // 16-byte units
-                const uint32_t acol = tmem + stage * 64;
+                const uint32_t acol = tmem + stage * 64, acc = dcol + (i & 1) * 2 * kRowsT;
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        umma_f16_ts(dcol, acol + 8 * k, b0 + (k < 4 ? 0 : kSlotBytesT / 32) + 2 * (k & 3), idesc, (i | k) != 0);
+                        umma_f16_ts(acc + (k & 1) * kRowsT, acol + 8 * k, b0 + (k < 4 ? 0 : kSlotBytesT / 32) + 2 * (k & 3), idesc, i > 1 || k > 1);
                     umma_commit(a_empty + 8 * stage);
                     if (!resident) umma_commit(b_empty + 8 * slot);
                 }
                 __syncwarp();
                 if (++slot == b_wrap) { slot = 0; if (!resident) use ^= 1; }  // a resident slot is filled once
-                if (++stage == kMaxAStages) { stage = 0; a_use ^= 1; }
+                if (++stage == kAStagesT) { stage = 0; a_use ^= 1; }
             }
             if (elect_one()) umma_commit(d_full + 8 * (seg & 1));
             done += len;
@@ -194,7 +202,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
         const int turn = warp >> 2, ctile = 2 * (warp & 3);
         DecodeState s{turn, turn, 1, false, turn % args.w_slots, (uint32_t)(turn / args.w_slots) & 1};
         decode_segment_rate<CB, kUnitGroups>(c.w.bits, s, my_units, w_ring, args.w_slots, w_stride, w_full, w_empty, a_full, a_empty,
-                                             tmem + ((uint32_t)(ctile * 16) << 16), kMaxAStages, ctile, lane, c.status);
+                                             tmem + ((uint32_t)(ctile * 16) << 16), kAStagesT, ctile, lane, c.status);
     } else {
         // ---- helper warps: input stages, then the epilogue of every other segment ---------------------
         const bool x_aligned = quads_aligned(c.x, c.x_dtype, c.x_stride);
@@ -249,11 +257,22 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
             bool good = mbar_wait(d_full + 8 * (seg & 1), (uint32_t)(seg >> 1) & 1, c.status, kTimeoutTensorPipe);
             __syncwarp();
             tc_fence_after_sync();
-            uint32_t r[16];
-            tmem_ld_32x16(tmem + ((uint32_t)(quarter * 32) << 16) + d_col + (seg & 1) * kRowsT, r);
-            tmem_ld_wait();
+            const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + d_col + (seg & 1) * kChains * kRowsT;
+            float v[kMaxRowsT];
+            uint32_t r[2][kMaxRowsT];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(r[j]));  // not before the wait
+            for (int pair = 0; pair < 2; ++pair) {  // the chains of the even units, then (if there are any) of the odd ones
+                if (pair && len < 2) break;
+                tmem_ld_32x8(at + pair * 2 * kRowsT, r[0]);
+                tmem_ld_32x8(at + pair * 2 * kRowsT + kRowsT, r[1]);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < kMaxRowsT; ++j) {
+                    asm volatile("" : "+r"(r[0][j]), "+r"(r[1][j]));  // not before the wait
+                    const float both = __fadd_rn(__uint_as_float(r[0][j]), __uint_as_float(r[1][j]));
+                    v[j] = pair ? __fadd_rn(v[j], both) : both;
+                }
+            }
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(d_empty + 8 * (seg & 1));
@@ -263,13 +282,12 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
                 if (good) {
 #pragma unroll
                     for (int j = 0; j < kMaxRowsT; ++j)
-                        if (j < rows) st_relaxed_gpu(words + ((size_t)cta * rows + j) * 128, r[j]);
+                        if (j < rows) st_relaxed_gpu(words + ((size_t)cta * rows + j) * 128, __float_as_uint(v[j]));
                 }
                 return;
             }
-            float v[kMaxRowsT];
 #pragma unroll
-            for (int j = 0; j < kMaxRowsT; ++j) v[j] = __fadd_rn(0.f, __uint_as_float(r[j]));
+            for (int j = 0; j < kMaxRowsT; ++j) v[j] = __fadd_rn(0.f, v[j]);
             // 16 words in flight, whatever the row count: R rows of 16 / R planes
             auto fold = [&](auto width) {
                 constexpr int R = decltype(width)::value, P = 16 / R;

@@ -32,3 +32,15 @@ def dev(a):
 
 def host(t):
     return t.detach().cpu().numpy()
+
+
+def linear64(w, layer, x):
+    """The linear of prepared weights `w` with the sums in 64 bits: the decoded weights and the core input
+    are the device's own (bit-exact by their own tests), everything after them is float64."""
+    h = torch.ones(1, 1, dtype=torch.float64)
+    while h.shape[0] < 128:
+        h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+    h = (h / 128 ** 0.5).cuda()
+    core = w.input_stages(x)[2].double() @ w.dequantize().double()
+    y = (core.view(x.shape[0], -1, 128) @ h).view(x.shape[0], -1) * dev(np.asarray(layer.svh).view(np.float16)).double()
+    return y if layer.bias is None else y + dev(layer.bias).double()

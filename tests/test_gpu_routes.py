@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import dev, gate, host
+from gpu_util import dev, gate, host, linear64
 from oracle import c_oracle
 from strix_trellis_b200 import synthetic
 from test_gpu_moe import MOE_NRMSE, MOE_REL, make_experts, oracle_block
@@ -38,6 +38,25 @@ def check(ctx, rows, inputs, outputs, bits=4, codebook="mul1", bias=False):
     (1, 6144, 14720, 2, "mul1"), (3, 6144, 14720, 2, "mul1"), (8, 16384, 4224, 3, "mul1")])  # rings, many units, long rows
 def test_decode_routes(ctx, rows, inputs, outputs, bits, codebook):
     check(ctx, rows, inputs, outputs, bits, codebook, bias=rows & 1 == 1)
+
+
+@pytest.mark.parametrize("rows,inputs,outputs,bits", [
+    (1, 4096, 129280, 5), (8, 16384, 4096, 5), (4, 5120, 5120, 4), (2, 16384, 14848, 2), (3, 128, 38144, 4)])
+def test_sums_of_the_tensor_memory_gemv(ctx, rows, inputs, outputs, bits):
+    """Four chains a column.  A truncating accumulation loses half a unit in the last place of the running
+    sum on average, at most 2^-24 of it; a running sum of k products of random sign is sqrt(k) of one.
+    Summed over the 2 L steps of a chain (L units in a CTA's segment of a column block) that is, of the
+    norm of the whole, 2^-24 * 4/3 * L for four chains a segment and four times as much for one.  The sums
+    that follow (chains, planes, H128) are roundings: a few 2^-25 each, together below 2^-22."""
+    layer = synthetic.make_layer(inputs, outputs, bits, seed=9050)
+    w = ctx.prepare(layer)
+    x = dev(synthetic.make_activations(rows, inputs, seed=9051))
+    want = linear64(w, layer, x)
+    error = float((w.gemv(x).double() - want).norm() / want.norm())
+    units = (inputs // 128) * (outputs // 128)
+    longest = min(inputs // 128, -(-units // min(units, torch.cuda.get_device_properties(0).multi_processor_count)))
+    assert error <= 2.0 ** -24 * 4 / 3 * longest + 2.0 ** -22, error
+    w.close()
 
 
 @pytest.mark.parametrize("rows", [9, 16, 17, 64, 128, 129, 176, 177, 256, 257, 513, 1024])
