@@ -260,7 +260,12 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     const int count = args.live ? (int)ld_acquire_gpu(reinterpret_cast<const unsigned int*>(args.live)) : args.count;
     const int units = count * args.nblocks * args.hblocks;
     const int grid = units < (int)gridDim.x ? units : (int)gridDim.x;
-    if (cta >= grid) return;
+    if (cta >= grid) {
+        // Without a live problem nobody else waits for the launch before, and a launch may only end after
+        // it has: the one after this counts on that when it overwrites what the one before reads.
+        if (!grid) pdl_wait_prior_grid();
+        return;
+    }
     const Split split = make_split(units, grid);
     const Range mine = cta_range(split, cta);
     const int my_units = mine.end - mine.begin;

@@ -121,6 +121,34 @@ def test_routed_rows_per_expert(ctx, tokens, n_exp, top_k):
             w.close()
 
 
+@pytest.mark.parametrize("tokens,n_exp,top_k", [(150, 1, 1), (64, 4, 2)])
+def test_submits_without_a_live_route(ctx, tokens, n_exp, top_k):
+    """Every route invalid, several submits in a row, then valid ones on the same plan: launches that have
+    nothing to do keep their place in the order of launches."""
+    from strix_trellis_b200.runtime import MoePlan
+    model, inter = 512, 256
+    layers = make_experts(n_exp, model, inter, 9250)
+    ws = [tuple(ctx.prepare(l[k]) for k in ("gate", "up", "down")) for l in layers]
+    x = synthetic.make_activations(tokens, model, seed=9251)
+    ids, scores = synthetic.make_routes(tokens, n_exp, top_k, seed=9252)
+    want, _ = oracle_block(x, layers, ids, scores, 1.0, 0.0, None)
+    device_ids, y = dev(np.full(ids.shape, n_exp, dtype=np.int32)), torch.zeros((tokens, model), device="cuda")
+    plan = MoePlan(ctx, ws, dev(x), y, device_ids, dev(scores), device_routed=True)
+    for _ in range(2):
+        device_ids.fill_(n_exp)
+        for _ in range(4):
+            plan.submit()
+        assert bool(torch.isnan(y).all())
+        device_ids.copy_(dev(ids.astype(np.uint32).view(np.int32)))
+        for _ in range(2):
+            plan.submit()
+        gate(host(y), want, "after submits without a route", MOE_REL, MOE_NRMSE)
+    plan.close()
+    for t in ws:
+        for w in t:
+            w.close()
+
+
 def test_immediate_calls_share_scratch_between_shapes(ctx):
     """Calls of changing shape, in turn on two streams; each stream's scratch serves them all."""
     shapes = [(1, 1152, 4096), (8, 2048, 640), (40, 512, 1280), (1, 256, 128), (300, 256, 384), (2, 6144, 2560)]
