@@ -17,7 +17,7 @@ struct strix_context_impl {
     size_t weights_count = 0;
     unsigned int* status = nullptr;  // device word: bounded-wait failures of any kernel
     bool programmatic_launch = true;
-    // Scratch areas of immediate calls that bring no workspace (direct_call.cu), one per stream, every
+    // Scratch areas of immediate calls that bring no workspace (api_call.cpp), one per stream, every
     // word empty between launches; freed with the context.
     struct StreamScratch { cudaStream_t stream; void* area; };
     std::vector<StreamScratch> stream_scratch;

@@ -427,6 +427,82 @@ void call_and_plan_rules(strix_context c) {
     CHECK(cudaFree(x) == cudaSuccess && cudaFree(y) == cudaSuccess && cudaFree(ws) == cudaSuccess);
 }
 
+// strix_b200_linear_call: the rules of strix_gemv / strix_gemm from plain arguments.
+void linear_call_rules(strix_context c) {
+    HostLayer layer;
+    auto stream = blank<strix_stream>();
+    auto parts = layer.parts();
+    strix_weights w = nullptr;
+    CHECK(strix_weights_prepare_parts(c, &parts, &stream, &w) == STRIX_SUCCESS);
+    void *x = nullptr, *y = nullptr, *ws = nullptr;
+    CHECK(cudaMalloc(&x, 16384) == cudaSuccess && cudaMalloc(&y, 16384) == cudaSuccess && cudaMalloc(&ws, 32768) == cudaSuccess);
+    const strix_b200_tensor x2{x, 2, 128, 128, 1, STRIX_DTYPE_F32, 2}, y2{y, 2, 256, 256, 1, STRIX_DTYPE_F32, 2};
+    strix_b200_tensor xt = x2, yt = y2;
+    auto call = [&](uint32_t operation, void* workspace, uint64_t bytes, void* on = nullptr) {
+        return strix_b200_linear_call(c, w, operation, &xt, &yt, 1.0f, 0.0f, workspace, bytes, on);
+    };
+    auto refused = [&](strix_status expected, uint32_t operation = STRIX_OPERATION_GEMV, void* workspace = nullptr, uint64_t bytes = 0,
+                       void* on = nullptr) {
+        const int launches = record().launches;
+        CHECK(call(operation, workspace, bytes, on) == expected && record().launches == launches);
+        xt = x2; yt = y2;
+    };
+
+    // what a call passes on
+    CHECK(call(STRIX_OPERATION_GEMV, nullptr, 0) == STRIX_SUCCESS);
+    CHECK(record().last.rows == 2 && record().last.x == x && record().last.y == y && !record().last_was_gemm);
+    const void* scratch = record().last_workspace;
+    CHECK(scratch && scratch != ws);
+    CHECK(call(STRIX_OPERATION_GEMV, ws, 32768) == STRIX_SUCCESS && record().last_workspace == ws);
+    xt = {x, 1, 128, 128, 1, STRIX_DTYPE_BF16, 1}; yt = {y, 1, 256, 256, 1, STRIX_DTYPE_F16, 1};
+    CHECK(call(STRIX_OPERATION_GEMV, nullptr, 0) == STRIX_SUCCESS && record().last.rows == 1);
+    CHECK(record().last.x_dtype == st::DT_BF16 && record().last.y_dtype == st::DT_F16 && record().last_workspace == scratch);
+    xt = x2; yt = y2;
+    CHECK(call(STRIX_OPERATION_GEMM, nullptr, 0) == STRIX_SUCCESS);  // a GEMM of few rows is a GEMV
+    xt.rows = yt.rows = 0; xt.data = yt.data = nullptr;
+    const int launches = record().launches;
+    CHECK(call(STRIX_OPERATION_GEMV, nullptr, 0) == STRIX_SUCCESS && record().launches == launches);  // nothing to do
+    xt = x2; yt = y2;
+
+    // refusals, nothing enqueued
+    refused(STRIX_ERROR_INVALID_ARGUMENT, 7);
+    CHECK(strix_b200_linear_call(c, nullptr, STRIX_OPERATION_GEMV, &xt, &yt, 1.0f, 0.0f, nullptr, 0, nullptr) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_call(c, w, STRIX_OPERATION_GEMV, nullptr, &yt, 1.0f, 0.0f, nullptr, 0, nullptr) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_call(c, w, STRIX_OPERATION_GEMV, &xt, nullptr, 1.0f, 0.0f, nullptr, 0, nullptr) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_call(c, w, STRIX_OPERATION_GEMV, &xt, &yt, INFINITY, 0.0f, nullptr, 0, nullptr) == STRIX_ERROR_INVALID_ARGUMENT);
+    refused(STRIX_ERROR_INVALID_ARGUMENT, STRIX_OPERATION_GEMV, nullptr, 32768);                        // bytes of no workspace
+    refused(STRIX_ERROR_INSUFFICIENT_BUFFER, STRIX_OPERATION_GEMV, ws, 256);
+    refused(STRIX_ERROR_INVALID_ARGUMENT, STRIX_OPERATION_GEMV, nullptr, 0, reinterpret_cast<void*>(uintptr_t(0x99)));  // no such stream
+    xt.rank = yt.rank = 3; refused(STRIX_ERROR_UNSUPPORTED_FORMAT);
+    xt.rank = 1; refused(STRIX_ERROR_UNSUPPORTED_FORMAT);
+    xt.column_stride = 2; refused(STRIX_ERROR_UNSUPPORTED_FORMAT);
+    xt.row_stride = 256; refused(STRIX_ERROR_UNSUPPORTED_FORMAT);
+    xt.dtype = 99; refused(STRIX_ERROR_UNSUPPORTED_FORMAT);
+    xt.data = nullptr; refused(STRIX_ERROR_INSUFFICIENT_BUFFER);
+    xt.data = static_cast<char*>(x) + 2; refused(STRIX_ERROR_INVALID_ARGUMENT);
+    yt.data = x; refused(STRIX_ERROR_INVALID_ARGUMENT);
+    xt.rows = yt.rows = 9; refused(STRIX_ERROR_UNSUPPORTED_FORMAT);
+    xt.rows = yt.rows = 9; refused(STRIX_ERROR_INSUFFICIENT_BUFFER, STRIX_OPERATION_GEMM);             // needs a workspace
+    xt.rows = yt.rows = 17; refused(STRIX_ERROR_INSUFFICIENT_BUFFER, STRIX_OPERATION_GEMM, nullptr, 0);  // rows outside the buffers' reach
+    // the span of such rows wraps 64 bits; strides and row counts are refused before it is used
+    xt.row_stride = uint64_t(1) << 63; refused(STRIX_ERROR_UNSUPPORTED_FORMAT);
+    xt.rows = yt.rows = (uint64_t(1) << 62) + 1; refused(STRIX_ERROR_UNSUPPORTED_FORMAT, STRIX_OPERATION_GEMM);
+    xt.rows = yt.rows = 0x7FFFFFFF; refused(STRIX_ERROR_INVALID_ARGUMENT, STRIX_OPERATION_GEMM);  // the spans meet
+    state().capturing = true;  // a captured launch replays anywhere: it brings its own workspace
+    refused(STRIX_ERROR_INSUFFICIENT_BUFFER);
+    CHECK(call(STRIX_OPERATION_GEMV, ws, 32768) == STRIX_SUCCESS);
+    state().capturing = false;
+    record().fail_launch = true;
+    refused(STRIX_ERROR_BACKEND);
+    record().fail_launch = false;
+    state().current_device = 1;
+    refused(STRIX_ERROR_INVALID_ARGUMENT);
+    state().current_device = 0;
+
+    CHECK(strix_weights_destroy(w) == STRIX_SUCCESS);
+    CHECK(cudaFree(x) == cudaSuccess && cudaFree(y) == cudaSuccess && cudaFree(ws) == cudaSuccess);
+}
+
 }  // namespace
 
 int main() {
@@ -441,6 +517,7 @@ int main() {
     CHECK(strix_context_create(&cd, &c) == STRIX_SUCCESS);
     prepare_rules(c);
     call_and_plan_rules(c);
+    linear_call_rules(c);
     CHECK(strix_context_destroy(c) == STRIX_SUCCESS);
     CHECK(state().blocks.empty());  // everything the library allocated was returned
     std::printf("contract ok: %d checks\n", g_checks);
