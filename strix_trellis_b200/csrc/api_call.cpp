@@ -12,12 +12,17 @@ namespace {
 
 constexpr size_t kMaxStreams = 16;  // areas a context keeps (0.6 MB each on 148 SMs)
 
-// The calling stream's scratch area, made on first use; null when the context has none to give.
+// The calling stream's scratch area, made on first use; null when the context has none to give.  Areas
+// belong to streams, not to their handles: cudaStreamPerThread is another stream in every thread, and
+// the handle of a destroyed stream may come back for a new one while the old one's work still runs.
 cudaError_t stream_scratch(strix_context c, const st::DeviceWeights& w, cudaStream_t stream, void** out) {
     *out = nullptr;
+    unsigned long long id = 0;
+    const cudaError_t found = cudaStreamGetId(stream, &id);
+    if (found != cudaSuccess) return found;
     std::lock_guard<std::mutex> hold(c->scratch_lock);
     for (const auto& s : c->stream_scratch)
-        if (s.stream == stream) { *out = s.area; return cudaSuccess; }
+        if (s.stream_id == id) { *out = s.area; return cudaSuccess; }
     if (c->stream_scratch.size() >= kMaxStreams) return cudaSuccess;
     st::GemvPlan area = st::plan_gemv(w, 8, c->sm_count);
     area.partial_bytes = st::align_up((size_t)c->sm_count * 8 * 128 * sizeof(float));  // any layer, any row count
@@ -28,7 +33,7 @@ cudaError_t stream_scratch(strix_context c, const st::DeviceWeights& w, cudaStre
         if (e != cudaSuccess) (void)cudaFree(p);
     }
     if (e != cudaSuccess) return e;
-    c->stream_scratch.push_back({stream, p});
+    c->stream_scratch.push_back({id, p});
     *out = p;
     return cudaSuccess;
 }

@@ -19,7 +19,7 @@ struct strix_context_impl {
     bool programmatic_launch = true;
     // Scratch areas of immediate calls that bring no workspace (api_call.cpp), one per stream, every
     // word empty between launches; freed with the context.
-    struct StreamScratch { cudaStream_t stream; void* area; };
+    struct StreamScratch { unsigned long long stream_id; void* area; };
     std::vector<StreamScratch> stream_scratch;
     std::mutex scratch_lock;
 };

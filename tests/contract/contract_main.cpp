@@ -499,6 +499,22 @@ void linear_call_rules(strix_context c) {
     refused(STRIX_ERROR_INVALID_ARGUMENT);
     state().current_device = 0;
 
+    // One scratch area per stream, not per handle: a handle may stand for another stream in every thread
+    // (cudaStreamPerThread), or for a new one after the old was destroyed with work of its still running.
+    void* const handle = reinterpret_cast<void*>(uintptr_t(0x2));
+    state().streams[handle] = 0;
+    auto area_of = [&](unsigned long long id) {
+        state().stream_ids[handle] = id;
+        CHECK(call(STRIX_OPERATION_GEMV, nullptr, 0, handle) == STRIX_SUCCESS);
+        return record().last_workspace;
+    };
+    const void *first = area_of(1001), *second = area_of(1002);
+    CHECK(first != second && first != scratch && second != scratch);
+    CHECK(area_of(1001) == first && area_of(1002) == second);
+    CHECK(call(STRIX_OPERATION_GEMV, nullptr, 0) == STRIX_SUCCESS && record().last_workspace == scratch);
+    state().stream_ids.clear();
+    state().streams.erase(handle);
+
     CHECK(strix_weights_destroy(w) == STRIX_SUCCESS);
     CHECK(cudaFree(x) == cudaSuccess && cudaFree(y) == cudaSuccess && cudaFree(ws) == cudaSuccess);
 }

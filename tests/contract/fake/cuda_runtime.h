@@ -37,6 +37,8 @@ struct State {
     int sm_count = 148;
     // streams other than the null stream that exist, with their device
     std::map<void*, int> streams;
+    // identity of a handle's stream where it is not the handle's own value
+    std::map<void*, unsigned long long> stream_ids;
     // live device allocations
     std::map<uintptr_t, Block> blocks;
     // counters
@@ -65,6 +67,7 @@ cudaError_t cudaStreamSynchronize(cudaStream_t s);
 cudaError_t cudaDeviceSynchronize();
 cudaError_t cudaStreamGetDevice(cudaStream_t s, int* device);
 cudaError_t cudaStreamGetFlags(cudaStream_t s, unsigned int* flags);
+cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long* id);
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* status);
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* out, const void* p);
 cudaError_t cudaGetDriverEntryPoint(const char* symbol, void** fn, unsigned long long flags,

@@ -73,6 +73,11 @@ cudaError_t cudaStreamGetFlags(cudaStream_t s, unsigned int* flags) {
     *flags = 0;
     return cudaSuccess;
 }
+cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long* id) {
+    auto it = state().stream_ids.find(s);
+    *id = it != state().stream_ids.end() ? it->second : static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(s));
+    return cudaSuccess;
+}
 cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* status) {
     *status = state().capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
