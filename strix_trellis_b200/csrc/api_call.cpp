@@ -10,31 +10,22 @@ using namespace sapi;
 
 namespace {
 
-constexpr size_t kMaxStreams = 16;  // areas a context keeps (0.6 MB each on 148 SMs)
-
-// The calling stream's scratch area, made on first use; null when the context has none to give.  Areas
-// belong to streams, not to their handles: cudaStreamPerThread is another stream in every thread, and
-// the handle of a destroyed stream may come back for a new one while the old one's work still runs.
-cudaError_t stream_scratch(strix_context c, const st::DeviceWeights& w, cudaStream_t stream, void** out) {
+// The calling stream's scratch area; null when all are taken.  Areas belong to streams, not to their
+// handles: cudaStreamPerThread is another stream in every thread, and the handle of a destroyed
+// stream may come back for a new one while the old one's work still runs.  They are there, and empty,
+// since the context is: an allocation here would fail, and end the capture, while another thread
+// captures in global mode.
+cudaError_t stream_scratch(strix_context c, cudaStream_t stream, void** out) {
     *out = nullptr;
     unsigned long long id = 0;
     const cudaError_t found = cudaStreamGetId(stream, &id);
     if (found != cudaSuccess) return found;
     std::lock_guard<std::mutex> hold(c->scratch_lock);
-    for (const auto& s : c->stream_scratch)
-        if (s.stream_id == id) { *out = s.area; return cudaSuccess; }
-    if (c->stream_scratch.size() >= kMaxStreams) return cudaSuccess;
-    st::GemvPlan area = st::plan_gemv(w, 8, c->sm_count);
-    area.partial_bytes = st::align_up((size_t)c->sm_count * 8 * 128 * sizeof(float));  // any layer, any row count
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, area.partial_bytes);
-    if (e == cudaSuccess) {
-        e = st::reset_gemv_scratch(p, area, stream);
-        if (e != cudaSuccess) (void)cudaFree(p);
-    }
-    if (e != cudaSuccess) return e;
-    c->stream_scratch.push_back({id, p});
-    *out = p;
+    size_t at = 0;
+    while (at < c->scratch_used && c->scratch_streams[at] != id) ++at;
+    if (at == kScratchStreams) return cudaSuccess;
+    if (at == c->scratch_used) c->scratch_streams[c->scratch_used++] = id;
+    *out = c->scratch + at * scratch_area_bytes(c);
     return cudaSuccess;
 }
 
@@ -96,7 +87,7 @@ extern "C" strix_status strix_b200_linear_call(strix_context c, strix_weights w,
     cudaError_t e = cudaStreamIsCapturing(cs, &capturing);
     if (e != cudaSuccess) return cuda_status(e);
     void* scratch = nullptr;
-    if (capturing == cudaStreamCaptureStatusNone) e = stream_scratch(c, w->device, cs, &scratch);
+    if (capturing == cudaStreamCaptureStatusNone) e = stream_scratch(c, cs, &scratch);
     if (e != cudaSuccess) return cuda_status(e);
     if (!scratch) return STRIX_ERROR_INSUFFICIENT_BUFFER;
     return cuda_status(st::launch_gemv(make_call(c, d, v), st::plan_gemv(w->device, v.rows, c->sm_count), scratch,

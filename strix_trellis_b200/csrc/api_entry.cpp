@@ -280,8 +280,13 @@ strix_status strix_context_create(const strix_context_desc* d, strix_context* ou
     c->sm_count = sms;
     e = cudaMalloc(reinterpret_cast<void**>(&c->status), kAlign);
     if (e == cudaSuccess) e = cudaMemset(c->status, 0, kAlign);
+    const size_t scratch_bytes = kScratchStreams * scratch_area_bytes(c);
+    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&c->scratch), scratch_bytes);
+    if (e == cudaSuccess) e = cudaMemset(c->scratch, 0xFF, scratch_bytes);  // every word empty
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // before any stream's launches
     if (e != cudaSuccess) {
-        if (c->status) (void)cudaFree(c->status);
+        (void)cudaFree(c->scratch);
+        (void)cudaFree(c->status);
         delete c;
         return cuda_status(e);
     }
@@ -291,7 +296,7 @@ strix_status strix_context_create(const strix_context_desc* d, strix_context* ou
 
 strix_status strix_context_destroy(strix_context c) {
     if (!c || c->weights_count) return STRIX_ERROR_INVALID_ARGUMENT;
-    for (const auto& s : c->stream_scratch) (void)cudaFree(s.area);
+    (void)cudaFree(c->scratch);
     (void)cudaFree(c->status);
     delete c;
     return STRIX_SUCCESS;

@@ -11,16 +11,20 @@
 #include "strix_trellis.h"
 #include "strix_trellis_b200.h"
 
+constexpr size_t kScratchStreams = 16;
+
 struct strix_context_impl {
     int device = 0;
     int sm_count = 148;
     size_t weights_count = 0;
     unsigned int* status = nullptr;  // device word: bounded-wait failures of any kernel
     bool programmatic_launch = true;
-    // Scratch areas of immediate calls that bring no workspace (api_call.cpp), one per stream, every
-    // word empty between launches; freed with the context.
-    struct StreamScratch { unsigned long long stream_id; void* area; };
-    std::vector<StreamScratch> stream_scratch;
+    // Scratch areas of immediate calls that bring no workspace (api_call.cpp), kScratchStreams of them side
+    // by side, every word empty between launches: area i belongs to the stream with identity
+    // scratch_streams[i].  Made and freed with the context.
+    unsigned char* scratch = nullptr;
+    unsigned long long scratch_streams[kScratchStreams] = {};
+    size_t scratch_used = 0;
     std::mutex scratch_lock;
 };
 
@@ -40,6 +44,8 @@ struct strix_weights_impl {
 namespace sapi {
 
 constexpr uint64_t kAlign = STRIX_TRELLIS_WORKSPACE_ALIGNMENT;
+// One plane of every CTA and row: any layer, up to eight rows (0.6 MB on 148 SMs).
+inline size_t scratch_area_bytes(strix_context c) { return st::align_up((size_t)c->sm_count * 8 * 128 * sizeof(float)); }
 
 // ---- small vocabulary of the validation code ---------------------------------------------
 // An enum field of a descriptor is whatever 32 bits the caller stored there; it is compared as

@@ -94,6 +94,8 @@ void context_rules() {
     // a failed status-word allocation leaves nothing behind
     state().alloc_failure_at = state().allocs;
     CHECK(strix_context_create(&cd, &c) == STRIX_ERROR_OUT_OF_MEMORY && !c && state().blocks.empty());
+    state().alloc_failure_at = state().allocs + 1;  // nor does the scratch of immediate calls
+    CHECK(strix_context_create(&cd, &c) == STRIX_ERROR_OUT_OF_MEMORY && !c && state().blocks.empty());
     state().alloc_failure_at = -1;
 
     // one process, two devices: each context sets up the kernels of ITS device
@@ -508,7 +510,14 @@ void linear_call_rules(strix_context c) {
         CHECK(call(STRIX_OPERATION_GEMV, nullptr, 0, handle) == STRIX_SUCCESS);
         return record().last_workspace;
     };
+    // The first call on a stream allocates, sets and waits for nothing: another thread may be capturing,
+    // and each of these would fail in it and end that capture.
+    const Counts b = Counts::now();
+    const int resets = record().scratch_resets;
     const void *first = area_of(1001), *second = area_of(1002);
+    CHECK(Counts::now().same_traffic(b) && record().scratch_resets == resets);
+    const auto* word = static_cast<const uint32_t*>(second);  // and finds every word empty
+    CHECK(word[0] == 0xFFFFFFFF && word[static_cast<size_t>(state().sm_count) * 8 * 128 - 1] == 0xFFFFFFFF);
     CHECK(first != second && first != scratch && second != scratch);
     CHECK(area_of(1001) == first && area_of(1002) == second);
     CHECK(call(STRIX_OPERATION_GEMV, nullptr, 0) == STRIX_SUCCESS && record().last_workspace == scratch);
