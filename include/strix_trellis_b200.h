@@ -77,7 +77,9 @@ strix_status strix_b200_gemv_partition(uint64_t inputs, uint64_t outputs, uint32
  * drain at exit, bit 3 tensor pipeline, bit 4 split-K fold, bit 5 a peer exchange that never
  * completed); results of that launch are invalid,
  * and after bit 4 the plan whose launch it was should be recreated (its fold scratch may hold
- * words of the abandoned launch; direct strix_gemv calls reset their scratch on every call).
+ * words of the abandoned launch; direct strix_gemv calls reset their scratch on every call, and
+ * this call resets the scratch that strix_b200_linear_call uses; until then the results of
+ * strix_b200_linear_call on the stream of the failed one are invalid too).
  * Synchronises the device.  No counterpart in the reference (its kernels never wait). */
 strix_status strix_b200_device_status(strix_context context, uint32_t *out_bits);
 

@@ -14,13 +14,13 @@ namespace {
 // handles: cudaStreamPerThread is another stream in every thread, and the handle of a destroyed
 // stream may come back for a new one while the old one's work still runs.  They are there, and empty,
 // since the context is: an allocation here would fail, and end the capture, while another thread
-// captures in global mode.
+// captures in global mode.  The caller holds scratch_lock, and holds it until its launch is enqueued:
+// strix_b200_device_status empties the areas between two launches.
 cudaError_t stream_scratch(strix_context c, cudaStream_t stream, void** out) {
     *out = nullptr;
     unsigned long long id = 0;
     const cudaError_t found = cudaStreamGetId(stream, &id);
     if (found != cudaSuccess) return found;
-    std::lock_guard<std::mutex> hold(c->scratch_lock);
     size_t at = 0;
     while (at < c->scratch_used && c->scratch_streams[at] != id) ++at;
     if (at == kScratchStreams) return cudaSuccess;
@@ -87,6 +87,7 @@ extern "C" strix_status strix_b200_linear_call(strix_context c, strix_weights w,
     cudaError_t e = cudaStreamIsCapturing(cs, &capturing);
     if (e != cudaSuccess) return cuda_status(e);
     void* scratch = nullptr;
+    std::lock_guard<std::mutex> hold(c->scratch_lock);
     if (capturing == cudaStreamCaptureStatusNone) e = stream_scratch(c, cs, &scratch);
     if (e != cudaSuccess) return cuda_status(e);
     if (!scratch) return STRIX_ERROR_INSUFFICIENT_BUFFER;

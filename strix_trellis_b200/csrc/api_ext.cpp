@@ -189,9 +189,13 @@ strix_status strix_b200_device_status(strix_context c, uint32_t* out_bits) {
     *out_bits = 0;
     const strix_status s = context_check(c);
     if (s != STRIX_SUCCESS) return s;
+    std::lock_guard<std::mutex> hold(c->scratch_lock);  // no immediate call between the wait and the end
     cudaError_t e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = cudaMemcpy(out_bits, c->status, sizeof(uint32_t), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemset(c->status, 0, sizeof(uint32_t));
+    // A launch that gave up may have left words in its scratch that every later call would add.
+    if (e == cudaSuccess && *out_bits) e = cudaMemset(c->scratch, 0xFF, kScratchStreams * scratch_area_bytes(c));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // the streams' next launches find both done
     return cuda_status(e);
 }
 

@@ -521,6 +521,15 @@ void linear_call_rules(strix_context c) {
     CHECK(first != second && first != scratch && second != scratch);
     CHECK(area_of(1001) == first && area_of(1002) == second);
     CHECK(call(STRIX_OPERATION_GEMV, nullptr, 0) == STRIX_SUCCESS && record().last_workspace == scratch);
+    // A launch that gave up may leave words in its area, and every later call would add them.  The failure
+    // is reported once, and from then on the areas are empty again.
+    uint32_t bits = 0;
+    static_cast<uint32_t*>(const_cast<void*>(second))[5] = 0x3F800000;
+    CHECK(strix_b200_device_status(c, &bits) == STRIX_SUCCESS && bits == 0 && word[5] == 0x3F800000);  // in use, for all it knows
+    *c->status = 16;
+    CHECK(strix_b200_device_status(c, &bits) == STRIX_SUCCESS && bits == 16 && word[5] == 0xFFFFFFFF);
+    CHECK(strix_b200_device_status(c, &bits) == STRIX_SUCCESS && bits == 0);
+    CHECK(area_of(1002) == second);
     state().stream_ids.clear();
     state().streams.erase(handle);
 
