@@ -266,7 +266,8 @@ strix_status strix_b200_gemv_noalloc(strix_context context, const strix_matmul_d
  * one device allocation.  `stream` is the stream handle itself.
  * With a workspace the call is strix_gemv / strix_gemm.  Without one (NULL/0) a call of up to eight
  * rows uses a scratch area that the context keeps for the stream (sixteen of 0.6 MB are made and freed
- * with the context, and assigned to streams in the order of their first such calls); where there is none to use -- more rows, a stream that is being captured,
+ * with the context, assigned to streams in the order of their first such calls and given back to all by
+ * strix_b200_device_status, which waits for everything in flight); where there is none to use -- more rows, a stream that is being captured,
  * more streams than the context keeps areas for -- it returns STRIX_ERROR_INSUFFICIENT_BUFFER with
  * nothing enqueued, and the caller brings a workspace. */
 typedef struct strix_b200_tensor {

@@ -196,6 +196,7 @@ strix_status strix_b200_device_status(strix_context c, uint32_t* out_bits) {
     // A launch that gave up may have left words in its scratch that every later call would add.
     if (e == cudaSuccess && *out_bits) e = cudaMemset(c->scratch, 0xFF, kScratchStreams * scratch_area_bytes(c));
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // the streams' next launches find both done
+    if (e == cudaSuccess) c->scratch_used = 0;  // nothing is in flight: the areas are anyone's again
     return cuda_status(e);
 }
 

@@ -35,6 +35,7 @@ class Context:
         desc.device_ordinal = self.device
         self.handle = N.vp()
         N.check(self.lib.strix_context_create(C.byref(desc), C.byref(self.handle)), "strix_context_create")
+        self._no_scratch = set()  # stream handles that the library had no scratch area for
 
     def close(self):
         if self.handle:
@@ -44,6 +45,7 @@ class Context:
     def device_status(self):
         bits = N.u32()
         N.check(self.lib.strix_b200_device_status(self.handle, C.byref(bits)), "strix_b200_device_status")
+        self._no_scratch.clear()  # the areas were given back
         return bits.value
 
     def set_programmatic_launch(self, enabled):
@@ -196,11 +198,16 @@ class Weights:
                     need = self.workspace_bytes(x, y)
                     if len(self._needs) < 64:
                         self._needs[x.shape[0]] = need
+            if not need and handle in self.ctx._no_scratch:
+                need = self.workspace_bytes(x, y)
             if not need:
                 status = call(self.ctx.handle, self.handle, operation, xt, yt, alpha, beta, None, 0, handle)
                 if status != N.INSUFFICIENT_BUFFER:
                     return N.check(status, where)
                 need = self.workspace_bytes(x, y)
+                # A hint only: the handle may stand for another stream one day, which then brings its own.
+                if need and len(self.ctx._no_scratch) < 4096 and not torch.cuda.is_current_stream_capturing():
+                    self.ctx._no_scratch.add(handle)
             workspace = torch.empty(max(need, 1), dtype=torch.uint8, device=x.device)
         size = workspace.numel() * workspace.element_size()
         N.check(call(self.ctx.handle, self.handle, operation, xt, yt, alpha, beta, workspace.data_ptr() if size else None, size,

@@ -6,6 +6,7 @@
 // cleared on failure, leak-free failure of every step of weight preparation, plans that
 // freeze their descriptor and submit with no query of any kind, lifetime rules, and the
 // per-device kernel set-up at context creation.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -529,7 +530,17 @@ void linear_call_rules(strix_context c) {
     *c->status = 16;
     CHECK(strix_b200_device_status(c, &bits) == STRIX_SUCCESS && bits == 16 && word[5] == 0xFFFFFFFF);
     CHECK(strix_b200_device_status(c, &bits) == STRIX_SUCCESS && bits == 0);
-    CHECK(area_of(1002) == second);
+    // Sixteen streams have areas.  The next one is told to bring a workspace, until the areas are given back:
+    // strix_b200_device_status waits for everything in flight anyway.
+    std::vector<const void*> areas;
+    for (unsigned long long id = 0; id < 16; ++id) areas.push_back(area_of(2000 + id));
+    std::sort(areas.begin(), areas.end());
+    CHECK(std::unique(areas.begin(), areas.end()) == areas.end());
+    state().stream_ids[handle] = 2016;
+    refused(STRIX_ERROR_INSUFFICIENT_BUFFER, STRIX_OPERATION_GEMV, nullptr, 0, handle);
+    CHECK(call(STRIX_OPERATION_GEMV, ws, 32768, handle) == STRIX_SUCCESS);
+    CHECK(strix_b200_device_status(c, &bits) == STRIX_SUCCESS && bits == 0);
+    CHECK(std::binary_search(areas.begin(), areas.end(), area_of(2016)));
     state().stream_ids.clear();
     state().streams.erase(handle);
 

@@ -169,3 +169,45 @@ def test_immediate_calls_share_scratch_between_shapes(ctx):
         gate(host(y), want, "immediate")
     for w, *_ in cases:
         w.close()
+
+
+def test_immediate_calls_on_more_streams_than_have_scratch(ctx):
+    """Streams beyond those that the context keeps scratch for: right results, and one refused C call per
+    stream, not one per call, until the areas are given back."""
+    layer = synthetic.make_layer(1152, 640, 4, seed=9400)
+    w = ctx.prepare(layer)
+    x = dev(synthetic.make_activations(2, 1152, seed=9401))
+    want = c_oracle.linear(layer.trellis, layer.suh, layer.svh, None, 4, 2, host(x))
+
+    class Counted:
+        calls = 0
+
+        def __getattr__(self, name):
+            return getattr(ctx.lib, name)
+
+        def strix_b200_linear_call(self, *args):
+            self.calls += 1
+            return ctx.lib.strix_b200_linear_call(*args)
+
+    w.lib = counted = Counted()
+    ctx.device_status()
+    streams = [torch.cuda.Stream() for _ in range(20)]
+    torch.cuda.synchronize()
+
+    def turn():
+        before = counted.calls
+        for s in streams:
+            with torch.cuda.stream(s):
+                results.append(w.gemv(x))
+        return counted.calls - before
+
+    results = []
+    assert turn() == 24 and turn() == 20 and turn() == 20
+    assert ctx.device_status() == 0
+    streams.reverse()
+    assert turn() == 24
+    torch.cuda.synchronize()
+    for y in results:
+        gate(host(y), want, "many streams")
+    ctx.device_status()
+    w.close()
