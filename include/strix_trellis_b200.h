@@ -280,6 +280,18 @@ strix_status strix_b200_linear_call(strix_context context, strix_weights weights
                                     float alpha, float beta, void *workspace, uint64_t workspace_bytes,
                                     void *stream);
 
+/* strix_linear_plan_submit of a plan of more than eight rows on another workspace than its own, which
+ * may be gone: 256-byte aligned device memory of at least strix_matmul_workspace_bytes, apart from
+ * the plan's tensors and weights, whatever its content.  It is the call's until the launches are
+ * done.  Such a workspace may hold the layer's decoded weights (up to 256 MB), so a program with a
+ * plan per layer shares one among the plans of a stream.  Like submit it makes no query and can be
+ * captured.  Plans of one to eight rows return STRIX_ERROR_UNSUPPORTED_FORMAT: their workspace has
+ * state. */
+strix_status strix_b200_linear_plan_submit_with(strix_linear_plan plan, void *workspace,
+                                                uint64_t workspace_bytes);
+/* The identity of the capture that the plan's stream takes part in, 0 when it is not captured. */
+strix_status strix_b200_linear_plan_capture_id(strix_linear_plan plan, uint64_t *out_id);
+
 #ifdef __cplusplus
 }
 #endif

@@ -10,6 +10,8 @@ struct strix_linear_plan_impl {
     st::LinearCall call;
     cudaStream_t stream;
     int rows;
+    View view;
+    uint64_t workspace_bytes;  // what a submit needs
 };
 
 namespace {
@@ -396,7 +398,7 @@ strix_status strix_linear_plan_create(strix_context c, const strix_matmul_desc* 
     s = storage_check(c, *d, v, needed, d->workspace, d->workspace_bytes);
     if (s != STRIX_SUCCESS) return s;
     if (d->weights->plan_refs == SIZE_MAX) return STRIX_ERROR_OUT_OF_MEMORY;
-    strix_linear_plan_impl* p = new (std::nothrow) strix_linear_plan_impl{c, *d, make_call(c, *d, v), cs, v.rows};
+    strix_linear_plan_impl* p = new (std::nothrow) strix_linear_plan_impl{c, *d, make_call(c, *d, v), cs, v.rows, v, needed};
     if (!p) return STRIX_ERROR_OUT_OF_MEMORY;
     if (v.rows && v.rows <= 8) {
         // The fold scratch starts empty and every launch leaves it empty, so submit is a
@@ -416,6 +418,35 @@ strix_status strix_linear_plan_submit(strix_linear_plan p) {
     const strix_status s = context_check(p->owner);
     if (s != STRIX_SUCCESS || !p->rows) return s;
     return cuda_status(enqueue_linear(p->owner, p->call, p->desc.workspace, false, p->stream));
+}
+
+strix_status strix_b200_linear_plan_submit_with(strix_linear_plan p, void* workspace, uint64_t bytes) {
+    if (!p) return STRIX_ERROR_INVALID_ARGUMENT;
+    const strix_status s = context_check(p->owner);
+    if (s != STRIX_SUCCESS) return s;
+    if (p->rows && p->rows <= 8) return STRIX_ERROR_UNSUPPORTED_FORMAT;  // its planes were marked empty at creation
+    if (bytes < p->workspace_bytes) return STRIX_ERROR_INSUFFICIENT_BUFFER;
+    const strix_weights_impl* w = p->desc.weights;
+    if (!range_ok(workspace, bytes) || (bytes && (!workspace || reinterpret_cast<uintptr_t>(workspace) % kAlign)) ||
+        overlap(workspace, bytes, p->desc.input.data, p->view.x_bytes) ||
+        overlap(workspace, bytes, p->desc.output.data, p->view.y_bytes) ||
+        overlap(workspace, bytes, w->allocation, w->allocation_bytes))
+        return STRIX_ERROR_INVALID_ARGUMENT;
+    if (!p->rows) return STRIX_SUCCESS;
+    return cuda_status(enqueue_linear(p->owner, p->call, workspace, false, p->stream));
+}
+
+strix_status strix_b200_linear_plan_capture_id(strix_linear_plan p, uint64_t* out) {
+    if (!out) return STRIX_ERROR_INVALID_ARGUMENT;
+    *out = 0;
+    if (!p) return STRIX_ERROR_INVALID_ARGUMENT;
+    const strix_status s = context_check(p->owner);
+    if (s != STRIX_SUCCESS) return s;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    const cudaError_t e = cudaStreamGetCaptureInfo(p->stream, &capturing, &id);
+    if (e == cudaSuccess && capturing == cudaStreamCaptureStatusActive) *out = id;
+    return cuda_status(e);
 }
 
 strix_status strix_linear_plan_destroy(strix_linear_plan p) {

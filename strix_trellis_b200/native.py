@@ -244,6 +244,8 @@ PROTOTYPES = {
     "strix_b200_device_status": (C.c_int, [vp, P(u32)]),
     "strix_b200_set_programmatic_launch": (C.c_int, [vp, u32]),
     "strix_b200_gemv_noalloc": (C.c_int, [vp, P(MatmulDesc), P(Stream)]),
+    "strix_b200_linear_plan_submit_with": (C.c_int, [vp, vp, u64]),
+    "strix_b200_linear_plan_capture_id": (C.c_int, [vp, P(u64)]),
     "strix_b200_linear_call": (C.c_int, [vp, vp, u32, P(Tensor), P(Tensor), f32, f32, vp, u64, vp]),
 }
 

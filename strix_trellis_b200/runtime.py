@@ -2,6 +2,7 @@
 memory (data_ptr) and of the current CUDA stream; all arithmetic happens inside
 libstrix_trellis.so."""
 import ctypes as C
+import weakref
 
 import numpy as np
 import torch
@@ -35,6 +36,7 @@ class Context:
         desc.device_ordinal = self.device
         self.handle = N.vp()
         N.check(self.lib.strix_context_create(C.byref(desc), C.byref(self.handle)), "strix_context_create")
+        self._capture_workspaces = weakref.WeakValueDictionary()  # of plans, by capture and stream
         self._no_scratch = set()  # stream handles that the library had no scratch area for
 
     def close(self):
@@ -168,10 +170,6 @@ class Weights:
         N.check(self.lib.strix_matmul_workspace_bytes(self.ctx.handle, C.byref(d), C.byref(out)), "workspace_bytes")
         return out.value
 
-    def _workspace(self, x, y):
-        n = self.workspace_bytes(x, y)
-        return torch.empty(max(n, 1), dtype=torch.uint8, device=x.device) if n else None
-
     def _call(self, operation, where, x, y, alpha, beta, workspace, stream):
         """One immediate call.  Without a workspace the library's scratch of this stream serves a GEMV;
         where it has none (many rows, graph capture) the call is repeated with a workspace of its own."""
@@ -281,22 +279,59 @@ class Weights:
         return out.value
 
 
+# A plan of more than eight rows without a workspace of the caller's owns one of up to this many bytes and
+# borrows a larger one for each submit.  Larger ones hold decoded weights (512 rows of 4096 -> 12288: 104 MB), and
+# a program has a prefill plan per layer.  Borrowing takes 7 us of host time, which the launches of such calls hide
+# (at least 50 us); smaller workspaces hold the planes of one launch (101 rows of 4096 -> 12288: 9 MB, 30 us).
+_OWN_WORKSPACE = 16 << 20
+
+
 class LinearPlan:
-    """strix_linear_plan: validated once, submitted many times (graph-capturable)."""
+    """strix_linear_plan: validated once, submitted many times (graph-capturable).  Large workspaces are
+    not the plan's own: outside a capture a submit takes one from torch's allocator on the plan's stream and gives
+    it back at once; the plans captured on one stream of one capture share one for as long as a plan of theirs lives."""
 
     def __init__(self, weights, x, y, operation, alpha, beta, workspace, stream):
         self.weights, self.lib = weights, weights.lib
+        self.borrows, self.captured = 0, None
         if workspace is None:
-            workspace = weights._workspace(x, y)
-        self.keep = (x, y, workspace)
+            need = weights.workspace_bytes(x, y)
+            if need:
+                workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
+            if need > _OWN_WORKSPACE and x.dim() == 2 and x.shape[0] > 8:
+                self.borrows = need
+        self.keep = (x, y) if self.borrows else (x, y, workspace)
         d = weights.matmul_desc(x, y, alpha, beta, workspace)
         sd = _cur_stream(stream)
         self.handle = N.vp()
         N.check(self.lib.strix_linear_plan_create(weights.ctx.handle, C.byref(d), C.byref(sd), operation,
                                                   C.byref(self.handle)), "strix_linear_plan_create")
+        self.stream, self.device = sd.hip_stream or 0, x.device
 
     def submit(self):
+        if self.borrows:
+            if torch.cuda.current_stream(self.device).cuda_stream == self.stream:
+                return self._submit_borrowed()
+            with torch.cuda.stream(torch.cuda.ExternalStream(self.stream, self.device)):
+                return self._submit_borrowed()
         N.check(self.lib.strix_linear_plan_submit(self.handle), "strix_linear_plan_submit")
+
+    def _submit_borrowed(self):
+        if torch.cuda.is_current_stream_capturing():  # the plan's stream, here
+            # Replays use the same memory again: it stays the plans', not the allocator's.  Launches of one
+            # capture on one stream are ordered, and a plan that is captured again keeps its workspace.
+            if self.captured is None:
+                capture = N.u64()
+                N.check(self.lib.strix_b200_linear_plan_capture_id(self.handle, C.byref(capture)), "capture_id")
+                shared, key = self.weights.ctx._capture_workspaces, (capture.value, self.stream)
+                self.captured = shared.get(key)
+                if self.captured is None or self.captured.numel() < self.borrows:
+                    self.captured = shared[key] = torch.empty(self.borrows, dtype=torch.uint8, device=self.device)
+            workspace = self.captured
+        else:
+            workspace = torch.empty(self.borrows, dtype=torch.uint8, device=self.device)
+        N.check(self.lib.strix_b200_linear_plan_submit_with(self.handle, workspace.data_ptr(), self.borrows),
+                "strix_linear_plan_submit")
 
     def close(self):
         if self.handle:

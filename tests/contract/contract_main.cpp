@@ -430,6 +430,62 @@ void call_and_plan_rules(strix_context c) {
     CHECK(cudaFree(x) == cudaSuccess && cudaFree(y) == cudaSuccess && cudaFree(ws) == cudaSuccess);
 }
 
+// strix_b200_linear_plan_submit_with: a plan of more than eight rows on a workspace of the moment.
+void plan_workspace_rules(strix_context c) {
+    HostLayer layer;
+    auto stream = blank<strix_stream>();
+    auto parts = layer.parts();
+    strix_weights w = nullptr;
+    CHECK(strix_weights_prepare_parts(c, &parts, &stream, &w) == STRIX_SUCCESS);
+    void *x = nullptr, *y = nullptr, *ws = nullptr;
+    CHECK(cudaMalloc(&x, 16384) == cudaSuccess && cudaMalloc(&y, 16384) == cudaSuccess && cudaMalloc(&ws, 32768) == cudaSuccess);
+    strix_matmul_desc d;
+    strix_matmul_desc_init(&d);
+    d.weights = w;
+    d.input.rank = d.output.rank = 2;
+    d.input.shape[0] = d.output.shape[0] = 16;
+    d.input.shape[1] = d.input.strides[0] = 128;
+    d.output.shape[1] = d.output.strides[0] = 256;
+    d.input.strides[1] = d.output.strides[1] = 1;
+    d.input.data = x; d.output.data = y;
+    d.input.buffer_bytes = d.output.buffer_bytes = 16384;
+    d.workspace = ws; d.workspace_bytes = 32768;
+    uint64_t need = 0, id = 9;
+    CHECK(strix_matmul_workspace_bytes(c, &d, &need) == STRIX_SUCCESS && need && need <= 16384);
+    strix_linear_plan plan = nullptr, small = nullptr;
+    CHECK(strix_linear_plan_create(c, &d, &stream, STRIX_OPERATION_GEMM, &plan) == STRIX_SUCCESS);
+    d.input.shape[0] = d.output.shape[0] = 8;
+    CHECK(strix_linear_plan_create(c, &d, &stream, STRIX_OPERATION_GEMM, &small) == STRIX_SUCCESS);
+
+    void* other = static_cast<char*>(ws) + 16384;
+    const Counts b = Counts::now();
+    CHECK(strix_b200_linear_plan_submit_with(plan, other, need) == STRIX_SUCCESS);
+    CHECK(record().last_workspace == other && record().last_was_gemm && record().last.rows == 16);
+    CHECK(strix_linear_plan_submit(plan) == STRIX_SUCCESS && record().last_workspace == ws);
+    CHECK(Counts::now().same_traffic(b) && Counts::now().same_queries(b) && record().launches == b.launches + 2);
+    CHECK(strix_b200_linear_plan_submit_with(nullptr, other, need) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_plan_submit_with(plan, other, need - 1) == STRIX_ERROR_INSUFFICIENT_BUFFER);
+    CHECK(strix_b200_linear_plan_submit_with(plan, nullptr, need) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_plan_submit_with(plan, static_cast<char*>(ws) + 16, need) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_plan_submit_with(plan, x, need) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_plan_submit_with(plan, y, need) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_plan_submit_with(plan, w->allocation, need) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_plan_submit_with(small, other, 16384) == STRIX_ERROR_UNSUPPORTED_FORMAT);  // its planes have state
+    state().current_device = 1;
+    CHECK(strix_b200_linear_plan_submit_with(plan, other, need) == STRIX_ERROR_INVALID_ARGUMENT);
+    state().current_device = 0;
+    CHECK(record().launches == b.launches + 2);
+    CHECK(strix_b200_linear_plan_capture_id(plan, nullptr) == STRIX_ERROR_INVALID_ARGUMENT);
+    CHECK(strix_b200_linear_plan_capture_id(nullptr, &id) == STRIX_ERROR_INVALID_ARGUMENT && id == 0);
+    CHECK(strix_b200_linear_plan_capture_id(plan, &id) == STRIX_SUCCESS && id == 0);
+    state().capturing = true;
+    CHECK(strix_b200_linear_plan_capture_id(plan, &id) == STRIX_SUCCESS && id == 77);
+    state().capturing = false;
+    CHECK(strix_linear_plan_destroy(plan) == STRIX_SUCCESS && strix_linear_plan_destroy(small) == STRIX_SUCCESS);
+    CHECK(strix_weights_destroy(w) == STRIX_SUCCESS);
+    CHECK(cudaFree(x) == cudaSuccess && cudaFree(y) == cudaSuccess && cudaFree(ws) == cudaSuccess);
+}
+
 // strix_b200_linear_call: the rules of strix_gemv / strix_gemm from plain arguments.
 void linear_call_rules(strix_context c) {
     HostLayer layer;
@@ -562,6 +618,7 @@ int main() {
     CHECK(strix_context_create(&cd, &c) == STRIX_SUCCESS);
     prepare_rules(c);
     call_and_plan_rules(c);
+    plan_workspace_rules(c);
     linear_call_rules(c);
     CHECK(strix_context_destroy(c) == STRIX_SUCCESS);
     CHECK(state().blocks.empty());  // everything the library allocated was returned

@@ -69,6 +69,7 @@ cudaError_t cudaStreamGetDevice(cudaStream_t s, int* device);
 cudaError_t cudaStreamGetFlags(cudaStream_t s, unsigned int* flags);
 cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long* id);
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* status);
+cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus* status, unsigned long long* id);
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* out, const void* p);
 cudaError_t cudaGetDriverEntryPoint(const char* symbol, void** fn, unsigned long long flags,
                                     cudaDriverEntryPointQueryResult* result);

@@ -82,6 +82,10 @@ cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* status)
     *status = state().capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
 }
+cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus* status, unsigned long long* id) {
+    *id = state().capturing ? 77 : 0;
+    return cudaStreamIsCapturing(s, status);
+}
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* out, const void* p) {
     ++state().pointer_queries;
     *out = cudaPointerAttributes{};

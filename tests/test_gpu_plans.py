@@ -259,3 +259,62 @@ def test_weights_from_container_slices(ctx, tmp_path):
                                        np.asarray(part.svh), bias, 4, 2, xs)
                 gate(got, want, f"{axis} shard {rank}")
                 w.close()
+
+
+def test_prefill_plans_do_not_each_hold_a_workspace():
+    """A plan per layer of 512 rows: the decoded weights (32 MB a layer) are in a workspace that each submit
+    borrows; captured plans share one per capture, apart from every other allocation."""
+    from strix_trellis_b200.runtime import Context
+    ctx = Context(0)
+    rows, inputs, outputs = 512, 4096, 4096
+    ws = [ctx.prepare(synthetic.make_layer(inputs, outputs, 2, seed=9500 + k)) for k in range(4)]
+    x = torch.from_numpy(synthetic.make_activations(rows, inputs, seed=9510)).cuda()
+    want = [w.gemm(x) for w in ws]
+    ys = [torch.empty_like(want[0]) for _ in ws]
+    need = ws[0].workspace_bytes(x, ys[0])
+    assert need > 32 << 20  # this call's weights are decoded first
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    side = torch.cuda.Stream()
+    plans = [w.plan(x, y, N.OP_GEMM, stream=s) for w, y, s in zip(ws, ys, (None, side, None, side))]
+    assert torch.cuda.memory_allocated() == before
+
+    def check(what):
+        torch.cuda.synchronize()
+        for k, (y, r) in enumerate(zip(ys, want)):
+            assert torch.equal(y, r), (what, k)
+            y.zero_()
+        torch.cuda.synchronize()
+
+    for plan in plans:  # two streams at the same time, neither of them current for half of the plans
+        plan.submit()
+    assert torch.cuda.memory_allocated() == before
+    check("submit")
+    with torch.cuda.stream(side):
+        for plan in plans:
+            plan.submit()
+    check("submit from the other stream")
+
+    graphs = []
+    for _ in range(2):
+        with torch.cuda.stream(side):
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=side):
+                plans[1].submit()
+                plans[3].submit()
+        graphs.append(g)
+    assert plans[1].captured is plans[3].captured
+    noise = [torch.full((need // 4,), 7.0, device="cuda") for _ in range(4)]  # where a workspace given back would be
+    for g in graphs:
+        g.replay()
+        plans[0].submit()
+        plans[2].submit()
+        check("replay")
+    assert all(bool((n == 7.0).all()) for n in noise)
+    del graphs, g
+    for plan in plans:
+        plan.close()
+    for w in ws:
+        w.close()
+    assert ctx.device_status() == 0
+    ctx.close()
