@@ -123,39 +123,29 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_row_kernel(const GemvArgs ar
     uint2* act = reinterpret_cast<uint2*>(ring + (size_t)stages * kStage);
 
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + stages);
-    // The producer sets up its ring and asks for the first units at once: weights are immutable, so
-    // this waits for nothing.  Only kFirstUnits of them: all CTAs start together, and a whole ring
-    // requested at once (19 MB over the chip) would put 3 us of other units before a CTA's first.
-    constexpr int kFirstUnits = 2;
-    auto load_unit = [&](int unit, int slot) {
-        mbar_expect_tx(full0 + 8 * slot, kStage);
-        bulk_load(smem_u32(ring) + slot * kStage,
-                  reinterpret_cast<const unsigned char*>(c.w.packed) + (size_t)(mine.begin + unit) * kStage, kStage, full0 + 8 * slot);
-    };
-    const int first = stages < kFirstUnits ? stages : kFirstUnits;
-    if (warp == kConsumers) {
-        if (lane < stages) {
-            mbar_init(full0 + 8 * lane, 1);
-            mbar_init(empty0 + 8 * lane, 8);
-            mbar_fence_init();
-        }
-        __syncwarp();
-        if (lane == 0)
-            for (int i = 0; i < first && i < my_units; ++i) load_unit(i, i);
+    // By the producer's lanes, one per ring slot.  Measured for a sweep of 96 launches and for the same sweep as
+    // two chains on two streams: 864 / 758 us so; by a decode warp 892 / 781; with the CTA's first two units
+    // asked for here, before the barrier, 885 / 790.
+    if (warp == kConsumers && lane < stages) {
+        mbar_init(full0 + 8 * lane, 1);
+        mbar_init(empty0 + 8 * lane, 8);
+        mbar_fence_init();
     }
     if (threadIdx.x == 0) *gave_up = 0;
     __syncthreads();
     pdl_launch_dependents();
 
     if (warp == kConsumers) {
-        // ---- producer: the other units ----
+        // ---- producer: weights are immutable, so this needs no wait on the launch before ----
         if (lane == 0) {
-            int issued = my_units < first ? my_units : first;
-            int st = issued == stages ? 0 : issued;
-            uint32_t prev_use = issued == stages ? 0 : 1;
+            int issued = 0;
+            int st = 0;  // ring slot of the next unit and the parity of its previous use, stepped without divisions
+            uint32_t prev_use = 1;
             for (; issued < my_units; ++issued) {
                 if (issued >= stages && !mbar_wait(empty0 + 8 * st, prev_use, c.status, kTimeoutRingEmpty)) break;
-                load_unit(issued, st);
+                mbar_expect_tx(full0 + 8 * st, kStage);
+                bulk_load(smem_u32(ring) + st * kStage,
+                          reinterpret_cast<const unsigned char*>(c.w.packed) + (size_t)(mine.begin + issued) * kStage, kStage, full0 + 8 * st);
                 if (++st == stages) { st = 0; prev_use ^= 1; }
             }
             // Never leave the CTA with a copy still landing in its shared memory.
