@@ -59,6 +59,18 @@ def test_sums_of_the_tensor_memory_gemv(ctx, rows, inputs, outputs, bits):
     w.close()
 
 
+def test_sums_of_sixteen_rows(ctx):
+    """Four chains of 2 L = 64 steps here too (see above), with the mean of a binade for the loss: half a unit is
+    0.72 * 2^-24 of a value on average, so 2^-24 * 0.96 * L; two chains would be twice as far off."""
+    layer = synthetic.make_layer(4096, 32768, 2, seed=9060)
+    w = ctx.prepare(layer)
+    x = dev(synthetic.make_activations(16, 4096, seed=9061))
+    want = linear64(w, layer, x)
+    error = float((w.gemm(x).double() - want).norm() / want.norm())
+    assert error <= 2.0 ** -24 * 0.96 * 32 + 2.0 ** -23, error
+    w.close()
+
+
 @pytest.mark.parametrize("rows", [9, 16, 17, 64, 128, 129, 176, 177, 256, 257, 513, 1024])
 @pytest.mark.parametrize("inputs,outputs", [(128, 128), (3072, 256), (640, 5120)])
 def test_wide_row_groups(ctx, rows, inputs, outputs):
