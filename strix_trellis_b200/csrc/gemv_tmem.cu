@@ -406,9 +406,13 @@ cudaError_t launch_gemv_few(const LinearCall& call, const GemvPlan& plan, Split 
 cudaError_t launch_gemv_row(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream);
 
 // One row with this many units per CTA takes this kernel: the decode loop then outweighs the longer
-// way from the last tile to the fold (measured, one row: 24 units of K4 15.4 against 16.5 us for
-// gemv_row.cu, 218 units of K5 115 against 129 us the other way round).
-constexpr int kTmemUnits = 96;
+// way from the last tile to the fold.  us per launch in a chain of one layer, K4, gemv_row.cu / this
+// kernel: 11 units 9.0 / 9.5, 21 14.9 / 14.3, 32 20.2 / 19.0, 48 29.2 / 26.2, 80 45.5 / 40.1, 192 101 / 88.
+// In a stack a layer pays for the change from one kernel to the other and back, so the line is higher
+// than where the two meet: 28 layers of up to 25 units (4096, 1024 and 14336 wide), K3 to K5, 320 us with
+// the widest in gemv_row.cu and 327 in this kernel; 16 layers of 28 and 7 units 206.3 / 207.4; 12 of 48
+// and 7 units 217 / 206.
+constexpr int kTmemUnits = 40;
 // Two or more rows with at most this many units per CTA go to gemv_few.cu.
 constexpr int kFewUnits = 4;
 

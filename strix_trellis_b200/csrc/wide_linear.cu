@@ -548,9 +548,10 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     // Even and odd K steps have accumulators of their own where there is room, half the truncating
     // accumulations in a row; calls of up to sixteen rows have four, as those of up to eight have (distance from the
     // sum in 64 bits, 16 rows of 5120 -> 5120: 8.4e-7 of its norm with two, 4.5e-7 with four, at
-    // 15.95 us instead of 15.55).  Beyond 128 rows there is room for one (129 rows of 4096 -> 12288: 2.6e-6 where two give
-    // 1.4e-6 for 128), as in the dense GEMM (4.9e-6).  A second buffer lets the MMAs of the next segment start under this one's epilogue.
-    // Four A stages (one for each decode group) are enough, half of the columns are the accumulators'.
+    // 15.95 us instead of 15.55).  Beyond 128 rows there is room for one (129 rows of 4096 -> 12288: 2.6e-6
+    // where two give 1.4e-6 for 128), as in the dense GEMM (4.9e-6).  A second buffer lets the MMAs of
+    // the next segment start under this one's epilogue.  Four A stages (one for each decode group) are
+    // enough, half of the columns are the accumulators'.
     a.d_accs = plan.n_max <= 16 && !set.table ? 4 : plan.n_max <= 128 ? 2 : 1;
     a.parts = plan.parts;
     while (a.parts > 1 && a.parts * a.d_accs * plan.n_max > 256) a.parts /= 2;
