@@ -6,8 +6,10 @@
 // accumulators into planes or outputs.  (src/gemv_lds.hip:93-167)
 //
 // Against gemv_tmem.cu, which serves the layers of more units: no tensor memory to allocate and no chain
-// tensor memory -> commit -> transposition before the fold (four rows, 1280 -> 2432, K5, in a chain of
-// launches: 5.4 against 6.7 us; from five units per CTA on it is the other way round, plan_gemv).
+// tensor memory -> commit -> transposition before the fold; both sides measured stand at kFewUnits.
+//
+// With at most kFewUnits units a CTA has a ring slot for each of them and a slot for the core input of
+// each H128 block they touch: nothing is recycled and nothing waits for a slot.
 //
 // Fold: a column block shared by several CTAs is finished by the CTA that holds its FIRST K range, the
 // end of its own.  The others publish planes word by word, a word being either "empty" (all ones, a
@@ -16,8 +18,7 @@
 // point to higher CTA indices and all CTAs are resident (grid <= SM count).
 #include <type_traits>
 
-#include "backend.h"
-#include "gemv_partition.h"
+#include "gemv_kernels.h"
 #include "hadamard.cuh"
 #include "sync_primitives.cuh"
 #include "trellis_decode.cuh"
@@ -30,17 +31,14 @@ constexpr int kConsumers = 8 * kGroups;          // decode warps
 constexpr int kThreads = (kConsumers + 2) * 32;  // + producer warp + epilogue warp
 constexpr int kDumpThreads = (kConsumers + 1) * 32;  // decode warps + epilogue warp
 constexpr uint32_t kEmptyWord = 0xFFFFFFFFu;      // a partial-plane word nobody has written yet
-constexpr int kActBytes = 64 * 1024;             // staged core input per CTA
-constexpr size_t kGemvSmemLimit = 200 * 1024;    // dynamic shared memory a launch may ask for
 constexpr int kTilesInFlight = 2;                // independent tile decodes per warp
 
 constexpr int kFewHeader = 16384 + 512;          // two fold buffers, barriers
+constexpr int kFewSmem = kFewHeader + kFewUnits * (unit_bytes(8) + 256 * 8);  // the most that a launch asks for
 
 struct GemvArgs {
     LinearCall call;
     Split split;               // unit range of every CTA (units / grid, units % grid)
-    int stages;
-    int act_blocks;            // H128 blocks of core input staged at a time
     float* partials;           // [grid][rows][128], every word empty on entry and on exit
 };
 
@@ -109,19 +107,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_few_kernel(const GemvArgs ar
     const int cta = (int)blockIdx.x;
     const Range mine = cta_range(args.split, cta);
     const int my_units = mine.end - mine.begin;
-    const int stages = args.stages;
     constexpr int kStage = unit_bytes(K);
 
     // shared memory: [2 x fold 8 KB][barriers 512 B][ring][core input]
     float* fold_base = reinterpret_cast<float*>(smem);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 16384);
     unsigned char* ring = smem + 16384 + 512;
-    uint2* act = reinterpret_cast<uint2*>(ring + (size_t)stages * kStage);
+    uint2* act = reinterpret_cast<uint2*>(ring + (size_t)my_units * kStage);
 
-    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + stages);
-    if ((int)threadIdx.x < stages) {  // one thread per ring slot
+    const uint32_t full0 = smem_u32(bars);
+    if ((int)threadIdx.x < my_units) {  // one thread per ring slot
         mbar_init(full0 + 8 * threadIdx.x, 1);
-        mbar_init(empty0 + 8 * threadIdx.x, 8);
         mbar_fence_init();
     }
     __syncthreads();
@@ -132,26 +128,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_few_kernel(const GemvArgs ar
         if (lane == 0) {
             const unsigned char* stream =
                 reinterpret_cast<const unsigned char*>(c.w.packed) + (size_t)mine.begin * kStage;
-            int issued = 0;
-            int st = 0;             // ring slot of unit i and the parity of its previous use,
-            uint32_t prev_use = 1;  // stepped without divisions
             for (int i = 0; i < my_units; ++i) {
-                if (i >= stages && !mbar_wait(empty0 + 8 * st, prev_use, c.status, kTimeoutRingEmpty)) break;
-                mbar_expect_tx(full0 + 8 * st, kStage);
-                bulk_load(smem_u32(ring + (size_t)st * kStage), stream + (size_t)i * kStage, kStage,
-                          full0 + 8 * st);
-                issued = i + 1;
-                if (++st == stages) { st = 0; prev_use ^= 1; }
+                mbar_expect_tx(full0 + 8 * i, kStage);
+                bulk_load(smem_u32(ring + (size_t)i * kStage), stream + (size_t)i * kStage, kStage, full0 + 8 * i);
             }
             // Never leave the CTA with a copy still landing in its shared memory.
-            for (int i = (issued > stages ? issued - stages : 0); i < issued; ++i)
-                mbar_wait(full0 + 8 * (i % stages), (i / stages) & 1, c.status, kTimeoutDrain);
+            for (int i = 0; i < my_units; ++i) mbar_wait(full0 + 8 * i, 0, c.status, kTimeoutDrain);
         }
         return;
     }
 
     // Segment walk shared by decode and epilogue warps: the CTA's unit range is cut at
-    // column-block ends (where a contribution is flushed) and at the staging capacity.
+    // column-block ends, where a contribution is flushed.
     // Each warp calls it once per segment, in order; the position is carried, not divided out.
     int walk_nb = mine.begin / hblocks, walk_hb0 = mine.begin - walk_nb * hblocks;
     auto segment = [&](int done, int& nb, int& hb0, int& len) {
@@ -159,7 +147,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_few_kernel(const GemvArgs ar
         hb0 = walk_hb0;
         len = my_units - done;
         if (len > hblocks - hb0) len = hblocks - hb0;
-        if (len > args.act_blocks) len = args.act_blocks;
         walk_hb0 += len;
         if (walk_hb0 == hblocks) { walk_hb0 = 0; ++walk_nb; }
     };
@@ -176,7 +163,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_few_kernel(const GemvArgs ar
             int nb, hb0, len;
             segment(done, nb, hb0, len);
             done += len;
-            if (!((hb0 + len == hblocks) || (done == my_units))) continue;
             const int buf = flush & 1;
             const int blk_lo = nb * hblocks, blk_hi = blk_lo + hblocks;
             const bool whole = mine.begin <= blk_lo && mine.end >= blk_hi;
@@ -216,15 +202,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_few_kernel(const GemvArgs ar
     }
 
     // ---- decode warps -------------------------------------------------------------------
-    // Resident mode: the whole core input fits the staging area, so every H128 block this
-    // CTA's range touches is staged exactly once, at its own slot, before the loop starts.
+    // Every H128 block this CTA's range touches is staged exactly once, before the loop starts: the block of
+    // unit u in slot u % hblocks.
     // The input scales of a warp's first block are weights (immutable): they are fetched
     // before the wait on the prior grid, so only the activation load follows it.
-    const bool resident = hblocks <= args.act_blocks;
     const int need = my_units < hblocks ? my_units : hblocks;
     const int hb_first = walk_hb0;
     uint16_t su_first[4] = {0, 0, 0, 0};
-    if (resident && warp < rows * need) {
+    if (warp < rows * need) {
         int hb = hb_first + warp % need;
         if (hb >= hblocks) hb -= hblocks;
 #pragma unroll
@@ -242,89 +227,67 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_few_kernel(const GemvArgs ar
 
     // (row, H128 block) items through the input stages, written in B-fragment order:
     // act[((slot*rows + r)*8 + kt)*4 + q] = {half2(k0,k0+1), half2(k0+8,k0+9)}, k0 = 2q.
-    // A warp keeps four items in flight so that their global loads overlap (eight rows of a
-    // 4096-input layer are 256 items, sixteen per warp).  where(item, r, hb, slot) names an item.
-    auto stage_items = [&](int n, bool first_scales_ready, auto&& where, auto width) {
-        constexpr int kInFlight = decltype(width)::value;
-        for (int base = warp; base < n; base += kInFlight * kConsumers) {
-            float xv[kInFlight][4];
-            uint16_t sc[kInFlight][4];
-            int rr[kInFlight], ss[kInFlight];
+    // A warp keeps its (at most two) items in flight so that their global loads overlap.
+    {
+        constexpr int kItems = kFewUnits * 8 / kConsumers;
+        float xv[kItems][4];
+        uint16_t sc[kItems][4];
+        int rr[kItems], ss[kItems];
 #pragma unroll
-            for (int u = 0; u < kInFlight; ++u) {
-                const int item = base + u * kConsumers;
-                if (item < n) {
-                    int hb;
-                    where(item, rr[u], hb, ss[u]);
-                    const long long xr = (long long)rr[u] * c.x_stride + (long long)hb * 128;
-                    const uint16_t* su = c.w.suh + (size_t)hb * 128;
-                    const bool ready = first_scales_ready && item == warp;
+        for (int u = 0; u < kItems; ++u) {
+            const int item = warp + u * kConsumers;
+            if (item < rows * need) {
+                rr[u] = item / need;
+                ss[u] = item % need;
+                int hb = hb_first + ss[u];
+                if (hb >= hblocks) hb -= hblocks;
+                const long long xr = (long long)rr[u] * c.x_stride + (long long)hb * 128;
+                const uint16_t* su = c.w.suh + (size_t)hb * 128;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        xv[u][j] = load_element(c.x, c.x_dtype, xr + lane + 32 * j);
-                        sc[u][j] = ready ? su_first[j] : su[lane + 32 * j];
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kInFlight; ++u) {
-                if (base + u * kConsumers < n) {
-                    float v[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) v[j] = __half2float(scale_input(xv[u][j], sc[u][j]));
-                    hadamard128_warp(v, lane);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int e = lane + 32 * j, kt = e >> 4, kk = e & 15;
-                        const int q = (kk & 7) >> 1, hi = kk >> 3, lo = kk & 1;
-                        act_h[((((size_t)ss[u] * rows + rr[u]) * 8 + kt) * 4 + q) * 4 + hi * 2 + lo] = __float2half_rn(v[j]);
-                    }
+                for (int j = 0; j < 4; ++j) {
+                    xv[u][j] = load_element(c.x, c.x_dtype, xr + lane + 32 * j);
+                    sc[u][j] = u == 0 ? su_first[j] : su[lane + 32 * j];
                 }
             }
         }
-    };
-    if (resident) {
-        auto where = [&](int item, int& r, int& hb, int& slot) {
-            r = item / need;
-            hb = hb_first + item % need;
-            if (hb >= hblocks) hb -= hblocks;
-            slot = hb;
-        };
-        stage_items(rows * need, true, where, std::integral_constant<int, 4>{});
+#pragma unroll
+        for (int u = 0; u < kItems; ++u) {
+            if (warp + u * kConsumers < rows * need) {
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = __half2float(scale_input(xv[u][j], sc[u][j]));
+                hadamard128_warp(v, lane);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int e = lane + 32 * j, kt = e >> 4, kk = e & 15;
+                    const int q = (kk & 7) >> 1, hi = kk >> 3, lo = kk & 1;
+                    act_h[((((size_t)ss[u] * rows + rr[u]) * 8 + kt) * 4 + q) * 4 + hi * 2 + lo] = __float2half_rn(v[j]);
+                }
+            }
+        }
         named_barrier(1, kConsumers * 32);
     }
 
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     bool ok = true;
     int done = 0, flush = 0, final_nb = 0;
-    int next = kgroup;  // the unit (relative to the range) this warp decodes next
-    int slot = kgroup % stages;
-    uint32_t use = (uint32_t)(kgroup / stages) & 1;
+    int next = kgroup;  // the unit (relative to the range) this warp decodes next, and the slot of its block
+    int slot = kgroup;
+    while (slot >= need) slot -= need;
     while (done < my_units) {
         int nb, hb0, len;
         segment(done, nb, hb0, len);
 
-        // chunked mode: input stages for H128 blocks [hb0, hb0+len) into slots 0..len-1
-        if (!resident) {
-            named_barrier(1, kConsumers * 32);  // previous chunk's readers are done
-            stage_items(rows * len, false, [&](int item, int& r, int& hb, int& slot) {
-                r = item / len;
-                slot = item % len;
-                hb = hb0 + slot;
-            }, std::integral_constant<int, 4>{});
-            named_barrier(1, kConsumers * 32);
-        }
-
-        // this warp group takes the units of its parity (ring slots alternate with them)
+        // this warp group takes the units of its parity
         for (; next < done + len && ok; next += 2) {
-            const int b = next - done, st = slot;
-            ok = mbar_wait(full0 + 8 * st, use, c.status, kTimeoutRingFull);
+            ok = mbar_wait(full0 + 8 * next, 0, c.status, kTimeoutRingFull);
             if (!ok) break;
-            slot += 2;  // ring slot and use parity of this warp's next unit, without divisions
-            while (slot >= stages) { slot -= stages; use ^= 1; }
+            __syncwarp();
             const uint32_t* tiles =
-                reinterpret_cast<const uint32_t*>(ring + (size_t)st * kStage) + ctile * tile_words(K);
-            const uint2* bsrc = act_lane + (size_t)(resident ? hb0 + b : b) * rows * 32;
+                reinterpret_cast<const uint32_t*>(ring + (size_t)next * kStage) + ctile * tile_words(K);
+            const uint2* bsrc = act_lane + (size_t)slot * rows * 32;
+            slot += 2;
+            while (slot >= need) slot -= need;
 #pragma unroll
             for (int kt = 0; kt < 8; kt += kTilesInFlight) {  // independent tiles in flight
                 uint32_t f[kTilesInFlight][4];
@@ -337,11 +300,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_few_kernel(const GemvArgs ar
 #pragma unroll
                 for (int q = 0; q < kTilesInFlight; ++q) mma_16816(acc[q & 1], f[q], bf[q].x, bf[q].y);
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty0 + 8 * st);
         }
         done += len;
-        if (!((hb0 + len == hblocks) || (done == my_units))) continue;
 
         // ---- drop this CTA's contribution to column block nb and move on --------------------
         // c0,c1: column ctile*16 + lane/4, rows 2(lane%4), +1; c2,c3: column + 8
@@ -389,22 +349,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_few_kernel(const GemvArgs ar
 }
 
 // ---- host side -------------------------------------------------------------------------
-// Shape of a launch of `rows` rows.
-void plan_gemv_few(const DeviceWeights& w, int rows, GemvPlan& plan) {
-    const int hblocks = w.inputs / 128, stride = unit_bytes(w.bits);
-    const long long units = (long long)hblocks * (w.outputs / 128);
-    const int per_cta = (int)((units + plan.grid - 1) / plan.grid);
-    int act_blocks = kActBytes / (256 * rows);
-    if (act_blocks > hblocks) act_blocks = hblocks;
-    int stages = ((int)kGemvSmemLimit - kFewHeader - act_blocks * 256 * rows) / stride;
-    const int want = (128 * 1024) / stride;  // enough bytes in flight per SM to cover HBM latency
-    if (stages > want) stages = want;
-    if (stages > per_cta) stages = per_cta;
-    if (stages > 28) stages = 28;
-    if (stages < 1) stages = 1;
-    plan.stages = stages;
-    plan.act_blocks = act_blocks;
-    plan.smem_bytes = kFewHeader + (size_t)stages * stride + (size_t)act_blocks * 256 * rows;
+void plan_gemv_few(const DeviceWeights& w, int rows, int units_per_cta, GemvPlan& plan) {
+    plan.stages = units_per_cta;
+    plan.act_blocks = units_per_cta < w.inputs / 128 ? units_per_cta : w.inputs / 128;
+    plan.smem_bytes = kFewHeader + (size_t)plan.stages * unit_bytes(w.bits) + (size_t)plan.act_blocks * 256 * rows;
 }
 
 template <int K, int CB>
@@ -449,7 +397,8 @@ static cudaError_t launch_few_rate(const GemvArgs& args, const GemvPlan& plan, b
 }
 
 cudaError_t launch_gemv_few(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream) {
-    const GemvArgs args{call, split, plan.stages, plan.act_blocks, planes};
+    if (split.q + (split.r != 0) > kFewUnits) return cudaErrorInvalidValue;
+    const GemvArgs args{call, split, planes};
     switch (call.w.codebook) {
     case CB_3INST: return launch_few_rate<CB_3INST>(args, plan, pdl, stream);
     case CB_MCG: return launch_few_rate<CB_MCG>(args, plan, pdl, stream);
@@ -466,7 +415,7 @@ static cudaError_t configure_few() {
     for (int bits = 1; bits <= (CB == CB_MUL1 ? kRateCodes : 8) && e == cudaSuccess; ++bits)
         e = for_rate<CB>(bits, [&](auto k) {
             return cudaFuncSetAttribute(gemv_few_kernel<decltype(k)::value, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kGemvSmemLimit);
+                                        kFewSmem);
         });
     return e;
 }

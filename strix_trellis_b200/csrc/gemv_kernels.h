@@ -1,0 +1,35 @@
+// The three kernels of a linear of 1..8 rows, between plan_gemv / launch_gemv (gemv_tmem.cu) and the
+// files of the two smaller ones.
+#pragma once
+#include "backend.h"
+#include "gemv_partition.h"
+
+namespace st {
+
+// One row with this many units per CTA takes gemv_tmem.cu, with fewer gemv_row.cu: the decode loop then
+// outweighs the longer way from the last tile to the fold.  us per launch in a chain of one layer, K4,
+// gemv_row.cu / gemv_tmem.cu: 11 units 9.0 / 9.5, 21 14.9 / 14.3, 32 20.2 / 19.0, 48 29.2 / 26.2, 80
+// 45.5 / 40.1, 192 101 / 88.  In a stack a layer pays for the change from one kernel to the other and
+// back, so the line is higher than where the two meet: 28 layers of up to 25 units (4096, 1024 and
+// 14336 wide), K3 to K5, 320 us with the widest in gemv_row.cu and 327 in gemv_tmem.cu; 16 layers of 28
+// and 7 units 206.3 / 207.4; 12 of 48 and 7 units 217 / 206.
+constexpr int kTmemUnits = 40;
+
+// Two or more rows with at most this many units per CTA take gemv_few.cu, with more gemv_tmem.cu.  us per
+// launch in a chain of one layer, 2 / 4 / 8 rows, gemv_few.cu against gemv_tmem.cu: two units of K4 4.5 / 4.6 /
+// 5.1 against 6.0 / 6.2 / 6.7; four of K6 6.0 / 6.2 / 7.0 against 7.2 / 7.3 / 7.7.  (With slots in turn instead of
+// one for every unit it was level at seven: 7.8 / 8.4 / 9.3 against 8.0 / 8.3 / 8.8.)  In a stack it depends on the
+// company, which a plan does not see.  84 layers of 1 to 5 units, four rows: at one rate 430 us with
+// gemv_few.cu and 582 without, at two 440 / 591, at five 501 / 594.  A few small layers among large ones pay for
+// the change of kernels, each rate an instantiation whose code is cold when it comes round again: 16 layers
+// of which four have two units 171 / 169, at five rates 181 / 179.
+constexpr int kFewUnits = 4;
+
+// One row, few units per CTA.  False when the row does not fit the staging area (gemv_tmem.cu then).
+bool plan_gemv_row(const DeviceWeights& w, GemvPlan& plan);
+cudaError_t launch_gemv_row(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream);
+// 2..8 rows, at most kFewUnits units per CTA.
+void plan_gemv_few(const DeviceWeights& w, int rows, int units_per_cta, GemvPlan& plan);
+cudaError_t launch_gemv_few(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream);
+
+}  // namespace st

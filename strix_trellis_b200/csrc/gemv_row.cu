@@ -16,8 +16,7 @@
 // Layers of many units per CTA are the other way round (plan_gemv).
 #include <type_traits>
 
-#include "backend.h"
-#include "gemv_partition.h"
+#include "gemv_kernels.h"
 #include "hadamard.cuh"
 #include "sync_primitives.cuh"
 #include "trellis_decode.cuh"
@@ -394,7 +393,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_row_kernel(const GemvArgs ar
 }
 
 // ---- host side -------------------------------------------------------------------------
-// Shape of a launch; false when the row does not fit the staging area (gemv_tmem.cu then).
 bool plan_gemv_row(const DeviceWeights& w, GemvPlan& plan) {
     const int hblocks = w.inputs / 128, stride = unit_bytes(w.bits);
     const long long units = (long long)hblocks * (w.outputs / 128);

@@ -26,8 +26,7 @@
 // rows, K5 29.6 -> 21.6 us; 4096 -> 129280, one row, K5 133 -> 116 us.
 #include <type_traits>
 
-#include "backend.h"
-#include "gemv_partition.h"
+#include "gemv_kernels.h"
 #include "hadamard.cuh"
 #include "tmem_decode.cuh"
 
@@ -398,24 +397,6 @@ __global__ void __launch_bounds__(256) empty_planes_kernel(uint4* planes, int co
 }
 
 // ---- host side -------------------------------------------------------------------------
-// gemv_row.cu: one row, few units per CTA
-bool plan_gemv_row(const DeviceWeights& w, GemvPlan& plan);
-// gemv_few.cu: 2..8 rows, very few units per CTA
-void plan_gemv_few(const DeviceWeights& w, int rows, GemvPlan& plan);
-cudaError_t launch_gemv_few(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream);
-cudaError_t launch_gemv_row(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream);
-
-// One row with this many units per CTA takes this kernel: the decode loop then outweighs the longer
-// way from the last tile to the fold.  us per launch in a chain of one layer, K4, gemv_row.cu / this
-// kernel: 11 units 9.0 / 9.5, 21 14.9 / 14.3, 32 20.2 / 19.0, 48 29.2 / 26.2, 80 45.5 / 40.1, 192 101 / 88.
-// In a stack a layer pays for the change from one kernel to the other and back, so the line is higher
-// than where the two meet: 28 layers of up to 25 units (4096, 1024 and 14336 wide), K3 to K5, 320 us with
-// the widest in gemv_row.cu and 327 in this kernel; 16 layers of 28 and 7 units 206.3 / 207.4; 12 of 48
-// and 7 units 217 / 206.
-constexpr int kTmemUnits = 40;
-// Two or more rows with at most this many units per CTA go to gemv_few.cu.
-constexpr int kFewUnits = 4;
-
 GemvPlan plan_gemv(const DeviceWeights& w, int rows, int sm_count) {
     GemvPlan plan{};
     const int hblocks = w.inputs / 128, nblocks = w.outputs / 128, stride = unit_bytes(w.bits);
@@ -444,7 +425,7 @@ GemvPlan plan_gemv(const DeviceWeights& w, int rows, int sm_count) {
     plan.partial_bytes = align_up((size_t)grid * rows * 128 * sizeof(float));
     plan.row_kernel = rows == 1 && per_cta < kTmemUnits && plan_gemv_row(w, plan);
     plan.few_kernel = rows > 1 && per_cta <= kFewUnits;
-    if (plan.few_kernel) plan_gemv_few(w, rows, plan);
+    if (plan.few_kernel) plan_gemv_few(w, rows, per_cta, plan);
     return plan;
 }
 
