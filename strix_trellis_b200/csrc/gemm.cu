@@ -57,7 +57,7 @@ double dense_us(const DeviceWeights& w, int rows, int sm_count) {
     return 14.5 + 0.59 * hblocks * nblocks / sm_count + (narrow ? 0.72 : 1.0) * step * 2 * hblocks;
 }
 WidePlan wide_plan(const DeviceWeights& w, const Cut& cut) {
-    return plan_wide(w.inputs, w.bits, cut.rows, (long long)cut.groups * (w.inputs / 128) * (w.outputs / 128), cut.ctas);
+    return plan_wide(w.bits, cut.rows, (long long)cut.groups * (w.inputs / 128) * (w.outputs / 128), cut.ctas);
 }
 }  // namespace
 

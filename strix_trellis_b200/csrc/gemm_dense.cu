@@ -28,6 +28,7 @@
 // one 16-byte store, and so are an activation lane's.
 #include "backend.h"
 #include "hadamard.cuh"
+#include "launch.h"
 #include "sync_primitives.cuh"
 #include "tcgen05.cuh"
 #include "trellis_decode.cuh"
@@ -372,40 +373,9 @@ cudaError_t launch_prologue(const DenseArgs& args, unsigned char* a, unsigned ch
     const long long decode_jobs = (long long)args.nb_count * (args.call.w.inputs / 64);
     const long long jobs = decode_jobs + (inputs ? (long long)(rows_padded / 32) * (args.call.w.inputs / 128) : 0);
     if (jobs > 0x3FFFFFFF) return cudaErrorInvalidValue;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(streaming_grid(jobs, 4));  // 64 registers x 256 threads: four CTAs per SM are resident
-    cfg.blockDim = dim3(256);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = programmatic ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, dense_prologue_kernel<K, CB>, args, a, b, (int)decode_jobs, (int)jobs, device_sm_count());
+    return launch_pdl(dense_prologue_kernel<K, CB>, streaming_grid(jobs, 4),  // 64 registers x 256 threads: four CTAs per SM are resident
+                      256, 0, programmatic, stream, args, a, b, (int)decode_jobs, (int)jobs, device_sm_count());
 }
-template <int CB>
-cudaError_t launch_prologue_bits(const DenseArgs& args, unsigned char* a, unsigned char* b, bool inputs, int padded,
-                                 bool pdl, cudaStream_t s) {
-    switch (args.call.w.bits) {
-    case 1: return launch_prologue<1, CB>(args, a, b, inputs, padded, pdl, s);
-    case 2: return launch_prologue<2, CB>(args, a, b, inputs, padded, pdl, s);
-    case 3: return launch_prologue<3, CB>(args, a, b, inputs, padded, pdl, s);
-    case 4: return launch_prologue<4, CB>(args, a, b, inputs, padded, pdl, s);
-    case 5: return launch_prologue<5, CB>(args, a, b, inputs, padded, pdl, s);
-    case 6: return launch_prologue<6, CB>(args, a, b, inputs, padded, pdl, s);
-    case 7: return launch_prologue<7, CB>(args, a, b, inputs, padded, pdl, s);
-    case 8: return launch_prologue<8, CB>(args, a, b, inputs, padded, pdl, s);
-    case 9: case 10: case 11:  // 1.5 / 2.5 / 3.5 bits per weight exist for mul1 only
-        if constexpr (CB == CB_MUL1) {
-            if (args.call.w.bits == 9) return launch_prologue<9, CB>(args, a, b, inputs, padded, pdl, s);
-            if (args.call.w.bits == 10) return launch_prologue<10, CB>(args, a, b, inputs, padded, pdl, s);
-            return launch_prologue<11, CB>(args, a, b, inputs, padded, pdl, s);
-        }
-        return cudaErrorInvalidValue;
-    default: return cudaErrorInvalidValue;
-    }
-}
-
 template <int NB>
 cudaError_t launch_dense(const DenseArgs& args, int sm_count, bool programmatic, cudaStream_t stream) {
     const int tiles = args.m_tiles * args.n_tiles, pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
@@ -460,13 +430,11 @@ cudaError_t launch_gemm_dense(const LinearCall& call, unsigned char* workspace, 
     for (int nb = 0; nb < nblocks; nb += range) {
         args.nb_first = nb;
         args.nb_count = nblocks - nb < range ? nblocks - nb : range;
-        cudaError_t e;
-        switch (call.w.codebook) {
-        case CB_3INST: e = launch_prologue_bits<CB_3INST>(args, workspace, b, nb == 0, rows_padded, programmatic, stream); break;
-        case CB_MCG: e = launch_prologue_bits<CB_MCG>(args, workspace, b, nb == 0, rows_padded, programmatic, stream); break;
-        case CB_MUL1: e = launch_prologue_bits<CB_MUL1>(args, workspace, b, nb == 0, rows_padded, programmatic, stream); break;
-        default: return cudaErrorInvalidValue;
-        }
+        cudaError_t e = for_codebook(call.w.codebook, [&](auto cb) {
+            return for_rate<decltype(cb)::value>(call.w.bits, [&](auto k) {
+                return launch_prologue<decltype(k)::value, decltype(cb)::value>(args, workspace, b, nb == 0, rows_padded, programmatic, stream);
+            });
+        });
         if (e != cudaSuccess) return e;
         const bool two = !gemm_dense_narrow(args.m_tiles, args.nb_count, sm_count / 2);
         args.n_tiles = two ? (args.nb_count + 1) / 2 : args.nb_count;

@@ -16,10 +16,9 @@
 // NaN no sum produces) or a value; the finishing CTA polls them (bounded), adds them in ascending K
 // order from +0, its own first (src/gemv_fused.hip:81-127), and marks them empty again.  Waits only
 // point to higher CTA indices and all CTAs are resident (grid <= SM count).
-#include <type_traits>
-
 #include "gemv_kernels.h"
 #include "hadamard.cuh"
+#include "launch.h"
 #include "sync_primitives.cuh"
 #include "trellis_decode.cuh"
 
@@ -355,56 +354,14 @@ void plan_gemv_few(const DeviceWeights& w, int rows, int units_per_cta, GemvPlan
     plan.smem_bytes = kFewHeader + (size_t)plan.stages * unit_bytes(w.bits) + (size_t)plan.act_blocks * 256 * rows;
 }
 
-template <int K, int CB>
-static cudaError_t launch_few(const GemvArgs& args, const GemvPlan& plan, bool pdl, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(plan.grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = plan.smem_bytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, gemv_few_kernel<K, CB>, args);
-}
-
-// launch(K) for the rate of the weights; half-integer rates exist for mul1 only.
-template <int CB, class Launch>
-static cudaError_t for_rate(int bits, Launch&& launch) {
-    switch (bits) {
-    case 1: return launch(std::integral_constant<int, 1>{});
-    case 2: return launch(std::integral_constant<int, 2>{});
-    case 3: return launch(std::integral_constant<int, 3>{});
-    case 4: return launch(std::integral_constant<int, 4>{});
-    case 5: return launch(std::integral_constant<int, 5>{});
-    case 6: return launch(std::integral_constant<int, 6>{});
-    case 7: return launch(std::integral_constant<int, 7>{});
-    case 8: return launch(std::integral_constant<int, 8>{});
-    default:
-        if constexpr (CB == CB_MUL1) {
-            if (bits == 9) return launch(std::integral_constant<int, 9>{});
-            if (bits == 10) return launch(std::integral_constant<int, 10>{});
-            if (bits == 11) return launch(std::integral_constant<int, 11>{});
-        }
-        return cudaErrorInvalidValue;
-    }
-}
-template <int CB>
-static cudaError_t launch_few_rate(const GemvArgs& args, const GemvPlan& plan, bool pdl, cudaStream_t stream) {
-    return for_rate<CB>(args.call.w.bits, [&](auto k) { return launch_few<decltype(k)::value, CB>(args, plan, pdl, stream); });
-}
-
 cudaError_t launch_gemv_few(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream) {
     if (split.q + (split.r != 0) > kFewUnits) return cudaErrorInvalidValue;
     const GemvArgs args{call, split, planes};
-    switch (call.w.codebook) {
-    case CB_3INST: return launch_few_rate<CB_3INST>(args, plan, pdl, stream);
-    case CB_MCG: return launch_few_rate<CB_MCG>(args, plan, pdl, stream);
-    case CB_MUL1: return launch_few_rate<CB_MUL1>(args, plan, pdl, stream);
-    default: return cudaErrorInvalidValue;
-    }
+    return for_codebook(call.w.codebook, [&](auto cb) {
+        return for_rate<decltype(cb)::value>(call.w.bits, [&](auto k) {
+            return launch_pdl(gemv_few_kernel<decltype(k)::value, decltype(cb)::value>, plan.grid, kThreads, plan.smem_bytes, pdl, stream, args);
+        });
+    });
 }
 
 // Opt-in dynamic shared memory is a per-device function attribute: set for every instantiation

@@ -14,10 +14,9 @@
 // rate, but nothing of the chain tensor memory -> commit -> epilogue warp -> transposition stands
 // between the last tile and the fold (16 layers of K4 in a chain of launches: 152 against 161 us).
 // Layers of many units per CTA are the other way round (plan_gemv).
-#include <type_traits>
-
 #include "gemv_kernels.h"
 #include "hadamard.cuh"
+#include "launch.h"
 #include "sync_primitives.cuh"
 #include "trellis_decode.cuh"
 
@@ -411,55 +410,13 @@ bool plan_gemv_row(const DeviceWeights& w, GemvPlan& plan) {
     return true;
 }
 
-template <int K, int CB>
-static cudaError_t launch_row(const GemvArgs& args, const GemvPlan& plan, bool pdl, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(plan.grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = plan.smem_bytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, gemv_row_kernel<K, CB>, args);
-}
-
-// launch(K) for the rate of the weights; half-integer rates exist for mul1 only.
-template <int CB, class Launch>
-static cudaError_t for_rate(int bits, Launch&& launch) {
-    switch (bits) {
-    case 1: return launch(std::integral_constant<int, 1>{});
-    case 2: return launch(std::integral_constant<int, 2>{});
-    case 3: return launch(std::integral_constant<int, 3>{});
-    case 4: return launch(std::integral_constant<int, 4>{});
-    case 5: return launch(std::integral_constant<int, 5>{});
-    case 6: return launch(std::integral_constant<int, 6>{});
-    case 7: return launch(std::integral_constant<int, 7>{});
-    case 8: return launch(std::integral_constant<int, 8>{});
-    default:
-        if constexpr (CB == CB_MUL1) {
-            if (bits == 9) return launch(std::integral_constant<int, 9>{});
-            if (bits == 10) return launch(std::integral_constant<int, 10>{});
-            if (bits == 11) return launch(std::integral_constant<int, 11>{});
-        }
-        return cudaErrorInvalidValue;
-    }
-}
-template <int CB>
-static cudaError_t launch_row_rate(const GemvArgs& args, const GemvPlan& plan, bool pdl, cudaStream_t stream) {
-    return for_rate<CB>(args.call.w.bits, [&](auto k) { return launch_row<decltype(k)::value, CB>(args, plan, pdl, stream); });
-}
-
 cudaError_t launch_gemv_row(const LinearCall& call, const GemvPlan& plan, Split split, float* planes, bool pdl, cudaStream_t stream) {
     const GemvArgs args{call, split, plan.stages, planes};
-    switch (call.w.codebook) {
-    case CB_3INST: return launch_row_rate<CB_3INST>(args, plan, pdl, stream);
-    case CB_MCG: return launch_row_rate<CB_MCG>(args, plan, pdl, stream);
-    case CB_MUL1: return launch_row_rate<CB_MUL1>(args, plan, pdl, stream);
-    default: return cudaErrorInvalidValue;
-    }
+    return for_codebook(call.w.codebook, [&](auto cb) {
+        return for_rate<decltype(cb)::value>(call.w.bits, [&](auto k) {
+            return launch_pdl(gemv_row_kernel<decltype(k)::value, decltype(cb)::value>, plan.grid, kThreads, plan.smem_bytes, pdl, stream, args);
+        });
+    });
 }
 
 // Opt-in dynamic shared memory is a per-device function attribute: set for every instantiation

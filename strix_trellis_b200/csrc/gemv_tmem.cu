@@ -28,6 +28,7 @@
 
 #include "gemv_kernels.h"
 #include "hadamard.cuh"
+#include "launch.h"
 #include "tmem_decode.cuh"
 
 namespace st {
@@ -429,22 +430,6 @@ GemvPlan plan_gemv(const DeviceWeights& w, int rows, int sm_count) {
     return plan;
 }
 
-template <class... Params, class... Args>
-static cudaError_t launch_pdl(void (*kernel)(Params...), int grid, int block, size_t smem, bool programmatic, cudaStream_t stream,
-                              Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = programmatic ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-}
-
 cudaError_t reset_gemv_scratch(void* workspace, const GemvPlan& plan, cudaStream_t stream) {
     const size_t words = (plan.counter_bytes + plan.partial_bytes) / 16;  // both are multiples of 256
     if (!words) return cudaSuccess;
@@ -465,12 +450,9 @@ cudaError_t launch_gemv(const LinearCall& call, const GemvPlan& plan, void* work
     args.planes = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + plan.counter_bytes);
     if (plan.row_kernel) return launch_gemv_row(call, plan, args.split, args.planes, programmatic_launch, stream);
     if (plan.few_kernel) return launch_gemv_few(call, plan, args.split, args.planes, programmatic_launch, stream);
-    switch (call.w.codebook) {
-    case CB_3INST: return launch_pdl(gemv_tmem_kernel<CB_3INST>, plan.grid, kThreadsT, plan.smem_bytes, programmatic_launch, stream, args);
-    case CB_MCG: return launch_pdl(gemv_tmem_kernel<CB_MCG>, plan.grid, kThreadsT, plan.smem_bytes, programmatic_launch, stream, args);
-    case CB_MUL1: return launch_pdl(gemv_tmem_kernel<CB_MUL1>, plan.grid, kThreadsT, plan.smem_bytes, programmatic_launch, stream, args);
-    default: return cudaErrorInvalidValue;
-    }
+    return for_codebook(call.w.codebook, [&](auto cb) {
+        return launch_pdl(gemv_tmem_kernel<decltype(cb)::value>, plan.grid, kThreadsT, plan.smem_bytes, programmatic_launch, stream, args);
+    });
 }
 
 // Opt-in dynamic shared memory is a per-device function attribute: set when a context is created

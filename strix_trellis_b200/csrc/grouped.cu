@@ -6,6 +6,7 @@
 // (src/dense_r1_group*.hip).
 #include "grouped.h"
 #include "hadamard.cuh"
+#include "launch.h"
 #include "sync_primitives.cuh"
 
 namespace st {
@@ -15,7 +16,7 @@ GroupedPlan plan_grouped(int inputs, int outputs, int max_bits, int rows, int sm
     const int hblocks = inputs / 128, nblocks = outputs / 128;
     if (rows > kGroupRows) rows = kGroupRows;
     if (problems < 1) problems = 1;
-    plan.wide = plan_wide(inputs, max_bits, rows, (long long)problems * nblocks * hblocks, sm_count);
+    plan.wide = plan_wide(max_bits, rows, (long long)problems * nblocks * hblocks, sm_count);
     expect_row_groups(plan, inputs, outputs, max_bits, (long long)problems * ((rows + 7) / 8), sm_count);
     plan.splits = (plan.wide.grid + problems * nblocks - 1) / (problems * nblocks);
     plan.scratch_splits = 1;
@@ -64,29 +65,12 @@ __global__ void swiglu_kernel(const float* __restrict__ gate, const float* __res
     }
 }
 
-// A small kernel of a routed-expert submit: launched programmatically when the context allows
-// it, so that it is resident and waiting when the launch before it ends.
-template <class... Params, class... Args>
-static cudaError_t launch_small(void (*kernel)(Params...), int grid, int block, bool programmatic, cudaStream_t stream,
-                                Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = programmatic ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-}
-
 cudaError_t launch_swiglu(const float* gate, const float* up, float* hidden, int rows, int width,
                           long long out_stride, bool programmatic, cudaStream_t stream) {
     const long long count = (long long)rows * width;
     if (count <= 0) return cudaSuccess;
     const long long want = (count + 255) / 256;
-    return launch_small(swiglu_kernel, streaming_grid(want), 256, programmatic, stream, gate, up, hidden, count, width,
+    return launch_pdl(swiglu_kernel, streaming_grid(want), 256, 0, programmatic, stream, gate, up, hidden, count, width,
                         out_stride);
 }
 
@@ -189,7 +173,7 @@ cudaError_t launch_moe_route(const unsigned int* route_ids, const float* route_s
     if (bank_count > 1024 || window.first_expert < 0 || window.experts_total < window.first_expert + bank_count ||
         window.group_rows < 1 || window.group_rows > kGroupRows)
         return cudaErrorInvalidValue;
-    return launch_small(moe_route_kernel, 1, 1024, programmatic, stream, route_ids, route_scores, tokens, top_k, bank,
+    return launch_pdl(moe_route_kernel, 1, 1024, 0, programmatic, stream, route_ids, route_scores, tokens, top_k, bank,
                         bank_count, window, gate_up, down, row_valid);
 }
 
@@ -228,7 +212,7 @@ cudaError_t launch_moe_combine(const float* each, const float* scores, const int
     const long long total = (long long)tokens * outputs;
     if (total <= 0) return cudaSuccess;
     const long long want = (total + 255) / 256;
-    return launch_small(moe_combine_kernel, streaming_grid(want), 256, programmatic, stream, each, scores, row_valid, tokens,
+    return launch_pdl(moe_combine_kernel, streaming_grid(want), 256, 0, programmatic, stream, each, scores, row_valid, tokens,
                         top_k, outputs, y, y_stride, alpha, beta, route_ids, first_expert, bank_count);
 }
 

@@ -10,6 +10,7 @@
 // (src/tp_moe.hip:60-164, src/tp_fused_device.hpp:19-126, src/dense_r1_group*.hip)
 #include "grouped.h"
 #include "hadamard.cuh"
+#include "launch.h"
 #include "sync_primitives.cuh"
 #include "trellis_decode.cuh"
 
@@ -210,33 +211,15 @@ cudaError_t configure_direct_kernels() {
     return e;
 }
 
-template <int CB>
-static cudaError_t launch_direct_cb(const DirectArgs& args, int grid, size_t smem, bool pdl, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kThreadsG);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, grouped_direct_kernel<CB>, args);
-}
-
 cudaError_t launch_grouped_direct(const GroupedProblem* problems, int problem_count, int inputs, int outputs, int codebook,
                                   const GroupedPlan& plan, unsigned int* status, bool programmatic, cudaStream_t stream) {
     const DirectArgs args{problems, plan.ctas_per_problem, plan.splits, plan.stages, inputs / 128, plan.stage_stride,
                           align_up((size_t)(outputs / 128) * sizeof(unsigned int)), status};
     const long long grid = (long long)problem_count * plan.ctas_per_problem;
     if (grid > 0x7FFFFFFF || plan.smem_bytes > kDirectSmemLimit) return cudaErrorInvalidValue;
-    switch (codebook) {
-    case CB_3INST: return launch_direct_cb<CB_3INST>(args, (int)grid, plan.smem_bytes, programmatic, stream);
-    case CB_MCG: return launch_direct_cb<CB_MCG>(args, (int)grid, plan.smem_bytes, programmatic, stream);
-    case CB_MUL1: return launch_direct_cb<CB_MUL1>(args, (int)grid, plan.smem_bytes, programmatic, stream);
-    default: return cudaErrorInvalidValue;
-    }
+    return for_codebook(codebook, [&](auto cb) {
+        return launch_pdl(grouped_direct_kernel<decltype(cb)::value>, (int)grid, kThreadsG, plan.smem_bytes, programmatic, stream, args);
+    });
 }
 
 }  // namespace st

@@ -23,6 +23,7 @@
 // Every wait is bounded and reports into the device status word.
 #include "gemv_partition.h"
 #include "hadamard.cuh"
+#include "launch.h"
 #include "sync_primitives.cuh"
 #include "tmem_decode.cuh"
 #include "wide_linear.h"
@@ -510,8 +511,7 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
 }
 
 // ---- host side -----------------------------------------------------------------------------------
-WidePlan plan_wide(int inputs, int heaviest, int rows_max, long long units, int sm_count) {
-    (void)inputs;
+WidePlan plan_wide(int heaviest, int rows_max, long long units, int sm_count) {
     WidePlan plan{};
     plan.grid = (int)(units < sm_count ? units : sm_count);
     plan.n_max = wide_n(rows_max < kWideRows ? rows_max : kWideRows);
@@ -565,22 +565,6 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     return a;
 }
 
-template <class... Params, class... Args>
-static cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, int block, size_t smem, bool programmatic,
-                              cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = programmatic ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-}
-
 cudaError_t launch_wide_inputs(const WideSet& set, const WidePlan& plan, unsigned int* flags, bool programmatic,
                                cudaStream_t stream) {
     const WideArgs a = wide_args(set, plan, flags, nullptr, nullptr);
@@ -592,12 +576,6 @@ cudaError_t launch_wide_inputs(const WideSet& set, const WidePlan& plan, unsigne
     return launch_pdl(wide_inputs_kernel, dim3(x, y), 32 * kInputWarps, 0, programmatic, stream, a, plan.grid);
 }
 
-template <int CB>
-static cudaError_t launch_wide_cb(const WideArgs& a, const WidePlan& plan, bool programmatic, cudaStream_t stream) {
-    if (a.parts > 1) return launch_pdl(wide_linear_kernel<CB, true>, dim3(plan.grid), kThreadsW, plan.smem_bytes, programmatic, stream, a);
-    return launch_pdl(wide_linear_kernel<CB, false>, dim3(plan.grid), kThreadsW, plan.smem_bytes, programmatic, stream, a);
-}
-
 cudaError_t launch_wide(const WideSet& set, const WidePlan& plan, unsigned int* flags, float* planes, unsigned int* status,
                         bool programmatic, cudaStream_t stream) {
     const WideArgs a = wide_args(set, plan, flags, planes, status);
@@ -605,12 +583,10 @@ cudaError_t launch_wide(const WideSet& set, const WidePlan& plan, unsigned int* 
     if (units < 1 || units > 0x7FFFFFFF || plan.b_slots < 1 || plan.w_slots < 2 || plan.smem_bytes > kSmemLimitW ||
         (size_t)plan.w_slots * plan.w_stride < kRingMin)
         return cudaErrorInvalidValue;
-    switch (set.codebook) {
-    case CB_3INST: return launch_wide_cb<CB_3INST>(a, plan, programmatic, stream);
-    case CB_MCG: return launch_wide_cb<CB_MCG>(a, plan, programmatic, stream);
-    case CB_MUL1: return launch_wide_cb<CB_MUL1>(a, plan, programmatic, stream);
-    default: return cudaErrorInvalidValue;
-    }
+    return for_codebook(set.codebook, [&](auto cb) {
+        return a.parts > 1 ? launch_pdl(wide_linear_kernel<decltype(cb)::value, true>, plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a)
+                           : launch_pdl(wide_linear_kernel<decltype(cb)::value, false>, plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a);
+    });
 }
 
 // Opt-in dynamic shared memory is a per-device function attribute: set when a context is created

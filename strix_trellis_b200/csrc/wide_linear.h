@@ -52,7 +52,7 @@ ST_RATE_FN int accumulator_parts(int hblocks, int nblocks, long long groups, int
     return parts;
 }
 // `heaviest`: the rate code with the largest tiles among the problems.
-WidePlan plan_wide(int inputs, int heaviest, int rows_max, long long units, int sm_count);
+WidePlan plan_wide(int heaviest, int rows_max, long long units, int sm_count);
 
 // A set of problems of one geometry.  `table` (device memory) holds them, `table_stride` bytes apart;
 // without a table the set is ONE layer whose `one.rows` rows are cut into problems of group_rows rows.
