@@ -2,6 +2,7 @@
 //   weights decoded on the fly into tensor memory, once for each row group (wide_linear.cu)
 //   weights decoded once into the workspace, dense GEMM (gemm_dense.cu)
 // Beyond kWideMaxRows always the second; below, whichever the estimates here say is faster.
+#include "strix_trellis_b200.h"
 #include "wide_linear.h"
 
 #include <cmath>
@@ -99,3 +100,28 @@ cudaError_t launch_gemm(const LinearCall& call, const GemmPlan& plan, void* work
 }
 
 }  // namespace st
+
+// Pure host arithmetic: no context, no device.
+extern "C" strix_status strix_b200_gemm_route(uint64_t inputs, uint64_t outputs, uint32_t bits_x2, uint32_t rows, uint32_t sm_count,
+                                              uint64_t out[4]) {
+    if (!out) return STRIX_ERROR_INVALID_ARGUMENT;
+    out[0] = out[1] = out[2] = out[3] = 0;
+    const int code = st::rate_code(bits_x2);
+    if (!inputs || !outputs || inputs % 128 || outputs % 128 || inputs > (1u << 30) || outputs > (1u << 30) ||
+        (inputs / 128) * (outputs / 128) > 0x7FFFFFFF || !code ||
+        rows <= 8 || rows > 0x7FFFFFFF || !sm_count || sm_count > 4096)
+        return STRIX_ERROR_INVALID_ARGUMENT;
+    st::DeviceWeights w{};
+    w.inputs = (int)inputs;
+    w.outputs = (int)outputs;
+    w.bits = code;
+    const st::GemmPlan plan = st::plan_gemm(w, (int)rows, (int)sm_count);
+    out[0] = plan.dense;
+    out[1] = plan.workspace_bytes;
+    if (!plan.dense) {
+        const st::Cut cut = st::cut_call(w, (int)rows, (int)sm_count);
+        out[2] = (uint64_t)cut.groups;
+        out[3] = (uint64_t)cut.ctas;
+    }
+    return STRIX_SUCCESS;
+}

@@ -1,0 +1,57 @@
+"""The choice between the two routes of a GEMM and its cut, checked on the CPU through the library's own
+arithmetic (strix_b200_gemm_route)."""
+import pytest
+
+from strix_trellis_b200 import native as N
+
+SHAPES = [(128, 128), (1152, 4096), (4096, 4096), (5120, 5120), (4096, 12288), (4096, 129280), (16384, 4096), (8192, 256), (128, 4096)]
+ROWS = [9, 15, 16, 17, 31, 64, 65, 100, 128, 129, 255, 256, 257, 300, 511, 512, 513, 777, 1023, 1024, 1025, 2048, 8192, 100000]
+
+
+def route(inputs, outputs, bits_x2, rows, sm_count=148):
+    out = (N.u64 * 4)()
+    status = N.load().strix_b200_gemm_route(inputs, outputs, bits_x2, rows, sm_count, out)
+    return status, list(out)
+
+
+@pytest.mark.parametrize("sm_count", [148, 132, 7, 1])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_cut_and_workspace(shape, sm_count):
+    inputs, outputs = shape
+    hblocks, nblocks = inputs // 128, outputs // 128
+    for bits_x2 in (2, 3, 5, 8, 12, 16):
+        for rows in ROWS:
+            if sm_count == 1 and rows > 1024:
+                continue
+            status, (dense, workspace, groups, ctas) = route(inputs, outputs, bits_x2, rows, sm_count)
+            assert status == N.SUCCESS
+            padded = (rows + 255) // 256 * 256
+            if dense:
+                assert sm_count >= 2 and groups == ctas == 0
+                decoded = workspace - padded * inputs * 2
+                assert 0 < decoded <= max(256 << 20, inputs * 512)  # a range of two column blocks at least
+                assert decoded % (inputs * 256) == 0 and decoded <= nblocks * inputs * 256
+            else:
+                assert rows <= 1024
+                each = -(-rows // groups)  # rows of a group, at most the MMA's N
+                assert 1 <= groups and each <= 256
+                assert 1 <= ctas <= sm_count
+                # input tiles of every group and a plane for every CTA fit
+                assert workspace >= rows * inputs * 2 + min(ctas, groups * hblocks * nblocks) * each * 512
+
+
+def test_measured_sides_of_the_line():
+    """Shapes whose two routes were timed, on the side that was faster."""
+    for rows, inputs, outputs, bits_x2, dense in [(16, 5120, 5120, 8, 0), (101, 4096, 12288, 8, 0), (178, 3072, 2048, 8, 0),
+                                                  (600, 7936, 7296, 8, 0), (546, 2176, 1024, 8, 0), (512, 4096, 12288, 10, 1),
+                                                  (1777, 5120, 5120, 12, 1), (8192, 4096, 12288, 8, 1)]:
+        assert route(inputs, outputs, bits_x2, rows)[1][0] == dense, (rows, inputs, outputs)
+    assert route(3072, 2048, 8, 178)[1][2] == 3  # 51 us in one group, 22 in three
+
+
+@pytest.mark.parametrize("args", [(0, 128, 8, 16), (128, 130, 8, 16), (128, 128, 0, 16), (128, 128, 9, 16), (128, 128, 17, 16),
+                                  (128, 128, 18, 16), (128, 128, 1, 16), (128, 128, 8, 8), (128, 128, 8, 0), (1 << 31, 128, 8, 16),
+                                  (128, 128, 8, 16, 0), (1 << 30, 1 << 30, 8, 16)])
+def test_refusals(args):
+    assert route(*args) == (N.INVALID_ARGUMENT, [0, 0, 0, 0])
+    assert N.load().strix_b200_gemm_route(128, 128, 8, 16, 148, None) == N.INVALID_ARGUMENT
