@@ -21,7 +21,7 @@ With N>1 (launched under torchrun) every rank runs the same workload on its own 
 the timed region: rates x rows on the largest shape, the prefill GEMM (K4/K5/K6), the
 routed-expert block on one rank's bank, and at every N the tensor-parallel dense layers
 (row-parallel + all-reduce, LM head + all-gather) and the expert-parallel block
-(all-to-all dispatch and return).  `--no-extra` skips them; `--case gemv|gemm|gemm-small|moe|decode` runs one
+(all-to-all dispatch and return).  `--no-extra` skips them; `--case gemv|gemv-rows|gemm|gemm-small|moe|decode` runs one
 small fixed workload of one kernel for profilers.
 
 `--impl reference` times the CPU contract (this repository's C restatement of the
@@ -474,11 +474,12 @@ def run_case(args):
     from strix_trellis_b200.runtime import Context
     ctx = Context(0)
     stream = torch.cuda.Stream()
-    if args.case == "gemv":
-        layer = synthetic.make_layer(4096, 14336, BITS, seed=synthetic.BASE_SEED + 3)
-        ws = [ctx.prepare(layer) for _ in range(8)]  # 8 x 29 MB: every launch reads cold weights
-        x = torch.from_numpy(synthetic.make_activations(ROWS, 4096)).cuda()
-        y = torch.empty((ROWS, 14336), dtype=torch.float32, device="cuda")
+    if args.case in ("gemv", "gemv-rows"):
+        inputs, outputs, bits, rows = (4096, 14336, BITS, ROWS) if args.case == "gemv" else (16384, 4096, 5, 8)
+        layer = synthetic.make_layer(inputs, outputs, bits, seed=synthetic.BASE_SEED + 3)
+        ws = [ctx.prepare(layer) for _ in range(8)]  # 8 x 29 or 42 MB: every launch reads cold weights
+        x = torch.from_numpy(synthetic.make_activations(rows, inputs)).cuda()
+        y = torch.empty((rows, outputs), dtype=torch.float32, device="cuda")
         with torch.cuda.stream(stream):
             plans = [w.plan(x, y, N.OP_GEMV, stream=stream) for w in ws]
 
@@ -486,7 +487,7 @@ def run_case(args):
             for p in plans:
                 p.submit()
         us = time_calls(torch, stream, one_pass, 3, warm=1) / len(plans)
-        print(json.dumps({"case": "gemv 4096x14336 K4 R1", "us_per_launch": round(us, 2),
+        print(json.dumps({"case": f"gemv {inputs}x{outputs} K{bits} R{rows}", "us_per_launch": round(us, 2),
                           "GBps": round(layer.packed_bytes / us / 1e3, 1), "status": ctx.device_status()}))
     elif args.case == "decode":
         # the decoder's own ceiling: decode + mma on tiles resident in shared memory, no memory traffic
@@ -843,7 +844,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--no-extra", action="store_true", help="skip the GEMM / MoE / TP side measurements")
-    ap.add_argument("--case", choices=["gemv", "gemm", "gemm-small", "moe", "decode"], help="run one small profiling workload and exit")
+    ap.add_argument("--case", choices=["gemv", "gemv-rows", "gemm", "gemm-small", "moe", "decode"], help="run one small profiling workload and exit")
     args = ap.parse_args()
     if args.case:
         run_case(args)

@@ -152,20 +152,29 @@ struct Epilogue {
                 const uint32_t at = taddr + part * a.d_accs * a.n_max + ch * kChunkRows;
                 __syncwarp();
                 tmem_ld_32x16(at, r);
-                if (a.d_accs == 1) {
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(r[j]));  // not before the wait
-                }
-#pragma unroll 1
-                for (int acc = 1; acc < a.d_accs; ++acc) {
+                if (a.d_accs > 1) {
                     uint32_t q[16];
-                    tmem_ld_32x16(at + acc * a.n_max, q);
+                    tmem_ld_32x16(at + a.n_max, q);
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        asm volatile("" : "+r"(r[j]), "+r"(q[j]));
+                        asm volatile("" : "+r"(r[j]), "+r"(q[j]));  // not before the wait
                         r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(q[j])));
+                    }
+                } else {
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(r[j]));
+                }
+                if (!PARTS && a.d_accs == 4) {  // one layer of up to sixteen rows
+                    uint32_t q[16], t[16];
+                    tmem_ld_32x16(at + 2 * a.n_max, q);
+                    tmem_ld_32x16(at + 3 * a.n_max, t);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        asm volatile("" : "+r"(q[j]), "+r"(t[j]));
+                        r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __fadd_rn(__uint_as_float(q[j]), __uint_as_float(t[j]))));
                     }
                 }
                 if (PARTS && part != first_part)
@@ -360,7 +369,8 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         for (Walk w(args, mine); w.unit < w.end && ok; ++seg) {
             const int len = w.length(args), n = wide_n(problem_rows(args, w.p));
             const uint32_t idesc = umma_idesc_f16_f32(128, n), dcol = tmem + d_column(seg);
-            const uint32_t accs = args.d_accs - 1;  // K step k goes to accumulator k % d_accs
+            // K step k goes to accumulator k % d_accs
+            const uint32_t odd = args.d_accs > 1 ? args.n_max : 0, two = !PARTS && args.d_accs == 4 ? 2 * args.n_max : 0;
             if (seg >= d_bufs && !mbar_wait(d_empty + 8 * d_index(seg), d_parity(seg) ^ 1, args.status, kTimeoutTensorPipe)) break;
             int part = PARTS ? part_of(args, w.hb) : 0, fresh = 1;
             for (int i = 0; i < len; ++i) {
@@ -377,7 +387,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        umma_f16_ts(acc + (k & accs) * args.n_max, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, !fresh || k >= args.d_accs);
+                        umma_f16_ts(acc + (k & 1) * odd + (k >> 1 & 1) * two, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, !fresh || k >= args.d_accs);
                     umma_commit(a_empty + 8 * stage);
                     umma_commit(b_empty + 8 * slot);
                 }
@@ -548,7 +558,7 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     // Even and odd K steps have accumulators of their own where there is room, half the truncating
     // accumulations in a row; calls of up to sixteen rows have four, as those of up to eight have (distance from the
     // sum in 64 bits, 16 rows of 5120 -> 5120: 8.4e-7 of its norm with two, 4.5e-7 with four, at
-    // 15.95 us instead of 15.55).  Beyond 128 rows there is room for one (129 rows of 4096 -> 12288: 2.6e-6
+    // 15.75 us instead of 15.55).  Beyond 128 rows there is room for one (129 rows of 4096 -> 12288: 2.6e-6
     // where two give 1.4e-6 for 128), as in the dense GEMM (4.9e-6).  A second buffer lets the MMAs of
     // the next segment start under this one's epilogue.  Four A stages (one for each decode group) are
     // enough, half of the columns are the accumulators'.
