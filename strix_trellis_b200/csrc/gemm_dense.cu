@@ -15,8 +15,9 @@
 // Launch 2 (gemm_dense_kernel): persistent CTA pairs (tcgen05 cta_group::2).  A pair's tile is
 // 256 rows x NB column blocks of 128; each CTA holds 128 rows of it, loads its own activation
 // image and its half of the weight image, the MMA reads the other half from the partner.
-// Bound by the tensor pipe: 8192 rows 549 us (1.50 PFLOP/s at the capped clock); the kernel before,
-// which decoded on the fly in 512 x 256 tiles, took 950 us.  What mattered most: the partner CTA's
+// Bound by the tensor pipe, which at 2048 rows is busy for 79 of 100 clocks that an SM is active, at a
+// clock that falls to 1.6 GHz under it; 8192 rows take 640 us with the prologue (1.29 PFLOP/s).  The kernel
+// before, which decoded on the fly in 512 x 256 tiles, took 950 us without one.  What mattered most: the partner CTA's
 // "my stage has landed" must not be a release-arrival on the leader's barrier (1250-1750 clocks each
 // beside bulk copies, longer than a K step); a four-byte st.async that counts as transaction bytes
 // took the same kernel from 950 to 557 us.

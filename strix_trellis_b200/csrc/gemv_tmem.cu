@@ -22,8 +22,8 @@
 // for another, measured 2.6 us per layer slower: the extra launch boundary costs more.)
 //
 // Measured in a chain of launches against the kernel before, which fed mma.sync and staged its rows
-// four 2-byte stores at a time: 16 layers, four rows, K2..K6 226 -> 178 us; 16384 -> 4096, eight
-// rows, K5 29.6 -> 21.6 us; 4096 -> 129280, one row, K5 133 -> 116 us.
+// four 2-byte stores at a time: 16 layers, four rows, K2..K6 226 -> 179 us (four of them small ones in
+// gemv_few.cu); 16384 -> 4096, eight rows, K5 29.6 -> 22.0 us; 4096 -> 129280, one row, K5 133 -> 118 us.
 #include <type_traits>
 
 #include "gemv_kernels.h"

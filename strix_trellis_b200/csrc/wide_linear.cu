@@ -260,7 +260,8 @@ struct Epilogue {
 };
 
 // At most 72 registers: a CTA of the next call's input stages (128 threads) then fits beside this
-// kernel's, is resident and has its operands in the L2 when this kernel ends.
+// kernel's, is resident and has its operands in the L2 when this kernel ends.  (ptxas spills for it in
+// the epilogue's chunk: 124 bytes stored and 188 loaded with K parts, 4 bytes without for mul1.)
 template <int CB, bool PARTS>
 __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];

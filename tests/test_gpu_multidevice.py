@@ -18,8 +18,8 @@ def test_second_device_in_the_same_process():
     from strix_trellis_b200.runtime import Context
     layer = synthetic.make_layer(2048, 1024, 4, 9700, bias=True)
     x1 = synthetic.make_activations(1, 2048, seed=9701)   # one-row kernel
-    x8 = synthetic.make_activations(8, 2048, seed=9702)   # multi-row kernel
-    xm = synthetic.make_activations(600, 2048, seed=9703)  # tensor-core pair kernel
+    x8 = synthetic.make_activations(8, 2048, seed=9702)   # few-rows kernel
+    xm = synthetic.make_activations(1100, 2048, seed=9703)  # weights decoded first, CTA-pair kernel
     want = {k: c_oracle.linear(layer.trellis, layer.suh, layer.svh, layer.bias, 4, 2, v)
             for k, v in (("r1", x1), ("r8", x8), ("m", xm))}
     got = {}

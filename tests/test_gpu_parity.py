@@ -215,7 +215,7 @@ def test_half_integer_rates_decode_bit_exact_and_multiply(ctx, golden_dir):
     """Rates 1.5 / 2.5 / 3.5 (stream positions alternate between floor(rate) and one bit more,
     mul1 only; reference python/strix_trellis/codec.py:12-20, CPU-only there).  The decoded Q of
     the golden tiles carries the hash the reference's own decoder produced; a larger layer goes
-    through the one-row kernel, the multi-row kernel, the 8-row chunks and the tensor-core GEMM
+    through the one-row kernel, the few-rows kernel and the GEMM that decodes on the fly
     against the NumPy contract."""
     meta = json.loads((golden_dir / "half_rates.json").read_text())
     rng = synthetic.rng_for(synthetic.BASE_SEED + 50)
@@ -249,7 +249,7 @@ def test_half_precision_tensors_widen_on_load_and_round_on_store(ctx, rows):
     include/strix_trellis.h:39-40; honoured here).  The arithmetic is the float32 contract: an
     input of either type gives the bits of the same values passed as float32, and an output of
     either type is the float32 output rounded to nearest even -- through the one-row kernel, the
-    multi-row kernel, the 8-row chunks and the tensor-core GEMM, with and without alpha / beta
+    few-rows kernel and the GEMM in one and in several row groups, with and without alpha / beta
     over an old output of that type."""
     layer = synthetic.make_layer(1024, 640, 4, seed=8100 + rows, bias=True)
     w = ctx.prepare(layer)
@@ -304,7 +304,8 @@ def test_config1_against_reference_golden(ctx, golden_dir):
 
 @pytest.mark.parametrize("rows", [9, 16, 17, 32])
 def test_gemm_small_rows(ctx, grid, rows):
-    """Up to 16 rows run as 8-row chunks of the fused GEMV, more rows take the tcgen05 kernel."""
+    """A few rows more than the GEMV takes: one row group of the kernel that decodes on the fly, whose
+    MMA has N = 16 or 32."""
     meta, outs = grid
     for case in meta["cases"][::7]:
         layer, _, _, _ = synthetic.grid_case(case["codebook"], case["bits"], case["wide"], meta["rows"])
@@ -352,10 +353,10 @@ def test_gemm_tensor_core_prefill_shape(ctx, bits, rows):
 
 @pytest.mark.parametrize("rows", [40, 130, 300])
 def test_gemm_more_column_stripes_than_sms(ctx, rows):
-    """A wide, short layer (256 -> 40960: 160 column stripes of 256, four K steps each): with up
-    to 256 rows some CTAs of the single-CTA kernel run two work items, so the weight prefetch and
-    the decoders' look-ahead cross from one item into the next and only the last item's
-    epilogue is shared with the decoder warps; 300 rows take the two-CTA kernel the same way."""
+    """A wide, short layer (256 -> 40960: 320 column blocks of two units each): with 40 rows
+    every CTA finishes several blocks, so the weight prefetch and the decoders' look-ahead cross
+    from one block into the next and only the last block's epilogue is shared with the
+    decode warps; with 130 and 300 rows the weights are decoded first and a CTA pair has several tiles."""
     layer = synthetic.make_layer(256, 40960, 2, seed=640, bias=True)
     x = synthetic.make_activations(rows, 256, seed=641)
     w = ctx.prepare(layer)
