@@ -11,7 +11,7 @@
 namespace st {
 
 // Prepared weights on the device.  `packed` holds the tiles regrouped per 128 output
-// columns: [N/128][I/16][8 column tiles][tile_words(rate) uint32 words]; a column block is one
+// columns: [N/128][I/64][8 column tiles][tile_words(rate) uint32 words][4 k-tiles]; a column block is one
 // contiguous stream of I/128 units of unit_bytes(rate) bytes.
 struct DeviceWeights {
     const uint32_t* packed;

@@ -78,12 +78,9 @@ __global__ void __launch_bounds__(256) dense_prologue_kernel(const DenseArgs arg
     // Weight images: a warp decodes one 16-column tile of four k-tiles, with the ring words of its
     // next job already on their way (a job is a DRAM round trip and only 200 instructions).
     auto decode = [&] {
-        const uint32_t* first = c.w.packed + ((size_t)args.nb_first * kt64 * 32 + warp) * tile_words(K);
+        const uint32_t* first = c.w.packed + ((size_t)args.nb_first * kt64 * 8 + warp) * quad_words(K);
         uint32_t w[4][3], next[4][3];
-        auto fetch = [&](int job, uint32_t (&words)[4][3]) {
-#pragma unroll
-            for (int t = 0; t < 4; ++t) load_window<K>(first + ((size_t)job * 32 + t * 8) * tile_words(K), geom, words[t]);
-        };
+        auto fetch = [&](int job, uint32_t (&words)[4][3]) { load_windows<K>(first + (size_t)job * 8 * quad_words(K), geom, words); };
         int job = blockIdx.x;
         if (job < decode_jobs) fetch(job, next);
         for (; job < decode_jobs; job += gridDim.x) {

@@ -30,7 +30,6 @@ constexpr int kConsumers = 8 * kGroups;          // decode warps
 constexpr int kThreads = (kConsumers + 2) * 32;  // + producer warp + epilogue warp
 constexpr int kDumpThreads = (kConsumers + 1) * 32;  // decode warps + epilogue warp
 constexpr uint32_t kEmptyWord = 0xFFFFFFFFu;      // a partial-plane word nobody has written yet
-constexpr int kTilesInFlight = 2;                // independent tile decodes per warp
 
 constexpr int kFewHeader = 16384 + 512;          // two fold buffers, barriers
 constexpr int kFewSmem = kFewHeader + kFewUnits * (unit_bytes(8) + 256 * 8);  // the most that a launch asks for
@@ -283,21 +282,19 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_few_kernel(const GemvArgs ar
             if (!ok) break;
             __syncwarp();
             const uint32_t* tiles =
-                reinterpret_cast<const uint32_t*>(ring + (size_t)next * kStage) + ctile * tile_words(K);
+                reinterpret_cast<const uint32_t*>(ring + (size_t)next * kStage) + ctile * quad_words(K);
             const uint2* bsrc = act_lane + (size_t)slot * rows * 32;
             slot += 2;
             while (slot >= need) slot -= need;
 #pragma unroll
-            for (int kt = 0; kt < 8; kt += kTilesInFlight) {  // independent tiles in flight
-                uint32_t f[kTilesInFlight][4];
-                uint2 bf[kTilesInFlight];
+            for (int half = 0; half < 2; ++half) {  // four independent tiles in flight
+                uint32_t f[4][4];
+                decode_quad_frag<K, CB>(tiles + half * 8 * quad_words(K), geom, f);
 #pragma unroll
-                for (int q = 0; q < kTilesInFlight; ++q) {
-                    decode_tile_frag<K, CB>(tiles + (kt + q) * 8 * tile_words(K), geom, f[q]);
-                    bf[q] = bsrc[(kt + q) * 4];
+                for (int t = 0; t < 4; ++t) {
+                    const uint2 bf = bsrc[(half * 4 + t) * 4];
+                    mma_16816(acc[t & 1], f[t], bf.x, bf.y);
                 }
-#pragma unroll
-                for (int q = 0; q < kTilesInFlight; ++q) mma_16816(acc[q & 1], f[q], bf[q].x, bf[q].y);
             }
         }
         done += len;

@@ -30,7 +30,6 @@ constexpr int kDumpThreads = (kConsumers + 1) * 32;  // decode warps + epilogue 
 constexpr uint32_t kEmptyWord = 0xFFFFFFFFu;      // a partial-plane word nobody has written yet
 constexpr int kActBytes = 64 * 1024;             // core input a CTA can stage
 constexpr size_t kGemvSmemLimit = 200 * 1024;    // dynamic shared memory a launch may ask for
-constexpr int kTilesInFlight = 2;                // independent tile decodes per warp
 
 struct GemvArgs {
     LinearCall call;
@@ -285,19 +284,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_row_kernel(const GemvArgs ar
             if (!ok) break;
             slot += 2;
             while (slot >= stages) { slot -= stages; use ^= 1; }
-            const uint32_t* tiles = reinterpret_cast<const uint32_t*>(ring + (size_t)st * kStage) + ctile * tile_words(K);
+            const uint32_t* tiles = reinterpret_cast<const uint32_t*>(ring + (size_t)st * kStage) + ctile * quad_words(K);
             const uint2* bsrc = act_lane + (size_t)(hb0 + b) * 32;
 #pragma unroll
-            for (int kt = 0; kt < 8; kt += kTilesInFlight) {
-                uint32_t f[kTilesInFlight][4];
-                uint2 bf[kTilesInFlight];
+            for (int half = 0; half < 2; ++half) {  // four independent tiles in flight
+                uint32_t f[4][4];
+                decode_quad_frag<K, CB>(tiles + half * 8 * quad_words(K), geom, f);
 #pragma unroll
-                for (int q = 0; q < kTilesInFlight; ++q) {
-                    decode_tile_frag<K, CB>(tiles + (kt + q) * 8 * tile_words(K), geom, f[q]);
-                    bf[q] = bsrc[(kt + q) * 4];
+                for (int t = 0; t < 4; ++t) {
+                    const uint2 bf = bsrc[(half * 4 + t) * 4];
+                    mma_16816(acc[t & 1], f[t], bf.x, bf.y);
                 }
-#pragma unroll
-                for (int q = 0; q < kTilesInFlight; ++q) mma_16816(acc[q & 1], f[q], bf[q].x, bf[q].y);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(empty0 + 8 * st);

@@ -42,16 +42,17 @@ __device__ __forceinline__ bool consume(const unsigned char* ring, int stage_str
     uint32_t use = 0;  // ring slot and use parity of unit i, stepped without divisions
     for (int i = 0; i < nblk; ++i, st = (st + 1 == stages ? 0 : st + 1), use ^= (st == 0)) {
         if (!mbar_wait(full0 + 8 * st, use, status, kTimeoutRingFull)) return false;
-        const uint32_t* tiles = reinterpret_cast<const uint32_t*>(ring + (size_t)st * stage_stride) + warp * tile_words(K);
+        const uint32_t* tiles = reinterpret_cast<const uint32_t*>(ring + (size_t)st * stage_stride) + warp * quad_words(K);
         const uint2* bsrc = act_lane + (size_t)i * rows * 32;
 #pragma unroll
-        for (int kt = 0; kt < 8; kt += 2) {
-            uint32_t fa[4], fb[4];
-            decode_tile_frag<K, CB>(tiles + kt * 8 * tile_words(K), geom, fa);
-            decode_tile_frag<K, CB>(tiles + (kt + 1) * 8 * tile_words(K), geom, fb);
-            const uint2 ba = bsrc[kt * 4], bb = bsrc[(kt + 1) * 4];
-            mma_16816(acc[0], fa, ba.x, ba.y);
-            mma_16816(acc[1], fb, bb.x, bb.y);
+        for (int half = 0; half < 2; ++half) {
+            uint32_t f[4][4];
+            decode_quad_frag<K, CB>(tiles + half * 8 * quad_words(K), geom, f);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const uint2 b = bsrc[(half * 4 + t) * 4];
+                mma_16816(acc[t & 1], f[t], b.x, b.y);
+            }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(empty0 + 8 * st);

@@ -9,18 +9,19 @@
 
 namespace st {
 
-// ---- regroup: [I/16][N/16][W] -> [N/128][I/16][8][W], W = 8*bits words ------------
+// ---- regroup: [I/16][N/16][W] -> [N/128][I/64][8][W][4], W words a tile: quads (trellis_decode.cuh) ----
 __global__ void regroup_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst,
                                int ktiles, int ntiles, int words) {
     // One thread per word; consecutive threads walk consecutive destination words.
     const long long total = (long long)ktiles * ntiles * words;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
-        const int word = (int)(i % words);
-        long long t = i / words;
+        const int in_quad = (int)(i & 3);
+        long long t = i >> 2;
+        const int word = (int)(t % words); t /= words;
         const int sub = (int)(t % 8); t /= 8;
-        const int kt = (int)(t % ktiles);
-        const int nb = (int)(t / ktiles);
+        const int kt = (int)(t % (ktiles / 4)) * 4 + in_quad;
+        const int nb = (int)(t / (ktiles / 4));
         dst[i] = src[((long long)kt * ntiles + nb * 8 + sub) * words + word];
     }
 }
@@ -36,9 +37,9 @@ cudaError_t launch_regroup(const uint32_t* src, uint32_t* dst, int inputs, int o
     return cudaGetLastError();
 }
 
-__device__ __forceinline__ const uint32_t* tile_ptr(const DeviceWeights& w, int kt, int nt) {
-    const int words = tile_words(w.bits), ktiles = w.inputs / 16;
-    return w.packed + (((long long)(nt >> 3) * ktiles + kt) * 8 + (nt & 7)) * words;
+// The quad that holds tile (kt, nt), as its tile kt % 4.
+__device__ __forceinline__ const uint32_t* quad_ptr(const DeviceWeights& w, int kt, int nt) {
+    return w.packed + (((long long)(nt >> 3) * (w.inputs / 64) + (kt >> 2)) * 8 + (nt & 7)) * quad_words(w.bits);
 }
 
 // ---- dequantise: one warp per tile, through decode_tile_frag ------------------------
@@ -51,7 +52,7 @@ __global__ void dequantize_kernel(DeviceWeights w, uint16_t* __restrict__ q) {
          t += (long long)gridDim.x * (blockDim.x >> 5)) {
         const int kt = (int)(t / ntiles), nt = (int)(t % ntiles);
         uint32_t frag[4];
-        decode_tile_frag<K, CB>(tile_ptr(w, kt, nt), lane, frag);
+        decode_tile_frag<K, CB>(quad_ptr(w, kt, nt), kt & 3, lane, frag);
         // frag order -> stream positions: frag[0]=(0,1) frag[2]=(2,3) frag[1]=(4,5) frag[3]=(6,7)
         const uint32_t by_pos[4] = {frag[0], frag[2], frag[1], frag[3]};
 #pragma unroll
@@ -191,7 +192,7 @@ __global__ void core_exact_kernel(DeviceWeights w, const uint16_t* __restrict__ 
     for (int i = 0; i < 32; ++i) acc[i] = 0.f;
     for (int kt = 0; kt < w.inputs / 16; ++kt) {
         uint32_t frag[4];
-        decode_tile_frag<K, CB>(tile_ptr(w, kt, nt), lane, frag);
+        decode_tile_frag<K, CB>(quad_ptr(w, kt, nt), kt & 3, lane, frag);
         const uint32_t by_pos[4] = {frag[0], frag[2], frag[1], frag[3]};
         __syncwarp();
 #pragma unroll
@@ -258,7 +259,7 @@ constexpr int kProbeUnits = 2;
 template <int K, int CB, int kWarps>
 __global__ void __launch_bounds__(kWarps * 32) decode_rate_kernel(const DeviceWeights w, int iters, float* sink,
                                                                        long long* clocks) {
-    extern __shared__ uint32_t probe_smem[];
+    extern __shared__ __align__(16) uint32_t probe_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kUnitWords = unit_bytes(K) / 4;
     const long long have = (long long)w.inputs * w.outputs / 256 * tile_words(K);  // words in the packed stream
@@ -269,14 +270,13 @@ __global__ void __launch_bounds__(kWarps * 32) decode_rate_kernel(const DeviceWe
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     const long long t0 = clock64();
     for (int it = 0; it < iters; ++it) {
-        const uint32_t* tiles = probe_smem + (it & (kProbeUnits - 1)) * kUnitWords + (warp & 7) * tile_words(K);
+        const uint32_t* tiles = probe_smem + (it & (kProbeUnits - 1)) * kUnitWords + (warp & 7) * quad_words(K);
 #pragma unroll
-        for (int kt = 0; kt < 8; kt += 2) {
-            uint32_t fa[4], fb[4];
-            decode_tile_frag<K, CB>(tiles + kt * 8 * tile_words(K), geom, fa);
-            decode_tile_frag<K, CB>(tiles + (kt + 1) * 8 * tile_words(K), geom, fb);
-            mma_16816(acc[0], fa, b0, b1);
-            mma_16816(acc[1], fb, b0, b1);
+        for (int half = 0; half < 2; ++half) {
+            uint32_t f[4][4];
+            decode_quad_frag<K, CB>(tiles + half * 8 * quad_words(K), geom, f);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) mma_16816(acc[t & 1], f[t], b0, b1);
         }
     }
     const long long t1 = clock64();

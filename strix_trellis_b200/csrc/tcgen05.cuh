@@ -103,12 +103,12 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
 }
 // 16 lanes x 32 columns stored: thread 4r + q holds, in registers 2m and 2m+1, column 4m + q of rows
 // r and r + 8 -- four decoded tiles in mma A-fragment order are one K = 64 slice of an A operand.
-__device__ __forceinline__ void tmem_st_16x32(uint32_t taddr, const uint32_t (&r)[16]) {
+__device__ __forceinline__ void tmem_st_16x32(uint32_t taddr, const uint32_t (&r)[4][4]) {
     asm volatile(
         "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], "
         "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+        ::"r"(taddr), "r"(r[0][0]), "r"(r[0][1]), "r"(r[0][2]), "r"(r[0][3]), "r"(r[1][0]), "r"(r[1][1]), "r"(r[1][2]), "r"(r[1][3]),
+          "r"(r[2][0]), "r"(r[2][1]), "r"(r[2][2]), "r"(r[2][3]), "r"(r[3][0]), "r"(r[3][1]), "r"(r[3][2]), "r"(r[3][3]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");

@@ -42,21 +42,15 @@ __device__ __forceinline__ bool decode_segment(DecodeState& s, int until, const 
         if (s.a_used && !mbar_wait(a_empty + 8 * stage, s.a_prev, status, kTimeoutTensorPipe))
             return false;
         tc_fence_after_sync();
-        const uint32_t* tiles = reinterpret_cast<const uint32_t*>(ring + (size_t)s.slot * w_stride) + ctile * tile_words(K);
+        const uint32_t* tiles = reinterpret_cast<const uint32_t*>(ring + (size_t)s.slot * w_stride) + ctile * quad_words(K);
         uint32_t to = taddr + stage * 64;
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c, tiles += tile_words(K), to += 16u << 16) {
+        for (int c = 0; c < 2; ++c, tiles += quad_words(K), to += 16u << 16) {
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                uint32_t r[16];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    uint32_t f[4];
-                    decode_tile_frag<K, CB>(tiles + (half * 4 + t) * 8 * tile_words(K), geom, f);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) r[4 * t + j] = f[j];
-                }
-                tmem_st_16x32(to + half * 32, r);
+                uint32_t f[4][4];
+                decode_quad_frag<K, CB>(tiles + half * 8 * quad_words(K), geom, f);
+                tmem_st_16x32(to + half * 32, f);
             }
         }
         if (lane == 0) mbar_arrive(w_empty + 8 * s.slot);

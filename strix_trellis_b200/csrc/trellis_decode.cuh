@@ -43,32 +43,69 @@ template <int K> struct Ring {
         return most;
     }
     static constexpr int kLoadWords = (max_offset() + kSpan <= 64) ? 2 : 3;
+    // Three-word rates whose span fits 64 bits are aligned by their END: the last bit of state 7 comes
+    // to bit kTail of the low word of a pair, two funnel shifts instead of three operations.  kTail = 2 at
+    // six bits puts two of the eight states on byte boundaries (one operation each instead of two).
+    static constexpr int kTail = K == 6 ? 2 : 0;
+    static constexpr bool kFromEnd = kLoadWords == 3 && kSpan + kTail <= 64;
+    __host__ __device__ static constexpr int end_bit(int lane) { return (lane + 1) * kLaneBits + kTail; }
 };
 static_assert(Ring<1>::kLoadWords == 2 && Ring<3>::kLoadWords == 2 && Ring<4>::kLoadWords == 2 &&
               Ring<5>::kLoadWords == 3 && Ring<8>::kLoadWords == 3 && Ring<9>::kLoadWords == 2 &&
               Ring<10>::kLoadWords == 2 && Ring<11>::kLoadWords == 3, "window words");
+static_assert(Ring<5>::kFromEnd && Ring<6>::kFromEnd && Ring<11>::kFromEnd && !Ring<7>::kFromEnd && !Ring<8>::kFromEnd, "alignment");
 
 // Per-lane constants of the window: word indices (with ring wrap) and the in-word bit
-// offset.  Computed once per thread, outside every loop.
+// offset (of the start or, kFromEnd, from the end; K = 3 uses both).  Computed once per thread, outside every loop.
 template <int K> struct LaneGeom {
-    int i0, i1, i2, shift;
+    int i0, i1, i2, shift, back;
     __device__ __forceinline__ explicit LaneGeom(int lane) {
-        const int s = Ring<K>::start_bit(lane);
-        i0 = s >> 5;
-        i1 = (i0 + 1 == Ring<K>::kWords) ? 0 : i0 + 1;
-        i2 = (i1 + 1 == Ring<K>::kWords) ? 0 : i1 + 1;
-        shift = s & 31;
+        if constexpr (Ring<K>::kFromEnd) {
+            const int e = Ring<K>::end_bit(lane);
+            i2 = ((e - 1) >> 5) % Ring<K>::kWords;
+            i1 = i2 ? i2 - 1 : Ring<K>::kWords - 1;
+            i0 = i1 ? i1 - 1 : Ring<K>::kWords - 1;
+            shift = back = -e & 31;
+        } else {
+            const int s = Ring<K>::start_bit(lane);
+            i0 = s >> 5;
+            i1 = (i0 + 1 == Ring<K>::kWords) ? 0 : i0 + 1;
+            i2 = (i1 + 1 == Ring<K>::kWords) ? 0 : i1 + 1;
+            shift = s & 31;
+            back = -Ring<K>::end_bit(lane) & 31;
+        }
     }
 };
 
-// The three (or two) ring words of a lane, read from a tile that starts at `tile`
-// (shared or global memory, 4-byte aligned).
+// ---- prepared tiles: quads ------------------------------------------------------
+// Four k-tiles of one column tile are stored word by word in turn: word i of tile t of a quad is at
+// 4 i + t.  A lane then reads its window of all four by two or three 16-byte loads instead of eight or twelve
+// loads of a word.  Clocks per tile per SM sub-partition at K2 / K3 / K4 / K5 / K6, tiles into tensor memory,
+// 16 warps per SM, each with the better split between the pipes (Balance) and the extraction of K3 and K6 that
+// was there then: plain tiles 41.5 / 48.6 / 41.2 / 49.9 / 54.0, quads 40.2 / 45.9 / 39.5 / 47.9 / 52.6.
+ST_RATE_FN int quad_words(int code) { return 4 * tile_words(code); }
+
+// The three (or two) ring words of a lane for tile t of a quad (global or shared memory, 4-byte aligned).
 template <int K>
-__device__ __forceinline__ void load_window(const uint32_t* tile, const LaneGeom<K>& g, uint32_t (&w)[3]) {
-    w[0] = tile[g.i0];
-    w[1] = tile[g.i1];
-    if constexpr (Ring<K>::kLoadWords == 3) w[2] = tile[g.i2];
+__device__ __forceinline__ void load_window(const uint32_t* quad, int t, const LaneGeom<K>& g, uint32_t (&w)[3]) {
+    w[0] = quad[4 * g.i0 + t];
+    w[1] = quad[4 * g.i1 + t];
+    if constexpr (Ring<K>::kLoadWords == 3) w[2] = quad[4 * g.i2 + t];
     else w[2] = 0;
+}
+// The same for all four tiles (16-byte aligned).
+template <int K>
+__device__ __forceinline__ void load_windows(const uint32_t* quad, const LaneGeom<K>& g, uint32_t (&w)[4][3]) {
+    const uint4* q = reinterpret_cast<const uint4*>(quad);
+    const uint4 a = q[g.i0], b = q[g.i1];
+    w[0][0] = a.x; w[1][0] = a.y; w[2][0] = a.z; w[3][0] = a.w;
+    w[0][1] = b.x; w[1][1] = b.y; w[2][1] = b.z; w[3][1] = b.w;
+    if constexpr (Ring<K>::kLoadWords == 3) {
+        const uint4 c = q[g.i2];
+        w[0][2] = c.x; w[1][2] = c.y; w[2][2] = c.z; w[3][2] = c.w;
+    } else {
+        w[0][2] = w[1][2] = w[2][2] = w[3][2] = 0;
+    }
 }
 
 // ---- state extraction ---------------------------------------------------------
@@ -76,9 +113,8 @@ __device__ __forceinline__ void load_window(const uint32_t* tile, const LaneGeom
 // the 16 bits at offset j*K of the big-endian bit string a[0]:a[1]:a[2].
 template <int K>
 __device__ __forceinline__ void align_window(const uint32_t (&w)[3], const LaneGeom<K>& g, uint32_t (&a)[3]) {
-    // In-word offsets: K=4 -> 20 and K=8 -> 24 for every lane; other rates depend on
-    // lane%4 (odd K) or lane%2 (K=2,6).
-    const int o = (K == 4) ? 20 : (K == 8) ? 24 : g.shift;
+    // In-word offsets: K=8 -> 24 for every lane; other rates depend on lane%4 (odd K).
+    const int o = (K == 8) ? 24 : g.shift;
     a[0] = __funnelshift_l(w[1], w[0], o);
     if constexpr (Ring<K>::kLoadWords == 3) {
         a[1] = __funnelshift_l(w[2], w[1], o);
@@ -99,9 +135,21 @@ __device__ __forceinline__ uint32_t field16(const uint32_t (&a)[3]) {
     else if constexpr (sh < 16) return (a[idx] >> (16 - sh)) & 0xFFFFu;
     else return __funnelshift_l(a[idx + 1], a[idx], sh) >> 16;
 }
+// 16-bit field whose last bit is bit P of hi:lo, zero-extended.
+template <int P>
+__device__ __forceinline__ uint32_t field16_up(uint32_t lo, uint32_t hi) {
+    constexpr int sh = P & 31;
+    const uint32_t word = P < 32 ? lo : hi;
+    if constexpr (sh == 0) return word & 0xFFFFu;
+    else if constexpr (sh == 8) return __byte_perm(word, 0, 0x4421);
+    else if constexpr (sh == 16) return word >> 16;
+    else if constexpr (sh < 16) return (word >> sh) & 0xFFFFu;
+    else return __funnelshift_r(lo, hi, sh) & 0xFFFFu;
+}
 
 template <int K>
 __device__ __forceinline__ void extract_states(const uint32_t (&w)[3], const LaneGeom<K>& g, uint32_t (&s)[8]) {
+    using R = Ring<K>;
     if constexpr (K == 4) {
         // Every lane's window is bits [20, 64) of w0:w1.  With U = bits [16,48) of the
         // pair, three shifts make all eight states byte aligned: 11 integer ops in all.
@@ -114,38 +162,38 @@ __device__ __forceinline__ void extract_states(const uint32_t (&w)[3], const Lan
         s[2] = u4 & 0xFFFFu;
         s[1] = __byte_perm(u, 0, 0x4421);
         s[0] = __byte_perm(u4, 0, 0x4421);
-        return;
-    }
-    uint32_t a[3];
-    align_window<K>(w, g, a);
-    if constexpr (K == 2 || K == 6) {
-        // Even rates: states at the same bit residue mod 8 share one pre-shifted copy
-        // of the window, after which every state is a single byte permute.
-        constexpr int step = 2;  // distinct residues {0,2,4,6}
+    } else if constexpr (K == 2) {
+        // The window is the first 30 bits of one word; states at the same bit residue mod 8 share a
+        // shifted copy: 12 ops.
+        const uint32_t a = __funnelshift_l(w[1], w[0], g.shift);
 #pragma unroll
-        for (int r = 0; r < 8; r += step) {
-            uint32_t b[3];
-            if (r == 0) { b[0] = a[0]; b[1] = a[1]; b[2] = a[2]; }
-            else {
-                b[0] = __funnelshift_l(a[1], a[0], r);
-                b[1] = __funnelshift_l(a[2], a[1], r);
-                b[2] = a[2] << r;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if ((j * K) % 8 == r) {
-                    const int p = j * K - r;  // byte aligned in b
-                    const int idx = p >> 5, sh = p & 31;
-                    // sh == 24 straddles two words: a byte permute has no zero source
-                    // left, so that one case costs a funnel shift plus a shift.
-                    s[j] = sh == 0 ? b[idx] >> 16
-                         : sh == 8 ? __byte_perm(b[idx], 0, 0x4421)
-                         : sh == 16 ? (b[idx] & 0xFFFFu)
-                         : __funnelshift_l(b[idx + 1 > 2 ? 2 : idx + 1], b[idx], 24) >> 16;
-                }
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t b = a << (2 * j);
+            s[j] = b >> 16;
+            s[j + 4] = __byte_perm(b, 0, 0x4421);
         }
+    } else if constexpr (K == 3) {
+        // 37 bits: the first two states from a word aligned by the start, the others from one aligned by
+        // the end: 16 ops (17 from one alignment).
+        const uint32_t a = __funnelshift_l(w[1], w[0], g.shift), b = __funnelshift_r(w[1], w[0], g.back);
+        s[0] = a >> 16;
+        s[1] = (a >> 13) & 0xFFFFu;
+        s[2] = (b >> 15) & 0xFFFFu;
+        s[3] = (b >> 12) & 0xFFFFu;
+        s[4] = (b >> 9) & 0xFFFFu;
+        s[5] = (b >> 6) & 0xFFFFu;
+        s[6] = (b >> 3) & 0xFFFFu;
+        s[7] = b & 0xFFFFu;
+    } else if constexpr (R::kFromEnd) {
+        const uint32_t lo = __funnelshift_r(w[2], w[1], g.back), hi = __funnelshift_r(w[1], w[0], g.back);
+        constexpr int last = R::field_pos(7) + R::kTail;
+        s[0] = field16_up<last - R::field_pos(0)>(lo, hi); s[1] = field16_up<last - R::field_pos(1)>(lo, hi);
+        s[2] = field16_up<last - R::field_pos(2)>(lo, hi); s[3] = field16_up<last - R::field_pos(3)>(lo, hi);
+        s[4] = field16_up<last - R::field_pos(4)>(lo, hi); s[5] = field16_up<last - R::field_pos(5)>(lo, hi);
+        s[6] = field16_up<last - R::field_pos(6)>(lo, hi); s[7] = field16_up<last - R::field_pos(7)>(lo, hi);
     } else {
-        using R = Ring<K>;
+        uint32_t a[3];
+        align_window<K>(w, g, a);
         s[0] = field16<R::field_pos(0)>(a); s[1] = field16<R::field_pos(1)>(a);
         s[2] = field16<R::field_pos(2)>(a); s[3] = field16<R::field_pos(3)>(a);
         s[4] = field16<R::field_pos(4)>(a); s[5] = field16<R::field_pos(5)>(a);
@@ -159,21 +207,39 @@ __device__ __forceinline__ uint32_t as_u32(__half2 h) { return *reinterpret_cast
 // ---- codebooks ------------------------------------------------------------------
 // mul1: p = s*0x83DCD12D, b = byte sum, value = fma(half(1024+b), 0x1EEE, 0xC931) with
 // ONE rounding.  A byte sum with accumulator 0x6400 yields the bit pattern of half(1024+b)
-// directly (b <= 1020).  The multiply, dp4a, the packing multiply-add and HFMA2 all issue on
-// the same half-rate pipe, so one of the two byte sums of a pair goes through the video
-// instruction vabsdiff4 (sum of |byte - 0|), which issues on the other integer pipe:
-// measured 49.6 against 52.0 clocks per K4 tile per scheduler.  Two states share one HFMA2.
+// directly (b <= 1020).  Two states share one HFMA2.
+//
+// Two pipes carry this, two clocks an instruction each (measured, clocks for one of each: IMAD + PRMT 2.0,
+// IMAD + DP4A 4.0, IMAD + HFMA2 4.0, PRMT + VABSDIFF4 4.0, PRMT + SHF 4.0): IMAD, DP4A and HFMA2 issue on
+// one, shifts, logic, PRMT and VABSDIFF4 on the other.  A byte sum may be a DP4A or a VABSDIFF4 (sum of
+// |byte - 0|), the packing of a pair an IMAD (d1*65536 + d0) or a PRMT, so the two kinds are dealt out
+// until the pipes carry the same, which depends on what extracting the states takes; the kernels' own address and
+// counter arithmetic is on the pipe of the shifts, so they want fewer sums there than the decoder alone (which is best at
+// five sums and two packings at K4).  Measured, us with (sums, packings) and with the (4, 0) that every rate had:
+// 4096 -> 129280, one row: K2 (4, 4) 99.8, 99.3; K3 (2, 0) 111.8, 114.5; K4 (3, 1) 95.0, 96.3; K5 (2, 0) 111.7, 118.7;
+// K6 (2, 0) 111.2, 115.8; eight tokens on an expert bank, K2: 188 and 190; the other rates by the count of their operations.
+template <int K> struct Balance {
+    // of the eight byte sums / four packings of a lane, those on the pipe of the shifts
+    static constexpr int kSums = K == 2 ? 4 : K == 1 || K == 4 || K == 8 || K == 9 || K == 10 ? 3 : K == 7 || K == 11 ? 1 : 2;
+    static constexpr int kPacks = K == 2 ? 4 : K == 4 || K == 8 ? 1 : 0;
+};
+
 __device__ __forceinline__ uint32_t bytesum_alu(uint32_t p) {
     uint32_t d;
     asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %3;" : "=r"(d) : "r"(p), "r"(0u), "r"(0x6400u));
     return d;
 }
+template <bool ALU> __device__ __forceinline__ uint32_t bytesum(uint32_t p) {
+    return ALU ? bytesum_alu(p) : __dp4a(p, 0x01010101u, 0x6400u);
+}
+// Pair `I` of a lane's four: its first sum is number I of the eight, its second number I + 4.
+template <int SUMS, int PACKS, int I>
 __device__ __forceinline__ uint32_t mul1_pair(uint32_t s0, uint32_t s1) {
-    const uint32_t d0 = bytesum_alu(s0 * 0x83DCD12Du);
-    const uint32_t d1 = __dp4a(s1 * 0x83DCD12Du, 0x01010101u, 0x6400u);
-    // d0, d1 < 2^16: d1*65536 + d0 packs them
-    uint32_t packed;
-    asm("mad.lo.u32 %0, %1, 65536, %2;" : "=r"(packed) : "r"(d1), "r"(d0));
+    const uint32_t d0 = bytesum<(I < SUMS)>(s0 * 0x83DCD12Du);
+    const uint32_t d1 = bytesum<(I + 4 < SUMS)>(s1 * 0x83DCD12Du);
+    uint32_t packed;  // d0, d1 < 2^16
+    if constexpr (I < PACKS) packed = __byte_perm(d0, d1, 0x5410);
+    else asm("mad.lo.u32 %0, %1, 65536, %2;" : "=r"(packed) : "r"(d1), "r"(d0));
     const __half2 v = __hfma2(as_h2(packed), as_h2(0x1EEE1EEEu), as_h2(0xC931C931u));
     return as_u32(v);
 }
@@ -189,39 +255,39 @@ __device__ __forceinline__ uint32_t mix_pair(uint32_t s0, uint32_t s1) {
     const uint32_t hi = __byte_perm(q0, q1, 0x7632);  // (hi16 q0, hi16 q1)
     return as_u32(__hadd2(as_h2(lo), as_h2(hi)));
 }
-template <int CB>
+template <int K, int CB, int I>
 __device__ __forceinline__ uint32_t codebook_pair(uint32_t s0, uint32_t s1) {
-    if constexpr (CB == CB_MUL1) return mul1_pair(s0, s1);
+    if constexpr (CB == CB_MUL1) return mul1_pair<Balance<K>::kSums, Balance<K>::kPacks, I>(s0, s1);
     else return mix_pair<CB>(s0, s1);
 }
 
-// Decode the lane's eight weights of one tile into mma A-fragment order.
-template <int K, int CB>
-__device__ __forceinline__ void decode_tile_frag(const uint32_t* tile, const LaneGeom<K>& g, uint32_t (&frag)[4]) {
-    uint32_t w[3], s[8];
-    load_window<K>(tile, g, w);
-    extract_states<K>(w, g, s);
-    frag[0] = codebook_pair<CB>(s[0], s[1]);
-    frag[2] = codebook_pair<CB>(s[2], s[3]);
-    frag[1] = codebook_pair<CB>(s[4], s[5]);
-    frag[3] = codebook_pair<CB>(s[6], s[7]);
-}
-
-// The same from ring words that are already in registers (software-pipelined callers).
+// The lane's eight weights of one tile, from its ring words, in mma A-fragment order.
 template <int K, int CB>
 __device__ __forceinline__ void decode_words_frag(const uint32_t (&w)[3], const LaneGeom<K>& g, uint32_t (&frag)[4]) {
     uint32_t s[8];
     extract_states<K>(w, g, s);
-    frag[0] = codebook_pair<CB>(s[0], s[1]);
-    frag[2] = codebook_pair<CB>(s[2], s[3]);
-    frag[1] = codebook_pair<CB>(s[4], s[5]);
-    frag[3] = codebook_pair<CB>(s[6], s[7]);
+    frag[0] = codebook_pair<K, CB, 0>(s[0], s[1]);
+    frag[2] = codebook_pair<K, CB, 1>(s[2], s[3]);
+    frag[1] = codebook_pair<K, CB, 2>(s[4], s[5]);
+    frag[3] = codebook_pair<K, CB, 3>(s[6], s[7]);
 }
 
+// The four tiles of a quad.
 template <int K, int CB>
-__device__ __forceinline__ void decode_tile_frag(const uint32_t* tile, int lane, uint32_t (&frag)[4]) {
+__device__ __forceinline__ void decode_quad_frag(const uint32_t* quad, const LaneGeom<K>& g, uint32_t (&frag)[4][4]) {
+    uint32_t w[4][3];
+    load_windows<K>(quad, g, w);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) decode_words_frag<K, CB>(w[t], g, frag[t]);
+}
+
+// Tile t of a quad alone (the probes).
+template <int K, int CB>
+__device__ __forceinline__ void decode_tile_frag(const uint32_t* quad, int t, int lane, uint32_t (&frag)[4]) {
     const LaneGeom<K> g(lane);
-    decode_tile_frag<K, CB>(tile, g, frag);
+    uint32_t w[3];
+    load_window<K>(quad, t, g, w);
+    decode_words_frag<K, CB>(w, g, frag);
 }
 
 // Logical coordinates of stream position 8*lane+j (docs/FORMAT.md:61-66).
