@@ -35,7 +35,7 @@ namespace st {
 
 namespace {
 constexpr int kUnitGroups = 4, kDecodeT = 4 * kUnitGroups, kHelpersT = 8;
-constexpr int kWarpMmaT = kDecodeT + kHelpersT, kWarpWeightsT = kWarpMmaT + 1;
+constexpr int kWarpMmaT = kDecodeT + kHelpersT, kWarpWeightsT = kWarpMmaT + kIssuers;
 constexpr int kThreadsT = (kWarpWeightsT + 1) * 32;
 constexpr int kRowsT = 16;                       // the MMA's N: the smallest it has; rows beyond the call's are never read
 constexpr int kMaxRowsT = 8;
@@ -47,9 +47,12 @@ constexpr int kMaxRowsT = 8;
 // 4.5e-7.  Four take 119.2 us instead of 118.0 for the first of these and 22.0 instead of 21.65 for the second.
 constexpr int kChains = 4, kAStagesT = 6;
 static_assert(kAStagesT * 64 + 2 * kChains * kRowsT <= 512 && kAStagesT >= kUnitGroups && kAStagesT <= kMaxAStages, "tensor memory");
-constexpr int kSlotBytesT = kRowsT * 256;        // activation operand of one H128 block
+// Activation operand of one H128 block: eight rows of both K = 64 halves.  The MMA's rows 8 to 15 are whatever
+// lies behind (the other half, the next slot, the weight ring): columns of the sums that nobody reads.  With room
+// for sixteen rows a layer of 4096 inputs left the weight ring 80 KB, too little for the trip to DRAM.
+constexpr int kSlotBytesT = kMaxRowsT * 256;
 constexpr int kStageFloats = kMaxRowsT * 128;    // transposition space of one helper group
-constexpr int kMaxWSlotsT = 32, kMaxBSlotsT = 48;
+constexpr int kMaxWSlotsT = 32, kMaxBSlotsT = 80;
 constexpr int kHeaderT = 2048 + 2 * kStageFloats * 4;
 constexpr size_t kSmemLimitT = 224 * 1024;
 constexpr uint32_t kEmptyWord = 0xFFFFFFFFu;      // a plane word nobody has written yet
@@ -123,7 +126,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
             for (int i = 0; i < first && i < my_units; ++i) load_unit(i, i);
     } else if (warp == kWarpMmaT) {
         tmem_alloc(smem_u32(&s_tmem_base), 512);
-    } else if (warp >= kDecodeT) {
+    } else if (warp >= kDecodeT && warp < kWarpMmaT) {
         // Scales of the first elements; the activations may be asked for early too (the L2 is the point
         // of coherence, so a line the previous kernel still writes is read correctly afterwards).
         load_scales(4 * h + e8);
@@ -135,11 +138,11 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
             if (l8 < x_bytes)
                 prefetch_line_l2(reinterpret_cast<const unsigned char*>(c.x) + ((size_t)row * c.x_stride + (size_t)hb * 128) * x_bytes + l8 * 128);
         }
-    } else {  // one decode thread per barrier
+    } else {  // one decode thread per barrier (and the second issuer, which has none)
         const int t = threadIdx.x;
         if (t < args.b_slots) { mbar_init(b_full + 8 * t, rows); mbar_init(b_empty + 8 * t, 1); }
         if (t < kAStagesT) { mbar_init(a_full + 8 * t, 4); mbar_init(a_empty + 8 * t, 1); }
-        if (t < 2) { mbar_init(d_full + 8 * t, 1); mbar_init(d_empty + 8 * t, 4); }
+        if (t < 2) { mbar_init(d_full + 8 * t, kIssuers); mbar_init(d_empty + 8 * t, 4); }
         mbar_fence_init();
     }
     tc_fence_before_sync();
@@ -155,44 +158,47 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
             int slot = issued == args.w_slots ? 0 : issued;
             uint32_t prev_use = issued == args.w_slots ? 0 : 1;
             for (; issued < my_units; ++issued) {
-                if (issued >= args.w_slots && !mbar_wait(w_empty + 8 * slot, prev_use, c.status, kTimeoutRingEmpty)) break;
+                if (issued >= args.w_slots && !mbar_wait_long(w_empty + 8 * slot, prev_use, c.status, kTimeoutRingEmpty)) break;
                 load_unit(issued, slot);
                 if (++slot == args.w_slots) { slot = 0; prev_use ^= 1; }
             }
             for (int i = (issued > args.w_slots ? issued - args.w_slots : 0); i < issued; ++i)  // nothing still landing at exit
                 mbar_wait(w_full + 8 * (i % args.w_slots), (uint32_t)(i / args.w_slots) & 1, c.status, kTimeoutDrain);
         }
-    } else if (warp == kWarpMmaT) {
-        // ---- MMA issuer: the whole warp walks, an elected lane issues ------------------------------
+    } else if (warp >= kWarpMmaT) {
+        // ---- MMA issuers, a unit each in turn: the whole warp walks, an elected lane issues ---------
         constexpr uint32_t idesc = umma_idesc_f16_f32(128, kRowsT);
         const uint64_t b_desc = umma_desc_k_major_sw128(smem_u32(b_ring));
-        const int b_wrap = resident ? hblocks : args.b_slots;
-        int slot = 0, stage = 0, seg = 0;
+        const int me = warp - kWarpMmaT, b_wrap = resident ? hblocks : args.b_slots;
+        int next = me, slot = me % b_wrap, stage = me, seg = 0;  // of this warp's next unit
         uint32_t use = 0, a_use = 0;
         bool ok = true;
         for (int done = 0, hb = first_hb; done < my_units && ok; ++seg, hb = 0) {
             const int left = my_units - done, len = left < hblocks - hb ? left : hblocks - hb;
-            const uint32_t dcol = tmem + d_col + (seg & 1) * kChains * kRowsT;
-            if (seg >= 2 && !mbar_wait(d_empty + 8 * (seg & 1), (uint32_t)((seg >> 1) - 1) & 1, c.status, kTimeoutTensorPipe)) break;
-            for (int i = 0; i < len; ++i) {
-                if (!mbar_wait(b_full + 8 * slot, use, c.status, kTimeoutTensorPipe) ||
-                    !mbar_wait(a_full + 8 * stage, a_use, c.status, kTimeoutTensorPipe)) {
+            const uint32_t acc = tmem + d_col + ((seg & 1) * kChains + me * (kChains / kIssuers)) * kRowsT;
+            // (Waited for without a unit in the segment too: the other issuer's commit of the segment two back
+            // must have come before this one's.)
+            if (seg >= 2 && !mbar_wait_long(d_empty + 8 * (seg & 1), (uint32_t)((seg >> 1) - 1) & 1, c.status, kTimeoutTensorPipe)) break;
+            for (bool fresh = true; next < done + len; next += kIssuers, fresh = false) {
+                if (!mbar_wait_long(b_full + 8 * slot, use, c.status, kTimeoutTensorPipe) ||
+                    !mbar_wait_long(a_full + 8 * stage, a_use, c.status, kTimeoutTensorPipe)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after_sync();
                 const uint64_t b0 = b_desc + (uint32_t)(slot * (kSlotBytesT / 16));  // 16-byte units
-                const uint32_t acol = tmem + stage * 64, acc = dcol + (i & 1) * 2 * kRowsT;
+                const uint32_t acol = tmem + stage * 64;
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        umma_f16_ts(acc + (k & 1) * kRowsT, acol + 8 * k, b0 + (k < 4 ? 0 : kSlotBytesT / 32) + 2 * (k & 3), idesc, i > 1 || k > 1);
+                        umma_f16_ts(acc + (k & 1) * kRowsT, acol + 8 * k, b0 + (k < 4 ? 0 : kSlotBytesT / 32) + 2 * (k & 3), idesc, !fresh || k > 1);
                     umma_commit(a_empty + 8 * stage);
                     if (!resident) umma_commit(b_empty + 8 * slot);
                 }
                 __syncwarp();
-                if (++slot == b_wrap) { slot = 0; if (!resident) use ^= 1; }  // a resident slot is filled once
-                if (++stage == kAStagesT) { stage = 0; a_use ^= 1; }
+                for (slot += kIssuers; slot >= b_wrap; slot -= b_wrap)
+                    if (!resident) use ^= 1;  // a resident slot is filled once
+                if ((stage += kIssuers) >= kAStagesT) { stage -= kAStagesT; a_use ^= 1; }
             }
             if (elect_one()) umma_commit(d_full + 8 * (seg & 1));
             done += len;
@@ -249,28 +255,29 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
         }
 
         float* stage = reinterpret_cast<float*>(smem + 2048) + group * kStageFloats;
-        auto epilogue = [&](int seg, int nb, int hb0, int len) {
+        auto epilogue = [&](int seg, int nb, int hb0, int len, int start) {
             const int c0 = nb * 128 + 4 * l8;
             const bool contributor = hb0 != 0;
             int last = cta;
             if (!contributor && len < hblocks) last = owner(args.split, (nb + 1) * hblocks - 1);
-            bool good = mbar_wait(d_full + 8 * (seg & 1), (uint32_t)(seg >> 1) & 1, c.status, kTimeoutTensorPipe);
+            bool good = mbar_wait_long(d_full + 8 * (seg & 1), (uint32_t)(seg >> 1) & 1, c.status, kTimeoutTensorPipe);
             __syncwarp();
             tc_fence_after_sync();
             const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + d_col + (seg & 1) * kChains * kRowsT;
             float v[kMaxRowsT];
             uint32_t r[2][kMaxRowsT];
 #pragma unroll
-            for (int pair = 0; pair < 2; ++pair) {  // the chains of the even units, then (if there are any) of the odd ones
-                if (pair && len < 2) break;
+            for (int j = 0; j < kMaxRowsT; ++j) v[j] = 0.f;
+#pragma unroll
+            for (int pair = 0; pair < kIssuers; ++pair) {  // the chains of one issuer, then of the other: both if there are two units
+                if (len < 2 && pair != (start & 1)) continue;
                 tmem_ld_32x8(at + pair * 2 * kRowsT, r[0]);
                 tmem_ld_32x8(at + pair * 2 * kRowsT + kRowsT, r[1]);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < kMaxRowsT; ++j) {
                     asm volatile("" : "+r"(r[0][j]), "+r"(r[1][j]));  // not before the wait
-                    const float both = __fadd_rn(__uint_as_float(r[0][j]), __uint_as_float(r[1][j]));
-                    v[j] = pair ? __fadd_rn(v[j], both) : both;
+                    v[j] = __fadd_rn(v[j], __fadd_rn(__uint_as_float(r[0][j]), __uint_as_float(r[1][j])));
                 }
             }
             tc_fence_before_sync();
@@ -286,8 +293,6 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
                 }
                 return;
             }
-#pragma unroll
-            for (int j = 0; j < kMaxRowsT; ++j) v[j] = __fadd_rn(0.f, v[j]);
             // 16 words in flight, whatever the row count: R rows of 16 / R planes
             auto fold = [&](auto width) {
                 constexpr int R = decltype(width)::value, P = 16 / R;
@@ -368,15 +373,15 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
             const int left = my_units - done, len = left < hblocks - hb ? left : hblocks - hb;
             if (!resident) {
                 stage_elements(done * rows, (done + len) * rows);
-                if (seg && ((seg - 1) & 1) == group) epilogue(seg - 1, nb - 1, prev_hb, prev_len);
+                if (seg && ((seg - 1) & 1) == group) epilogue(seg - 1, nb - 1, prev_hb, prev_len, done - prev_len);
                 prev_hb = hb;
                 prev_len = len;
             } else if ((seg & 1) == group) {
-                epilogue(seg, nb, hb, len);
+                epilogue(seg, nb, hb, len, done);
             }
             done += len;
         }
-        if (!resident && ((seg - 1) & 1) == group) epilogue(seg - 1, nb - 1, prev_hb, prev_len);
+        if (!resident && ((seg - 1) & 1) == group) epilogue(seg - 1, nb - 1, prev_hb, prev_len, done - prev_len);
     }
 
     tc_fence_before_sync();

@@ -75,6 +75,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
     if (status) atomicOr(status, fail_bit);
     return false;
 }
+// The same for waits that are long as a rule (a role that is ahead of the others): it sleeps at once, since tries in a
+// loop take issue slots from the warps it waits for.
+__device__ __forceinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, unsigned int* status, unsigned int fail_bit) {
+    if (mbar_try(bar, parity)) return true;
+#pragma unroll 1
+    for (uint32_t i = 0; i < (1u << 17); ++i)
+        if (mbar_try_sleep(bar, parity)) return true;
+    if (status) atomicOr(status, fail_bit);
+    return false;
+}
 // Arrive on a barrier given by its shared::cluster address (see map_to_rank).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");

@@ -108,7 +108,7 @@ __device__ __forceinline__ void tmem_st_16x32(uint32_t taddr, const uint32_t (&r
         "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], "
         "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
         ::"r"(taddr), "r"(r[0][0]), "r"(r[0][1]), "r"(r[0][2]), "r"(r[0][3]), "r"(r[1][0]), "r"(r[1][1]), "r"(r[1][2]), "r"(r[1][3]),
-          "r"(r[2][0]), "r"(r[2][1]), "r"(r[2][2]), "r"(r[2][3]), "r"(r[3][0]), "r"(r[3][1]), "r"(r[3][2]), "r"(r[3][3]) : "memory");
+          "r"(r[2][0]), "r"(r[2][1]), "r"(r[2][2]), "r"(r[2][3]), "r"(r[3][0]), "r"(r[3][1]), "r"(r[3][2]), "r"(r[3][3]));
 }
 __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");

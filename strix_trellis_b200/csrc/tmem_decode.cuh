@@ -19,6 +19,7 @@
 namespace st {
 
 constexpr int kMaxAStages = 7;  // decoded units in tensor memory
+constexpr int kIssuers = 2;
 
 // Decodes this warp's two column tiles of the units of its turn in one segment:
 // two K = 64 halves per column tile, four tiles each, one tensor-memory store per half.

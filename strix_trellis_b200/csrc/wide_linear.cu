@@ -32,7 +32,7 @@ namespace st {
 
 namespace {
 constexpr int kUnitGroups = 4, kDecodeW = 4 * kUnitGroups, kEpiW = 4;
-constexpr int kWarpMma = kDecodeW + kEpiW, kWarpWeights = kWarpMma + 1, kWarpRows = kWarpMma + 2;
+constexpr int kWarpMma = kDecodeW + kEpiW, kWarpWeights = kWarpMma + kIssuers, kWarpRows = kWarpWeights + 1;
 constexpr int kThreadsW = (kWarpRows + 1) * 32;
 constexpr int kChunkRows = 16;                       // rows of one epilogue chunk
 constexpr int kStageFloats = kChunkRows * 128;       // 8 KB of transposition space per warp group
@@ -115,7 +115,7 @@ __device__ __forceinline__ void red_release_gpu(unsigned int* p, unsigned int v)
 template <bool PARTS>  // K in more than one part
 struct Epilogue {
     const WideArgs& a;
-    int cta, quarter, lane, bar;
+    int cta, origin, quarter, lane, bar;  // origin: first unit of the range
     float* areas;      // staging: two areas in turn (one barrier per chunk instead of two), or one
     int area_floats;   // from one to the other; 0: one
 
@@ -149,33 +149,43 @@ struct Epilogue {
             // Parts in ascending K order; the running sum of a column waits in its place in `stage`.
 #pragma unroll 1
             for (int part = first_part; part <= last_part; ++part) {
-                const uint32_t at = taddr + part * a.d_accs * a.n_max + ch * kChunkRows;
-                __syncwarp();
-                tmem_ld_32x16(at, r);
-                if (a.d_accs > 1) {
+                // The units of this part in this segment: from two on both issuers have had some.
+                const int lo = PARTS && part_begin(a, part) > w.hb ? part_begin(a, part) : w.hb;
+                const int hi = PARTS && part_begin(a, part + 1) < w.hb + len ? part_begin(a, part + 1) : w.hb + len;
+                const bool both = a.d_accs > 1 && hi - lo > 1;
+                const int set = a.d_accs > 1 && !both ? (w.unit - origin + lo - w.hb) & 1 : 0;
+                const uint32_t at = taddr + (part * a.d_accs + set * (a.d_accs >> 1)) * a.n_max + ch * kChunkRows;
+                auto add = [&](uint32_t from) {
                     uint32_t q[16];
-                    tmem_ld_32x16(at + a.n_max, q);
+                    tmem_ld_32x16(from, q);
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        asm volatile("" : "+r"(r[j]), "+r"(q[j]));  // not before the wait
+                        asm volatile("" : "+r"(q[j]), "+r"(r[j]));  // not before the wait
                         r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(q[j])));
                     }
+                };
+                __syncwarp();
+                tmem_ld_32x16(at, r);
+                if (!PARTS && a.d_accs == 4) {  // one layer of up to sixteen rows
+                    add(at + a.n_max);
+                    if (both) {
+                        uint32_t q[16], t[16];
+                        tmem_ld_32x16(at + 2 * a.n_max, q);
+                        tmem_ld_32x16(at + 3 * a.n_max, t);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            asm volatile("" : "+r"(q[j]), "+r"(t[j]));
+                            r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __fadd_rn(__uint_as_float(q[j]), __uint_as_float(t[j]))));
+                        }
+                    }
+                } else if (both) {
+                    add(at + a.n_max);
                 } else {
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(r[j]));
-                }
-                if (!PARTS && a.d_accs == 4) {  // one layer of up to sixteen rows
-                    uint32_t q[16], t[16];
-                    tmem_ld_32x16(at + 2 * a.n_max, q);
-                    tmem_ld_32x16(at + 3 * a.n_max, t);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        asm volatile("" : "+r"(q[j]), "+r"(t[j]));
-                        r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __fadd_rn(__uint_as_float(q[j]), __uint_as_float(t[j]))));
-                    }
                 }
                 if (PARTS && part != first_part)
 #pragma unroll
@@ -292,12 +302,13 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * kMaxWSlots, b_full = w_empty + 8 * kMaxWSlots,
                    b_empty = b_full + 8 * kMaxBSlots, a_full = b_empty + 8 * kMaxBSlots, a_empty = a_full + 8 * kMaxAStages,
                    d_full = a_empty + 8 * kMaxAStages, d_empty = d_full + 16, all_done = d_empty + 16;
+    const int issuers = args.d_accs > 1 ? kIssuers : 1;
     if (threadIdx.x == 0) {
         for (int i = 0; i < args.w_slots; ++i) { mbar_init(w_full + 8 * i, 1); mbar_init(w_empty + 8 * i, 4); }
         for (int i = 0; i < args.b_slots; ++i) { mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, 1); }
         for (int i = 0; i < a_stages; ++i) { mbar_init(a_full + 8 * i, 4); mbar_init(a_empty + 8 * i, 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, 1); mbar_init(d_empty + 8 * i, kEpiW); }
-        mbar_init(all_done, 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, issuers); mbar_init(d_empty + 8 * i, kEpiW); }
+        mbar_init(all_done, issuers);
         mbar_fence_init();
     }
     if (warp == kWarpMma) tmem_alloc(smem_u32(&s_tmem_base), 512);
@@ -323,7 +334,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                 const unsigned char* src = reinterpret_cast<const unsigned char*>(dw.packed) +
                                            ((size_t)w.nb * args.hblocks + w.hb) * bytes;
                 for (int i = 0; i < len; ++i, src += bytes) {
-                    if (issued >= args.w_slots && !mbar_wait(w_empty + 8 * slot, prev_use, args.status, kTimeoutRingEmpty)) {
+                    if (issued >= args.w_slots && !mbar_wait_long(w_empty + 8 * slot, prev_use, args.status, kTimeoutRingEmpty)) {
                         ok = false;
                         break;
                     }
@@ -348,7 +359,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                 const uint32_t bytes = (uint32_t)wide_tile_bytes(problem_rows(args, w.p));
                 const unsigned char* src = problem_tiles(args, w.p) + (size_t)w.hb * bytes;
                 for (int i = 0; i < len; ++i, src += bytes) {
-                    if (issued >= args.b_slots && !mbar_wait(b_empty + 8 * slot, prev_use, args.status, kTimeoutTensorPipe)) {
+                    if (issued >= args.b_slots && !mbar_wait_long(b_empty + 8 * slot, prev_use, args.status, kTimeoutTensorPipe)) {
                         ok = false;
                         break;
                     }
@@ -362,45 +373,50 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             for (int i = (issued > args.b_slots ? issued - args.b_slots : 0); i < issued; ++i)
                 mbar_wait(b_full + 8 * (i % args.b_slots), (uint32_t)(i / args.b_slots) & 1, args.status, kTimeoutDrain);
         }
-    } else if (warp == kWarpMma) {
-        // ---- MMA issuer: the whole warp walks, an elected lane issues -------------------------------
-        int slot = 0, stage = 0, seg = 0;
-        uint32_t use = 0, a_use = 0;
-        bool ok = true;
-        for (Walk w(args, mine); w.unit < w.end && ok; ++seg) {
-            const int len = w.length(args), n = wide_n(problem_rows(args, w.p));
-            const uint32_t idesc = umma_idesc_f16_f32(128, n), dcol = tmem + d_column(seg);
-            // K step k goes to accumulator k % d_accs
-            const uint32_t odd = args.d_accs > 1 ? args.n_max : 0, two = !PARTS && args.d_accs == 4 ? 2 * args.n_max : 0;
-            if (seg >= d_bufs && !mbar_wait(d_empty + 8 * d_index(seg), d_parity(seg) ^ 1, args.status, kTimeoutTensorPipe)) break;
-            int part = PARTS ? part_of(args, w.hb) : 0, fresh = 1;
-            for (int i = 0; i < len; ++i) {
-                if (PARTS && part_begin(args, part + 1) == w.hb + i) { ++part; fresh = 1; }
-                const uint32_t acc = dcol + part * args.d_accs * args.n_max;
-                if (!mbar_wait(b_full + 8 * slot, use, args.status, kTimeoutTensorPipe) ||
-                    !mbar_wait(a_full + 8 * stage, a_use, args.status, kTimeoutTensorPipe)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after_sync();
-                const uint32_t rows0 = smem_u32(b_ring) + slot * args.b_stride, acol = tmem + stage * 64;
-                const uint64_t b0 = umma_desc_k_major_sw128(rows0), b1 = umma_desc_k_major_sw128(rows0 + n * 128);
-                if (elect_one()) {
+    } else if (warp >= kWarpMma) {
+        // ---- MMA issuers, a unit each in turn: the whole warp walks, an elected lane issues ---------
+        const int me = warp - kWarpMma;
+        if (me < issuers) {
+            // K step k of a unit goes to accumulator `me` of two, or (four) 2 me + k % 2.
+            const uint32_t mine_acc = me * (args.d_accs >> 1) * args.n_max, odd = args.d_accs == 4 ? args.n_max : 0;
+            int next = me, slot = me, stage = me, seg = 0;  // of this warp's next unit
+            uint32_t use = 0, a_use = 0;
+            bool ok = true;
+            for (Walk w(args, mine); w.unit < w.end && ok; ++seg) {
+                const int len = w.length(args), n = wide_n(problem_rows(args, w.p)), start = w.unit - mine.begin;
+                const uint32_t idesc = umma_idesc_f16_f32(128, n), dcol = tmem + d_column(seg) + mine_acc;
+                // (Waited for without a unit in the segment too: the other issuer's commit of the buffer's segment
+                // before must have come before this one's.)
+                if (seg >= d_bufs && !mbar_wait_long(d_empty + 8 * d_index(seg), d_parity(seg) ^ 1, args.status, kTimeoutTensorPipe)) break;
+                int part = PARTS ? part_of(args, w.hb) : 0, fresh = 1;
+                for (; next < start + len; next += issuers) {
+                    while (PARTS && part_begin(args, part + 1) <= w.hb + next - start) { ++part; fresh = 1; }
+                    const uint32_t acc = dcol + part * args.d_accs * args.n_max;
+                    if (!mbar_wait_long(b_full + 8 * slot, use, args.status, kTimeoutTensorPipe) ||
+                        !mbar_wait_long(a_full + 8 * stage, a_use, args.status, kTimeoutTensorPipe)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    const uint32_t rows0 = smem_u32(b_ring) + slot * args.b_stride, acol = tmem + stage * 64;
+                    const uint64_t b0 = umma_desc_k_major_sw128(rows0), b1 = umma_desc_k_major_sw128(rows0 + n * 128);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        umma_f16_ts(acc + (k & 1) * odd + (k >> 1 & 1) * two, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, !fresh || k >= args.d_accs);
-                    umma_commit(a_empty + 8 * stage);
-                    umma_commit(b_empty + 8 * slot);
+                        for (int k = 0; k < 8; ++k)
+                            umma_f16_ts(acc + (k & 1) * odd, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, !fresh || k > 1 || (k == 1 && !odd));
+                        umma_commit(a_empty + 8 * stage);
+                        umma_commit(b_empty + 8 * slot);
+                    }
+                    __syncwarp();
+                    fresh = 0;
+                    if ((slot += issuers) >= args.b_slots) { slot -= args.b_slots; use ^= 1; }
+                    if ((stage += issuers) >= a_stages) { stage -= a_stages; a_use ^= 1; }
                 }
-                __syncwarp();
-                fresh = 0;
-                if (++slot == args.b_slots) { slot = 0; use ^= 1; }
-                if (++stage == a_stages) { stage = 0; a_use ^= 1; }
+                if (elect_one()) umma_commit(d_full + 8 * d_index(seg));
+                w.next(args, len);
             }
-            if (elect_one()) umma_commit(d_full + 8 * d_index(seg));
-            w.next(args, len);
+            if (elect_one()) umma_commit(all_done);
         }
-        if (elect_one()) umma_commit(all_done);
     } else if (warp >= kDecodeW) {
         // ---- epilogue group: every segment, all of it except the last, which the decoders share ----
         // Output scales and bias are cold in DRAM and needed at the very end: ask the L2 for them now.
@@ -410,12 +426,12 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             if (lane < 2) prefetch_line_l2(dw.svh + (size_t)nb * 128 + lane * 64);
             else if (lane < 6 && dw.bias) prefetch_line_l2(dw.bias + (size_t)nb * 128 + (lane - 2) * 32);
         }
-        const Epilogue<PARTS> epi{args, cta, warp & 3, lane, 1, epi_stage, kStageFloats};
+        const Epilogue<PARTS> epi{args, cta, mine.begin, warp & 3, lane, 1, epi_stage, kStageFloats};
         int seg = 0;
         for (Walk w(args, mine); w.unit < w.end; ++seg) {
             const int len = w.length(args);
             const bool final = w.unit + len == w.end;
-            const bool ok = mbar_wait(d_full + 8 * d_index(seg), d_parity(seg), args.status, kTimeoutTensorPipe);
+            const bool ok = mbar_wait_long(d_full + 8 * d_index(seg), d_parity(seg), args.status, kTimeoutTensorPipe);
             if (group_any(1, !ok)) break;
             tc_fence_after_sync();
             if (!epi.segment(split, w, len, tmem + d_column(seg), 0, final ? 1 + kDecodeW / 4 : 1, d_empty + 8 * d_index(seg))) break;
@@ -444,10 +460,10 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         const int group = warp >> 2;
         // (Not d_full: these warps may be several segments ahead of the accumulators, where its parity
         // would already look like the last segment's.)
-        if (ok) ok = mbar_wait(all_done, 0, args.status, kTimeoutTensorPipe);
+        if (ok) ok = mbar_wait_long(all_done, 0, args.status, kTimeoutTensorPipe);
         if (!group_any(2 + group, !ok)) {
             tc_fence_after_sync();
-            const Epilogue<PARTS> epi{args, cta, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, 0};
+            const Epilogue<PARTS> epi{args, cta, mine.begin, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, 0};
             epi.segment(split, w, w.length(args), tmem + d_column(seg), 1 + group, 1 + kDecodeW / 4, 0);
             tc_fence_before_sync();
         }
