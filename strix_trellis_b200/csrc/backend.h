@@ -108,10 +108,10 @@ cudaError_t launch_gemv(const LinearCall& call, const GemvPlan& plan, void* work
 
 // ---- GEMM (rows > 8) --------------------------------------------------------------------
 struct GemmPlan {
-    size_t act_bytes;        // core input as binary16 operand images
     size_t workspace_bytes;
     int sm_count;
     bool dense;  // weights decoded once, dense GEMM (else decoded on the fly)
+    bool pairs;  // instead of either: decoded on the fly by CTA pairs, in the workspace planned
 };
 GemmPlan plan_gemm(const DeviceWeights& w, int rows, int sm_count);
 cudaError_t launch_gemm(const LinearCall& call, const GemmPlan& plan, void* workspace,

@@ -1,7 +1,8 @@
 // Routes of a GEMM (more than 8 rows) and their workspace.
 //   weights decoded on the fly into tensor memory, once for each row group (wide_linear.cu)
+//   the same by CTA pairs, 257 to 1024 rows (wide_linear.cu)
 //   weights decoded once into the workspace, dense GEMM (gemm_dense.cu)
-// Beyond kWideMaxRows always the second; below, whichever the estimates here say is faster.
+// Beyond kWideMaxRows always the last; below, whichever the estimates here say is faster.
 #include "strix_trellis_b200.h"
 #include "wide_linear.h"
 
@@ -18,6 +19,9 @@ cudaError_t launch_gemm_dense(const LinearCall& call, unsigned char* workspace, 
 namespace {
 // As far as the estimates are fitted and measured; beyond, four and more decodes of a unit hardly pay.
 constexpr int kWideMaxRows = 1024;
+// Beyond, decoding once is level with decoding in CTA pairs or better.  (From 257 rows on: below, one tile is too
+// little for 74 pairs on most layers.)
+constexpr int kPairMaxRows = 1024;
 
 // How a call's rows are cut into groups that each decode the weights, and how many CTAs run them: one
 // group and every SM, unless so few column blocks are left that many CTAs share one and the CTA that
@@ -57,6 +61,33 @@ double dense_us(const DeviceWeights& w, int rows, int sm_count) {
     const double step = 0.485 * full + (rest ? 0.28 + 0.205 * rest / pairs : 0.0);
     return 14.5 + 0.59 * hblocks * nblocks / sm_count + (narrow ? 0.72 : 1.0) * step * 2 * hblocks;
 }
+// The same for CTA pairs (256 columns a pair, one tile of up to 256 rows): whole tiles in equal numbers, or
+// every pair and the tiles cut between them.  Estimates in us, fitted to 280 timings of 70 shapes of 257 to 2600 rows (rms
+// error 7 %): 8.6 and 1.5 a million inputs for the input stages; a unit 0.38 + 0.001 a row (the MMAs; the decode beside
+// them is shorter); 0.024 a row for a tile's epilogue, which has no second accumulator buffer to hide under; 0.009 a
+// row and 3 for the planes of tiles that pairs share and for pairs that end unevenly.  Measured against the better of the two other routes: 512 rows,
+// 4096 -> 12288, K5 86 -> 60 us; 625 rows, 6144 -> 12672, K6 146 -> 99; 370 rows, 6144 -> 8704 72 -> 45; 283 rows, 1536 -> 8320 29 -> 20;
+// 1885 rows, 5376 -> 8448 164 -> 157; 2329 rows, 3456 -> 3456 64 -> 69.
+Cut cut_pairs(const DeviceWeights& w, int rows, int sm_count) {
+    const int hblocks = w.inputs / 128, pairs = sm_count / 2;
+    Cut best{};
+    for (int count = (rows + kWideRows - 1) / kWideRows; (rows + count - 1) / count > 128; ++count) {
+        const int each = (rows + count - 1) / count, n = pair_n(each), groups = (rows + n - 1) / n;
+        const long long tiles = (long long)groups * ((w.outputs / 128 + 1) / 2);
+        const double unit = 0.38 + 0.001 * n, base = 8.6 + 1.5e-6 * rows * (double)w.inputs;
+        const long long turns = (tiles + pairs - 1) / pairs;
+        const double whole = base + turns * (hblocks * unit + 0.024 * n);
+        const double share = (double)tiles / pairs;  // tiles a pair
+        const double cut = base + share * hblocks * unit + 0.024 * n * (1.0 + share) + 0.009 * n / std::fmin(share, 1.0) + 3.0;
+        const bool split = cut < whole && tiles * hblocks >= pairs;
+        const double us = split ? cut : whole;
+        if (!best.groups || us < best.us) best = Cut{groups, n < rows ? n : rows, split ? pairs : (int)((tiles + turns - 1) / turns), us};
+    }
+    return best;
+}
+WidePlan pair_plan(const DeviceWeights& w, const Cut& cut) {
+    return plan_wide(w.bits, cut.rows, (long long)cut.groups * (w.inputs / 128) * ((w.outputs / 128 + 1) / 2), 2 * cut.ctas, true);
+}
 WidePlan wide_plan(const DeviceWeights& w, const Cut& cut) {
     return plan_wide(w.bits, cut.rows, (long long)cut.groups * (w.inputs / 128) * (w.outputs / 128), cut.ctas);
 }
@@ -66,15 +97,27 @@ GemmPlan plan_gemm(const DeviceWeights& w, int rows, int sm_count) {
     GemmPlan plan{};
     plan.sm_count = sm_count;
     const Cut cut = cut_call(w, rows, sm_count);
-    plan.dense = sm_count >= 2 && (rows > kWideMaxRows || dense_us(w, rows, sm_count) < cut.us);
+    const double dense = sm_count >= 2 ? dense_us(w, rows, sm_count) : 0.0;
+    plan.dense = sm_count >= 2 && (rows > kWideMaxRows || dense < cut.us);
     if (plan.dense) {
-        plan.act_bytes = align_up((size_t)gemm_dense_rows_padded(rows) * w.inputs * 2);
-        plan.workspace_bytes = plan.act_bytes + gemm_dense_scratch(w);
-        return plan;
+        plan.workspace_bytes = align_up((size_t)gemm_dense_rows_padded(rows) * w.inputs * 2) + gemm_dense_scratch(w);
+    } else {
+        const WidePlan wide = wide_plan(w, cut);
+        plan.workspace_bytes = wide.flag_bytes + wide.plane_bytes + align_up((size_t)cut.groups * (w.inputs / 128) * wide_tile_bytes(cut.rows));
     }
-    const WidePlan wide = wide_plan(w, cut);
-    plan.act_bytes = align_up((size_t)cut.groups * (w.inputs / 128) * wide_tile_bytes(cut.rows));
-    plan.workspace_bytes = wide.flag_bytes + wide.plane_bytes + plan.act_bytes;
+    if (rows > kWideRows && rows <= kPairMaxRows && sm_count >= 2) {
+        const Cut pairs = cut_pairs(w, rows, sm_count);
+        plan.pairs = pairs.us < (plan.dense ? dense : cut.us);
+        if (plan.pairs) {
+            const WidePlan wide = pair_plan(w, pairs);
+            const size_t need = wide.flag_bytes + wide.plane_bytes + align_up((size_t)pairs.groups * (w.inputs / 128) * pair_n(pairs.rows) * 256);
+            if (need > plan.workspace_bytes) {
+                // In the space of the decoded weights as a rule; a layer too small for that stays with its route.
+                if (plan.dense) plan.pairs = false;
+                else plan.workspace_bytes = need;
+            }
+        }
+    }
     return plan;
 }
 
@@ -82,9 +125,9 @@ cudaError_t launch_gemm(const LinearCall& call, const GemmPlan& plan, void* work
                         cudaStream_t stream) {
     if (!workspace) return cudaErrorInvalidValue;
     unsigned char* base = static_cast<unsigned char*>(workspace);
-    if (plan.dense) return launch_gemm_dense(call, base, plan.sm_count, programmatic_launch, stream);
-    const Cut cut = cut_call(call.w, call.rows, plan.sm_count);
-    const WidePlan wide = wide_plan(call.w, cut);
+    if (plan.dense && !plan.pairs) return launch_gemm_dense(call, base, plan.sm_count, programmatic_launch, stream);
+    const Cut cut = plan.pairs ? cut_pairs(call.w, call.rows, plan.sm_count) : cut_call(call.w, call.rows, plan.sm_count);
+    const WidePlan wide = plan.pairs ? pair_plan(call.w, cut) : wide_plan(call.w, cut);
     WideSet set{};
     set.count = cut.groups;
     set.group_rows = cut.rows;
@@ -101,20 +144,28 @@ cudaError_t launch_gemm(const LinearCall& call, const GemmPlan& plan, void* work
 
 }  // namespace st
 
+namespace {
+// A layer and a device of these sizes, for the host arithmetic; false: refused.
+bool route_layer(uint64_t inputs, uint64_t outputs, uint32_t bits_x2, uint32_t rows, uint32_t sm_count, st::DeviceWeights& w) {
+    const int code = st::rate_code(bits_x2);
+    if (!inputs || !outputs || inputs % 128 || outputs % 128 || inputs > (1u << 30) || outputs > (1u << 30) ||
+        (inputs / 128) * (outputs / 128) > 0x7FFFFFFF || !code ||
+        rows <= 8 || rows > 0x7FFFFFFF || !sm_count || sm_count > 4096)
+        return false;
+    w.inputs = (int)inputs;
+    w.outputs = (int)outputs;
+    w.bits = code;
+    return true;
+}
+}  // namespace
+
 // Pure host arithmetic: no context, no device.
 extern "C" strix_status strix_b200_gemm_route(uint64_t inputs, uint64_t outputs, uint32_t bits_x2, uint32_t rows, uint32_t sm_count,
                                               uint64_t out[4]) {
     if (!out) return STRIX_ERROR_INVALID_ARGUMENT;
     out[0] = out[1] = out[2] = out[3] = 0;
-    const int code = st::rate_code(bits_x2);
-    if (!inputs || !outputs || inputs % 128 || outputs % 128 || inputs > (1u << 30) || outputs > (1u << 30) ||
-        (inputs / 128) * (outputs / 128) > 0x7FFFFFFF || !code ||
-        rows <= 8 || rows > 0x7FFFFFFF || !sm_count || sm_count > 4096)
-        return STRIX_ERROR_INVALID_ARGUMENT;
     st::DeviceWeights w{};
-    w.inputs = (int)inputs;
-    w.outputs = (int)outputs;
-    w.bits = code;
+    if (!route_layer(inputs, outputs, bits_x2, rows, sm_count, w)) return STRIX_ERROR_INVALID_ARGUMENT;
     const st::GemmPlan plan = st::plan_gemm(w, (int)rows, (int)sm_count);
     out[0] = plan.dense;
     out[1] = plan.workspace_bytes;
@@ -123,5 +174,20 @@ extern "C" strix_status strix_b200_gemm_route(uint64_t inputs, uint64_t outputs,
         out[2] = (uint64_t)cut.groups;
         out[3] = (uint64_t)cut.ctas;
     }
+    return STRIX_SUCCESS;
+}
+
+extern "C" strix_status strix_b200_gemm_pairs(uint64_t inputs, uint64_t outputs, uint32_t bits_x2, uint32_t rows, uint32_t sm_count,
+                                              uint64_t out[3]) {
+    if (!out) return STRIX_ERROR_INVALID_ARGUMENT;
+    out[0] = out[1] = out[2] = 0;
+    st::DeviceWeights w{};
+    if (!route_layer(inputs, outputs, bits_x2, rows, sm_count, w)) return STRIX_ERROR_INVALID_ARGUMENT;
+    if (!st::plan_gemm(w, (int)rows, (int)sm_count).pairs) return STRIX_SUCCESS;
+    const st::Cut cut = st::cut_pairs(w, (int)rows, (int)sm_count);
+    const st::WidePlan wide = st::pair_plan(w, cut);
+    out[0] = (uint64_t)cut.groups;
+    out[1] = (uint64_t)wide.grid;
+    out[2] = wide.flag_bytes + wide.plane_bytes + st::align_up((size_t)cut.groups * (w.inputs / 128) * st::pair_n(cut.rows) * 256);
     return STRIX_SUCCESS;
 }

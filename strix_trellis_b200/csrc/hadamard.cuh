@@ -77,6 +77,73 @@ __device__ __forceinline__ void hadamard128_oct(float (&v)[4][4], int lane) {
         for (int i = 0; i < 4; ++i) v[i][j] = __fmul_rn(v[i][j], scale);
     }
 }
+// Two binary32 values in one register pair: one instruction for both, each rounded on its own (sm_100).
+struct Pair { unsigned long long bits; };
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+    Pair p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p.bits) : "f"(lo), "f"(hi));
+    return p;
+}
+__device__ __forceinline__ void split_pair(Pair p, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p.bits)); }
+__device__ __forceinline__ Pair add_pair(Pair a, Pair b) {
+    Pair p;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(p.bits) : "l"(a.bits), "l"(b.bits));
+    return p;
+}
+__device__ __forceinline__ Pair mul_pair(Pair a, Pair b) {
+    Pair p;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p.bits) : "l"(a.bits), "l"(b.bits));
+    return p;
+}
+__device__ __forceinline__ Pair fma_pair(Pair a, Pair b, Pair c) {
+    Pair p;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p.bits) : "l"(a.bits), "l"(b.bits), "l"(c.bits));
+    return p;
+}
+// hadamard128_oct with v[j][h] = elements 32 * 2h + 4(l % 8) + j and 32 * (2h + 1) + 4(l % 8) + j of the lane's block:
+// all stages but stride 32 work on pairs.  Same pairs, same ascending stage order, same operand sides
+// (a - b as the fused a + -1 * b: the product is exact): identical bits.
+__device__ __forceinline__ void hadamard128_oct_pairs(Pair (&v)[4][2], int lane) {
+    const Pair minus = pair_of(-1.0f, -1.0f);
+    auto butterfly = [&](Pair& lo, Pair& hi) {
+        const Pair a = lo, b = hi;
+        lo = add_pair(a, b);
+        hi = fma_pair(b, minus, a);
+    };
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        butterfly(v[0][h], v[1][h]);  // stride 1
+        butterfly(v[2][h], v[3][h]);
+        butterfly(v[0][h], v[2][h]);  // stride 2
+        butterfly(v[1][h], v[3][h]);
+    }
+#pragma unroll
+    for (int mask = 1; mask < 8; mask <<= 1) {  // strides 4, 8, 16
+        const float side = (lane & mask) ? -1.0f : 1.0f;
+        const Pair sign = pair_of(side, side);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float lo, hi;
+                split_pair(v[j][h], lo, hi);
+                v[j][h] = fma_pair(v[j][h], sign, pair_of(__shfl_xor_sync(0xFFFFFFFFu, lo, mask), __shfl_xor_sync(0xFFFFFFFFu, hi, mask)));
+            }
+    }
+    const Pair scale = pair_of(0x1.6a09e6p-4f, 0x1.6a09e6p-4f);  // RN32(1/sqrt(128))
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // stride 32
+            float lo, hi;
+            split_pair(v[j][h], lo, hi);
+            v[j][h] = pair_of(__fadd_rn(lo, hi), __fsub_rn(lo, hi));
+        }
+        butterfly(v[j][0], v[j][1]);  // stride 64
+        v[j][0] = mul_pair(v[j][0], scale);
+        v[j][1] = mul_pair(v[j][1], scale);
+    }
+}
 // The same transform of a block that one thread holds alone (a row of a tensor-memory tile).
 __device__ __forceinline__ void hadamard128_thread(float (&v)[128]) {
 #pragma unroll

@@ -7,6 +7,26 @@
 
 namespace st {
 
+// The launch of clusters of `cluster` CTAs below, with programmatic start or without.
+template <class... Params, class... Args>
+inline cudaError_t launch_clusters(void (*kernel)(Params...), int cluster, dim3 grid, int block, size_t smem, bool programmatic,
+                                   cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[programmatic].id = cudaLaunchAttributeClusterDimension;
+    attr[programmatic].val.clusterDim.x = cluster;
+    attr[programmatic].val.clusterDim.y = 1;
+    attr[programmatic].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = programmatic ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
 // One launch; `programmatic`: it may start while the launch before it in the stream still runs (the
 // kernel then waits with griddepcontrol.wait).
 template <class... Params, class... Args>

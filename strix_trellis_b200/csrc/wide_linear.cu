@@ -20,6 +20,16 @@
 // range holds the block's first K part finishes the block at the end of its own range and adds the
 // planes in ascending K order.  Waits only point to higher CTA indices and every CTA is resident.
 // The decode warps, idle at the end of the range, share the last segment's epilogue.
+//
+// CTA pairs (PAIR; one layer, groups of 129 to 256 rows, tcgen05 cta_group::2): each CTA decodes a column block of
+// its own into its own tensor memory and loads half of the activation rows; one MMA multiplies both blocks by
+// all rows.  Alone, a CTA of 256 rows waits for the 64 KB of every unit's activations, two in its ring (1.19 us a unit);
+// in a pair it loads half of them and the MMAs follow each other at the tensor pipe's rate (1080 clocks a unit
+// at 256 rows, 1024 of them MMAs; the decode beside them takes 750).  The accumulators of 256 rows leave no room for a
+// second buffer, so all warps share every segment's epilogue: about 10 000 clocks a tile against 35 000 of MMAs at
+// K = 4096.  512 rows, 4096 -> 12288, K5: 86 -> 60 us (decoding once, with its 23 us prologue, before).
+// The partner tells the leader by four transaction bytes on the leader's own barriers that a unit is decoded and
+// its rows have landed, and that a segment's accumulators are read.
 // Every wait is bounded and reports into the device status word.
 #include "gemv_partition.h"
 #include "hadamard.cuh"
@@ -36,7 +46,8 @@ constexpr int kWarpMma = kDecodeW + kEpiW, kWarpWeights = kWarpMma + kIssuers, k
 constexpr int kThreadsW = (kWarpRows + 1) * 32;
 constexpr int kChunkRows = 16;                       // rows of one epilogue chunk
 constexpr int kStageFloats = kChunkRows * 128;       // 8 KB of transposition space per warp group
-constexpr int kHeaderW = 1024 + 2 * kStageFloats * 4;  // barriers, the epilogue group's two staging areas
+constexpr int kHeaderW = 1024 + 2 * kStageFloats * 4;  // barriers, the epilogue warps' two staging areas
+constexpr int kPairHeader = 1024 + (1 + kUnitGroups) * kStageFloats * 4;  // a pair: one for each group of warps
 constexpr size_t kSmemLimitW = 224 * 1024;
 constexpr int kMaxWSlots = 24, kMaxBSlots = 8;
 constexpr int kRingMin = kDecodeW / 4 * kStageFloats * 4;       // the decode groups' staging of the last segment
@@ -50,10 +61,14 @@ struct WideArgs {
     int n_max, w_slots, w_stride, b_slots, b_stride;
     // tensor memory: a_stages x 64 columns of A, then d_bufs buffers of `parts` times d_accs accumulators of n_max
     int a_stages, d_bufs, d_accs, parts, parts_log2;
+    // CTA pairs: `nblocks` above counts pairs of column blocks; the layer's own count
+    int pair, layer_nblocks;
     unsigned int* flags;
     float* planes;
     unsigned int* status;
 };
+// The MMA's N for `rows` rows: a CTA pair splits it in two.
+__device__ __forceinline__ int tile_n(const WideArgs& a, int rows) { return a.pair ? pair_n(rows) : wide_n(rows); }
 
 // Problem p of the set: from the table, or row group p of the one layer.
 __device__ __forceinline__ const WideProblem& problem(const WideArgs& a, int p) {
@@ -65,7 +80,7 @@ __device__ __forceinline__ int problem_rows(const WideArgs& a, int p) {
     return left < a.group_rows ? left : a.group_rows;
 }
 __device__ __forceinline__ const unsigned char* problem_tiles(const WideArgs& a, int p) {
-    return a.table ? problem(a, p).tiles : a.one.tiles + (size_t)p * a.hblocks * wide_tile_bytes(a.group_rows);
+    return a.table ? problem(a, p).tiles : a.one.tiles + (size_t)p * a.hblocks * tile_n(a, a.group_rows) * 256;
 }
 
 // First block of K part s: the blocks [part_begin(s), part_begin(s + 1)) have accumulators of their own.
@@ -112,13 +127,15 @@ __device__ __forceinline__ void red_release_gpu(unsigned int* p, unsigned int v)
 // chunk, adds the other CTAs' planes (finisher) or stores the sums to this CTA's plane
 // (contributor); for outputs the chunk is transposed through `stage` and each warp finishes four
 // rows, eight lanes per row.
-template <bool PARTS>  // K in more than one part
+template <bool PARTS, bool PAIR>  // K in more than one part; CTA pairs
 struct Epilogue {
     const WideArgs& a;
-    int cta, origin, quarter, lane, bar;  // origin: first unit of the range
+    int cta, rank, origin, quarter, lane, bar;  // cta: of the split (a pair is one); origin: first unit of the range
     float* areas;      // staging: two areas in turn (one barrier per chunk instead of two), or one
     int area_floats;   // from one to the other; 0: one
 
+    // Index of the flag and the plane of `c`.
+    __device__ __forceinline__ int of(int c) const { return PAIR ? 2 * c + rank : c; }
     // false: a wait ran out (the whole group returns together)
     __device__ __forceinline__ bool segment(const Split& split, const Walk& w, int len, uint32_t dcol, int first_chunk, int step,
                                             uint32_t d_empty) const {
@@ -127,13 +144,13 @@ struct Epilogue {
         const bool contributor = w.hb != 0;
         int last = cta;
         if (!contributor && w.hb + len < a.hblocks) last = owner(split, hi - 1);
-        const WideProblem& pr = problem(a, w.p);
+        const WideProblem& pr = PAIR ? a.one : problem(a, w.p);
         // The flag of CTA c counts the chunks of its plane that are there.
         bool late = false;
         for (int c = cta + 1; c <= last && !late; ++c) {
             late = true;
             for (uint32_t tries = 0; tries < (1u << 20); ++tries)
-                if (ld_acquire_gpu(a.flags + c) >= (unsigned int)chunks) { late = false; break; }
+                if (ld_acquire_gpu(a.flags + of(c)) >= (unsigned int)chunks) { late = false; break; }
         }
         if (group_any(bar, late)) {
             if (late && lane == 0) atomicOr(a.status, kTimeoutFold);
@@ -142,6 +159,8 @@ struct Epilogue {
         const int col = quarter * 32 + lane;
         const uint32_t taddr = ((uint32_t)(quarter * 32) << 16) + dcol;
         float* stage = areas;
+        const bool live = !PAIR || 2 * w.nb + rank < a.layer_nblocks;  // an odd block count: the last pair's second half is padding
+        if (PAIR && d_empty && first_chunk >= chunks && lane == 0) mbar_arrive(d_empty);
         const int first_part = PARTS ? part_of(a, w.hb) : 0, last_part = PARTS ? part_of(a, w.hb + len - 1) : 0;  // of this segment
         int dumped = 0;
         for (int ch = first_chunk; ch < chunks; ch += step) {
@@ -200,7 +219,7 @@ struct Epilogue {
                 if (lane == 0) mbar_arrive(d_empty);
             }
             if (contributor) {
-                float* plane = a.planes + ((size_t)cta * a.n_max + ch * kChunkRows) * 128 + col;
+                float* plane = a.planes + ((size_t)of(cta) * a.n_max + ch * kChunkRows) * 128 + col;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) __stcg(plane + j * 128, __uint_as_float(r[j]));
                 ++dumped;
@@ -210,7 +229,7 @@ struct Epilogue {
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = __fadd_rn(0.f, __uint_as_float(r[j]));
             for (int c = cta + 1; c <= last; ++c) {
-                const float* plane = a.planes + ((size_t)c * a.n_max + ch * kChunkRows) * 128 + col;
+                const float* plane = a.planes + ((size_t)of(c) * a.n_max + ch * kChunkRows) * 128 + col;
                 float other[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) other[j] = __ldcg(plane + j * 128);
@@ -220,51 +239,94 @@ struct Epilogue {
 #pragma unroll
             for (int j = 0; j < 16; ++j) stage[j * 128 + col] = v[j];
             named_barrier(bar, 128);
-            finish_rows(pr, w, ch, rows, stage);
+            if (live) finish_rows(pr, w, ch, rows, stage);
             if (!area_floats) named_barrier(bar, 128);  // (two areas: the next chunk's barrier does)
             stage = stage == areas ? areas + area_floats : areas;
         }
         if (contributor && dumped) {
             named_barrier(bar, 128);  // the group's stores are ordered before the count below
-            if (quarter == 0 && lane == 0) red_release_gpu(a.flags + cta, (unsigned int)dumped);
+            if (quarter == 0 && lane == 0) red_release_gpu(a.flags + of(cta), (unsigned int)dumped);
         }
         return true;
     }
 
+    // Four rows per warp, eight lanes per row: H128, output scales, bias, alpha and beta.
     __device__ __forceinline__ void finish_rows(const WideProblem& pr, const Walk& w, int ch, int rows, const float* stage) const {
         const int l8 = lane & 7;
         const int in_chunk = quarter * 4 + (lane >> 3);
-        float v[4][4];
+        Pair v[4][2];  // column 32i + 4 l8 + j is half i % 2 of v[j][i / 2]
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 t = *reinterpret_cast<const float4*>(stage + in_chunk * 128 + 32 * i + 4 * l8);
-            v[i][0] = t.x; v[i][1] = t.y; v[i][2] = t.z; v[i][3] = t.w;
+        for (int h = 0; h < 2; ++h) {
+            const float4 t = *reinterpret_cast<const float4*>(stage + in_chunk * 128 + 64 * h + 4 * l8);
+            const float4 u = *reinterpret_cast<const float4*>(stage + in_chunk * 128 + 64 * h + 32 + 4 * l8);
+            v[0][h] = pair_of(t.x, u.x);
+            v[1][h] = pair_of(t.y, u.y);
+            v[2][h] = pair_of(t.z, u.z);
+            v[3][h] = pair_of(t.w, u.w);
         }
-        hadamard128_oct(v, lane);
+        hadamard128_oct_pairs(v, lane);
         const int r = ch * kChunkRows + in_chunk;
         if (r >= rows) return;
-        uint2 sv[4];
-        float4 bi[4];
+        const int nb = PAIR ? 2 * w.nb + rank : w.nb, c0 = nb * 128 + 4 * l8;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {  // all loads before the first store
-            const int c0 = w.nb * 128 + 32 * i + 4 * l8;
-            sv[i] = __ldg(reinterpret_cast<const uint2*>(pr.w.svh + c0));
-            bi[i] = pr.w.bias ? __ldg(reinterpret_cast<const float4*>(pr.w.bias + c0)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int h = 0; h < 2; ++h) {
+            const uint2 lo = __ldg(reinterpret_cast<const uint2*>(pr.w.svh + c0 + 64 * h)), hi = __ldg(reinterpret_cast<const uint2*>(pr.w.svh + c0 + 64 * h + 32));
+            auto scale = [&](Pair& p, uint32_t l, uint32_t u, int shift) {
+                p = mul_pair(p, pair_of(half_bits_to_float((uint16_t)(l >> shift)), half_bits_to_float((uint16_t)(u >> shift))));
+            };
+            scale(v[0][h], lo.x, hi.x, 0);
+            scale(v[1][h], lo.x, hi.x, 16);
+            scale(v[2][h], lo.y, hi.y, 0);
+            scale(v[3][h], lo.y, hi.y, 16);
         }
-        const int out_row = a.table ? (pr.y_rows ? pr.y_rows[r] : r) : w.p * a.group_rows + r;
-        const bool aligned = quads_aligned(pr.y, pr.y_dtype, pr.y_stride);
+        if (pr.w.bias) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int c0 = w.nb * 128 + 32 * i + 4 * l8;
-            const uint32_t sw[2] = {sv[i].x, sv[i].y};
-            const float bias[4] = {bi[i].x, bi[i].y, bi[i].z, bi[i].w};
-            float o[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                o[j] = __fmul_rn(v[i][j], half_bits_to_float((uint16_t)(sw[j >> 1] >> (16 * (j & 1)))));
-                if (pr.w.bias) o[j] = __fadd_rn(o[j], bias[j]);
+            for (int h = 0; h < 2; ++h) {
+                const float4 lo = __ldg(reinterpret_cast<const float4*>(pr.w.bias + c0 + 64 * h)), hi = __ldg(reinterpret_cast<const float4*>(pr.w.bias + c0 + 64 * h + 32));
+                v[0][h] = add_pair(v[0][h], pair_of(lo.x, hi.x));
+                v[1][h] = add_pair(v[1][h], pair_of(lo.y, hi.y));
+                v[2][h] = add_pair(v[2][h], pair_of(lo.z, hi.z));
+                v[3][h] = add_pair(v[3][h], pair_of(lo.w, hi.w));
             }
-            scale_and_store_quad(pr.y, pr.y_dtype, (long long)out_row * pr.y_stride + c0, aligned, o, pr.alpha, pr.beta);
+        }
+        const int out_row = !PAIR && a.table ? (pr.y_rows ? pr.y_rows[r] : r) : w.p * a.group_rows + r;
+        const long long at = (long long)out_row * pr.y_stride + c0;
+        float o[4][4];  // [i][j]
+        auto unpack = [&] {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) split_pair(v[j][h], o[2 * h][j], o[2 * h + 1][j]);
+        };
+        if (pr.beta != 0.0f || !quads_aligned(pr.y, pr.y_dtype, pr.y_stride)) {
+            unpack();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) scale_and_store_quad(pr.y, pr.y_dtype, at + 32 * i, false, o[i], pr.alpha, pr.beta);
+            return;
+        }
+        const Pair alpha = pair_of(pr.alpha, pr.alpha);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) v[j][h] = mul_pair(v[j][h], alpha);
+        unpack();
+        if (pr.y_dtype == DT_F32) {
+            float4* out = reinterpret_cast<float4*>(static_cast<float*>(pr.y) + at);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) out[8 * i] = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
+        } else {
+            uint2* out = reinterpret_cast<uint2*>(static_cast<uint16_t*>(pr.y) + at);
+            if (pr.y_dtype == DT_F16) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    out[8 * i] = make_uint2(as_u32(__floats2half2_rn(o[i][0], o[i][1])), as_u32(__floats2half2_rn(o[i][2], o[i][3])));
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const __nv_bfloat162 lo = __floats2bfloat162_rn(o[i][0], o[i][1]), hi = __floats2bfloat162_rn(o[i][2], o[i][3]);
+                    out[8 * i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                }
+            }
         }
     }
 };
@@ -272,17 +334,18 @@ struct Epilogue {
 // At most 72 registers: a CTA of the next call's input stages (128 threads) then fits beside this
 // kernel's, is resident and has its operands in the L2 when this kernel ends.  (ptxas spills for it in
 // the epilogue's chunk: 124 bytes stored and 188 loaded with K parts, 4 bytes without for mul1.)
-template <int CB, bool PARTS>
+template <int CB, bool PARTS, bool PAIR>
 __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (still a shared-memory pointer to the compiler)
-    const int warp = uniform_warp(), lane = threadIdx.x & 31, cta = (int)blockIdx.x;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    const int cta = (int)blockIdx.x >> (PAIR ? 1 : 0), rank = PAIR ? (int)cluster_ctarank() : 0;  // rank 0 leads its pair
     // Weights are immutable and a table is there before the launch before lets this one start (its own
     // wait comes first, see wide_inputs_kernel; acquiring the count acquires the table), so only the
     // activation producer waits.
     const int count = args.live ? (int)ld_acquire_gpu(reinterpret_cast<const unsigned int*>(args.live)) : args.count;
     const int units = count * args.nblocks * args.hblocks;
-    const int grid = units < (int)gridDim.x ? units : (int)gridDim.x;
+    const int ctas = (int)gridDim.x >> (PAIR ? 1 : 0), grid = units < ctas ? units : ctas;
     if (cta >= grid) {
         // Without a live problem nobody else waits for the launch before, and a launch may only end after
         // it has: the one after this counts on that when it overwrites what the one before reads.
@@ -296,24 +359,30 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
 
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
     float* epi_stage = reinterpret_cast<float*>(smem + 1024);
-    unsigned char* b_ring = smem + kHeaderW;                                    // 1024-byte aligned images
+    unsigned char* b_ring = smem + (PAIR ? kPairHeader : kHeaderW);                                    // 1024-byte aligned images
     unsigned char* w_ring = b_ring + (size_t)args.b_slots * args.b_stride;
     __shared__ uint32_t s_tmem_base;
+    __shared__ __align__(16) uint32_t s_sink[4];
     const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * kMaxWSlots, b_full = w_empty + 8 * kMaxWSlots,
                    b_empty = b_full + 8 * kMaxBSlots, a_full = b_empty + 8 * kMaxBSlots, a_empty = a_full + 8 * kMaxAStages,
-                   d_full = a_empty + 8 * kMaxAStages, d_empty = d_full + 16, all_done = d_empty + 16;
+                   d_full = a_empty + 8 * kMaxAStages, d_empty = d_full + 16, all_done = d_empty + 16, d_peer = all_done + 8;  // d_peer: of a pair, the partner's accumulators are read
     const int issuers = args.d_accs > 1 ? kIssuers : 1;
     if (threadIdx.x == 0) {
         for (int i = 0; i < args.w_slots; ++i) { mbar_init(w_full + 8 * i, 1); mbar_init(w_empty + 8 * i, 4); }
         for (int i = 0; i < args.b_slots; ++i) { mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, 1); }
         for (int i = 0; i < a_stages; ++i) { mbar_init(a_full + 8 * i, 4); mbar_init(a_empty + 8 * i, 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, issuers); mbar_init(d_empty + 8 * i, kEpiW); }
+        for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, issuers); mbar_init(d_empty + 8 * i, PAIR ? kEpiW + kDecodeW : kEpiW); }
         mbar_init(all_done, issuers);
+        mbar_init(d_peer, 1);
         mbar_fence_init();
     }
-    if (warp == kWarpMma) tmem_alloc(smem_u32(&s_tmem_base), 512);
+    if (warp == kWarpMma) {
+        if (PAIR) tmem_alloc_pair(smem_u32(&s_tmem_base), 512);
+        else tmem_alloc(smem_u32(&s_tmem_base), 512);
+    }
     tc_fence_before_sync();
-    __syncthreads();
+    if (PAIR) cluster_sync_all();  // the partner signals these barriers
+    else __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = s_tmem_base;
     pdl_launch_dependents();
@@ -331,8 +400,9 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                 const int len = w.length(args);
                 const DeviceWeights& dw = problem(args, w.p).w;
                 const uint32_t bytes = unit_bytes(dw.bits);
-                const unsigned char* src = reinterpret_cast<const unsigned char*>(dw.packed) +
-                                           ((size_t)w.nb * args.hblocks + w.hb) * bytes;
+                int nb = PAIR ? 2 * w.nb + rank : w.nb;
+                if (PAIR && nb >= args.layer_nblocks) nb = args.layer_nblocks - 1;  // padding: decoded, never written out
+                const unsigned char* src = reinterpret_cast<const unsigned char*>(dw.packed) + ((size_t)nb * args.hblocks + w.hb) * bytes;
                 for (int i = 0; i < len; ++i, src += bytes) {
                     if (issued >= args.w_slots && !mbar_wait_long(w_empty + 8 * slot, prev_use, args.status, kTimeoutRingEmpty)) {
                         ok = false;
@@ -356,15 +426,24 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             bool ok = true;
             for (Walk w(args, mine); w.unit < w.end && ok;) {
                 const int len = w.length(args);
-                const uint32_t bytes = (uint32_t)wide_tile_bytes(problem_rows(args, w.p));
+                const uint32_t bytes = (uint32_t)tile_n(args, problem_rows(args, w.p)) * 256;
                 const unsigned char* src = problem_tiles(args, w.p) + (size_t)w.hb * bytes;
                 for (int i = 0; i < len; ++i, src += bytes) {
                     if (issued >= args.b_slots && !mbar_wait_long(b_empty + 8 * slot, prev_use, args.status, kTimeoutTensorPipe)) {
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(b_full + 8 * slot, bytes);
-                    bulk_load(smem_u32(b_ring + (size_t)slot * args.b_stride), src, bytes, b_full + 8 * slot);
+                    const uint32_t dst = smem_u32(b_ring + (size_t)slot * args.b_stride);
+                    if (PAIR) {
+                        // this CTA's half of the rows, of both halves of K; the leader's stage also counts the partner's signal
+                        const uint32_t part = bytes / 4;
+                        mbar_expect_tx(b_full + 8 * slot, 2 * part + (rank == 0 ? 4 : 0));
+                        bulk_load(dst, src + rank * part, part, b_full + 8 * slot);
+                        bulk_load(dst + part, src + bytes / 2 + rank * part, part, b_full + 8 * slot);
+                    } else {
+                        mbar_expect_tx(b_full + 8 * slot, bytes);
+                        bulk_load(dst, src, bytes, b_full + 8 * slot);
+                    }
                     ++issued;
                     if (++slot == args.b_slots) { slot = 0; prev_use ^= 1; }
                 }
@@ -376,18 +455,49 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     } else if (warp >= kWarpMma) {
         // ---- MMA issuers, a unit each in turn: the whole warp walks, an elected lane issues ---------
         const int me = warp - kWarpMma;
-        if (me < issuers) {
+        if (PAIR && rank) {
+            // ---- partner CTA: one signal per unit that is decoded and whose rows have landed ----------
+            if (me == 0 && lane == 0) {
+                const uint32_t leader_full = map_to_rank(b_full, 0), sink = map_to_rank(smem_u32(s_sink), 0);
+                int slot = 0, stage = 0;
+                uint32_t use = 0, a_use = 0;
+                for (int unit = 0; unit < my_units; ++unit) {
+                    if (!mbar_wait_long(b_full + 8 * slot, use, args.status, kTimeoutTensorPipe) ||
+                        !mbar_wait_long(a_full + 8 * stage, a_use, args.status, kTimeoutTensorPipe))
+                        break;
+                    tc_fence_after_sync();
+                    signal_cluster_tx(leader_full + 8 * slot, sink);
+                    if (++slot == args.b_slots) { slot = 0; use ^= 1; }
+                    if (++stage == a_stages) { stage = 0; a_use ^= 1; }
+                }
+            } else if (me == 1 && lane == 0) {
+                // ---- and one per segment but the last whose accumulators are read -----------------------
+                const uint32_t leader_peer = map_to_rank(d_peer, 0), sink = map_to_rank(smem_u32(s_sink + 1), 0);
+                Walk w(args, mine);
+                w.next(args, w.length(args));
+                for (int seg = 0; w.unit < w.end; ++seg, w.next(args, w.length(args))) {
+                    if (!mbar_wait_long(d_empty, (uint32_t)seg & 1, args.status, kTimeoutTensorPipe)) break;
+                    signal_cluster_tx(leader_peer, sink);
+                }
+            }
+        } else if (me < issuers) {
             // K step k of a unit goes to accumulator `me` of two, or (four) 2 me + k % 2.
             const uint32_t mine_acc = me * (args.d_accs >> 1) * args.n_max, odd = args.d_accs == 4 ? args.n_max : 0;
             int next = me, slot = me, stage = me, seg = 0;  // of this warp's next unit
             uint32_t use = 0, a_use = 0;
             bool ok = true;
             for (Walk w(args, mine); w.unit < w.end && ok; ++seg) {
-                const int len = w.length(args), n = wide_n(problem_rows(args, w.p)), start = w.unit - mine.begin;
-                const uint32_t idesc = umma_idesc_f16_f32(128, n), dcol = tmem + d_column(seg) + mine_acc;
+                const int len = w.length(args), n = tile_n(args, problem_rows(args, w.p)), start = w.unit - mine.begin;
+                const uint32_t idesc = umma_idesc_f16_f32(PAIR ? 256 : 128, n), dcol = tmem + d_column(seg) + mine_acc;
                 // (Waited for without a unit in the segment too: the other issuer's commit of the buffer's segment
                 // before must have come before this one's.)
-                if (seg >= d_bufs && !mbar_wait_long(d_empty + 8 * d_index(seg), d_parity(seg) ^ 1, args.status, kTimeoutTensorPipe)) break;
+                if (seg >= d_bufs) {
+                    if (!mbar_wait_long(d_empty + 8 * d_index(seg), d_parity(seg) ^ 1, args.status, kTimeoutTensorPipe)) break;
+                    if (PAIR) {
+                        if (elect_one()) mbar_expect_tx(d_peer, 4);
+                        if (!mbar_wait_long(d_peer, (uint32_t)(seg - 1) & 1, args.status, kTimeoutTensorPipe)) break;
+                    }
+                }
                 int part = PARTS ? part_of(args, w.hb) : 0, fresh = 1;
                 for (; next < start + len; next += issuers) {
                     while (PARTS && part_begin(args, part + 1) <= w.hb + next - start) { ++part; fresh = 1; }
@@ -399,8 +509,14 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                     }
                     tc_fence_after_sync();
                     const uint32_t rows0 = smem_u32(b_ring) + slot * args.b_stride, acol = tmem + stage * 64;
-                    const uint64_t b0 = umma_desc_k_major_sw128(rows0), b1 = umma_desc_k_major_sw128(rows0 + n * 128);
-                    if (elect_one()) {
+                    const uint64_t b0 = umma_desc_k_major_sw128(rows0), b1 = umma_desc_k_major_sw128(rows0 + (PAIR ? n * 64 : n * 128));
+                    if (PAIR && elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            umma_f16_ts_pair(acc, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, !fresh || k > 0);
+                        umma_commit_pair(a_empty + 8 * stage, 3);
+                        umma_commit_pair(b_empty + 8 * slot, 3);
+                    } else if (!PAIR && elect_one()) {
 #pragma unroll
                         for (int k = 0; k < 8; ++k)
                             umma_f16_ts(acc + (k & 1) * odd, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, !fresh || k > 1 || (k == 1 && !odd));
@@ -412,21 +528,29 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                     if ((slot += issuers) >= args.b_slots) { slot -= args.b_slots; use ^= 1; }
                     if ((stage += issuers) >= a_stages) { stage -= a_stages; a_use ^= 1; }
                 }
-                if (elect_one()) umma_commit(d_full + 8 * d_index(seg));
+                if (elect_one()) {
+                    if (PAIR) umma_commit_pair(d_full + 8 * d_index(seg), 3);
+                    else umma_commit(d_full + 8 * d_index(seg));
+                }
                 w.next(args, len);
             }
-            if (elect_one()) umma_commit(all_done);
+            if (elect_one()) {
+                if (PAIR) umma_commit_pair(all_done, 3);
+                else umma_commit(all_done);
+            }
         }
     } else if (warp >= kDecodeW) {
         // ---- epilogue group: every segment, all of it except the last, which the decoders share ----
         // Output scales and bias are cold in DRAM and needed at the very end: ask the L2 for them now.
-        for (int b = mine.begin / args.hblocks + (warp & 3), e = (mine.end - 1) / args.hblocks; b <= e; b += kEpiW) {
-            const int p = b / args.nblocks, nb = b - p * args.nblocks;
+        for (int b = mine.begin / args.hblocks + (warp & 3), e = (mine.end - 1) / args.hblocks; b <= e; b += 4) {
+            const int p = b / args.nblocks;
+            int nb = b - p * args.nblocks;
+            if (PAIR) nb = 2 * nb + rank < args.layer_nblocks ? 2 * nb + rank : args.layer_nblocks - 1;
             const DeviceWeights& dw = problem(args, p).w;
             if (lane < 2) prefetch_line_l2(dw.svh + (size_t)nb * 128 + lane * 64);
             else if (lane < 6 && dw.bias) prefetch_line_l2(dw.bias + (size_t)nb * 128 + (lane - 2) * 32);
         }
-        const Epilogue<PARTS> epi{args, cta, mine.begin, warp & 3, lane, 1, epi_stage, kStageFloats};
+        const Epilogue<PARTS, PAIR> epi{args, cta, rank, mine.begin, warp & 3, lane, 1, epi_stage, PAIR ? 0 : kStageFloats};
         int seg = 0;
         for (Walk w(args, mine); w.unit < w.end; ++seg) {
             const int len = w.length(args);
@@ -434,7 +558,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             const bool ok = mbar_wait_long(d_full + 8 * d_index(seg), d_parity(seg), args.status, kTimeoutTensorPipe);
             if (group_any(1, !ok)) break;
             tc_fence_after_sync();
-            if (!epi.segment(split, w, len, tmem + d_column(seg), 0, final ? 1 + kDecodeW / 4 : 1, d_empty + 8 * d_index(seg))) break;
+            if (!epi.segment(split, w, len, tmem + d_column(seg), 0, 1 + (PAIR || final ? kDecodeW / 4 : 0), d_empty + 8 * d_index(seg))) break;
             w.next(args, len);
         }
     } else {
@@ -445,36 +569,68 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         bool ok = true;
         int seg = 0, until = 0;
         Walk w(args, mine);
-        while (true) {
-            const int len = w.length(args);
-            until += len;
-            const int bits = problem(args, w.p).w.bits;
-            ok = decode_segment_rate<CB, kUnitGroups>(bits, s, until, w_ring, args.w_slots, args.w_stride, w_full, w_empty, a_full, a_empty,
-                                         taddr, a_stages, ctile, lane, args.status);
-            if (!ok || until >= my_units) break;
-            w.next(args, len);
-            ++seg;
-        }
-        // The range is decoded: a quarter of these warps each is a group that takes its share of the
-        // last segment's epilogue, with staging space in the idle weight ring.
-        const int group = warp >> 2;
-        // (Not d_full: these warps may be several segments ahead of the accumulators, where its parity
-        // would already look like the last segment's.)
-        if (ok) ok = mbar_wait_long(all_done, 0, args.status, kTimeoutTensorPipe);
-        if (!group_any(2 + group, !ok)) {
-            tc_fence_after_sync();
-            const Epilogue<PARTS> epi{args, cta, mine.begin, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, 0};
-            epi.segment(split, w, w.length(args), tmem + d_column(seg), 1 + group, 1 + kDecodeW / 4, 0);
+        const int group = turn;
+        auto decode_until = [&](int end) {
+            return decode_segment_rate<CB, kUnitGroups>((PAIR ? args.one : problem(args, w.p)).w.bits, s, end, w_ring, args.w_slots, args.w_stride, w_full, w_empty,
+                                                        a_full, a_empty, taddr, a_stages, ctile, lane, args.status);
+        };
+        if (PAIR) {
+            // The accumulators of a group of rows leave no room for a second buffer, so these warps share the
+            // epilogue of every segment, each once it has a unit of the next one decoded.
+            const Epilogue<PARTS, PAIR> epi{args, cta, rank, mine.begin, warp & 3, lane, 2 + group, epi_stage + (1 + group) * kStageFloats, 0};
+            auto share = [&](const Walk& at, int len, int of) {
+                if (group_any(2 + group, !mbar_wait_long(d_full, (uint32_t)of & 1, args.status, kTimeoutTensorPipe))) return false;
+                tc_fence_after_sync();
+                return epi.segment(split, at, len, tmem + d_column(of), 1 + group, 1 + kDecodeW / 4, d_empty);
+            };
+            Walk before = w;
+            int before_len = 0;
+            for (; w.unit < w.end && ok; ++seg) {
+                const int len = w.length(args);
+                until += len;
+                if (seg) {
+                    ok = decode_until(s.unit + 1 < until ? s.unit + 1 : until);
+                    // (A group whose wait ran out leaves together; the others' waits end by their own limit.)
+                    if (group_any(2 + group, !ok) || !share(before, before_len, seg - 1)) { ok = false; break; }
+                }
+                ok = decode_until(until);
+                before = w;
+                before_len = len;
+                w.next(args, len);
+            }
+            if (!group_any(2 + group, !ok)) share(before, before_len, seg - 1);
             tc_fence_before_sync();
+        } else {
+            while (true) {
+                const int len = w.length(args);
+                until += len;
+                ok = decode_until(until);
+                if (!ok || until >= my_units) break;
+                w.next(args, len);
+                ++seg;
+            }
+            // The range is decoded: a quarter of these warps each is a group that takes its share of the
+            // last segment's epilogue, with staging space in the idle weight ring.
+            // (Not d_full: these warps may be several segments ahead of the accumulators, where its parity
+            // would already look like the last segment's.)
+            if (ok) ok = mbar_wait_long(all_done, 0, args.status, kTimeoutTensorPipe);
+            if (!group_any(2 + group, !ok)) {
+                tc_fence_after_sync();
+                const Epilogue<PARTS, PAIR> epi{args, cta, rank, mine.begin, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, 0};
+                epi.segment(split, w, w.length(args), tmem + d_column(seg), 1 + group, 1 + kDecodeW / 4, 0);
+                tc_fence_before_sync();
+            }
         }
     }
 
     tc_fence_before_sync();
-    __syncthreads();
+    if (PAIR) cluster_sync_all();  // both CTAs are done with each other's memory
+    else __syncthreads();
     if (warp == kWarpMma) {
         __syncwarp();
         tc_fence_after_sync();
-        tmem_dealloc(tmem, 512);
+        if (PAIR) tmem_dealloc_pair(tmem, 512);
+        else tmem_dealloc(tmem, 512);
     }
 }
 
@@ -506,7 +662,7 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
     for (int p = blockIdx.y; p < count; p += gridDim.y) {
         const WideProblem& pr = problem(args, p);
         const int rows = problem_rows(args, p), quads = (rows + 3) / 4;
-        const size_t tile_bytes = wide_tile_bytes(rows);
+        const size_t tile_bytes = (size_t)tile_n(args, rows) * 256;
         unsigned char* tiles = const_cast<unsigned char*>(problem_tiles(args, p));
         const bool aligned = quads_aligned(pr.x, pr.x_dtype, pr.x_stride);
         for (int item = first; item < quads * args.hblocks; item += gridDim.x * kInputWarps) {
@@ -538,22 +694,25 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
 }
 
 // ---- host side -----------------------------------------------------------------------------------
-WidePlan plan_wide(int heaviest, int rows_max, long long units, int sm_count) {
+WidePlan plan_wide(int heaviest, int rows_max, long long units, int sm_count, bool pair) {
     WidePlan plan{};
-    plan.grid = (int)(units < sm_count ? units : sm_count);
-    plan.n_max = wide_n(rows_max < kWideRows ? rows_max : kWideRows);
+    plan.pair = pair;
+    const int most = pair ? sm_count / 2 : sm_count;
+    plan.grid = (int)(units < most ? units : most);
+    plan.n_max = pair ? pair_n(rows_max) : wide_n(rows_max < kWideRows ? rows_max : kWideRows);
     plan.parts = 1;
     plan.w_stride = unit_bytes(heaviest);
-    plan.w_slots = (64 * 1024) / plan.w_stride;
+    plan.w_slots = (pair ? 80 * 1024 : 64 * 1024) / plan.w_stride;
     if (plan.w_slots > kMaxWSlots) plan.w_slots = kMaxWSlots;
     while ((size_t)plan.w_slots * plan.w_stride < kRingMin) ++plan.w_slots;  // 1 and 1.5 bits per weight
     const size_t ring = (size_t)plan.w_slots * plan.w_stride;
-    plan.b_stride = plan.n_max * 256;
-    plan.b_slots = (int)((kSmemLimitW - 1024 - kHeaderW - ring) / plan.b_stride);
+    plan.b_stride = plan.n_max * (pair ? 128 : 256);
+    const size_t header = pair ? kPairHeader : kHeaderW;
+    plan.b_slots = (int)((kSmemLimitW - 1024 - header - ring) / plan.b_stride);
     if (plan.b_slots > kMaxBSlots) plan.b_slots = kMaxBSlots;
-    plan.smem_bytes = 1024 + kHeaderW + ring + (size_t)plan.b_slots * plan.b_stride;
+    plan.smem_bytes = 1024 + header + ring + (size_t)plan.b_slots * plan.b_stride;
     plan.flag_bytes = align_up((size_t)sm_count * sizeof(unsigned int));
-    plan.plane_bytes = align_up((size_t)plan.grid * plan.n_max * 128 * sizeof(float));
+    plan.plane_bytes = align_up((size_t)plan.grid * (pair ? 2 : 1) * plan.n_max * 128 * sizeof(float));
     return plan;
 }
 
@@ -566,7 +725,9 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     a.count = set.count;
     a.group_rows = set.group_rows;
     a.hblocks = set.inputs / 128;
-    a.nblocks = set.outputs / 128;
+    a.pair = plan.pair;
+    a.layer_nblocks = set.outputs / 128;
+    a.nblocks = plan.pair ? (a.layer_nblocks + 1) / 2 : a.layer_nblocks;
     a.n_max = plan.n_max;
     a.w_slots = plan.w_slots;
     a.w_stride = plan.w_stride;
@@ -600,19 +761,22 @@ cudaError_t launch_wide_inputs(const WideSet& set, const WidePlan& plan, unsigne
     const int y = set.count < 1024 ? set.count : 1024;
     int x = streaming_grid((long long)per_problem * y, 8) / y;
     x = x < 1 ? 1 : x > per_problem ? per_problem : x;
-    return launch_pdl(wide_inputs_kernel, dim3(x, y), 32 * kInputWarps, 0, programmatic, stream, a, plan.grid);
+    return launch_pdl(wide_inputs_kernel, dim3(x, y), 32 * kInputWarps, 0, programmatic, stream, a, plan.grid * (plan.pair ? 2 : 1));
 }
 
 cudaError_t launch_wide(const WideSet& set, const WidePlan& plan, unsigned int* flags, float* planes, unsigned int* status,
                         bool programmatic, cudaStream_t stream) {
     const WideArgs a = wide_args(set, plan, flags, planes, status);
     const long long units = (long long)set.count * a.nblocks * a.hblocks;
+    if (plan.pair && (set.table || a.d_accs != 1 || a.parts != 1)) return cudaErrorInvalidValue;  // one layer, more than 128 rows a group
     if (units < 1 || units > 0x7FFFFFFF || plan.b_slots < 1 || plan.w_slots < 2 || plan.smem_bytes > kSmemLimitW ||
         (size_t)plan.w_slots * plan.w_stride < kRingMin)
         return cudaErrorInvalidValue;
     return for_codebook(set.codebook, [&](auto cb) {
-        return a.parts > 1 ? launch_pdl(wide_linear_kernel<decltype(cb)::value, true>, plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a)
-                           : launch_pdl(wide_linear_kernel<decltype(cb)::value, false>, plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a);
+        constexpr int CB = decltype(cb)::value;
+        if (plan.pair) return launch_clusters(wide_linear_kernel<CB, false, true>, 2, 2 * plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a);
+        return a.parts > 1 ? launch_pdl(wide_linear_kernel<CB, true, false>, plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a)
+                           : launch_pdl(wide_linear_kernel<CB, false, false>, plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a);
     });
 }
 
@@ -620,9 +784,10 @@ cudaError_t launch_wide(const WideSet& set, const WidePlan& plan, unsigned int* 
 // on a device (configure_device), never on the launch path.
 template <int CB>
 static cudaError_t configure_wide_cb() {
-    const cudaError_t e = cudaFuncSetAttribute(wide_linear_kernel<CB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(wide_linear_kernel<CB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    cudaError_t e = cudaFuncSetAttribute(wide_linear_kernel<CB, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_linear_kernel<CB, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_linear_kernel<CB, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    return e;
 }
 cudaError_t configure_wide_kernels() {
     cudaError_t e = configure_wide_cb<CB_3INST>();

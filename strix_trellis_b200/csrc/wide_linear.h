@@ -23,17 +23,19 @@ struct WideProblem {
 };
 
 ST_RATE_FN int wide_n(int rows) { return rows <= 16 ? 16 : (rows + 15) & ~15; }  // MMA N
+ST_RATE_FN int pair_n(int rows) { return (rows + 31) & ~31; }  // in a CTA pair, which halves it
 ST_RATE_FN size_t wide_tile_bytes(int rows) { return (size_t)wide_n(rows) * 256; }
 
 struct WidePlan {
-    int grid;
+    bool pair;              // CTA pairs, of one layer with more than 128 rows a group
+    int grid;               // CTAs, or pairs
     int n_max;              // widest problem's N
     int w_slots, w_stride;  // weight ring: slots of one unit, bytes apart
     int b_slots, b_stride;  // activation ring
     int parts;              // K parts that are summed apart (accumulator_parts), 1, 2 or 4
     size_t smem_bytes;
-    size_t flag_bytes;      // [grid] counters, zeroed by launch_wide_inputs
-    size_t plane_bytes;     // [grid][n_max][128] partial sums
+    size_t flag_bytes;      // [CTAs] counters, zeroed by launch_wide_inputs
+    size_t plane_bytes;     // [CTAs][n_max][128] partial sums
 };
 // K parts, each with accumulators of its own, for `groups` problems of at most eight rows.  The tensor
 // cores truncate as they accumulate, so the error of a sum grows with the steps it is made of, and a
@@ -52,7 +54,7 @@ ST_RATE_FN int accumulator_parts(int hblocks, int nblocks, long long groups, int
     return parts;
 }
 // `heaviest`: the rate code with the largest tiles among the problems.
-WidePlan plan_wide(int heaviest, int rows_max, long long units, int sm_count);
+WidePlan plan_wide(int heaviest, int rows_max, long long units, int sm_count, bool pair = false);
 
 // A set of problems of one geometry.  `table` (device memory) holds them, `table_stride` bytes apart;
 // without a table the set is ONE layer whose `one.rows` rows are cut into problems of group_rows rows.

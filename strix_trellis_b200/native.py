@@ -242,6 +242,7 @@ PROTOTYPES = {
     "strix_b200_peer_gather": (C.c_int, [vp, P(PeerGatherDesc), P(Stream)]),
     "strix_b200_peer_return_routes": (C.c_int, [vp, P(PeerReturnDesc), P(Stream)]),
     "strix_b200_gemm_route": (C.c_int, [u64, u64, u32, u32, u32, P(u64)]),
+    "strix_b200_gemm_pairs": (C.c_int, [u64, u64, u32, u32, u32, P(u64)]),
     "strix_b200_device_status": (C.c_int, [vp, P(u32)]),
     "strix_b200_set_programmatic_launch": (C.c_int, [vp, u32]),
     "strix_b200_gemv_noalloc": (C.c_int, [vp, P(MatmulDesc), P(Stream)]),

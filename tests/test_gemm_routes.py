@@ -55,3 +55,27 @@ def test_measured_sides_of_the_line():
 def test_refusals(args):
     assert route(*args) == (N.INVALID_ARGUMENT, [0, 0, 0, 0])
     assert N.load().strix_b200_gemm_route(128, 128, 8, 16, 148, None) == N.INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize("sm_count", [148, 132, 7, 2, 1])
+@pytest.mark.parametrize("shape", SHAPES + [(1024, 9600), (1280, 6016), (256, 4224)])
+def test_cta_pairs(shape, sm_count):
+    """Groups of 129 to 256 rows, no more pairs than the device has, all of it within the workspace."""
+    inputs, outputs = shape
+    tiles = (outputs // 128 + 1) // 2
+    for bits_x2 in (2, 8, 12):
+        for rows in ROWS:
+            if sm_count == 1 and rows > 1024:
+                continue
+            out = (N.u64 * 3)()
+            assert N.load().strix_b200_gemm_pairs(inputs, outputs, bits_x2, rows, sm_count, out) == N.SUCCESS
+            groups, pairs, used = list(out)
+            if not groups:
+                assert pairs == used == 0
+                continue
+            assert 256 < rows <= 1024 and sm_count >= 2
+            assert 128 < -(-rows // groups) <= 256 and 1 <= pairs <= min(sm_count // 2, groups * tiles * (inputs // 128))
+            planes = 2 * pairs * 512 * -(-rows // groups)
+            assert rows * inputs * 2 + planes <= used <= route(inputs, outputs, bits_x2, rows, sm_count)[1][1]
+    assert N.load().strix_b200_gemm_pairs(0, 128, 8, 300, 148, (N.u64 * 3)()) == N.INVALID_ARGUMENT
+    assert N.load().strix_b200_gemm_pairs(128, 128, 8, 300, 148, None) == N.INVALID_ARGUMENT

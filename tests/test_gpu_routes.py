@@ -80,6 +80,43 @@ def test_wide_row_groups(ctx, rows, inputs, outputs):
     check(ctx, rows, inputs, outputs, bits=5, bias=inputs == 640)
 
 
+def pairs_of(inputs, outputs, bits, rows, sm_count):
+    from strix_trellis_b200 import native as N
+    out = (N.u64 * 3)()
+    assert N.load().strix_b200_gemm_pairs(inputs, outputs, 2 * bits, rows, sm_count, out) == N.SUCCESS
+    return list(out)
+
+
+@pytest.mark.parametrize("rows,inputs,outputs,bits,codebook", [
+    (257, 1536, 8320, 5, "mul1"),                              # smallest, whole tiles, an odd number of column blocks
+    (289, 1024, 9600, 4, "mcg"), (384, 1024, 9600, 2, "3inst"),  # tiles cut between pairs, odd blocks
+    (512, 1024, 9600, 8, "mul1"), (513, 2048, 2176, 3, "mul1"), (1024, 1280, 6016, 6, "mul1"),  # two and more tiles a pair
+    (700, 2048, 2176, 1, "mul1")])
+def test_cta_pairs(ctx, rows, inputs, outputs, bits, codebook):
+    assert pairs_of(inputs, outputs, bits, rows, torch.cuda.get_device_properties(0).multi_processor_count)[0]
+    check(ctx, rows, inputs, outputs, bits, codebook, bias=bits != 4)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+def test_cta_pairs_tensors(ctx, dtype):
+    """Tensor types, alpha and beta, and rows that are not aligned, against the contract in the tensor's type."""
+    rows, inputs, outputs = 300, 1024, 9600
+    layer = synthetic.make_layer(inputs, outputs, 4, seed=9110, bias=True)
+    w = ctx.prepare(layer)
+    x = dev(synthetic.make_activations(rows, inputs, seed=9111)).to(dtype)
+    want = c_oracle.linear(layer.trellis, layer.suh, layer.svh, layer.bias, 4, 2, host(x.float()))
+    rounding = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 0.0}[dtype]
+    limit = 1e-3 * np.abs(want).max()
+    buffer = torch.full((rows * outputs + 2,), 0.5, dtype=dtype, device="cuda")
+    for y, alpha, beta in ((torch.empty((rows, outputs), dtype=dtype, device="cuda"), 1.0, 0.0),
+                           (torch.full((rows, outputs), 0.5, dtype=dtype, device="cuda"), -2.0, 0.25),
+                           (buffer[1:-1].view(rows, outputs), 1.0, 0.0)):
+        w.gemm(x, y, alpha=alpha, beta=beta)
+        np.testing.assert_allclose(host(y.float()), alpha * want + beta * 0.5, rtol=2 * rounding + 1e-3, atol=abs(alpha) * limit)
+    assert buffer[0] == 0.5 and buffer[-1] == 0.5
+    w.close()
+
+
 @pytest.mark.parametrize("rows", [1025, 1151, 1281])
 @pytest.mark.parametrize("inputs,outputs,bits,codebook", [(128, 128, 2, "mul1"), (1152, 384, 6, "mcg"), (256, 4480, 4, "3inst")])
 def test_dense_tiles(ctx, rows, inputs, outputs, bits, codebook):
