@@ -191,6 +191,17 @@ __device__ __forceinline__ void scale_and_store(void* y, int dtype, long long in
     store_element(y, dtype, index, value);
 }
 
+// Four 16-bit elements that were loaded as one word.
+__device__ __forceinline__ void widen_quad(uint2 t, int dtype, float (&v)[4]) {
+    if (dtype == DT_F16) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&t.x));
+        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&t.y));
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    } else {
+        v[0] = __uint_as_float(t.x << 16); v[1] = __uint_as_float(t.x & 0xFFFF0000u);
+        v[2] = __uint_as_float(t.y << 16); v[3] = __uint_as_float(t.y & 0xFFFF0000u);
+    }
+}
 // Four neighbouring elements; `quads_aligned` says whether they may be read as one word.
 __device__ __forceinline__ bool quads_aligned(const void* base, int dtype, long long stride) {
     return (stride & 3) == 0 && (reinterpret_cast<uintptr_t>(base) & (dtype == DT_F32 ? 15 : 7)) == 0;
@@ -203,15 +214,7 @@ __device__ __forceinline__ void load_quad(const void* base, int dtype, long long
         const float4 t = *reinterpret_cast<const float4*>(static_cast<const float*>(base) + index);
         v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
     } else {
-        const uint2 t = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + index);
-        if (dtype == DT_F16) {
-            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&t.x));
-            const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&t.y));
-            v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-        } else {
-            v[0] = __uint_as_float(t.x << 16); v[1] = __uint_as_float(t.x & 0xFFFF0000u);
-            v[2] = __uint_as_float(t.y << 16); v[3] = __uint_as_float(t.y & 0xFFFF0000u);
-        }
+        widen_quad(*reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + index), dtype, v);
     }
 }
 // scale_and_store of four neighbours.
