@@ -8,12 +8,12 @@ namespace st {
 
 // One row with this many units per CTA takes gemv_tmem.cu, with fewer gemv_row.cu: the decode loop then
 // outweighs the longer way from the last tile to the fold.  us per launch in a chain of one layer, K4,
-// gemv_row.cu / gemv_tmem.cu: 11 units 9.0 / 9.5, 21 14.9 / 14.3, 32 20.2 / 19.0, 48 29.2 / 26.2, 80
-// 45.5 / 40.1, 192 101 / 88.  In a stack a layer pays for the change from one kernel to the other and
-// back, so the line is higher than where the two meet: 28 layers of up to 25 units (4096, 1024 and
-// 14336 wide), K3 to K5, 320 us with the widest in gemv_row.cu and 327 in gemv_tmem.cu; 16 layers of 28
-// and 7 units 206.3 / 207.4; 12 of 48 and 7 units 217 / 206.
-constexpr int kTmemUnits = 40;
+// gemv_row.cu / gemv_tmem.cu (before the two MMA issuers): 11 units 9.0 / 9.5, 21 14.9 / 14.3, 32 20.2 / 19.0, 48
+// 29.2 / 26.2, 80 45.5 / 40.1, 192 101 / 88.  In a stack a layer pays for the change from one kernel to the other and
+// back, so the line is higher than where the two meet.  Stacks whose widest layers have 25 units, those in
+// gemv_row.cu / gemv_tmem.cu: 16 layers K4 149.0 / 148.0, K2 to K6 160.8 / 160.8; 28 layers K4 288.8 / 285.2, K3 to K5 311.8 /
+// 313.4.  With the line at 8 units the first of these takes 151.6 for 145.
+constexpr int kTmemUnits = 24;
 
 // Two or more rows with at most this many units per CTA take gemv_few.cu, with more gemv_tmem.cu.  us per
 // launch in a chain of one layer, 2 / 4 / 8 rows, gemv_few.cu against gemv_tmem.cu: two units of K4 4.5 / 4.6 /
