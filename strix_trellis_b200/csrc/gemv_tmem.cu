@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) gemv_tmem_kernel(const TmemArgs 
         // ---- decode warps ---------------------------------------------------------------------------
         const int turn = warp >> 2, ctile = 2 * (warp & 3);
         DecodeState s{turn, turn, 1, false, turn % args.w_slots, (uint32_t)(turn / args.w_slots) & 1};
-        decode_segment_rate<CB, kUnitGroups>(c.w.bits, s, my_units, w_ring, args.w_slots, w_stride, w_full, w_empty, a_full, a_empty,
+        decode_segment_rate<CB, kUnitGroups, false>(c.w.bits, s, my_units, w_ring, args.w_slots, w_stride, w_full, w_empty, a_full, a_empty,
                                              tmem + ((uint32_t)(ctile * 16) << 16), kAStagesT, ctile, lane, c.status);
     } else {
         // ---- helper warps: input stages, then the epilogue of every other segment ---------------------

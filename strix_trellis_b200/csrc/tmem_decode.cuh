@@ -31,8 +31,10 @@ struct DecodeState {
     int slot;      // its ring slot
     uint32_t use;  // and the slot's use parity
 };
-// GROUPS of four warps take turns.
-template <int K, int CB, int GROUPS>
+// GROUPS of four warps take turns.  LONG: the unit's sixteen tiles of a warp unrolled, not eight; faster where a
+// CTA decodes hundreds of units (expert bank of 32, K2: 185 -> 180 us), slower where the code is cold for most of
+// the launch (sixteen rows 15.1 -> 15.6, 16 layers of four rows 170.7 -> 174).
+template <int K, int CB, int GROUPS, bool LONG>
 __device__ __forceinline__ bool decode_segment(DecodeState& s, int until, const unsigned char* ring, int w_slots, int w_stride,
                                                uint32_t w_full, uint32_t w_empty, uint32_t a_full, uint32_t a_empty,
                                                uint32_t taddr, int a_stages, int ctile, int lane, unsigned int* status) {
@@ -45,7 +47,7 @@ __device__ __forceinline__ bool decode_segment(DecodeState& s, int until, const 
         tc_fence_after_sync();
         const uint32_t* tiles = reinterpret_cast<const uint32_t*>(ring + (size_t)s.slot * w_stride) + ctile * quad_words(K);
         uint32_t to = taddr + stage * 64;
-#pragma unroll 1
+#pragma unroll(LONG ? 2 : 1)
         for (int c = 0; c < 2; ++c, tiles += quad_words(K), to += 16u << 16) {
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
@@ -68,12 +70,12 @@ __device__ __forceinline__ bool decode_segment(DecodeState& s, int until, const 
 }
 
 // The same for a run-time rate.
-template <int CB, int GROUPS>
+template <int CB, int GROUPS, bool LONG>
 __device__ __forceinline__ bool decode_segment_rate(int bits, DecodeState& s, int until, const unsigned char* ring, int w_slots,
                                                     int w_stride, uint32_t w_full, uint32_t w_empty, uint32_t a_full,
                                                     uint32_t a_empty, uint32_t taddr, int a_stages, int ctile, int lane,
                                                     unsigned int* status) {
-#define ST_DECODE(K) decode_segment<K, CB, GROUPS>(s, until, ring, w_slots, w_stride, w_full, w_empty, a_full, a_empty, taddr, a_stages, ctile, lane, status)
+#define ST_DECODE(K) decode_segment<K, CB, GROUPS, LONG>(s, until, ring, w_slots, w_stride, w_full, w_empty, a_full, a_empty, taddr, a_stages, ctile, lane, status)
     switch (bits) {
     case 1: return ST_DECODE(1);
     case 2: return ST_DECODE(2);

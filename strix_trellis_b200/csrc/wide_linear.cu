@@ -70,17 +70,23 @@ struct WideArgs {
 // The MMA's N for `rows` rows: a CTA pair splits it in two.
 __device__ __forceinline__ int tile_n(const WideArgs& a, int rows) { return a.pair ? pair_n(rows) : wide_n(rows); }
 
+// One layer, its row groups the problems; a table of problems; one layer on CTA pairs.  The kernel knows at compile
+// time, so that a layer's descriptor is read where the launch put it and not through a pointer.
+enum : int { kLayer = 0, kTable = 1, kPairs = 2 };
 // Problem p of the set: from the table, or row group p of the one layer.
+template <int MODE>
 __device__ __forceinline__ const WideProblem& problem(const WideArgs& a, int p) {
-    return a.table ? *reinterpret_cast<const WideProblem*>(reinterpret_cast<const unsigned char*>(a.table) + p * a.table_stride) : a.one;
+    return MODE == kTable ? *reinterpret_cast<const WideProblem*>(reinterpret_cast<const unsigned char*>(a.table) + p * a.table_stride) : a.one;
 }
+template <int MODE>
 __device__ __forceinline__ int problem_rows(const WideArgs& a, int p) {
-    if (a.table) return problem(a, p).rows;
+    if (MODE == kTable) return problem<MODE>(a, p).rows;
     const int left = a.one.rows - p * a.group_rows;
     return left < a.group_rows ? left : a.group_rows;
 }
+template <int MODE>
 __device__ __forceinline__ const unsigned char* problem_tiles(const WideArgs& a, int p) {
-    return a.table ? problem(a, p).tiles : a.one.tiles + (size_t)p * a.hblocks * tile_n(a, a.group_rows) * 256;
+    return MODE == kTable ? problem<MODE>(a, p).tiles : a.one.tiles + (size_t)p * a.hblocks * tile_n(a, a.group_rows) * 256;
 }
 
 // First block of K part s: the blocks [part_begin(s), part_begin(s + 1)) have accumulators of their own.
@@ -127,8 +133,9 @@ __device__ __forceinline__ void red_release_gpu(unsigned int* p, unsigned int v)
 // chunk, adds the other CTAs' planes (finisher) or stores the sums to this CTA's plane
 // (contributor); for outputs the chunk is transposed through `stage` and each warp finishes four
 // rows, eight lanes per row.
-template <bool PARTS, bool PAIR>  // K in more than one part; CTA pairs
+template <bool PARTS, int MODE>  // PARTS: K in more than one part
 struct Epilogue {
+    static constexpr bool PAIR = MODE == kPairs;
     const WideArgs& a;
     int cta, rank, origin, quarter, lane, bar;  // cta: of the split (a pair is one); origin: first unit of the range
     float* areas;      // staging: two areas in turn (one barrier per chunk instead of two), or one
@@ -139,12 +146,12 @@ struct Epilogue {
     // false: a wait ran out (the whole group returns together)
     __device__ __forceinline__ bool segment(const Split& split, const Walk& w, int len, uint32_t dcol, int first_chunk, int step,
                                             uint32_t d_empty) const {
-        const int rows = problem_rows(a, w.p), chunks = (rows + kChunkRows - 1) / kChunkRows;
+        const int rows = problem_rows<MODE>(a, w.p), chunks = (rows + kChunkRows - 1) / kChunkRows;
         const int lo = (w.p * a.nblocks + w.nb) * a.hblocks, hi = lo + a.hblocks;
         const bool contributor = w.hb != 0;
         int last = cta;
         if (!contributor && w.hb + len < a.hblocks) last = owner(split, hi - 1);
-        const WideProblem& pr = PAIR ? a.one : problem(a, w.p);
+        const WideProblem& pr = problem<MODE>(a, w.p);
         // The flag of CTA c counts the chunks of its plane that are there.
         bool late = false;
         for (int c = cta + 1; c <= last && !late; ++c) {
@@ -289,7 +296,7 @@ struct Epilogue {
                 v[3][h] = add_pair(v[3][h], pair_of(lo.w, hi.w));
             }
         }
-        const int out_row = !PAIR && a.table ? (pr.y_rows ? pr.y_rows[r] : r) : w.p * a.group_rows + r;
+        const int out_row = MODE == kTable ? (pr.y_rows ? pr.y_rows[r] : r) : w.p * a.group_rows + r;
         const long long at = (long long)out_row * pr.y_stride + c0;
         float o[4][4];  // [i][j]
         auto unpack = [&] {
@@ -334,8 +341,9 @@ struct Epilogue {
 // At most 72 registers: a CTA of the next call's input stages (128 threads) then fits beside this
 // kernel's, is resident and has its operands in the L2 when this kernel ends.  (ptxas spills for it in
 // the epilogue's chunk: 124 bytes stored and 188 loaded with K parts, 4 bytes without for mul1.)
-template <int CB, bool PARTS, bool PAIR>
+template <int CB, bool PARTS, int MODE>
 __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
+    constexpr bool PAIR = MODE == kPairs;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (still a shared-memory pointer to the compiler)
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -343,7 +351,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     // Weights are immutable and a table is there before the launch before lets this one start (its own
     // wait comes first, see wide_inputs_kernel; acquiring the count acquires the table), so only the
     // activation producer waits.
-    const int count = args.live ? (int)ld_acquire_gpu(reinterpret_cast<const unsigned int*>(args.live)) : args.count;
+    const int count = MODE == kTable && args.live ? (int)ld_acquire_gpu(reinterpret_cast<const unsigned int*>(args.live)) : args.count;
     const int units = count * args.nblocks * args.hblocks;
     const int ctas = (int)gridDim.x >> (PAIR ? 1 : 0), grid = units < ctas ? units : ctas;
     if (cta >= grid) {
@@ -398,7 +406,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             bool ok = true;
             for (Walk w(args, mine); w.unit < w.end && ok;) {
                 const int len = w.length(args);
-                const DeviceWeights& dw = problem(args, w.p).w;
+                const DeviceWeights& dw = problem<MODE>(args, w.p).w;
                 const uint32_t bytes = unit_bytes(dw.bits);
                 int nb = PAIR ? 2 * w.nb + rank : w.nb;
                 if (PAIR && nb >= args.layer_nblocks) nb = args.layer_nblocks - 1;  // padding: decoded, never written out
@@ -426,8 +434,8 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             bool ok = true;
             for (Walk w(args, mine); w.unit < w.end && ok;) {
                 const int len = w.length(args);
-                const uint32_t bytes = (uint32_t)tile_n(args, problem_rows(args, w.p)) * 256;
-                const unsigned char* src = problem_tiles(args, w.p) + (size_t)w.hb * bytes;
+                const uint32_t bytes = (uint32_t)tile_n(args, problem_rows<MODE>(args, w.p)) * 256;
+                const unsigned char* src = problem_tiles<MODE>(args, w.p) + (size_t)w.hb * bytes;
                 for (int i = 0; i < len; ++i, src += bytes) {
                     if (issued >= args.b_slots && !mbar_wait_long(b_empty + 8 * slot, prev_use, args.status, kTimeoutTensorPipe)) {
                         ok = false;
@@ -487,7 +495,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             uint32_t use = 0, a_use = 0;
             bool ok = true;
             for (Walk w(args, mine); w.unit < w.end && ok; ++seg) {
-                const int len = w.length(args), n = tile_n(args, problem_rows(args, w.p)), start = w.unit - mine.begin;
+                const int len = w.length(args), n = tile_n(args, problem_rows<MODE>(args, w.p)), start = w.unit - mine.begin;
                 const uint32_t idesc = umma_idesc_f16_f32(PAIR ? 256 : 128, n), dcol = tmem + d_column(seg) + mine_acc;
                 // (Waited for without a unit in the segment too: the other issuer's commit of the buffer's segment
                 // before must have come before this one's.)
@@ -546,11 +554,11 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             const int p = b / args.nblocks;
             int nb = b - p * args.nblocks;
             if (PAIR) nb = 2 * nb + rank < args.layer_nblocks ? 2 * nb + rank : args.layer_nblocks - 1;
-            const DeviceWeights& dw = problem(args, p).w;
+            const DeviceWeights& dw = problem<MODE>(args, p).w;
             if (lane < 2) prefetch_line_l2(dw.svh + (size_t)nb * 128 + lane * 64);
             else if (lane < 6 && dw.bias) prefetch_line_l2(dw.bias + (size_t)nb * 128 + (lane - 2) * 32);
         }
-        const Epilogue<PARTS, PAIR> epi{args, cta, rank, mine.begin, warp & 3, lane, 1, epi_stage, PAIR ? 0 : kStageFloats};
+        const Epilogue<PARTS, MODE> epi{args, cta, rank, mine.begin, warp & 3, lane, 1, epi_stage, PAIR ? 0 : kStageFloats};
         int seg = 0;
         for (Walk w(args, mine); w.unit < w.end; ++seg) {
             const int len = w.length(args);
@@ -571,13 +579,13 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         Walk w(args, mine);
         const int group = turn;
         auto decode_until = [&](int end) {
-            return decode_segment_rate<CB, kUnitGroups>((PAIR ? args.one : problem(args, w.p)).w.bits, s, end, w_ring, args.w_slots, args.w_stride, w_full, w_empty,
+            return decode_segment_rate<CB, kUnitGroups, MODE == kTable>(problem<MODE>(args, w.p).w.bits, s, end, w_ring, args.w_slots, args.w_stride, w_full, w_empty,
                                                         a_full, a_empty, taddr, a_stages, ctile, lane, args.status);
         };
         if (PAIR) {
             // The accumulators of a group of rows leave no room for a second buffer, so these warps share the
             // epilogue of every segment, each once it has a unit of the next one decoded.
-            const Epilogue<PARTS, PAIR> epi{args, cta, rank, mine.begin, warp & 3, lane, 2 + group, epi_stage + (1 + group) * kStageFloats, 0};
+            const Epilogue<PARTS, MODE> epi{args, cta, rank, mine.begin, warp & 3, lane, 2 + group, epi_stage + (1 + group) * kStageFloats, 0};
             auto share = [&](const Walk& at, int len, int of) {
                 if (group_any(2 + group, !mbar_wait_long(d_full, (uint32_t)of & 1, args.status, kTimeoutTensorPipe))) return false;
                 tc_fence_after_sync();
@@ -616,7 +624,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
             if (ok) ok = mbar_wait_long(all_done, 0, args.status, kTimeoutTensorPipe);
             if (!group_any(2 + group, !ok)) {
                 tc_fence_after_sync();
-                const Epilogue<PARTS, PAIR> epi{args, cta, rank, mine.begin, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, 0};
+                const Epilogue<PARTS, MODE> epi{args, cta, rank, mine.begin, warp & 3, lane, 2 + group, reinterpret_cast<float*>(w_ring) + group * kStageFloats, 0};
                 epi.segment(split, w, w.length(args), tmem + d_column(seg), 1 + group, 1 + kDecodeW / 4, 0);
                 tc_fence_before_sync();
             }
@@ -636,15 +644,16 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
 
 // ---- input stages: four rows of one 128-block per warp, eight lanes per row --------------------
 constexpr int kInputWarps = 4;
+template <int MODE>  // kLayer (pairs too) or kTable
 __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const WideArgs args, int grid_ctas) {
-    if (!args.table) pdl_launch_dependents();
+    if (MODE != kTable) pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l8 = lane & 7;
     const int first = blockIdx.x * kInputWarps + warp;
     uint2 su[4];
-    if (!args.table) {
+    if (MODE != kTable) {
         // One layer: the scales are weights, and the activations may be asked for early (the L2 is
         // the point of coherence); both are there when the launch before ends.
-        const int p = blockIdx.y, rows = problem_rows(args, p), quad = first / args.hblocks, blk = first - quad * args.hblocks;
+        const int p = blockIdx.y, rows = problem_rows<MODE>(args, p), quad = first / args.hblocks, blk = first - quad * args.hblocks;
         const int row = quad * 4 + (lane >> 3);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -655,20 +664,20 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
                              ((size_t)(p * args.group_rows + row) * args.one.x_stride + blk * 128) * (row_bytes / 128) + l8 * 128);
     }
     pdl_wait_prior_grid();  // x may come from the launch before; the tiles may still be read by it
-    if (args.table) pdl_launch_dependents();  // not earlier: that launch reads the table at once
+    if (MODE == kTable) pdl_launch_dependents();  // not earlier: that launch reads the table at once
     if (blockIdx.x == 0 && blockIdx.y == 0)
         for (int i = threadIdx.x; i < grid_ctas; i += blockDim.x) args.flags[i] = 0;
-    const int count = args.live ? *args.live : args.count;
+    const int count = MODE == kTable && args.live ? *args.live : args.count;
     for (int p = blockIdx.y; p < count; p += gridDim.y) {
-        const WideProblem& pr = problem(args, p);
-        const int rows = problem_rows(args, p), quads = (rows + 3) / 4;
+        const WideProblem& pr = problem<MODE>(args, p);
+        const int rows = problem_rows<MODE>(args, p), quads = (rows + 3) / 4;
         const size_t tile_bytes = (size_t)tile_n(args, rows) * 256;
-        unsigned char* tiles = const_cast<unsigned char*>(problem_tiles(args, p));
+        unsigned char* tiles = const_cast<unsigned char*>(problem_tiles<MODE>(args, p));
         const bool aligned = quads_aligned(pr.x, pr.x_dtype, pr.x_stride);
         for (int item = first; item < quads * args.hblocks; item += gridDim.x * kInputWarps) {
             const int quad = item / args.hblocks, blk = item - quad * args.hblocks;
             const int row = quad * 4 + (lane >> 3);
-            const int x_row = row >= rows ? 0 : !args.table ? p * args.group_rows + row : pr.x_rows ? pr.x_rows[row] : row;
+            const int x_row = row >= rows ? 0 : MODE != kTable ? p * args.group_rows + row : pr.x_rows ? pr.x_rows[row] : row;
             float v[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -676,7 +685,7 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
                 if (row < rows)
                     load_quad(pr.x, pr.x_dtype, (long long)x_row * pr.x_stride + blk * 128 + 32 * i + 4 * l8, aligned, v[i]);
             }
-            if (args.table || item != first) {
+            if (MODE == kTable || item != first) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     su[i] = __ldg(reinterpret_cast<const uint2*>(pr.w.suh + blk * 128 + 32 * i + 4 * l8));
@@ -761,22 +770,23 @@ cudaError_t launch_wide_inputs(const WideSet& set, const WidePlan& plan, unsigne
     const int y = set.count < 1024 ? set.count : 1024;
     int x = streaming_grid((long long)per_problem * y, 8) / y;
     x = x < 1 ? 1 : x > per_problem ? per_problem : x;
-    return launch_pdl(wide_inputs_kernel, dim3(x, y), 32 * kInputWarps, 0, programmatic, stream, a, plan.grid * (plan.pair ? 2 : 1));
+    return launch_pdl(set.table ? wide_inputs_kernel<kTable> : wide_inputs_kernel<kLayer>, dim3(x, y), 32 * kInputWarps, 0, programmatic, stream, a,
+                      plan.grid * (plan.pair ? 2 : 1));
 }
 
 cudaError_t launch_wide(const WideSet& set, const WidePlan& plan, unsigned int* flags, float* planes, unsigned int* status,
                         bool programmatic, cudaStream_t stream) {
     const WideArgs a = wide_args(set, plan, flags, planes, status);
     const long long units = (long long)set.count * a.nblocks * a.hblocks;
-    if (plan.pair && (set.table || a.d_accs != 1 || a.parts != 1)) return cudaErrorInvalidValue;  // one layer, more than 128 rows a group
+    if ((plan.pair && (set.table || a.d_accs != 1)) || (!set.table && a.parts != 1)) return cudaErrorInvalidValue;  // one layer, more than 128 rows a group
     if (units < 1 || units > 0x7FFFFFFF || plan.b_slots < 1 || plan.w_slots < 2 || plan.smem_bytes > kSmemLimitW ||
         (size_t)plan.w_slots * plan.w_stride < kRingMin)
         return cudaErrorInvalidValue;
     return for_codebook(set.codebook, [&](auto cb) {
         constexpr int CB = decltype(cb)::value;
-        if (plan.pair) return launch_clusters(wide_linear_kernel<CB, false, true>, 2, 2 * plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a);
-        return a.parts > 1 ? launch_pdl(wide_linear_kernel<CB, true, false>, plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a)
-                           : launch_pdl(wide_linear_kernel<CB, false, false>, plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a);
+        if (plan.pair) return launch_clusters(wide_linear_kernel<CB, false, kPairs>, 2, 2 * plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a);
+        return launch_pdl(!set.table ? wide_linear_kernel<CB, false, kLayer> : a.parts > 1 ? wide_linear_kernel<CB, true, kTable> : wide_linear_kernel<CB, false, kTable>,
+                          plan.grid, kThreadsW, plan.smem_bytes, programmatic, stream, a);
     });
 }
 
@@ -784,9 +794,10 @@ cudaError_t launch_wide(const WideSet& set, const WidePlan& plan, unsigned int* 
 // on a device (configure_device), never on the launch path.
 template <int CB>
 static cudaError_t configure_wide_cb() {
-    cudaError_t e = cudaFuncSetAttribute(wide_linear_kernel<CB, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_linear_kernel<CB, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_linear_kernel<CB, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    cudaError_t e = cudaFuncSetAttribute(wide_linear_kernel<CB, false, kLayer>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_linear_kernel<CB, false, kTable>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_linear_kernel<CB, true, kTable>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_linear_kernel<CB, false, kPairs>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitW);
     return e;
 }
 cudaError_t configure_wide_kernels() {
@@ -795,7 +806,8 @@ cudaError_t configure_wide_kernels() {
     if (e == cudaSuccess) e = configure_wide_cb<CB_MUL1>();
     // The same shared-memory carve-out as the kernel that follows: an SM that has to change its split
     // between L1 and shared memory drains first, and nothing of the two launches overlaps.
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_inputs_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_inputs_kernel<kLayer>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(wide_inputs_kernel<kTable>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     return e;
 }
 
