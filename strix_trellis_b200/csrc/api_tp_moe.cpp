@@ -220,7 +220,10 @@ strix_status host_routing(const strix_tp_moe_desc* d, int tokens, int top_k, std
     return STRIX_SUCCESS;
 }
 
-strix_status enqueue_gate_up(strix_tp_moe_plan_impl* p) {
+// `hidden`: with the SwiGLU of the rows; without it the down projection of the same submit makes them
+// (enqueue_down with `fused`), one launch and one pass over the rows less.
+bool down_makes_hidden(const strix_tp_moe_plan_impl* p) { return !p->down_plan.direct; }
+strix_status enqueue_gate_up(strix_tp_moe_plan_impl* p, bool hidden = true) {
     cudaError_t e = cudaSuccess;
     if (p->device_routed)
         e = st::launch_moe_route(p->route_ids, p->scores, p->tokens, p->top_k, p->bank, p->bank_count, p->window, p->gu,
@@ -228,7 +231,7 @@ strix_status enqueue_gate_up(strix_tp_moe_plan_impl* p) {
     if (e == cudaSuccess)
         e = st::launch_grouped(p->gu, p->gu_count, p->model, p->inter, p->codebook, p->gu_plan, p->owner->status,
                                p->owner->programmatic_launch, p->stream);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && hidden)
         e = st::launch_swiglu(p->g, p->u, p->hidden, p->tokens * p->top_k, p->inter, p->inter,
                               p->owner->programmatic_launch, p->stream);
     return cuda_status(e);
@@ -272,8 +275,10 @@ void plan_projections(strix_tp_moe_plan_impl* p, const Geometry& g, int group_ro
     }
 }
 
-strix_status enqueue_down(strix_tp_moe_plan_impl* p, bool combine = true) {
-    cudaError_t e = st::launch_grouped(p->down, p->down_count, p->inter, p->model, p->codebook, p->down_plan,
+strix_status enqueue_down(strix_tp_moe_plan_impl* p, bool combine = true, bool fused = false) {
+    st::GroupedPlan plan = p->down_plan;
+    if (fused) plan.swiglu = st::SwigluRows{p->g, p->u, p->hidden};
+    cudaError_t e = st::launch_grouped(p->down, p->down_count, p->inter, p->model, p->codebook, plan,
                                        p->owner->status, p->owner->programmatic_launch, p->stream);
     if (e == cudaSuccess && combine) {
         const bool partial = p->device_routed && p->window.experts_total != p->bank_count;  // other ranks own some slots
@@ -535,8 +540,8 @@ strix_status strix_tp_moe_plan_down(strix_tp_moe_plan p) {
 strix_status strix_tp_moe_plan_submit(strix_tp_moe_plan p) {
     if (!p) return STRIX_ERROR_INVALID_ARGUMENT;
     strix_status s = context_check(p->owner);
-    if (s == STRIX_SUCCESS) s = enqueue_gate_up(p);
-    if (s == STRIX_SUCCESS) s = enqueue_down(p);
+    if (s == STRIX_SUCCESS) s = enqueue_gate_up(p, !down_makes_hidden(p));
+    if (s == STRIX_SUCCESS) s = enqueue_down(p, true, down_makes_hidden(p));
     return s;
 }
 // ---- expert parallelism: the bank as a window of the router's id space ------------------------
@@ -554,8 +559,8 @@ strix_status strix_b200_moe_plan_set_window(strix_tp_moe_plan p, uint32_t first_
 strix_status strix_b200_moe_plan_projections(strix_tp_moe_plan p) {
     if (!p) return STRIX_ERROR_INVALID_ARGUMENT;
     strix_status s = context_check(p->owner);
-    if (s == STRIX_SUCCESS) s = enqueue_gate_up(p);
-    if (s == STRIX_SUCCESS) s = enqueue_down(p, false);
+    if (s == STRIX_SUCCESS) s = enqueue_gate_up(p, !down_makes_hidden(p));
+    if (s == STRIX_SUCCESS) s = enqueue_down(p, false, down_makes_hidden(p));
     return s;
 }
 strix_status strix_b200_moe_plan_rows(strix_tp_moe_plan p, const float** each, const int32_t** row_valid) {

@@ -108,6 +108,7 @@ cudaError_t launch_gemv(const LinearCall& call, const GemvPlan& plan, void* work
 
 // ---- GEMM (rows > 8) --------------------------------------------------------------------
 struct GemmPlan {
+    size_t act_bytes;        // core input as binary16 operand images
     size_t workspace_bytes;
     int sm_count;
     bool dense;  // weights decoded once, dense GEMM (else decoded on the fly)

@@ -100,22 +100,26 @@ GemmPlan plan_gemm(const DeviceWeights& w, int rows, int sm_count) {
     const double dense = sm_count >= 2 ? dense_us(w, rows, sm_count) : 0.0;
     plan.dense = sm_count >= 2 && (rows > kWideMaxRows || dense < cut.us);
     if (plan.dense) {
-        plan.workspace_bytes = align_up((size_t)gemm_dense_rows_padded(rows) * w.inputs * 2) + gemm_dense_scratch(w);
+        plan.act_bytes = align_up((size_t)gemm_dense_rows_padded(rows) * w.inputs * 2);
+        plan.workspace_bytes = plan.act_bytes + gemm_dense_scratch(w);
     } else {
         const WidePlan wide = wide_plan(w, cut);
-        plan.workspace_bytes = wide.flag_bytes + wide.plane_bytes + align_up((size_t)cut.groups * (w.inputs / 128) * wide_tile_bytes(cut.rows));
+        plan.act_bytes = align_up((size_t)cut.groups * (w.inputs / 128) * wide_tile_bytes(cut.rows));
+        plan.workspace_bytes = wide.flag_bytes + wide.plane_bytes + plan.act_bytes;
     }
     if (rows > kWideRows && rows <= kPairMaxRows && sm_count >= 2) {
         const Cut pairs = cut_pairs(w, rows, sm_count);
         plan.pairs = pairs.us < (plan.dense ? dense : cut.us);
         if (plan.pairs) {
             const WidePlan wide = pair_plan(w, pairs);
-            const size_t need = wide.flag_bytes + wide.plane_bytes + align_up((size_t)pairs.groups * (w.inputs / 128) * pair_n(pairs.rows) * 256);
+            const size_t act = align_up((size_t)pairs.groups * (w.inputs / 128) * pair_n(pairs.rows) * 256);
+            const size_t need = wide.flag_bytes + wide.plane_bytes + act;
             if (need > plan.workspace_bytes) {
                 // In the space of the decoded weights as a rule; a layer too small for that stays with its route.
                 if (plan.dense) plan.pairs = false;
                 else plan.workspace_bytes = need;
             }
+            if (plan.pairs) plan.act_bytes = act;
         }
     }
     return plan;

@@ -39,6 +39,7 @@ struct GroupedPlan {
     size_t partial_bytes_per_problem;  // core input tiles of one problem; direct: counters (zero at first) and planes
     size_t shared_bytes;               // flags and planes of a launch
     unsigned char* shared;             // the caller's memory for them
+    SwigluRows swiglu;                 // not direct: input rows that the launch makes itself
 };
 // `rows` = most rows of one problem, `problems` = most problems of a launch; for up to kDirectRows rows
 // the plan may be a direct one (direct_pays).

@@ -164,6 +164,14 @@ __device__ __forceinline__ float half_bits_to_float(uint16_t h) {
     return __half2float(__ushort_as_half(h));
 }
 
+// SiLU(gate) * up with the stable sigmoid (src/tp_moe_activation.hpp:52-59).
+__device__ __forceinline__ float swiglu(float g, float u) {
+    const float e = expf(g < 0.0f ? g : -g);
+    const float d = __fadd_rn(1.0f, e);
+    const float sig = g < 0.0f ? __fdiv_rn(e, d) : __fdiv_rn(1.0f, d);
+    return __fmul_rn(__fmul_rn(g, sig), u);
+}
+
 // RN16(RN32(x * f32(suh))) as a float holding the binary16 value.  The product is
 // rounded to float32 first; converting the exact product straight to binary16 would
 // round differently on ties (reference tests/test_numerics.py:46-54).

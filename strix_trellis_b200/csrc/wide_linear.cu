@@ -63,6 +63,7 @@ struct WideArgs {
     int a_stages, d_bufs, d_accs, parts, parts_log2;
     // CTA pairs: `nblocks` above counts pairs of column blocks; the layer's own count
     int pair, layer_nblocks;
+    SwigluRows swiglu;
     unsigned int* flags;
     float* planes;
     unsigned int* status;
@@ -646,6 +647,9 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
 constexpr int kInputWarps = 4;
 template <int MODE>  // kLayer (pairs too) or kTable
 __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const WideArgs args, int grid_ctas) {
+    // Rows that are still to be made come from the launch before, their table from launches before that, which were
+    // over when the launch before let this one start: everything up to the rows themselves is read ahead of the wait.
+    const bool early = MODE == kTable && args.swiglu.gate;
     if (MODE != kTable) pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l8 = lane & 7;
     const int first = blockIdx.x * kInputWarps + warp;
@@ -663,11 +667,16 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
             prefetch_line_l2(static_cast<const unsigned char*>(args.one.x) +
                              ((size_t)(p * args.group_rows + row) * args.one.x_stride + blk * 128) * (row_bytes / 128) + l8 * 128);
     }
-    pdl_wait_prior_grid();  // x may come from the launch before; the tiles may still be read by it
-    if (MODE == kTable) pdl_launch_dependents();  // not earlier: that launch reads the table at once
-    if (blockIdx.x == 0 && blockIdx.y == 0)
-        for (int i = threadIdx.x; i < grid_ctas; i += blockDim.x) args.flags[i] = 0;
-    const int count = MODE == kTable && args.live ? *args.live : args.count;
+    bool waited = false;
+    auto wait = [&] {  // x may come from the launch before; the tiles may still be read by it
+        pdl_wait_prior_grid();
+        if (MODE == kTable) pdl_launch_dependents();  // not earlier: that launch reads the table at once, and decodes beside this one
+        if (blockIdx.x == 0 && blockIdx.y == 0)
+            for (int i = threadIdx.x; i < grid_ctas; i += blockDim.x) args.flags[i] = 0;
+        waited = true;
+    };
+    if (!early) wait();
+    const int count = MODE == kTable && args.live ? (int)ld_acquire_gpu(reinterpret_cast<const unsigned int*>(args.live)) : args.count;
     for (int p = blockIdx.y; p < count; p += gridDim.y) {
         const WideProblem& pr = problem<MODE>(args, p);
         const int rows = problem_rows<MODE>(args, p), quads = (rows + 3) / 4;
@@ -678,17 +687,40 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
             const int quad = item / args.hblocks, blk = item - quad * args.hblocks;
             const int row = quad * 4 + (lane >> 3);
             const int x_row = row >= rows ? 0 : MODE != kTable ? p * args.group_rows + row : pr.x_rows ? pr.x_rows[row] : row;
-            float v[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0.f;
-                if (row < rows)
-                    load_quad(pr.x, pr.x_dtype, (long long)x_row * pr.x_stride + blk * 128 + 32 * i + 4 * l8, aligned, v[i]);
-            }
             if (MODE == kTable || item != first) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     su[i] = __ldg(reinterpret_cast<const uint2*>(pr.w.suh + blk * 128 + 32 * i + 4 * l8));
+            }
+            if (MODE == kTable && !waited) wait();
+            float v[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0.f;
+                if (row < rows && !(MODE == kTable && args.swiglu.gate))
+                    load_quad(pr.x, pr.x_dtype, (long long)x_row * pr.x_stride + blk * 128 + 32 * i + 4 * l8, aligned, v[i]);
+            }
+            if (MODE == kTable && args.swiglu.gate && row < rows) {
+                const long long at = (long long)x_row * args.hblocks * 128 + blk * 128 + 4 * l8;
+                float4 g[4], u[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    g[i] = __ldcg(reinterpret_cast<const float4*>(args.swiglu.gate + at + 32 * i));
+                    u[i] = __ldcg(reinterpret_cast<const float4*>(args.swiglu.up + at + 32 * i));
+                }
+                const bool whole = (reinterpret_cast<uintptr_t>(args.swiglu.hidden) & 15) == 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    v[i][0] = swiglu(g[i].x, u[i].x);
+                    v[i][1] = swiglu(g[i].y, u[i].y);
+                    v[i][2] = swiglu(g[i].z, u[i].z);
+                    v[i][3] = swiglu(g[i].w, u[i].w);
+                    float* out = args.swiglu.hidden + at + 32 * i;
+                    if (whole) *reinterpret_cast<float4*>(out) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+                    else
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) out[j] = v[i][j];
+                }
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) scale_quad(v[i], su[i]);
@@ -700,6 +732,7 @@ __global__ void __launch_bounds__(32 * kInputWarps) wide_inputs_kernel(const Wid
                     make_uint2(as_u32(__floats2half2_rn(v[i][0], v[i][1])), as_u32(__floats2half2_rn(v[i][2], v[i][3])));
         }
     }
+    if (MODE == kTable && !waited) wait();
 }
 
 // ---- host side -----------------------------------------------------------------------------------
@@ -733,6 +766,7 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     a.one = set.one;
     a.count = set.count;
     a.group_rows = set.group_rows;
+    a.swiglu = set.swiglu;
     a.hblocks = set.inputs / 128;
     a.pair = plan.pair;
     a.layer_nblocks = set.outputs / 128;

@@ -56,6 +56,13 @@ ST_RATE_FN int accumulator_parts(int hblocks, int nblocks, long long groups, int
 // `heaviest`: the rate code with the largest tiles among the problems.
 WidePlan plan_wide(int heaviest, int rows_max, long long units, int sm_count, bool pair = false);
 
+// Input rows that are still to be made: row r is SwiGLU of rows r of `gate` and `up`, and is also written to `hidden`
+// (all [rows][inputs]).
+struct SwigluRows {
+    const float* gate;
+    const float* up;
+    float* hidden;
+};
 // A set of problems of one geometry.  `table` (device memory) holds them, `table_stride` bytes apart;
 // without a table the set is ONE layer whose `one.rows` rows are cut into problems of group_rows rows.
 // `live` (device memory, may be null) overrides `count` at run time.
@@ -66,6 +73,7 @@ struct WideSet {
     WideProblem one;
     int count, group_rows;
     int inputs, outputs, codebook;
+    SwigluRows swiglu;  // of a table whose x rows they are; gate null: x is there
 };
 // Input stages of every row of every problem into its tiles; also zeroes the flags.
 cudaError_t launch_wide_inputs(const WideSet& set, const WidePlan& plan, unsigned int* flags, bool programmatic,

@@ -171,6 +171,42 @@ def test_routed_rows_per_expert(ctx, tokens, n_exp, top_k):
             w.close()
 
 
+@pytest.mark.parametrize("tokens,n_exp,top_k", [(1, 4, 2), (150, 1, 1), (130, 2, 2), (200, 16, 6)])
+def test_hidden_rows_of_a_submit(ctx, tokens, n_exp, top_k):
+    """Hidden rows and outputs of a submit, whose down projection makes the rows itself (except where the direct kernel
+    serves it), have the bits of the three stages one by one; more routes than the routing kernel has threads, and
+    a row with an id twice."""
+    from strix_trellis_b200.runtime import MoePlan
+    model, inter = 512, 384
+    layers = make_experts(n_exp, model, inter, 9260, bits_of=lambda e, k: 2)
+    ws = [tuple(ctx.prepare(l[k]) for k in ("gate", "up", "down")) for l in layers]
+    x = dev(synthetic.make_activations(tokens, model, seed=9261))
+    ids, scores = synthetic.make_routes(tokens, n_exp, top_k, seed=9262)
+    ids = ids.astype(np.uint32)
+    bad = tokens - 1 if top_k > 1 and tokens > 1 else None
+    if bad is not None:
+        ids[bad, top_k - 1] = ids[bad, 0]
+    y = torch.zeros((tokens, model), device="cuda")
+    plan = MoePlan(ctx, ws, x, y, dev(ids.view(np.int32)), dev(scores), device_routed=True)
+    plan.gate_up()
+    plan.down()
+    torch.cuda.synchronize()
+    valid = [t for t in range(tokens) if t != bad]
+    rows, out = plan.hidden().clone(), y.clone()
+    plan.hidden().fill_(float("nan"))
+    y.fill_(7.0)
+    for _ in range(2):
+        plan.submit()
+    torch.cuda.synchronize()
+    assert torch.equal(plan.hidden()[valid], rows[valid])
+    assert torch.equal(y[valid], out[valid]) and torch.isfinite(y[valid]).all()
+    assert bad is None or torch.isnan(y[bad]).all()
+    plan.close()
+    for t in ws:
+        for w in t:
+            w.close()
+
+
 @pytest.mark.parametrize("tokens,n_exp,top_k", [(150, 1, 1), (64, 4, 2)])
 def test_submits_without_a_live_route(ctx, tokens, n_exp, top_k):
     """Every route invalid, several submits in a row, then valid ones on the same plan: launches that have
