@@ -81,7 +81,7 @@ strix_status strix_b200_gemv_partition(uint64_t inputs, uint64_t outputs, uint32
 strix_status strix_b200_gemm_route(uint64_t inputs, uint64_t outputs, uint32_t bits_x2, uint32_t rows,
                                    uint32_t sm_count, uint64_t out[4]);
 
-/* The same for CTA pairs, which 257 to 1024 rows may take: out[0] = the groups that the rows are cut into
+/* The same for CTA pairs, which 257 to 4096 rows may take: out[0] = the groups that the rows are cut into
  * (0: another route), out[1] = the pairs, out[2] = the bytes that they use of the workspace. */
 strix_status strix_b200_gemm_pairs(uint64_t inputs, uint64_t outputs, uint32_t bits_x2, uint32_t rows,
                                    uint32_t sm_count, uint64_t out[3]);

@@ -1,8 +1,8 @@
 // Routes of a GEMM (more than 8 rows) and their workspace.
 //   weights decoded on the fly into tensor memory, once for each row group (wide_linear.cu)
-//   the same by CTA pairs, 257 to 1024 rows (wide_linear.cu)
+//   the same by CTA pairs, 257 to 4096 rows (wide_linear.cu)
 //   weights decoded once into the workspace, dense GEMM (gemm_dense.cu)
-// Beyond kWideMaxRows always the last; below, whichever the estimates here say is faster.
+// Whichever the estimates here say is faster; beyond kWideMaxRows not the first, beyond kPairMaxRows the last.
 #include "strix_trellis_b200.h"
 #include "wide_linear.h"
 
@@ -19,9 +19,11 @@ cudaError_t launch_gemm_dense(const LinearCall& call, unsigned char* workspace, 
 namespace {
 // As far as the estimates are fitted and measured; beyond, four and more decodes of a unit hardly pay.
 constexpr int kWideMaxRows = 1024;
-// Beyond, decoding once is level with decoding in CTA pairs or better.  (From 257 rows on: below, one tile is too
-// little for 74 pairs on most layers.)
-constexpr int kPairMaxRows = 1024;
+// CTA pairs: from 257 rows on (below, one tile is too little for 74 pairs on most layers).  The estimates are less
+// sure beyond 1024 rows, where decoding once is paid by more rows: there the pairs' has to be lower by 8 %, with which
+// they were never slower among 25 shapes of 1042 to 3863 rows (1777 rows, 5120 -> 5120 94.8 -> 90.9 us; 2122 rows, 6272 -> 7040
+// 182 -> 170; with equal estimates 2851 rows, 2304 -> 11520 142 -> 158).
+constexpr int kPairMaxRows = 4096;
 
 // How a call's rows are cut into groups that each decode the weights, and how many CTAs run them: one
 // group and every SM, unless so few column blocks are left that many CTAs share one and the CTA that
@@ -109,7 +111,7 @@ GemmPlan plan_gemm(const DeviceWeights& w, int rows, int sm_count) {
     }
     if (rows > kWideRows && rows <= kPairMaxRows && sm_count >= 2) {
         const Cut pairs = cut_pairs(w, rows, sm_count);
-        plan.pairs = pairs.us < (plan.dense ? dense : cut.us);
+        plan.pairs = pairs.us < (rows > kWideMaxRows ? 0.92 * dense : plan.dense ? dense : cut.us);
         if (plan.pairs) {
             const WidePlan wide = pair_plan(w, pairs);
             const size_t act = align_up((size_t)pairs.groups * (w.inputs / 128) * pair_n(pairs.rows) * 256);

@@ -73,7 +73,7 @@ def test_cta_pairs(shape, sm_count):
             if not groups:
                 assert pairs == used == 0
                 continue
-            assert 256 < rows <= 1024 and sm_count >= 2
+            assert 256 < rows <= 4096 and sm_count >= 2
             assert 128 < -(-rows // groups) <= 256 and 1 <= pairs <= min(sm_count // 2, groups * tiles * (inputs // 128))
             planes = 2 * pairs * 512 * -(-rows // groups)
             assert rows * inputs * 2 + planes <= used <= route(inputs, outputs, bits_x2, rows, sm_count)[1][1]

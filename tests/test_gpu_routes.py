@@ -91,7 +91,7 @@ def pairs_of(inputs, outputs, bits, rows, sm_count):
     (257, 1536, 8320, 5, "mul1"),                              # smallest, whole tiles, an odd number of column blocks
     (289, 1024, 9600, 4, "mcg"), (384, 1024, 9600, 2, "3inst"),  # tiles cut between pairs, odd blocks
     (512, 1024, 9600, 8, "mul1"), (513, 2048, 2176, 3, "mul1"), (1024, 1280, 6016, 6, "mul1"),  # two and more tiles a pair
-    (700, 2048, 2176, 1, "mul1")])
+    (700, 2048, 2176, 1, "mul1"), (1100, 3072, 2176, 4, "mul1"), (1254, 3072, 2048, 6, "mul1")])
 def test_cta_pairs(ctx, rows, inputs, outputs, bits, codebook):
     assert pairs_of(inputs, outputs, bits, rows, torch.cuda.get_device_properties(0).multi_processor_count)[0]
     check(ctx, rows, inputs, outputs, bits, codebook, bias=bits != 4)
