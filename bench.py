@@ -21,7 +21,7 @@ With N>1 (launched under torchrun) every rank runs the same workload on its own 
 the timed region: rates x rows on the largest shape, the prefill GEMM (K4/K5/K6), the
 routed-expert block on one rank's bank, and at every N the tensor-parallel dense layers
 (row-parallel + all-reduce, LM head + all-gather) and the expert-parallel block
-(all-to-all dispatch and return).  `--no-extra` skips them; `--case gemv|gemv-rows|gemm|gemm-small|moe|decode` runs one
+(all-to-all dispatch and return).  `--no-extra` skips them; `--case gemv|gemv-rows|gemm|gemm-small|gemm-mid|moe|decode` runs one
 small fixed workload of one kernel for profilers.
 
 `--impl reference` times the CPU contract (this repository's C restatement of the
@@ -512,6 +512,9 @@ def run_case(args):
     elif args.case == "gemm-small":
         print(json.dumps({"case": "gemm 4096->12288 K4, one row tile with K partitions",
                           **gemm_case(torch, ctx, stream, [128], reps=2), "status": ctx.device_status()}))
+    elif args.case == "gemm-mid":
+        print(json.dumps({"case": "gemm 4096->12288 K4, 512 rows in CTA pairs",
+                          **gemm_case(torch, ctx, stream, [512], reps=2), "status": ctx.device_status()}))
     else:
         print(json.dumps({"case": "moe bank 32, top-8, 4096/2048 K2", **moe_case(torch, ctx, stream, [8], reps=2),
                           "status": ctx.device_status()}))
@@ -822,7 +825,7 @@ def run_gpu(args):
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
                          "traffic": None if traffic is None else round(traffic * total_bytes / launches),
-                         "kernel": "gemv_row_kernel<4, mul1>",
+                         "kernel": "gemv_row_kernel<4, mul1>; 4096x14336: gemv_tmem_kernel<mul1>",
                          "algorithmic_bytes_per_launch": round(total_bytes / launches)},
             "e2e": {"value": round(e2e_value, 2), "unit": "GB/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h},
@@ -844,7 +847,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--no-extra", action="store_true", help="skip the GEMM / MoE / TP side measurements")
-    ap.add_argument("--case", choices=["gemv", "gemv-rows", "gemm", "gemm-small", "moe", "decode"], help="run one small profiling workload and exit")
+    ap.add_argument("--case", choices=["gemv", "gemv-rows", "gemm", "gemm-small", "gemm-mid", "moe", "decode"], help="run one small profiling workload and exit")
     args = ap.parse_args()
     if args.case:
         run_case(args)

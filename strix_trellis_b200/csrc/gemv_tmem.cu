@@ -23,7 +23,8 @@
 //
 // Measured in a chain of launches against the kernel before, which fed mma.sync and staged its rows
 // four 2-byte stores at a time: 16 layers, four rows, K2..K6 226 -> 179 us (four of them small ones in
-// gemv_few.cu); 16384 -> 4096, eight rows, K5 29.6 -> 22.0 us; 4096 -> 129280, one row, K5 133 -> 118 us.
+// gemv_few.cu); 16384 -> 4096, eight rows, K5 29.6 -> 22.0 us; 4096 -> 129280, one row, K5 133 -> 118 us.  With two MMA
+// issuers, tiles in quads and the decoder balanced between the pipes 171, 21.1 and 113 us.
 #include <type_traits>
 
 #include "gemv_kernels.h"

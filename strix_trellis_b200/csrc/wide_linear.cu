@@ -340,8 +340,7 @@ struct Epilogue {
 };
 
 // At most 72 registers: a CTA of the next call's input stages (128 threads) then fits beside this
-// kernel's, is resident and has its operands in the L2 when this kernel ends.  (ptxas spills for it in
-// the epilogue's chunk: 124 bytes stored and 188 loaded with K parts, 4 bytes without for mul1.)
+// kernel's, is resident and has its operands in the L2 when this kernel ends.
 template <int CB, bool PARTS, int MODE>
 __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
     constexpr bool PAIR = MODE == kPairs;
@@ -776,8 +775,9 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     a.w_stride = plan.w_stride;
     a.b_slots = plan.b_slots;
     a.b_stride = plan.b_stride;
-    // Even and odd K steps have accumulators of their own where there is room, half the truncating
-    // accumulations in a row; calls of up to sixteen rows have four, as those of up to eight have (distance from the
+    // The two issuers have accumulators of their own where there is room, half the truncating accumulations in a row
+    // (with one issuer it was even and odd K steps: 64 rows of 4096 -> 4096 5.6e-7, now 5.7e-7; 101 rows of 4096 -> 12288 1.36e-6
+    // both); calls of up to sixteen rows have four, as those of up to eight have (distance from the
     // sum in 64 bits, 16 rows of 5120 -> 5120: 8.4e-7 of its norm with two, 4.5e-7 with four, at
     // 15.75 us instead of 15.55).  Beyond 128 rows there is room for one (129 rows of 4096 -> 12288: 2.6e-6
     // where two give 1.4e-6 for 128), as in the dense GEMM (4.9e-6).  A second buffer lets the MMAs of
