@@ -176,10 +176,10 @@ struct Epilogue {
             // Parts in ascending K order; the running sum of a column waits in its place in `stage`.
 #pragma unroll 1
             for (int part = first_part; part <= last_part; ++part) {
-                // The units of this part in this segment: from two on both issuers have had some.
+                // The units of this part in this segment: from two on both issuers have had some (halves of each: always).
                 const int lo = PARTS && part_begin(a, part) > w.hb ? part_begin(a, part) : w.hb;
                 const int hi = PARTS && part_begin(a, part + 1) < w.hb + len ? part_begin(a, part + 1) : w.hb + len;
-                const bool both = a.d_accs > 1 && hi - lo > 1;
+                const bool both = a.d_accs > 1 && (MODE == kLayer || hi - lo > 1);
                 const int set = a.d_accs > 1 && !both ? (w.unit - origin + lo - w.hb) & 1 : 0;
                 const uint32_t at = taddr + (part * a.d_accs + set * (a.d_accs >> 1)) * a.n_max + ch * kChunkRows;
                 auto add = [&](uint32_t from) {
@@ -375,10 +375,14 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                    b_empty = b_full + 8 * kMaxBSlots, a_full = b_empty + 8 * kMaxBSlots, a_empty = a_full + 8 * kMaxAStages,
                    d_full = a_empty + 8 * kMaxAStages, d_empty = d_full + 16, all_done = d_empty + 16, d_peer = all_done + 8;  // d_peer: of a pair, the partner's accumulators are read
     const int issuers = args.d_accs > 1 ? kIssuers : 1;
+    // Of one layer each issuer takes a K = 64 half of every unit, so that the sums' chains are of one length; of a
+    // table, whose segments are whole blocks as a rule, the units in turn, which halves the waits.
+    constexpr bool kHalves = MODE == kLayer;
+    const int unit_commits = kHalves ? issuers : 1;
     if (threadIdx.x == 0) {
         for (int i = 0; i < args.w_slots; ++i) { mbar_init(w_full + 8 * i, 1); mbar_init(w_empty + 8 * i, 4); }
-        for (int i = 0; i < args.b_slots; ++i) { mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, 1); }
-        for (int i = 0; i < a_stages; ++i) { mbar_init(a_full + 8 * i, 4); mbar_init(a_empty + 8 * i, 1); }
+        for (int i = 0; i < args.b_slots; ++i) { mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, unit_commits); }
+        for (int i = 0; i < a_stages; ++i) { mbar_init(a_full + 8 * i, 4); mbar_init(a_empty + 8 * i, unit_commits); }
         for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, issuers); mbar_init(d_empty + 8 * i, PAIR ? kEpiW + kDecodeW : kEpiW); }
         mbar_init(all_done, issuers);
         mbar_init(d_peer, 1);
@@ -461,7 +465,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                 mbar_wait(b_full + 8 * (i % args.b_slots), (uint32_t)(i / args.b_slots) & 1, args.status, kTimeoutDrain);
         }
     } else if (warp >= kWarpMma) {
-        // ---- MMA issuers, a unit each in turn: the whole warp walks, an elected lane issues ---------
+        // ---- MMA issuers, a half of each unit or the units in turn: the whole warp walks, an elected lane issues
         const int me = warp - kWarpMma;
         if (PAIR && rank) {
             // ---- partner CTA: one signal per unit that is decoded and whose rows have landed ----------
@@ -491,7 +495,8 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
         } else if (me < issuers) {
             // K step k of a unit goes to accumulator `me` of two, or (four) 2 me + k % 2.
             const uint32_t mine_acc = me * (args.d_accs >> 1) * args.n_max, odd = args.d_accs == 4 ? args.n_max : 0;
-            int next = me, slot = me, stage = me, seg = 0;  // of this warp's next unit
+            const int turns = kHalves ? 1 : issuers, half0 = kHalves ? me : 0, halves = kHalves && issuers > 1 ? 1 : 2;
+            int next = kHalves ? 0 : me, slot = next, stage = next, seg = 0;  // of this warp's next unit
             uint32_t use = 0, a_use = 0;
             bool ok = true;
             for (Walk w(args, mine); w.unit < w.end && ok; ++seg) {
@@ -507,7 +512,7 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                     }
                 }
                 int part = PARTS ? part_of(args, w.hb) : 0, fresh = 1;
-                for (; next < start + len; next += issuers) {
+                for (; next < start + len; next += turns) {
                     while (PARTS && part_begin(args, part + 1) <= w.hb + next - start) { ++part; fresh = 1; }
                     const uint32_t acc = dcol + part * args.d_accs * args.n_max;
                     if (!mbar_wait_long(b_full + 8 * slot, use, args.status, kTimeoutTensorPipe) ||
@@ -525,16 +530,21 @@ __global__ void __maxnreg__(72) wide_linear_kernel(const WideArgs args) {
                         umma_commit_pair(a_empty + 8 * stage, 3);
                         umma_commit_pair(b_empty + 8 * slot, 3);
                     } else if (!PAIR && elect_one()) {
+#pragma unroll(kHalves ? 1 : 2)
+                        for (int h = 0; h < halves; ++h) {
+                            const uint64_t b = (kHalves ? half0 + h : h) ? b1 : b0;
+                            const uint32_t from = acol + 32 * (kHalves ? half0 + h : h);
 #pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            umma_f16_ts(acc + (k & 1) * odd, acol + 8 * k, (k < 4 ? b0 : b1) + 2 * (k & 3), idesc, !fresh || k > 1 || (k == 1 && !odd));
+                            for (int k = 0; k < 4; ++k)
+                                umma_f16_ts(acc + (k & 1) * odd, from + 8 * k, b + 2 * k, idesc, !fresh || h || k > 1 || (k == 1 && !odd));
+                        }
                         umma_commit(a_empty + 8 * stage);
                         umma_commit(b_empty + 8 * slot);
                     }
                     __syncwarp();
                     fresh = 0;
-                    if ((slot += issuers) >= args.b_slots) { slot -= args.b_slots; use ^= 1; }
-                    if ((stage += issuers) >= a_stages) { stage -= a_stages; a_use ^= 1; }
+                    if ((slot += turns) >= args.b_slots) { slot -= args.b_slots; use ^= 1; }
+                    if ((stage += turns) >= a_stages) { stage -= a_stages; a_use ^= 1; }
                 }
                 if (elect_one()) {
                     if (PAIR) umma_commit_pair(d_full + 8 * d_index(seg), 3);
@@ -776,8 +786,7 @@ static WideArgs wide_args(const WideSet& set, const WidePlan& plan, unsigned int
     a.b_slots = plan.b_slots;
     a.b_stride = plan.b_stride;
     // The two issuers have accumulators of their own where there is room, half the truncating accumulations in a row
-    // (with one issuer it was even and odd K steps: 64 rows of 4096 -> 4096 5.6e-7, now 5.7e-7; 101 rows of 4096 -> 12288 1.36e-6
-    // both); calls of up to sixteen rows have four, as those of up to eight have (distance from the
+    // (64 rows of 4096 -> 4096: 5.6e-7 of the norm from the sum in 64 bits); calls of up to sixteen rows have four, as those of up to eight have (distance from the
     // sum in 64 bits, 16 rows of 5120 -> 5120: 8.4e-7 of its norm with two, 4.5e-7 with four, at
     // 15.75 us instead of 15.55).  Beyond 128 rows there is room for one (129 rows of 4096 -> 12288: 2.6e-6
     // where two give 1.4e-6 for 128), as in the dense GEMM (4.9e-6).  A second buffer lets the MMAs of
