@@ -14,7 +14,7 @@
 // contiguous range of units (gemv_partition.h), whatever the shapes are.
 // Roles: 16 decode warps (warp w feeds tensor-memory lane quarter w % 4, i.e. column tiles
 // 2(w % 4) and +1, of every fourth unit), 4 epilogue warps, one producer thread each for
-// the weight ring and the activation ring, one MMA issuer.
+// the weight ring and the activation ring, two MMA issuers (one beyond 128 rows).
 // Fold: a CTA whose range BEGINS inside a column block dumps its raw sums to its plane in global
 // scratch (that is its first segment, done early) and counts the chunks in its flag; the CTA whose
 // range holds the block's first K part finishes the block at the end of its own range and adds the
